@@ -7,7 +7,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB_DIR = os.path.join(HERE, "_lib")
 LIB_PATH = os.path.join(LIB_DIR, "libmorello_b200.so")
-SOURCES = ["combine.cu", "plan.cpp", "capi.cpp"]
+SOURCES = ["combine.cu", "devplan.cu", "plan.cpp", "optable.cpp", "capi.cpp"]
 
 
 def _nvcc():

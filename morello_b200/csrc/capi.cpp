@@ -10,10 +10,26 @@
 
 using namespace mrl;
 
+// What was planned, to plan it again where the host's form of the plan is asked for.
+struct Job {
+  bool precompute = false;
+  uint32_t size = 0;
+  Through through = THROUGH_MOVE;
+  std::vector<Dtype> dtypes;
+  std::vector<LogicalSpec> goals;
+};
+
 struct mrl_ctx {
   int device = 0;
   int n_threads = 1;
-  Plan plan;
+  Plan plan;                      // the host's form of the plan (with on_device: only once it was asked for)
+  // Plans are made on the device where one fill on one GPU is planned; sharded fills, planning-only
+  // contexts and the cross-check modes plan on the host.
+  bool on_device = false;
+  bool host_plan = false;         // `plan` holds the current job
+  Job job;
+  OpTables tab;                   // of a plan made on the device
+  std::vector<uint64_t> specs;    // its Specs by id (packed), once they were asked for
   bool planned = false, uploaded = false, filled = false;
   DeviceFill dev;
   mrl_stats stats;
@@ -76,42 +92,130 @@ void copy_fill_stats(mrl_ctx* ctx) {
   for (int k = 0; k < 8; k++) ctx->stats.phase_ms[k] = fs.phase_ms[k];
 }
 
-// Upload + fill of the planned tables.
-int upload_and_fill(mrl_ctx* ctx) {
-  if (ctx->device < 0) return fail(ctx, -2, "planning-only context: no device to fill on");
-  ctx->filled = false;
+int dev_rc(int rc) { return (rc == -5 || rc == -6 || rc == -3) ? rc : -2; }
+
+int upload_plan(mrl_ctx* ctx) {
   double t0 = now_s();
-  int rc = ctx->dev.upload(ctx->plan);
-  if (rc != 0) return fail(ctx, (rc == -5 || rc == -6 || rc == -3) ? rc : -2, ctx->dev.error());
+  ctx->filled = false;
+  int rc = ctx->on_device ? ctx->dev.prepare_fill() : ctx->dev.upload(ctx->plan, ctx->cands_elsewhere);
+  if (rc != 0) return fail(ctx, dev_rc(rc), ctx->dev.error());
   ctx->uploaded = true;
   ctx->stats.upload_seconds = now_s() - t0;
   ctx->stats.h2d_bytes = ctx->dev.h2d_bytes();
-  rc = ctx->dev.run(ctx->plan);
+  return 0;
+}
+
+// Upload + fill of the planned tables.
+int upload_and_fill(mrl_ctx* ctx) {
+  if (ctx->device < 0) return fail(ctx, -2, "planning-only context: no device to fill on");
+  int rc = upload_plan(ctx);
+  if (rc) return rc;
+  rc = ctx->dev.run();
   copy_fill_stats(ctx);
-  if (rc != 0) return fail(ctx, (rc == -5 || rc == -6 || rc == -3) ? rc : -2, ctx->dev.error());
+  if (rc != 0) return fail(ctx, dev_rc(rc), ctx->dev.error());
   ctx->filled = true;
   return 0;
 }
 
-int set_plan(mrl_ctx* ctx, const std::vector<LogicalSpec>& goals, int mirror_dtype = -1) {
-  double t0 = now_s();
+Plan plan_on_host(const mrl_ctx* ctx, const Job& job, double* goal_seconds) {
+  if (!job.precompute) return build_plan(job.goals, ctx->n_threads, nullptr, ctx->rank, ctx->world, -1, ctx->plan_flags);
+  // u32 + f32: the goal sets mirror each other by construction, so only the u32 goals are
+  // enumerated and the planner derives the f32 half (plan.cpp, "dtype twins")
+  std::vector<Dtype> dts = job.dtypes;
+  int mirror = -1;
+  if (dts.size() == 2 && dts[0] == DT_U32 && dts[1] == DT_F32 && !(ctx->plan_flags & PLAN_NO_TWINS)) {
+    dts.pop_back();
+    mirror = DT_F32;
+  }
+  const double t0 = now_s();
+  const std::vector<LogicalSpec> goals = precompute_goals(job.size, job.through, dts, ctx->n_threads);
+  *goal_seconds = now_s() - t0;
+  return build_plan(goals, ctx->n_threads, nullptr, ctx->rank, ctx->world, mirror, ctx->plan_flags);
+}
+
+// The host's form of a plan that was made on the device (sharding tables, plan sharing).
+void need_host_plan(mrl_ctx* ctx) {
+  if (!ctx->on_device || ctx->host_plan) return;
+  double goal_seconds = 0;
+  ctx->plan = plan_on_host(ctx, ctx->job, &goal_seconds);
+  ctx->host_plan = true;
+}
+
+int set_plan(mrl_ctx* ctx, Job&& job) {
+  // What can fail on account of the job fails before the context's present plan is touched.
+  const double t0 = now_s();
+  double goal_seconds = 0;
+  OpTables tab;
+  bool factored = ctx->device >= 0 && ctx->world == 1 && ctx->plan_flags == 0;
+  if (factored) {
+    try {
+      if (job.precompute) tab.build_precompute(job.size, job.through, job.dtypes);
+      else tab.build_goals(job.goals);
+      goal_seconds = now_s() - t0;
+    } catch (const ModelError&) {
+      factored = false;   // outside the factored form, or an error in the job itself: the host planner tells
+    }
+  }
+  Plan host;
+  if (!factored) host = plan_on_host(ctx, job, &goal_seconds);
+  ctx->planned = ctx->uploaded = ctx->filled = false;
   ctx->cands_elsewhere = false;
   ctx->table_only = false;
-  ctx->dev.wait_upload();   // a background upload may still be reading the old plan
-  ctx->plan = build_plan(goals, ctx->n_threads, nullptr, ctx->rank, ctx->world, mirror_dtype, ctx->plan_flags);
-  ctx->planned = true;
-  ctx->uploaded = ctx->filled = false;
-  const PlanStats& ps = ctx->plan.stats;
+  ctx->on_device = ctx->host_plan = false;
+  ctx->specs.clear();
+  ctx->job = std::move(job);
   memset(&ctx->stats, 0, sizeof(ctx->stats));
+  ctx->dev.wait_upload();   // a background upload may still be reading the old plan
+  if (factored) {
+    const int rc = ctx->dev.plan(tab);
+    if (rc < 0) return fail(ctx, dev_rc(rc), ctx->dev.error());
+    if (rc == 0) {
+      ctx->tab = std::move(tab);
+      ctx->plan = Plan();
+      ctx->on_device = ctx->planned = true;
+      ctx->stats.n_specs = ctx->dev.n_specs();
+      ctx->stats.n_goal_specs = ctx->dev.n_goals();
+      ctx->stats.n_candidates = ctx->dev.n_cands();
+      ctx->stats.n_stages = ctx->dev.stages().size();
+      ctx->stats.plan_seconds = now_s() - t0;
+      ctx->stats.plan_goal_seconds = goal_seconds;
+      ctx->stats.plan_discover_seconds = ctx->stats.plan_seconds - goal_seconds;
+      return 0;
+    }
+    host = plan_on_host(ctx, ctx->job, &goal_seconds);
+  }
+  ctx->plan = std::move(host);
+  ctx->planned = ctx->host_plan = true;
+  const PlanStats& ps = ctx->plan.stats;
   ctx->stats.n_specs = ps.n_specs;
   ctx->stats.n_goal_specs = ps.n_goal_specs;
   ctx->stats.n_candidates = ps.n_cands;
   ctx->stats.n_stages = ps.n_stages;
   ctx->stats.plan_seconds = now_s() - t0;
+  ctx->stats.plan_goal_seconds = goal_seconds;
   ctx->stats.plan_discover_seconds = ps.seconds_discover;
   ctx->stats.plan_layout_seconds = ps.seconds_layout;
   for (int k = 0; k < 8; k++) ctx->stats.plan_layout_step_seconds[k] = ps.seconds_layout_step[k];
   return 0;
+}
+
+uint64_t spec_count(const mrl_ctx* ctx) { return ctx->on_device ? ctx->dev.n_specs() : ctx->plan.specs.size(); }
+uint32_t top_code_of(const mrl_ctx* ctx, int k) { return ctx->on_device ? ctx->tab.top_code[k] : ctx->plan.top_code[k]; }
+
+// Specs by id. The packed Specs of a plan made on the device are fetched once.
+void need_specs(mrl_ctx* ctx) {
+  if (!ctx->on_device || ctx->specs.size() == ctx->dev.n_specs()) return;
+  ctx->specs.resize(ctx->dev.n_specs());
+  if (ctx->dev.read_specs(ctx->specs.data()) != 0) {
+    ctx->specs.clear();
+    throw ModelError(ctx->dev.error());
+  }
+}
+LogicalSpec spec_at(const mrl_ctx* ctx, uint64_t id) { return ctx->on_device ? ctx->tab.spec_of(ctx->specs[id]) : ctx->plan.specs[id]; }
+uint64_t job_fingerprint(mrl_ctx* ctx) {
+  if (!ctx->on_device) return ctx->plan.fingerprint(ctx->n_threads);
+  need_specs(ctx);
+  return fingerprint_of(ctx->specs.size(), [&](size_t i) { return ctx->tab.spec_of(ctx->specs[i]); }, ctx->tab.top_code, ctx->n_threads);
 }
 
 int parse_goals(const uint8_t* blobs, const uint64_t* off, size_t n, std::vector<LogicalSpec>& out) {
@@ -238,20 +342,12 @@ int mrl_plan_precompute(mrl_ctx* ctx, uint32_t size, int through, int dtype_mask
     if (through < 0 || through > THROUGH_MATMUL) return fail(ctx, -1, "bad `through`");
     std::vector<Dtype> dts = dtypes_of(dtype_mask);
     if (dts.empty()) return fail(ctx, -1, "empty dtype mask");
-    double t0 = now_s();
-    // u32 + f32: the goal sets mirror each other by construction, so only the u32 goals are
-    // enumerated and the planner derives the f32 half (plan.cpp, "dtype twins")
-    int mirror = -1;
-    if (dts.size() == 2 && dts[0] == DT_U32 && dts[1] == DT_F32 && !(ctx->plan_flags & PLAN_NO_TWINS)) {
-      dts.pop_back();
-      mirror = DT_F32;
-    }
-    std::vector<LogicalSpec> goals = precompute_goals(size, (Through)through, dts, ctx->n_threads);
-    const double t_goals = now_s() - t0;
-    int rc = set_plan(ctx, goals, mirror);
-    ctx->stats.plan_seconds = now_s() - t0;
-    ctx->stats.plan_goal_seconds = t_goals;
-    return rc;
+    Job job;
+    job.precompute = true;
+    job.size = size;
+    job.through = (Through)through;
+    job.dtypes = dts;
+    return set_plan(ctx, std::move(job));
   } catch (const std::exception& e) {
     return fail(ctx, -1, e.what());
   }
@@ -260,9 +356,9 @@ int mrl_plan_precompute(mrl_ctx* ctx, uint32_t size, int through, int dtype_mask
 int mrl_plan_goals(mrl_ctx* ctx, const uint8_t* blobs, const uint64_t* blob_off, size_t n) {
   if (!ctx) return -1;
   try {
-    std::vector<LogicalSpec> goals;
-    if (parse_goals(blobs, blob_off, n, goals) != 0) return fail(ctx, -4, "goal Spec is not canonicalizable");
-    return set_plan(ctx, goals);
+    Job job;
+    if (parse_goals(blobs, blob_off, n, job.goals) != 0) return fail(ctx, -4, "goal Spec is not canonicalizable");
+    return set_plan(ctx, std::move(job));
   } catch (const std::exception& e) {
     return fail(ctx, -1, e.what());
   }
@@ -280,23 +376,16 @@ int mrl_upload(mrl_ctx* ctx) {
   if (ctx->device < 0) return fail(ctx, -2, "planning-only context: no device to fill on");
   if (!ctx->planned) return fail(ctx, -1, "nothing planned");
   if (ctx->table_only) return fail(ctx, -1, "the tables were loaded from a file without their plan: nothing to upload or fill");
-  double t0 = now_s();
-  int urc = ctx->dev.upload(ctx->plan, ctx->cands_elsewhere);
-  if (urc != 0) return fail(ctx, urc == -6 ? -6 : -2, ctx->dev.error());
-  ctx->uploaded = true;
-  ctx->filled = false;
-  ctx->stats.upload_seconds = now_s() - t0;
-  ctx->stats.h2d_bytes = ctx->dev.h2d_bytes();
-  return 0;
+  return upload_plan(ctx);
 }
 
 int mrl_fill(mrl_ctx* ctx) {
   if (!ctx) return -1;
   if (!ctx->uploaded || ctx->table_only) return fail(ctx, -1, "plan not uploaded");
   ctx->filled = false;
-  int rc = ctx->dev.run(ctx->plan);
+  int rc = ctx->dev.run();
   copy_fill_stats(ctx);
-  if (rc != 0) return fail(ctx, (rc == -5 || rc == -6 || rc == -3) ? rc : -2, ctx->dev.error());
+  if (rc != 0) return fail(ctx, dev_rc(rc), ctx->dev.error());
   ctx->filled = true;
   return 0;
 }
@@ -320,18 +409,51 @@ static void resolve_queries(const Plan& plan, const uint8_t* blobs, const uint64
   }
 }
 
+// The same for a plan in factored form: (packed Spec, packed limit codes).
+static void resolve_packed(const OpTables& tab, const uint8_t* blobs, const uint64_t* blob_off, size_t n, const uint64_t* limits,
+                           mrl_decision* out, std::vector<uint64_t>& specs, std::vector<uint32_t>& packs, std::vector<size_t>& where) {
+  specs.reserve(n);
+  packs.reserve(n);
+  where.reserve(n);
+  for (size_t i = 0; i < n; i++) {
+    memset(&out[i], 0, sizeof(out[i]));
+    out[i].found = -1;
+    const uint8_t* const blob = blobs + blob_off[i];
+    const size_t len = blob_off[i + 1] - blob_off[i];
+    uint64_t at;
+    if (!tab.locate_blob(blob, len, &at)) {   // not in canonical form, or not in the tables
+      LogicalSpec ls = LogicalSpec::from_key(std::string((const char*)blob, len));
+      if (logicalspec_canonicalize(ls) != CANON_OK || !tab.locate(ls, &at)) continue;
+    }
+    uint32_t pack;
+    if (!pack_limit_codes(limits + 4 * i, tab.top_code, &pack)) continue;
+    specs.push_back(at);
+    packs.push_back(pack);
+    where.push_back(i);
+  }
+}
+
 int mrl_get_many(mrl_ctx* ctx, const uint8_t* blobs, const uint64_t* blob_off, size_t n, const uint64_t* limits,
                  mrl_decision* out) {
   if (!ctx) return -1;
   if (!ctx->filled) return fail(ctx, -1, "tables are not filled");
   try {
     std::vector<uint32_t> ids, packs;
+    std::vector<uint64_t> specs;
     std::vector<size_t> where;
-    resolve_queries(ctx->plan, blobs, blob_off, n, limits, out, ids, packs, where);
-    std::vector<MrlRow> rows(ids.size());
-    if (ctx->dev.lookup(ids.data(), packs.data(), ids.size(), rows.data()) != 0) return fail(ctx, -2, ctx->dev.error());
-    for (size_t j = 0; j < ids.size(); j++) decode_row(rows[j], &out[where[j]]);
-    ctx->stats.d2h_bytes = ids.size() * sizeof(MrlRow);
+    std::vector<MrlRow> rows;
+    if (ctx->on_device) {
+      resolve_packed(ctx->tab, blobs, blob_off, n, limits, out, specs, packs, where);
+      rows.resize(where.size());
+      if (ctx->dev.lookup_packed(specs.data(), packs.data(), where.size(), rows.data()) != 0) return fail(ctx, -2, ctx->dev.error());
+    } else {
+      resolve_queries(ctx->plan, blobs, blob_off, n, limits, out, ids, packs, where);
+      rows.resize(where.size());
+      if (ctx->dev.lookup(ids.data(), packs.data(), where.size(), rows.data()) != 0) return fail(ctx, -2, ctx->dev.error());
+    }
+    for (size_t j = 0; j < where.size(); j++)
+      if (!(ctx->on_device && rows[j].aux)) decode_row(rows[j], &out[where[j]]);
+    ctx->stats.d2h_bytes = where.size() * sizeof(MrlRow);
     return 0;
   } catch (const std::exception& e) {
     return fail(ctx, -1, e.what());
@@ -354,6 +476,29 @@ int mrl_top_down_many_noalloc(mrl_ctx* ctx, const uint8_t* blobs, const uint64_t
     std::vector<LogicalSpec> goals;
     if (parse_goals(blobs, blob_off, n, goals) != 0) return fail(ctx, -4, "goal Spec is not canonicalizable");
     // A plan of its own: the context's tables (and their device memory) are left as they are.
+    if (ctx->plan_flags == 0) {
+      char err[256] = {0};
+      int rc = 1;
+      std::vector<uint64_t> specs;
+      std::vector<uint32_t> packs;
+      std::vector<size_t> where;
+      std::vector<MrlRow> rows;
+      try {
+        OpTables tab;
+        tab.build_goals(goals);
+        resolve_packed(tab, blobs, blob_off, n, limits, out, specs, packs, where);
+        rows.resize(where.size());
+        rc = fill_static(ctx->dev.device(), ctx->dev.stream(), tab, specs.data(), packs.data(), specs.size(), rows.data(), err, sizeof(err));
+      } catch (const ModelError&) {
+        rc = 1;   // outside the factored form: plan on the host
+      }
+      if (rc < 0) return fail(ctx, rc, err);
+      if (rc == 0) {
+        for (size_t j = 0; j < where.size(); j++)
+          if (!rows[j].aux) decode_row(rows[j], &out[where[j]]);
+        return 0;
+      }
+    }
     Plan plan = build_plan(goals, ctx->n_threads, nullptr, 0, 1, -1, ctx->plan_flags);
     std::vector<uint32_t> ids, packs;
     std::vector<size_t> where;
@@ -394,6 +539,11 @@ int mrl_plan_share(mrl_ctx* ctx, void* ptrs[8], uint64_t sizes[8]) {
   if (!ctx || !ptrs || !sizes) return -1;
   if (!ctx->planned) return fail(ctx, -1, "nothing planned");
   u64 sz[Plan::N_BLOBS];
+  try {
+    need_host_plan(ctx);
+  } catch (const std::exception& e) {
+    return fail(ctx, -1, e.what());
+  }
   ctx->plan.share_blobs(ptrs, sz);
   for (int k = 0; k < Plan::N_BLOBS; k++) sizes[k] = sz[k];
   return 0;
@@ -407,6 +557,8 @@ int mrl_plan_adopt(mrl_ctx* ctx, const uint64_t sizes[8], void* ptrs[8], int can
     ctx->dev.wait_upload();   // a background upload may still be reading the old plan
     ctx->plan = Plan();
     ctx->planned = ctx->uploaded = ctx->filled = false;
+    ctx->on_device = false;
+    ctx->host_plan = true;
     ctx->table_only = false;
     ctx->plan.adopt_alloc(sz);
     ctx->plan.share_blobs(ptrs, sz);
@@ -436,12 +588,24 @@ int mrl_plan_adopt_done(mrl_ctx* ctx, double plan_seconds) {
   }
 }
 
-uint64_t mrl_num_stages(const mrl_ctx* ctx) { return ctx && ctx->planned ? ctx->plan.stages.size() : 0; }
-uint64_t mrl_num_families(const mrl_ctx* ctx) { return ctx && ctx->planned ? ctx->plan.families.size() : 0; }
+uint64_t mrl_num_stages(const mrl_ctx* ctx) { return ctx && ctx->planned ? (ctx->on_device ? ctx->dev.stages().size() : ctx->plan.stages.size()) : 0; }
+
+// Families and owners are of the host's form of a plan.
+static bool host_plan_ready(const mrl_ctx* ctx) {
+  if (!ctx || !ctx->planned) return false;
+  try {
+    need_host_plan(const_cast<mrl_ctx*>(ctx));
+    return true;
+  } catch (const std::exception&) {
+    return false;
+  }
+}
+
+uint64_t mrl_num_families(const mrl_ctx* ctx) { return host_plan_ready(ctx) ? ctx->plan.families.size() : 0; }
 
 int mrl_stage_info(const mrl_ctx* ctx, uint64_t stage, uint32_t* spec_lo, uint32_t* spec_hi, uint32_t* family_lo,
                    uint32_t* family_hi) {
-  if (!ctx || !ctx->planned || stage >= ctx->plan.stages.size()) return -1;
+  if (!host_plan_ready(ctx) || stage >= ctx->plan.stages.size()) return -1;
   const Stage& st = ctx->plan.stages[stage];
   if (spec_lo) *spec_lo = st.spec_lo;
   if (spec_hi) *spec_hi = st.spec_hi;
@@ -452,7 +616,7 @@ int mrl_stage_info(const mrl_ctx* ctx, uint64_t stage, uint32_t* spec_lo, uint32
 
 int mrl_family_info(const mrl_ctx* ctx, uint64_t family, uint32_t* stage, uint32_t* owner, uint32_t* spec_lo,
                     uint32_t* spec_hi) {
-  if (!ctx || !ctx->planned || family >= ctx->plan.families.size()) return -1;
+  if (!host_plan_ready(ctx) || family >= ctx->plan.families.size()) return -1;
   const Family& f = ctx->plan.families[family];
   if (stage) *stage = f.stage;
   if (owner) *owner = f.owner;
@@ -462,7 +626,7 @@ int mrl_family_info(const mrl_ctx* ctx, uint64_t family, uint32_t* stage, uint32
 }
 
 int mrl_spec_owners(const mrl_ctx* ctx, uint8_t* out, uint64_t n) {
-  if (!ctx || !ctx->planned || !out || n != ctx->plan.hdrs.size()) return -1;
+  if (!ctx || !ctx->planned || !out || n != spec_count(ctx)) return -1;
   if (ctx->plan.owner.empty()) memset(out, 0, n);
   else memcpy(out, ctx->plan.owner.data(), n);
   return 0;
@@ -503,9 +667,9 @@ int mrl_fill_begin(mrl_ctx* ctx) {
 
 int mrl_fill_stage_solve(mrl_ctx* ctx, uint64_t stage, void** masks, uint64_t* mask_bytes) {
   if (!ctx || !ctx->uploaded) return -1;
-  int rc = ctx->dev.solve_stage(ctx->plan, (uint32_t)stage);
-  if (rc != 0) return fail(ctx, (rc == -5 || rc == -6 || rc == -3) ? rc : -2, ctx->dev.error());
-  if (ctx->dev.stage_masks(ctx->plan, (uint32_t)stage, masks, mask_bytes) != 0) return fail(ctx, -2, ctx->dev.error());
+  int rc = ctx->dev.solve_stage((uint32_t)stage);
+  if (rc != 0) return fail(ctx, dev_rc(rc), ctx->dev.error());
+  if (ctx->dev.stage_masks((uint32_t)stage, masks, mask_bytes) != 0) return fail(ctx, -2, ctx->dev.error());
   return 0;
 }
 
@@ -513,8 +677,8 @@ int mrl_fill_stage_place(mrl_ctx* ctx, uint64_t stage, void** rows, uint64_t* ro
   if (!ctx || !ctx->uploaded) return -1;
   void* p = nullptr;
   uint64_t b = 0;
-  int rc = ctx->dev.place_stage(ctx->plan, (uint32_t)stage, &p, &b);
-  if (rc != 0) return fail(ctx, (rc == -5 || rc == -6 || rc == -3) ? rc : -2, ctx->dev.error());
+  int rc = ctx->dev.place_stage((uint32_t)stage, &p, &b);
+  if (rc != 0) return fail(ctx, dev_rc(rc), ctx->dev.error());
   if (rows) *rows = p;
   if (row_bytes) *row_bytes = b;
   return 0;
@@ -533,12 +697,19 @@ namespace {
 // One node of the reconstruction and, below it, its sub-Specs at the limits the stored action
 // leaves them (morello/src/reconstruct.rs:14-80).
 void reconstruct(mrl_ctx* ctx, const LogicalSpec& ls, const u64 limits[4], int level, std::string& out) {
-  const long id = ctx->plan.find(ls);
-  uint32_t pack = 0;
-  if (id < 0 || !ctx->plan.pack_limits(limits, &pack)) throw ModelError("not in the tables: " + ls.str());
-  const uint32_t id32 = (uint32_t)id;
   MrlRow row;
-  if (ctx->dev.lookup(&id32, &pack, 1, &row) != 0) throw ModelError(ctx->dev.error());
+  uint32_t pack = 0;
+  if (ctx->on_device) {
+    uint64_t at = 0;
+    if (!ctx->tab.locate(ls, &at) || !pack_limit_codes(limits, ctx->tab.top_code, &pack)) throw ModelError("not in the tables: " + ls.str());
+    if (ctx->dev.lookup_packed(&at, &pack, 1, &row) != 0) throw ModelError(ctx->dev.error());
+    if (row.aux) throw ModelError("not in the tables: " + ls.str());
+  } else {
+    const long id = ctx->plan.find(ls);
+    if (id < 0 || !ctx->plan.pack_limits(limits, &pack)) throw ModelError("not in the tables: " + ls.str());
+    const uint32_t id32 = (uint32_t)id;
+    if (ctx->dev.lookup(&id32, &pack, 1, &row) != 0) throw ModelError(ctx->dev.error());
+  }
   mrl_decision d;
   decode_row(row, &d);
   if (d.found != 1) throw ModelError("no implementation for " + ls.str());
@@ -580,7 +751,7 @@ int mrl_verify(mrl_ctx* ctx, uint64_t n_samples, uint64_t seed, uint64_t* n_chec
   if (!ctx->filled) return fail(ctx, -1, "tables are not filled");
   if (ctx->table_only) return fail(ctx, -1, "the tables were loaded from a file without their plan: plan the job, then load, to verify");
   uint64_t first_bad = 0;
-  if (ctx->dev.verify(ctx->plan, n_samples, seed, n_checked, n_mismatch, &first_bad) != 0) return fail(ctx, -2, ctx->dev.error());
+  if (ctx->dev.verify(n_samples, seed, n_checked, n_mismatch, &first_bad) != 0) return fail(ctx, -2, ctx->dev.error());
   return 0;
 }
 
@@ -590,18 +761,24 @@ int mrl_get_stats(const mrl_ctx* ctx, mrl_stats* out) {
   return 0;
 }
 
-uint64_t mrl_num_specs(const mrl_ctx* ctx) { return ctx && ctx->planned ? ctx->plan.specs.size() : 0; }
+uint64_t mrl_num_specs(const mrl_ctx* ctx) { return ctx && ctx->planned ? spec_count(ctx) : 0; }
 
 int mrl_spec_blob(const mrl_ctx* ctx, uint64_t spec_id, uint8_t* out, size_t cap) {
-  if (!ctx || !ctx->planned || spec_id >= ctx->plan.specs.size()) return -1;
-  std::string k = ctx->plan.specs[spec_id].key();
+  if (!ctx || !ctx->planned || spec_id >= spec_count(ctx)) return -1;
+  std::string k;
+  try {
+    need_specs(const_cast<mrl_ctx*>(ctx));
+    k = spec_at(ctx, spec_id).key();
+  } catch (const std::exception&) {
+    return -2;
+  }
   if (k.size() > cap) return -3;
   memcpy(out, k.data(), k.size());
   return (int)k.size();
 }
 
 int mrl_spec_grid(mrl_ctx* ctx, uint64_t spec_id, uint32_t masks[4], uint64_t* n_cells) {
-  if (!ctx || !ctx->filled || spec_id >= ctx->plan.specs.size()) return -1;
+  if (!ctx || !ctx->filled || spec_id >= spec_count(ctx)) return -1;
   SpecHdr h;
   if (ctx->dev.read_hdr((uint32_t)spec_id, &h) != 0) return fail(ctx, -2, ctx->dev.error());
   uint64_t n = 1;
@@ -611,7 +788,7 @@ int mrl_spec_grid(mrl_ctx* ctx, uint64_t spec_id, uint32_t masks[4], uint64_t* n
 }
 
 int mrl_export_rows(mrl_ctx* ctx, uint64_t spec_id, mrl_decision* out, size_t cap) {
-  if (!ctx || !ctx->filled || spec_id >= ctx->plan.specs.size()) return -1;
+  if (!ctx || !ctx->filled || spec_id >= spec_count(ctx)) return -1;
   SpecHdr h;
   if (ctx->dev.read_hdr((uint32_t)spec_id, &h) != 0) return fail(ctx, -2, ctx->dev.error());
   uint64_t n = 1;
@@ -641,7 +818,7 @@ int mrl_export_all(mrl_ctx* ctx, uint32_t* masks, uint64_t* first_row, mrl_row* 
   if (!ctx->filled) return fail(ctx, -1, "tables are not filled");
   static_assert(sizeof(mrl_row) == sizeof(MrlRow), "exported rows are the device rows");
   try {
-    const uint64_t n = ctx->plan.hdrs.size(), n_rows = ctx->dev.stats().n_rows;
+    const uint64_t n = spec_count(ctx), n_rows = ctx->dev.stats().n_rows;
     if (rows_cap < n_rows) return fail(ctx, -3, "export buffer too small");
     std::vector<SpecHdr> h(n);
     if (ctx->dev.read_table(h.data(), reinterpret_cast<MrlRow*>(rows)) != 0) return fail(ctx, -2, ctx->dev.error());
@@ -658,7 +835,7 @@ int mrl_export_all(mrl_ctx* ctx, uint32_t* masks, uint64_t* first_row, mrl_row* 
 }
 
 long mrl_export_rects(mrl_ctx* ctx, uint64_t spec_id, uint8_t* lo, uint8_t* hi, mrl_decision* out, size_t cap) {
-  if (!ctx || !ctx->filled || spec_id >= ctx->plan.specs.size()) return -1;
+  if (!ctx || !ctx->filled || spec_id >= spec_count(ctx)) return -1;
   try {
     SpecHdr h;
     if (ctx->dev.read_hdr((uint32_t)spec_id, &h) != 0) return fail(ctx, -2, ctx->dev.error());
@@ -683,7 +860,7 @@ long mrl_export_rects(mrl_ctx* ctx, uint64_t spec_id, uint8_t* lo, uint8_t* hi, 
         const uint32_t s = (uint32_t)(rest % nn[k]);
         rest /= nn[k];
         r.lo[k] = (uint8_t)codes[k][s];
-        r.hi[k] = (uint8_t)(s + 1 < nn[k] ? codes[k][s + 1] - 1 : ctx->plan.top_code[k]);
+        r.hi[k] = (uint8_t)(s + 1 < nn[k] ? codes[k][s + 1] - 1 : top_code_of(ctx, k));
       }
       r.row = (uint32_t)i;
       r.dead = false;
@@ -773,7 +950,7 @@ int mrl_save(mrl_ctx* ctx, const char* path) {
   if (!ctx || !path) return -1;
   if (!ctx->filled) return fail(ctx, -1, "tables are not filled");
   try {
-    const uint64_t n = ctx->plan.hdrs.size(), n_rows = ctx->dev.stats().n_rows;
+    const uint64_t n = spec_count(ctx), n_rows = ctx->dev.stats().n_rows;
     std::vector<SpecHdr> h(n);
     std::vector<MrlRow> rows(n_rows);
     if (ctx->dev.read_table(h.data(), rows.data()) != 0) return fail(ctx, -2, ctx->dev.error());
@@ -781,15 +958,16 @@ int mrl_save(mrl_ctx* ctx, const char* path) {
     memset(&fh, 0, sizeof(fh));
     memcpy(fh.magic, kMagic, 8);
     fh.version = 1; fh.target = 1; fh.tile_scale = 1;
-    for (int k = 0; k < 4; k++) fh.top_code[k] = ctx->plan.top_code[k];
+    for (int k = 0; k < 4; k++) fh.top_code[k] = top_code_of(ctx, k);
     fh.n_specs = n; fh.n_rows = n_rows;
-    fh.fingerprint = ctx->plan.fingerprint(ctx->n_threads);
+    fh.fingerprint = job_fingerprint(ctx);
+    need_specs(ctx);
     if (ctx->dev.checksum(&fh.table_checksum) != 0) return fail(ctx, -2, ctx->dev.error());
     std::string blobs;
     std::vector<uint32_t> blob_end(n);
     for (uint64_t i = 0; i < n; i++) {
       char kb[LogicalSpec::MAX_KEY];
-      const int kl = ctx->plan.specs[i].key_into(kb);
+      const int kl = spec_at(ctx, i).key_into(kb);
       blobs.append(kb, (size_t)kl);
       blob_end[i] = (uint32_t)blobs.size();
     }
@@ -853,8 +1031,7 @@ int mrl_load(mrl_ctx* ctx, const char* path) {
     }
     // the file is sound as far as the host can tell; from here on a device is needed
     if (ctx->device < 0) return fail(ctx, -2, "planning-only context: no device to load onto");
-    const bool same_job = ctx->planned && !ctx->table_only && ctx->plan.hdrs.size() == n &&
-                          ctx->plan.fingerprint(ctx->n_threads) == fh.fingerprint;
+    const bool same_job = ctx->planned && !ctx->table_only && spec_count(ctx) == n && job_fingerprint(ctx) == fh.fingerprint;
     if (!same_job) {
       RawVec<LogicalSpec> specs;
       specs.reset(n);
@@ -866,7 +1043,8 @@ int mrl_load(mrl_ctx* ctx, const char* path) {
       ctx->dev.wait_upload();
       ctx->plan = table_only_plan(std::move(specs), std::move(hdrs), fh.top_code, ctx->n_threads);
       if (ctx->plan.fingerprint(ctx->n_threads) != fh.fingerprint) return fail(ctx, -8, "the database file is corrupt (Spec fingerprint)");
-      ctx->planned = true;
+      ctx->planned = ctx->host_plan = true;
+      ctx->on_device = false;
       ctx->table_only = true;
       ctx->cands_elsewhere = false;
       memset(&ctx->stats, 0, sizeof(ctx->stats));
@@ -874,16 +1052,17 @@ int mrl_load(mrl_ctx* ctx, const char* path) {
       int rc = ctx->dev.upload(ctx->plan);
       if (rc != 0) return fail(ctx, rc == -6 ? -6 : -2, ctx->dev.error());
       ctx->uploaded = true;
-      if (ctx->dev.load_table(ctx->plan, ctx->plan.hdrs.data(), rows.data(), fh.n_rows) != 0) return fail(ctx, -2, ctx->dev.error());
+      if (ctx->dev.load_table(ctx->plan.hdrs.data(), rows.data(), fh.n_rows) != 0) return fail(ctx, -2, ctx->dev.error());
     } else {
       if (!ctx->uploaded) {
-        int rc = ctx->dev.upload(ctx->plan, ctx->cands_elsewhere);
-        if (rc != 0) return fail(ctx, rc == -6 ? -6 : -2, ctx->dev.error());
-        ctx->uploaded = true;
+        int rc = upload_plan(ctx);
+        if (rc) return rc;
       }
       // the plan's own candidate ranges stay; masks and first rows come from the file
-      for (uint64_t i = 0; i < n; i++) { hdrs[i].cand_off = ctx->plan.hdrs[i].cand_off; hdrs[i].ncand = ctx->plan.hdrs[i].ncand; }
-      if (ctx->dev.load_table(ctx->plan, hdrs.data(), rows.data(), fh.n_rows) != 0) return fail(ctx, -2, ctx->dev.error());
+      std::vector<SpecHdr> own(n);
+      if (ctx->dev.read_hdrs(own.data()) != 0) return fail(ctx, -2, ctx->dev.error());
+      for (uint64_t i = 0; i < n; i++) { hdrs[i].cand_off = own[i].cand_off; hdrs[i].ncand = own[i].ncand; }
+      if (ctx->dev.load_table(hdrs.data(), rows.data(), fh.n_rows) != 0) return fail(ctx, -2, ctx->dev.error());
     }
     ctx->filled = true;
     ctx->stats.n_rows = fh.n_rows;

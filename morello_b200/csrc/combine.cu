@@ -42,6 +42,7 @@
 // Integer-only work; no tensor cores.
 #include "device_types.h"
 #include "fill.hpp"
+#include "devplan.hpp"
 #include "../../include/morello_b200.h"
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
@@ -1500,6 +1501,26 @@ __global__ void lookup_rows_kernel(const SpecHdr* hdrs, const MrlRow* rows, cons
   *reinterpret_cast<uint4*>(out + i) = r;
 }
 
+// The same for Specs of a plan made on the device, named by family and operands: a Spec's id is the
+// number of existing Specs before its position. aux = 1 in the answer: the Spec does not exist.
+struct PackedQuery { unsigned long long spec; uint32_t cpack, pad; };
+__global__ void __launch_bounds__(kBlock)
+lookup_packed_kernel(const mrl::DpTables t, const SpecHdr* hdrs, const MrlRow* rows, const PackedQuery* queries, unsigned long long n,
+                     MrlRow* out) {
+  const unsigned long long i = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const PackedQuery q = queries[i];
+  const uint32_t pos = mrl::dp_pos(t, t.fams[q.spec >> 48], (uint32_t)(q.spec >> 32) & 0xFFFFu, (uint32_t)(q.spec >> 16) & 0xFFFFu,
+                                   (uint32_t)q.spec & 0xFFFFu);
+  uint4 r = make_uint4(MRL_UNSAT, MRL_UNSAT, MRL_UNSAT, 1u);
+  if ((t.rank[pos >> 5].x >> (pos & 31u)) & 1u) {
+    r = lookup(hdrs, rows, rows, mrl::dp_id(t, pos), below(code_of(q.cpack, 0)), below(code_of(q.cpack, 1)), below(code_of(q.cpack, 2)),
+               below(code_of(q.cpack, 3)));
+    r.w = 0;
+  }
+  *reinterpret_cast<uint4*>(out + i) = r;
+}
+
 __device__ __forceinline__ unsigned long long mix64(unsigned long long z) {
   z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ull;
   z = (z ^ (z >> 27)) * 0x94D049BB133111EBull;
@@ -1563,6 +1584,11 @@ namespace mrl {
 
 static size_t align256(size_t x) { return (x + 255) & ~size_t(255); }
 
+struct DeviceFill::DevTables {
+  DpTables t;
+};
+
+DeviceFill::DeviceFill() {}
 DeviceFill::~DeviceFill() { release(); }
 
 int DeviceFill::too_large_() {
@@ -1590,22 +1616,57 @@ int DeviceFill::alloc_(void** p, size_t bytes) {
   return 0;
 }
 
-void DeviceFill::free_(void* p) {
-  if (p && !fixed_) cudaFree(p);
+void DeviceFill::drop_(DevBuf& b) {
+  if (b.p && !fixed_) cudaFree(b.p);
+  b.p = nullptr;
+  b.cap = 0;
+}
+
+// A cudaMalloc or cudaFree costs 50 us to milliseconds (seconds, in the tail) against the 1 to 60
+// ms of a small fill, and a plan has some twenty buffers, so buffers stay from plan to plan. What
+// a large plan leaves behind is given back when the next plan needs less than 1/16 of it.
+int DeviceFill::reserve_(DevBuf& b, size_t bytes, bool give_back) {
+  bytes = std::max<size_t>(bytes, 256);
+  if (!fixed_ && b.cap >= bytes && !(give_back && b.cap > (size_t(256) << 20) && b.cap / 16 > bytes)) return 0;
+  if (!fixed_ && b.p) {
+    CK(cudaStreamSynchronize(stream_));
+    drop_(b);
+  }
+  const size_t want = fixed_ ? bytes : (bytes < (size_t(64) << 20) ? bytes + bytes / 4 : bytes);
+  int rc = alloc_(&b.p, want);
+  if (rc) { b.p = nullptr; b.cap = 0; return rc; }
+  b.cap = want;
+  return 0;
+}
+
+int DeviceFill::reserve_host_(size_t bytes) {
+  if (h_stage_bytes_ >= bytes) return 0;
+  if (fixed_) {   // pinning memory is an allocation the no-allocation entry point does not make
+    h_pageable_.resize(bytes);
+    h_stage_ = h_pageable_.data();
+    h_stage_bytes_ = bytes;
+    return 0;
+  }
+  if (h_stage_) cudaFreeHost(h_stage_);
+  h_stage_ = nullptr;
+  h_stage_bytes_ = 0;
+  const size_t want = std::max<size_t>(bytes + bytes / 2, size_t(64) << 10);
+  CK(cudaHostAlloc(&h_stage_, want, cudaHostAllocDefault));
+  h_stage_bytes_ = want;
+  return 0;
 }
 
 void DeviceFill::release() {
   wait_upload();
-  free_(d_hdrs_); free_(d_cands_); free_(d_rmask_); free_(d_mine_); free_(d_chunks_); free_(d_items_); free_(d_minsat_); free_(d_corner_); free_(d_stamp_); free_(d_ehdr_); free_(d_rows_);
-  free_(d_temp_); free_(d_fcount_); free_(d_block_sums_); free_(d_ctl_); free_(d_stage_);
-  free_(d_dirty_);
-  d_hdrs_ = nullptr; d_cands_ = nullptr; d_rmask_ = nullptr; d_mine_ = nullptr; d_chunks_ = nullptr; d_items_ = nullptr; d_minsat_ = nullptr; d_corner_ = nullptr; d_stamp_ = nullptr; d_ehdr_ = nullptr;
-  d_rows_ = nullptr; d_temp_ = nullptr; d_fcount_ = nullptr; d_block_sums_ = nullptr; d_ctl_ = nullptr;
-  d_stage_ = nullptr; d_dirty_ = nullptr;
-  stage_bytes_ = 0;
-  row_cap_ = temp_cap_ = chunk_cap_ = item_cap_ = 0;
+  for (DevBuf* b : {&b_ctl_, &b_hdrs_, &b_cands_, &b_spec_, &b_stage_specs_, &b_mine_, &b_chunks_, &b_items_, &b_temp_, &b_rows_,
+                    &b_lookup_, &b_tables_, &b_bits_, &b_rank_, &b_desc_, &b_stage_lo_})
+    drop_(*b);
+  tab_.reset();
   buf_off_ = 0;
   cands_present_ = false;
+  if (h_stage_ && !fixed_) cudaFreeHost(h_stage_);
+  h_stage_ = nullptr;
+  h_stage_bytes_ = 0;
   if (h_ctl_ && h_ctl_ != &ctl_pageable_) cudaFreeHost(h_ctl_);
   h_ctl_ = nullptr;
   if (ev0_) cudaEventDestroy(ev0_);
@@ -1636,6 +1697,8 @@ int DeviceFill::init_events() {
   CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, stage_kernel, kBlock, 0));
   if (per_sm < 1) { snprintf(err_, sizeof(err_), "the stage kernel does not fit an SM"); return -1; }
   coop_blocks_ = per_sm * n_sm_;
+  plan_blocks_ = plan_kernel_blocks_per_sm();
+  if (plan_blocks_ < 1) { snprintf(err_, sizeof(err_), "the plan kernel does not fit an SM"); return -1; }
   return 0;
 }
 
@@ -1678,38 +1741,53 @@ int DeviceFill::wait_cands_(uint64_t upto_bytes) {
 
 int DeviceFill::wait_upload() { return wait_cands_(~uint64_t(0) >> 1); }
 
-int DeviceFill::upload(const Plan& plan, bool skip_cands) {
-  CK(cudaSetDevice(device_));
+// Forgets the plan the device holds.
+void DeviceFill::begin_plan_() {
   wait_upload();   // of an earlier plan
-  free_(d_hdrs_); free_(d_cands_); free_(d_rmask_); free_(d_mine_); free_(d_chunks_); free_(d_items_); free_(d_minsat_); free_(d_corner_); free_(d_stamp_); free_(d_ehdr_); free_(d_rows_);
-  free_(d_temp_); free_(d_fcount_); free_(d_block_sums_); free_(d_ctl_); free_(d_stage_);
-  free_(d_dirty_);
-  d_hdrs_ = nullptr; d_cands_ = nullptr; d_rmask_ = nullptr; d_mine_ = nullptr; d_chunks_ = nullptr; d_items_ = nullptr; d_minsat_ = nullptr; d_corner_ = nullptr; d_stamp_ = nullptr; d_ehdr_ = nullptr;
-  d_rows_ = nullptr; d_temp_ = nullptr; d_fcount_ = nullptr; d_block_sums_ = nullptr; d_ctl_ = nullptr;
-  d_stage_ = nullptr; d_dirty_ = nullptr;
-  stage_bytes_ = 0;
-  buf_off_ = 0;
+  if (fixed_) {    // carved afresh by every plan
+    for (DevBuf* b : {&b_ctl_, &b_hdrs_, &b_cands_, &b_spec_, &b_stage_specs_, &b_mine_, &b_chunks_, &b_items_, &b_temp_, &b_rows_,
+                      &b_lookup_, &b_tables_, &b_bits_, &b_rank_, &b_desc_, &b_stage_lo_})
+      drop_(*b);
+    buf_off_ = 0;
+  }
+  tab_.reset();
   cands_present_ = false;
-  n_specs_ = (uint32_t)plan.hdrs.size();
+  stages_.clear();
+  n_specs_ = 0;
   max_stage_ = 1;
-  for (const Stage& st : plan.stages) max_stage_ = std::max(max_stage_, st.spec_hi - st.spec_lo);
+  n_cand_bytes_ = 0;
+}
+
+// Buffers a fill works in, for n_specs_ Specs in stages_ (of which a rank of `world` computes its share).
+int DeviceFill::working_buffers_(bool with_mine, uint32_t world) {
   int rc;
-  if ((rc = alloc_((void**)&d_ctl_, 512))) return rc;
-  if ((rc = alloc_((void**)&d_hdrs_, plan.hdrs.size() * sizeof(SpecHdr)))) return rc;
-  if ((rc = alloc_((void**)&d_cands_, plan.cands.size() * sizeof(CandRec)))) return rc;
-  if ((rc = alloc_((void**)&d_rmask_, plan.hdrs.size() * sizeof(uint4)))) return rc;
-  if ((rc = alloc_((void**)&d_dirty_, plan.hdrs.size()))) return rc;
-  if ((rc = alloc_((void**)&d_minsat_, plan.hdrs.size() * sizeof(uint32_t)))) return rc;
-  if ((rc = alloc_((void**)&d_corner_, (size_t)max_stage_ * sizeof(uint32_t)))) return rc;
-  if ((rc = alloc_((void**)&d_stamp_, (size_t)max_stage_ * sizeof(uint32_t)))) return rc;
-  if ((rc = alloc_((void**)&d_ehdr_, (size_t)max_stage_ * sizeof(SpecHdr)))) return rc;
-  if (!plan.mine.empty() && (rc = alloc_((void**)&d_mine_, plan.mine.size()))) return rc;
-  if ((rc = alloc_((void**)&d_fcount_, (size_t)max_stage_ * sizeof(uint32_t)))) return rc;
-  if ((rc = alloc_((void**)&d_block_sums_, ((size_t)max_stage_ / kBlock + 1) * sizeof(unsigned long long)))) return rc;
+  max_stage_ = 1;
+  for (const StageIds& st : stages_) max_stage_ = std::max(max_stage_, st.hi - st.lo);
+  const size_t n = std::max<uint32_t>(n_specs_, 1), ms = max_stage_;
+  // per Spec: real-breakpoint masks, corner, marks; per Spec of a stage: grid of the unordered phase, corner, stamp, final cells
+  const size_t o_minsat = align256(n * sizeof(uint4)), o_dirty = o_minsat + align256(n * sizeof(uint32_t));
+  if ((rc = reserve_(b_spec_, o_dirty + align256(n)))) return rc;
+  unsigned char* p = static_cast<unsigned char*>(b_spec_.p);
+  d_rmask_ = reinterpret_cast<uint4*>(p);
+  d_minsat_ = reinterpret_cast<uint32_t*>(p + o_minsat);
+  d_dirty_ = p + o_dirty;
+  const size_t o_corner = align256(ms * sizeof(SpecHdr)), o_stamp = o_corner + align256(ms * sizeof(uint32_t)),
+               o_fcount = o_stamp + align256(ms * sizeof(uint32_t)), o_sums = o_fcount + align256(ms * sizeof(uint32_t));
+  if ((rc = reserve_(b_stage_specs_, o_sums + (ms / kBlock + 1) * sizeof(unsigned long long)))) return rc;
+  p = static_cast<unsigned char*>(b_stage_specs_.p);
+  d_ehdr_ = reinterpret_cast<SpecHdr*>(p);
+  d_corner_ = reinterpret_cast<uint32_t*>(p + o_corner);
+  d_stamp_ = reinterpret_cast<uint32_t*>(p + o_stamp);
+  d_fcount_ = reinterpret_cast<uint32_t*>(p + o_fcount);
+  d_block_sums_ = reinterpret_cast<unsigned long long*>(p + o_sums);
+  d_mine_ = nullptr;
+  if (with_mine) {
+    if ((rc = reserve_(b_mine_, n))) return rc;
+    d_mine_ = static_cast<uint8_t*>(b_mine_.p);
+  }
   if (fixed_) {
     // Everything left is split once: lookup staging, chunks, work items, working rows and final rows.
-    stage_bytes_ = 64 << 10;
-    if ((rc = alloc_(&d_stage_, stage_bytes_))) return rc;
+    if ((rc = reserve_(b_lookup_, 64 << 10))) return rc;
     const size_t left = buf_bytes_ > align256(buf_off_) + 2048 ? buf_bytes_ - align256(buf_off_) - 2048 : 0;
     // per working cell: two rows of 16 bytes (the cell and what the unordered phase found for it),
     // under 1 byte of chunks and work items; the rest is the table
@@ -1726,20 +1804,57 @@ int DeviceFill::upload(const Plan& plan, bool skip_cands) {
     // share), each within a part of the free memory. The table gets the largest
     // part: enlarging it later needs the old and the new copy at once. A stage that needs more than
     // these reports what it needs and is run again with larger buffers.
-    size_t free_b = 0, total_b = 0;
-    CK(cudaMemGetInfo(&free_b, &total_b));
-    const uint64_t shard = std::max<uint32_t>(1, plan.world);
+    const uint64_t shard = std::max<uint32_t>(1, world);
     const uint64_t stage_part = ((uint64_t)max_stage_ * 3 / 2 + shard - 1) / shard;   // Specs of the largest stage a rank solves, with slack
+    uint64_t temp = std::max<uint64_t>(1u << 20, stage_part * 1000), rows = std::max<uint64_t>(1u << 20, (uint64_t)n_specs_ * 48);
+    if (temp * 2 * sizeof(MrlRow) > b_temp_.cap || rows * sizeof(MrlRow) > b_rows_.cap) {
+      size_t free_b = 0, total_b = 0;
+      CK(cudaMemGetInfo(&free_b, &total_b));
+      free_b += b_temp_.cap + b_rows_.cap;
+      temp = std::max<uint64_t>(1u << 20, std::min<uint64_t>(temp, free_b / 4 / (2 * sizeof(MrlRow))));
+      rows = std::max<uint64_t>(1u << 20, std::min<uint64_t>(rows, free_b / 2 / sizeof(MrlRow)));
+    }
+    if ((rc = reserve_(b_temp_, temp * 2 * sizeof(MrlRow))) || (rc = reserve_(b_rows_, rows * sizeof(MrlRow)))) return rc;
+    temp_cap_ = b_temp_.cap / (2 * sizeof(MrlRow));
+    row_cap_ = b_rows_.cap / sizeof(MrlRow);
     chunk_cap_ = std::max<uint64_t>(1u << 16, stage_part * 32);
-    temp_cap_ = std::max<uint64_t>(1u << 20, std::min<uint64_t>(stage_part * 1000, free_b / 4 / (2 * sizeof(MrlRow))));
-    row_cap_ = std::max<uint64_t>(1u << 20, std::min<uint64_t>((uint64_t)n_specs_ * 48, free_b / 2 / sizeof(MrlRow)));
     item_cap_ = temp_cap_ / 32 + max_stage_ + 1;   // a work item holds at least 32 cells, and every Spec at most one partial item
     if (!h_ctl_) CK(cudaHostAlloc((void**)&h_ctl_, sizeof(FillCtl), cudaHostAllocDefault));
   }
-  if ((rc = alloc_((void**)&d_chunks_, chunk_cap_ * sizeof(Chunk)))) return rc;
-  if ((rc = alloc_((void**)&d_items_, item_cap_ * sizeof(WorkItem)))) return rc;
-  if ((rc = alloc_((void**)&d_temp_, temp_cap_ * 2 * sizeof(MrlRow)))) return rc;   // the cells, then what the unordered phase found for them
-  if ((rc = alloc_((void**)&d_rows_, row_cap_ * sizeof(MrlRow)))) return rc;
+  if ((rc = reserve_(b_chunks_, chunk_cap_ * sizeof(Chunk)))) return rc;
+  if ((rc = reserve_(b_items_, item_cap_ * sizeof(WorkItem)))) return rc;
+  if (fixed_) {
+    if ((rc = reserve_(b_temp_, temp_cap_ * 2 * sizeof(MrlRow)))) return rc;   // the cells, then what the unordered phase found for them
+    if ((rc = reserve_(b_rows_, row_cap_ * sizeof(MrlRow)))) return rc;
+  } else {
+    chunk_cap_ = b_chunks_.cap / sizeof(Chunk);
+  }
+  d_chunks_ = static_cast<Chunk*>(b_chunks_.p);
+  d_items_ = static_cast<WorkItem*>(b_items_.p);
+  d_temp_ = static_cast<MrlRow*>(b_temp_.p);
+  d_rows_ = static_cast<MrlRow*>(b_rows_.p);
+  return 0;
+}
+
+int DeviceFill::upload(const Plan& plan, bool skip_cands) {
+  CK(cudaSetDevice(device_));
+  begin_plan_();
+  n_specs_ = (uint32_t)plan.hdrs.size();
+  top_pack_ = plan.top_pack();
+  n_goals_ = plan.stats.n_goal_specs;
+  for (const Stage& st : plan.stages) {
+    StageIds s = {st.spec_lo, st.spec_hi, 0};
+    if (st.spec_hi > st.spec_lo) s.cand_end = (uint64_t)plan.hdrs[st.spec_hi - 1].cand_off + plan.hdrs[st.spec_hi - 1].ncand;
+    stages_.push_back(s);
+  }
+  int rc;
+  if ((rc = reserve_(b_ctl_, 512))) return rc;
+  if ((rc = reserve_(b_hdrs_, plan.hdrs.size() * sizeof(SpecHdr)))) return rc;
+  if ((rc = reserve_(b_cands_, plan.cands.size() * sizeof(CandRec)))) return rc;
+  d_ctl_ = static_cast<FillCtl*>(b_ctl_.p);
+  d_hdrs_ = static_cast<SpecHdr*>(b_hdrs_.p);
+  d_cands_ = static_cast<CandRec*>(b_cands_.p);
+  if ((rc = working_buffers_(!plan.mine.empty(), plan.world))) return rc;
   h2d_bytes_ = plan.hdrs.size() * sizeof(SpecHdr) + (skip_cands ? 0 : plan.cands.size() * sizeof(CandRec)) + plan.mine.size();
   CK(cudaMemsetAsync(d_ctl_, 0, 512, stream_));
   if (!plan.hdrs.empty())
@@ -1820,6 +1935,123 @@ int DeviceFill::upload(const Plan& plan, bool skip_cands) {
   return 0;
 }
 
+int DeviceFill::plan(const OpTables& tab) {
+  CK(cudaSetDevice(device_));
+  if (tab.max_records > DP_MAX_RECORDS || tab.n_positions == 0) return 1;
+  begin_plan_();
+  int rc;
+  // tables, in one copy
+  struct Part { const void* src; size_t bytes, off; };
+  Part parts[] = {{tab.shapes.data(), tab.shapes.size() * sizeof(DpShape), 0},   {tab.ops.data(), tab.ops.size() * sizeof(DpOp), 0},
+                  {tab.moves.data(), tab.moves.size() * sizeof(DpMove), 0},      {tab.tiles.data(), tab.tiles.size() * sizeof(u32), 0},
+                  {tab.fams.data(), tab.fams.size() * sizeof(DpFam), 0},         {tab.fam_child.data(), tab.fam_child.size() * sizeof(u16), 0},
+                  {tab.stage_base.data(), tab.stage_base.size() * sizeof(u32), 0},
+                  {tab.products.data(), tab.products.size() * sizeof(DpProduct), 0}, {tab.lists.data(), tab.lists.size() * sizeof(u16), 0},
+                  {tab.seeds.data(), tab.seeds.size() * sizeof(u64), 0}};
+  size_t bytes = 0;
+  for (Part& q : parts) { q.off = bytes; bytes += align256(q.bytes); }
+  const u32 n_words = (tab.n_positions + 31) / 32, n_stages = (u32)tab.stage_base.size();
+  const size_t back = align256(sizeof(PlanCtl)) + align256((n_stages + 1) * sizeof(u32));   // what comes back
+  if ((rc = reserve_host_(std::max(bytes, back)))) return rc;
+  for (const Part& q : parts) if (q.bytes) memcpy(static_cast<unsigned char*>(h_stage_) + q.off, q.src, q.bytes);
+  const size_t word_bytes = align256((size_t)n_words * sizeof(u32));
+  if ((rc = reserve_(b_ctl_, 512)) || (rc = reserve_(b_tables_, bytes)) || (rc = reserve_(b_bits_, word_bytes + (size_t)tab.n_positions * sizeof(u64))) ||
+      (rc = reserve_(b_rank_, (size_t)n_words * sizeof(uint2))) || (rc = reserve_(b_stage_lo_, back + (size_t)coop_blocks_ * 16)))
+    return rc == -5 ? 1 : rc;
+  d_ctl_ = static_cast<FillCtl*>(b_ctl_.p);
+  CK(cudaMemcpyAsync(b_tables_.p, h_stage_, bytes, cudaMemcpyHostToDevice, stream_));
+  CK(cudaMemsetAsync(b_bits_.p, 0, word_bytes, stream_));
+  CK(cudaMemsetAsync(b_stage_lo_.p, 0, sizeof(PlanCtl), stream_));
+  PlanArgs a;
+  memset(&a, 0, sizeof(a));
+  const unsigned char* const base = static_cast<unsigned char*>(b_tables_.p);
+  a.t.shapes = reinterpret_cast<const DpShape*>(base + parts[0].off);
+  a.t.ops = reinterpret_cast<const DpOp*>(base + parts[1].off);
+  a.t.moves = reinterpret_cast<const DpMove*>(base + parts[2].off);
+  a.t.tiles = reinterpret_cast<const u32*>(base + parts[3].off);
+  a.t.fams = reinterpret_cast<const DpFam*>(base + parts[4].off);
+  a.t.fam_child = reinterpret_cast<const u16*>(base + parts[5].off);
+  a.stage_base = reinterpret_cast<const u32*>(base + parts[6].off);
+  a.products = reinterpret_cast<const DpProduct*>(base + parts[7].off);
+  a.lists = reinterpret_cast<const u16*>(base + parts[8].off);
+  a.seeds = reinterpret_cast<const u64*>(base + parts[9].off);
+  a.t.n_positions = tab.n_positions;
+  a.n_stages = n_stages;
+  a.n_products = (u32)tab.products.size();
+  a.n_seeds = (u32)tab.seeds.size();
+  a.n_words = n_words;
+  a.found = static_cast<u32*>(b_bits_.p);
+  a.queue = reinterpret_cast<u64*>(static_cast<unsigned char*>(b_bits_.p) + word_bytes);
+  a.rank = static_cast<uint2*>(b_rank_.p);
+  a.t.rank = a.rank;
+  unsigned char* const res = static_cast<unsigned char*>(b_stage_lo_.p);
+  a.ctl = reinterpret_cast<PlanCtl*>(res);
+  a.stage_lo = reinterpret_cast<u32*>(res + align256(sizeof(PlanCtl)));
+  a.block_sums = reinterpret_cast<unsigned long long*>(res + back);
+  const PlanCtl* const ctl = static_cast<const PlanCtl*>(h_stage_);
+  const u32* const lo = reinterpret_cast<const u32*>(static_cast<unsigned char*>(h_stage_) + align256(sizeof(PlanCtl)));
+  // A warp per Spec: the grid follows the positions, up to what is co-resident. While positions are
+  // few, headers and records for all of them are reserved ahead and one launch does everything;
+  // otherwise the sizes come back after the closure, and again after the records are counted.
+  const u32 max_blocks = (u32)std::min(plan_blocks_ * n_sm_, coop_blocks_);
+  auto blocks = [&](uint64_t specs) { return (int)std::min<uint64_t>(max_blocks, std::max<uint64_t>(8, (specs + 7) / 8)); };
+  uint64_t want_specs = 0, want_cands = 0;
+  if (!fixed_) {
+    const uint64_t most = (uint64_t)tab.n_positions * tab.max_records;
+    want_specs = std::min<uint64_t>(tab.n_positions, 1u << 16);
+    want_cands = std::min<uint64_t>(most, 1u << 17);
+    if (b_cands_.cap > (size_t(256) << 20) && b_cands_.cap / sizeof(CandRec) / 16 > most) drop_(b_cands_);   // of a far larger plan
+  }
+  int phases = fixed_ ? DPP_CLOSURE : DPP_CLOSURE | DPP_SPECS | DPP_RECORDS;
+  for (int attempt = 0;; attempt++) {
+    if (phases & DPP_SPECS) {
+      if ((rc = reserve_(b_hdrs_, want_specs * sizeof(SpecHdr), false)) || (rc = reserve_(b_desc_, want_specs * sizeof(u64), false)))
+        return rc == -5 ? 1 : rc;
+      if ((phases & DPP_RECORDS) && (rc = reserve_(b_cands_, want_cands * sizeof(CandRec), false))) return rc == -5 ? 1 : rc;
+    }
+    a.hdrs = static_cast<SpecHdr*>(b_hdrs_.p);
+    a.desc = static_cast<u64*>(b_desc_.p);
+    a.cands = static_cast<CandRec*>(b_cands_.p);
+    a.cap_specs = (u32)std::min<uint64_t>(0xFFFFFFF0u, std::min(b_hdrs_.cap / sizeof(SpecHdr), b_desc_.cap / sizeof(u64)));
+    a.cap_cands = b_cands_.cap / sizeof(CandRec);
+    a.phases = phases;
+    CK(launch_plan_kernel(a, blocks(attempt == 0 ? tab.n_positions / 2 : want_specs), stream_));
+    CK(cudaMemcpyAsync(h_stage_, res, back, cudaMemcpyDeviceToHost, stream_));
+    CK(cudaStreamSynchronize(stream_));
+    if (ctl->n_specs > 0xFFFFFFF0u || ctl->n_cands > 0xFFFFFFFFull || attempt > 3) return 1;
+    want_specs = ctl->n_specs;
+    want_cands = ctl->n_cands;
+    if (ctl->n_specs > a.cap_specs || !b_hdrs_.p) phases = fixed_ ? DPP_SPECS : DPP_SPECS | DPP_RECORDS;
+    else if (ctl->n_cands > a.cap_cands || !b_cands_.p || !(phases & DPP_RECORDS)) phases = DPP_RECORDS;
+    else break;
+    if (phases == DPP_RECORDS && (rc = reserve_(b_cands_, std::max<uint64_t>(want_cands, 1) * sizeof(CandRec), false))) return rc == -5 ? 1 : rc;
+  }
+  d_hdrs_ = a.hdrs;
+  d_cands_ = a.cands;
+  n_specs_ = ctl->n_specs;
+  n_goals_ = ctl->n_goals;
+  n_cand_bytes_ = ctl->n_cands * sizeof(CandRec);
+  for (u32 g = 0; g < n_stages; g++)
+    if (lo[g + 1] > lo[g]) stages_.push_back(StageIds{lo[g], lo[g + 1], 0});
+  top_pack_ = 0;
+  for (int k = 0; k < NMEM; k++) top_pack_ |= tab.top_code[k] << (8 * k);
+  h2d_bytes_ = bytes;
+  tab_.reset(new DevTables());
+  tab_->t = a.t;
+  stats_ = FillStats();
+  return 0;
+}
+
+int DeviceFill::prepare_fill() {
+  CK(cudaSetDevice(device_));
+  int rc = working_buffers_(false, 1);
+  if (rc) return rc;
+  CK(cudaMemsetAsync(d_ctl_, 0, 512, stream_));
+  cands_present_ = true;
+  stats_ = FillStats();
+  return 0;
+}
+
 int DeviceFill::cands_arrived() {
   CK(cudaSetDevice(device_));
   if (cands_present_) return 0;
@@ -1850,22 +2082,20 @@ int DeviceFill::grow_after_error_(uint32_t bits) {
   if (fixed_) return too_large_();
   stats_.growths++;
   CK(cudaStreamSynchronize(stream_));
-  auto regrow = [&](void** p, uint64_t* cap, uint64_t need, size_t elem) -> int {
-    if (need <= *cap) return 0;
-    cudaFree(*p);
-    *p = nullptr;
-    *cap = 0;
-    const uint64_t want = need + need / 4;
-    int rc = alloc_(p, want * elem);
-    if (rc) return rc;
-    *cap = want;
-    return 0;
+  auto regrow = [&](DevBuf& b, uint64_t need, size_t elem) -> int {
+    return need * elem <= b.cap ? 0 : reserve_(b, (need + need / 4) * elem);
   };
-  int rc;
+  int rc = 0;
   if (bits & MRL_ERR_WORKING) {
-    if ((rc = regrow((void**)&d_temp_, &temp_cap_, h_ctl_->need_temp, 2 * sizeof(MrlRow)))) return rc;
-    if ((rc = regrow((void**)&d_chunks_, &chunk_cap_, h_ctl_->need_chunks, sizeof(Chunk)))) return rc;
-    if ((rc = regrow((void**)&d_items_, &item_cap_, h_ctl_->need_items, sizeof(WorkItem)))) return rc;
+    if ((rc = regrow(b_temp_, h_ctl_->need_temp, 2 * sizeof(MrlRow))) == 0 && (rc = regrow(b_chunks_, h_ctl_->need_chunks, sizeof(Chunk))) == 0)
+      rc = regrow(b_items_, h_ctl_->need_items, sizeof(WorkItem));
+    temp_cap_ = b_temp_.cap / (2 * sizeof(MrlRow));
+    chunk_cap_ = b_chunks_.cap / sizeof(Chunk);
+    item_cap_ = b_items_.cap / sizeof(WorkItem);
+    d_temp_ = static_cast<MrlRow*>(b_temp_.p);
+    d_chunks_ = static_cast<Chunk*>(b_chunks_.p);
+    d_items_ = static_cast<WorkItem*>(b_items_.p);
+    if (rc) return rc;
   }
   if (bits & MRL_ERR_TABLE) {
     const uint64_t need = h_ctl_->need_rows;
@@ -1880,8 +2110,9 @@ int DeviceFill::grow_after_error_(uint32_t bits) {
     }
     if (h_ctl_->final_top) CK(cudaMemcpyAsync(nr, d_rows_, h_ctl_->final_top * sizeof(MrlRow), cudaMemcpyDeviceToDevice, stream_));
     CK(cudaStreamSynchronize(stream_));
-    cudaFree(d_rows_);
-    d_rows_ = nr;
+    drop_(b_rows_);
+    b_rows_.p = d_rows_ = nr;
+    b_rows_.cap = cap * sizeof(MrlRow);
     row_cap_ = cap;
   }
   return 0;
@@ -1901,24 +2132,27 @@ int DeviceFill::begin_fill() {
   return 0;
 }
 
-int DeviceFill::launch_solve_(const Plan& plan, uint32_t si, bool place_too) {
-  const Stage& st = plan.stages[si];
-  const uint32_t n = st.spec_hi - st.spec_lo;
-  if (n == 0) return 0;
-  {
-    // the stage reads its own Specs' candidate records (ids, and with them the records, are in
-    // stage order): wait for that much of a background upload
-    const SpecHdr& last = plan.hdrs[st.spec_hi - 1];
-    int rc = wait_cands_(((uint64_t)last.cand_off + last.ncand) * sizeof(CandRec));
-    if (rc) return rc;
-  }
-  StageArgs a;
+void DeviceFill::stage_args_(void* args, uint32_t si) const {
+  StageArgs& a = *static_cast<StageArgs*>(args);
+  const StageIds& st = stages_[si];
   a.hdrs = d_hdrs_; a.cands = d_cands_; a.rmask = d_rmask_; a.mine = d_mine_; a.dirty = d_dirty_;
   a.chunks = d_chunks_; a.items = d_items_; a.rows = d_rows_; a.temp = d_temp_; a.base = d_temp_ + temp_cap_; a.ehdr = d_ehdr_;
   a.fcount = d_fcount_; a.block_sums = d_block_sums_; a.minsat = d_minsat_; a.corner = d_corner_; a.stamp = d_stamp_; a.ctl = d_ctl_;
-  a.lo = st.spec_lo; a.hi = st.spec_hi; a.top_pack = plan.top_pack(); a.stage = si;
-  a.prev_lo = si ? plan.stages[si - 1].spec_lo : 0; a.prev_hi = si ? plan.stages[si - 1].spec_hi : 0;
+  a.lo = st.lo; a.hi = st.hi; a.top_pack = top_pack_; a.stage = si;
+  a.prev_lo = si ? stages_[si - 1].lo : 0; a.prev_hi = si ? stages_[si - 1].hi : 0;
   a.temp_cap = temp_cap_; a.chunk_cap = chunk_cap_; a.item_cap = item_cap_; a.row_cap = row_cap_;
+}
+
+int DeviceFill::launch_solve_(uint32_t si, bool place_too) {
+  const StageIds& st = stages_[si];
+  const uint32_t n = st.hi - st.lo;
+  if (n == 0) return 0;
+  // the stage reads its own Specs' candidate records (ids, and with them the records, are in
+  // stage order): wait for that much of a background upload
+  int rc = wait_cands_(st.cand_end * sizeof(CandRec));
+  if (rc) return rc;
+  StageArgs a;
+  stage_args_(&a, si);
   a.solve = 1;
   a.place = place_too ? 1 : 0;
   // Small stages run on fewer blocks: a grid-wide barrier costs less, and there is no work for more.
@@ -1930,17 +2164,12 @@ int DeviceFill::launch_solve_(const Plan& plan, uint32_t si, bool place_too) {
   return 0;
 }
 
-int DeviceFill::launch_place_(const Plan& plan, uint32_t si) {
-  const Stage& st = plan.stages[si];
-  const uint32_t n = st.spec_hi - st.spec_lo;
+int DeviceFill::launch_place_(uint32_t si) {
+  const StageIds& st = stages_[si];
+  const uint32_t n = st.hi - st.lo;
   if (n == 0) return 0;
   StageArgs a;
-  a.hdrs = d_hdrs_; a.cands = d_cands_; a.rmask = d_rmask_; a.mine = d_mine_; a.dirty = d_dirty_;
-  a.chunks = d_chunks_; a.items = d_items_; a.rows = d_rows_; a.temp = d_temp_; a.base = d_temp_ + temp_cap_; a.ehdr = d_ehdr_;
-  a.fcount = d_fcount_; a.block_sums = d_block_sums_; a.minsat = d_minsat_; a.corner = d_corner_; a.stamp = d_stamp_; a.ctl = d_ctl_;
-  a.lo = st.spec_lo; a.hi = st.spec_hi; a.top_pack = plan.top_pack(); a.stage = si;
-  a.prev_lo = si ? plan.stages[si - 1].spec_lo : 0; a.prev_hi = si ? plan.stages[si - 1].spec_hi : 0;
-  a.temp_cap = temp_cap_; a.chunk_cap = chunk_cap_; a.item_cap = item_cap_; a.row_cap = row_cap_;
+  stage_args_(&a, si);
   a.solve = 0;
   a.place = 1;
   const uint64_t want = ((uint64_t)n + kBlock - 1) / kBlock;
@@ -1951,10 +2180,10 @@ int DeviceFill::launch_place_(const Plan& plan, uint32_t si) {
   return 0;
 }
 
-int DeviceFill::solve_stage(const Plan& plan, uint32_t si) {
-  if (si >= plan.stages.size()) { snprintf(err_, sizeof(err_), "stage index out of range"); return -3; }
+int DeviceFill::solve_stage(uint32_t si) {
+  if (si >= stages_.size()) { snprintf(err_, sizeof(err_), "stage index out of range"); return -3; }
   if (!filling_) { snprintf(err_, sizeof(err_), "no fill in progress"); return -3; }
-  return launch_solve_(plan, si, false);
+  return launch_solve_(si, false);
 }
 
 static const char* kErrorBits = "(1: candidate record out of range, 2: working buffers too small, 4: row table too small, "
@@ -1964,10 +2193,10 @@ static const char* kErrorBits = "(1: candidate record out of range, 2: working b
 // the stage). The masks must be final before they travel, so this is where a rank learns that its
 // solve ran out of working room: it enlarges its own buffers and solves the stage again; the other
 // ranks wait in the exchange.
-int DeviceFill::stage_masks(const Plan& plan, uint32_t si, void** ptr, uint64_t* bytes) {
-  if (si >= plan.stages.size()) { snprintf(err_, sizeof(err_), "stage index out of range"); return -3; }
-  const Stage& st = plan.stages[si];
-  if (filling_ && st.spec_hi != st.spec_lo) {
+int DeviceFill::stage_masks(uint32_t si, void** ptr, uint64_t* bytes) {
+  if (si >= stages_.size()) { snprintf(err_, sizeof(err_), "stage index out of range"); return -3; }
+  const StageIds& st = stages_[si];
+  if (filling_ && st.hi != st.lo) {
     int rc;
     if (read_ctl_() != 0) return -1;
     if (h_ctl_->error & MRL_ERR_WORKING) {
@@ -1978,7 +2207,7 @@ int DeviceFill::stage_masks(const Plan& plan, uint32_t si, void** ptr, uint64_t*
       }
       if ((rc = grow_after_error_(MRL_ERR_WORKING))) return rc;
       CK(cudaMemsetAsync(&d_ctl_->error, 0, sizeof(uint32_t), stream_));
-      if ((rc = launch_solve_(plan, si, false))) return rc;
+      if ((rc = launch_solve_(si, false))) return rc;
       if (read_ctl_() != 0) return -1;
       if (h_ctl_->error) {
         snprintf(err_, sizeof(err_), "stage %u failed again after its working buffers were enlarged (0x%x)", si, h_ctl_->error);
@@ -1986,23 +2215,23 @@ int DeviceFill::stage_masks(const Plan& plan, uint32_t si, void** ptr, uint64_t*
       }
     }
   }
-  if (ptr) *ptr = d_rmask_ + st.spec_lo;
-  if (bytes) *bytes = (uint64_t)(st.spec_hi - st.spec_lo) * sizeof(uint4);
+  if (ptr) *ptr = d_rmask_ + st.lo;
+  if (bytes) *bytes = (uint64_t)(st.hi - st.lo) * sizeof(uint4);
   return 0;
 }
 
 // Appends the stage's compacted grids to the table and reports where they went (the slice other
 // ranks need), which costs the one synchronisation of the stage. A stage that ran out of room is
 // run again here, whole, after its buffers have grown: its masks cannot have been exchanged yet.
-int DeviceFill::place_stage(const Plan& plan, uint32_t si, void** rows_ptr, uint64_t* bytes) {
-  if (si >= plan.stages.size()) { snprintf(err_, sizeof(err_), "stage index out of range"); return -3; }
+int DeviceFill::place_stage(uint32_t si, void** rows_ptr, uint64_t* bytes) {
+  if (si >= stages_.size()) { snprintf(err_, sizeof(err_), "stage index out of range"); return -3; }
   if (!filling_) { snprintf(err_, sizeof(err_), "no fill in progress"); return -3; }
   if (rows_ptr) *rows_ptr = d_rows_;
   if (bytes) *bytes = 0;
-  const Stage& st = plan.stages[si];
-  if (st.spec_hi == st.spec_lo) return 0;
+  const StageIds& st = stages_[si];
+  if (st.hi == st.lo) return 0;
   int rc;
-  if ((rc = launch_place_(plan, si))) return rc;
+  if ((rc = launch_place_(si))) return rc;
   if (read_ctl_() != 0) return -1;
   if (h_ctl_->error) {
     const uint32_t bits = h_ctl_->error;
@@ -2018,7 +2247,7 @@ int DeviceFill::place_stage(const Plan& plan, uint32_t si, void** rows_ptr, uint
     }
     if ((rc = grow_after_error_(bits))) return rc;
     CK(cudaMemsetAsync(&d_ctl_->error, 0, sizeof(uint32_t), stream_));
-    if ((rc = launch_place_(plan, si))) return rc;
+    if ((rc = launch_place_(si))) return rc;
     if (read_ctl_() != 0) return -1;
     if (h_ctl_->error) { snprintf(err_, sizeof(err_), "stage %u failed again after its buffers were enlarged (0x%x)", si, h_ctl_->error); return -2; }
   }
@@ -2062,13 +2291,13 @@ int DeviceFill::end_fill() {
 // geometry are all decided on the device. A stage that runs out of room raises an error word
 // that turns the stages behind it into no-ops; the host then enlarges the buffers it named and
 // resumes from that stage.
-int DeviceFill::run(const Plan& plan) {
+int DeviceFill::run() {
   int rc;
   if ((rc = begin_fill())) return rc;
   uint32_t from = 0;
   for (int attempt = 0;; attempt++) {
-    for (uint32_t s = from; s < plan.stages.size(); s++)
-      if ((rc = launch_solve_(plan, s, true))) return rc;
+    for (uint32_t s = from; s < stages_.size(); s++)
+      if ((rc = launch_solve_(s, true))) return rc;
     CK(cudaEventRecord(ev1_, stream_));
     if (read_ctl_() != 0) return -1;
     const uint32_t bits = h_ctl_->error;
@@ -2089,47 +2318,89 @@ int DeviceFill::run(const Plan& plan) {
   return 0;
 }
 
+// Point lookups: the queries go up from pinned staging and the rows come back into it, in batches.
+template <class Fill, class Launch>
+int DeviceFill::lookup_batches_(size_t n, size_t query_bytes, MrlRow* out, Fill fill, Launch launch) {
+  const size_t per = std::max(query_bytes, sizeof(MrlRow));
+  size_t batch = std::min<size_t>(n, size_t(1) << 20);
+  if (fixed_) batch = std::min(n, b_lookup_.cap / 2 / per);
+  else {
+    int rc = reserve_(b_lookup_, 2 * align256(batch * per));
+    if (rc) return rc;
+  }
+  if (batch == 0) { snprintf(err_, sizeof(err_), "lookup staging too small"); return -5; }
+  int rc = reserve_host_(batch * per);
+  if (rc) return rc;
+  unsigned char* const d_q = static_cast<unsigned char*>(b_lookup_.p);
+  MrlRow* const d_out = reinterpret_cast<MrlRow*>(d_q + b_lookup_.cap / 2 / 256 * 256);
+  for (size_t done = 0; done < n; done += batch) {
+    const size_t m = std::min(batch, n - done);
+    fill(h_stage_, done, m);
+    CK(cudaMemcpyAsync(d_q, h_stage_, m * query_bytes, cudaMemcpyHostToDevice, stream_));
+    launch(d_q, m, d_out);
+    CK(cudaGetLastError());
+    CK(cudaMemcpyAsync(h_stage_, d_out, m * sizeof(MrlRow), cudaMemcpyDeviceToHost, stream_));
+    CK(cudaStreamSynchronize(stream_));
+    memcpy(out + done, h_stage_, m * sizeof(MrlRow));
+  }
+  return 0;
+}
+
 int DeviceFill::lookup(const uint32_t* spec_ids, const uint32_t* cpacks, size_t n, MrlRow* out) {
-  std::lock_guard<std::mutex> guard(lookup_mu_);   // callers on several threads share the staging buffer and the stream
+  std::lock_guard<std::mutex> guard(lookup_mu_);   // callers on several threads share the staging buffers and the stream
   CK(cudaSetDevice(device_));
   if (n == 0) return 0;
   for (size_t i = 0; i < n; i++)
     if (spec_ids[i] >= n_specs_) { snprintf(err_, sizeof(err_), "Spec id out of range"); return -3; }
-  const size_t per = sizeof(uint2) + sizeof(MrlRow);
-  size_t batch = std::min<size_t>(n, size_t(1) << 22);
-  if (fixed_) batch = std::min(n, stage_bytes_ / 2 / per);
-  else if (stage_bytes_ < 2 * align256(batch * sizeof(MrlRow))) {
-    CK(cudaStreamSynchronize(stream_));
-    if (d_stage_) cudaFree(d_stage_);
-    d_stage_ = nullptr;
-    stage_bytes_ = 0;
-    int rc = alloc_(&d_stage_, 2 * align256(batch * sizeof(MrlRow)));
-    if (rc) return rc;
-    stage_bytes_ = 2 * align256(batch * sizeof(MrlRow));
-  }
-  if (batch == 0) { snprintf(err_, sizeof(err_), "lookup staging too small"); return -5; }
-  std::vector<uint2> q(batch);
-  for (size_t done = 0; done < n; done += batch) {
-    const size_t m = std::min(batch, n - done);
-    for (size_t i = 0; i < m; i++) q[i] = make_uint2(spec_ids[done + i], cpacks[done + i]);
-    uint2* d_q = static_cast<uint2*>(d_stage_);
-    MrlRow* d_out = reinterpret_cast<MrlRow*>(static_cast<unsigned char*>(d_stage_) + stage_bytes_ / 2);
-    CK(cudaMemcpyAsync(d_q, q.data(), m * sizeof(uint2), cudaMemcpyHostToDevice, stream_));
-    lookup_rows_kernel<<<(unsigned)((m + 255) / 256), 256, 0, stream_>>>(d_hdrs_, d_rows_, d_q, m, d_out);
-    CK(cudaGetLastError());
-    CK(cudaMemcpyAsync(out + done, d_out, m * sizeof(MrlRow), cudaMemcpyDeviceToHost, stream_));
-    CK(cudaStreamSynchronize(stream_));
-  }
+  return lookup_batches_(n, sizeof(uint2), out,
+                         [&](void* to, size_t at, size_t m) {
+                           uint2* q = static_cast<uint2*>(to);
+                           for (size_t i = 0; i < m; i++) q[i] = make_uint2(spec_ids[at + i], cpacks[at + i]);
+                         },
+                         [&](const void* q, size_t m, MrlRow* d_out) {
+                           lookup_rows_kernel<<<(unsigned)((m + kBlock - 1) / kBlock), kBlock, 0, stream_>>>(
+                               d_hdrs_, d_rows_, static_cast<const uint2*>(q), m, d_out);
+                         });
+}
+
+int DeviceFill::lookup_packed(const uint64_t* specs, const uint32_t* cpacks, size_t n, MrlRow* out) {
+  std::lock_guard<std::mutex> guard(lookup_mu_);
+  CK(cudaSetDevice(device_));
+  if (n == 0) return 0;
+  if (!tab_) { snprintf(err_, sizeof(err_), "no plan made on the device"); return -3; }
+  return lookup_batches_(n, sizeof(PackedQuery), out,
+                         [&](void* to, size_t at, size_t m) {
+                           PackedQuery* q = static_cast<PackedQuery*>(to);
+                           for (size_t i = 0; i < m; i++) q[i] = PackedQuery{specs[at + i], cpacks[at + i], 0u};
+                         },
+                         [&](const void* q, size_t m, MrlRow* d_out) {
+                           lookup_packed_kernel<<<(unsigned)((m + kBlock - 1) / kBlock), kBlock, 0, stream_>>>(
+                               tab_->t, d_hdrs_, d_rows_, static_cast<const PackedQuery*>(q), m, d_out);
+                         });
+}
+
+int DeviceFill::read_specs(uint64_t* out) {
+  CK(cudaSetDevice(device_));
+  if (!tab_) { snprintf(err_, sizeof(err_), "no plan made on the device"); return -3; }
+  CK(cudaMemcpyAsync(out, b_desc_.p, (size_t)n_specs_ * sizeof(uint64_t), cudaMemcpyDeviceToHost, stream_));
+  CK(cudaStreamSynchronize(stream_));
+  return 0;
+}
+
+int DeviceFill::read_hdrs(SpecHdr* out) {
+  CK(cudaSetDevice(device_));
+  if (n_specs_) CK(cudaMemcpyAsync(out, d_hdrs_, (size_t)n_specs_ * sizeof(SpecHdr), cudaMemcpyDeviceToHost, stream_));
+  CK(cudaStreamSynchronize(stream_));
   return 0;
 }
 
 // Checks the finished table against its defining recurrence at n_samples pseudo-random points of
 // (Spec x limits lattice), or at every point when n_samples == 0.
-int DeviceFill::verify(const Plan& plan, uint64_t n_samples, uint64_t seed, uint64_t* checked, uint64_t* mismatches,
+int DeviceFill::verify(uint64_t n_samples, uint64_t seed, uint64_t* checked, uint64_t* mismatches,
                        uint64_t* first_bad) {
   CK(cudaSetDevice(device_));
   if (wait_upload()) return -1;
-  const uint32_t top = plan.top_pack();
+  const uint32_t top = top_pack_;
   unsigned long long per_spec = 1;
   for (int k = 0; k < 4; k++) per_spec *= ((top >> (8 * k)) & 0xFFu) + 1u;
   const unsigned long long total = per_spec * n_specs_;
@@ -2178,18 +2449,14 @@ int DeviceFill::read_table(SpecHdr* hdrs_out, MrlRow* rows_out) {
   return 0;
 }
 
-int DeviceFill::load_table(const Plan& plan, const SpecHdr* hdrs, const MrlRow* rows, uint64_t n_rows) {
+int DeviceFill::load_table(const SpecHdr* hdrs, const MrlRow* rows, uint64_t n_rows) {
   CK(cudaSetDevice(device_));
-  if (plan.hdrs.size() != n_specs_) { snprintf(err_, sizeof(err_), "the saved table belongs to another plan"); return -3; }
   if (n_rows > row_cap_) {
     if (fixed_) return too_large_();
-    CK(cudaStreamSynchronize(stream_));
-    cudaFree(d_rows_);
-    d_rows_ = nullptr;
-    row_cap_ = 0;
-    int rc = alloc_((void**)&d_rows_, n_rows * sizeof(MrlRow));
+    int rc = reserve_(b_rows_, n_rows * sizeof(MrlRow));
+    d_rows_ = static_cast<MrlRow*>(b_rows_.p);
+    row_cap_ = b_rows_.cap / sizeof(MrlRow);
     if (rc) return rc;
-    row_cap_ = n_rows;
   }
   if (n_specs_) CK(cudaMemcpyAsync(d_hdrs_, hdrs, (size_t)n_specs_ * sizeof(SpecHdr), cudaMemcpyHostToDevice, stream_));
   if (n_rows) CK(cudaMemcpyAsync(d_rows_, rows, n_rows * sizeof(MrlRow), cudaMemcpyHostToDevice, stream_));
@@ -2275,9 +2542,30 @@ int fill_static(int device, cudaStream_t stream, const Plan& plan, const uint32_
   f.attach_buffer(base, (size_t)MRL_STATIC_SCRATCH_BYTES, stream, device);
   int rc = f.init_events();
   if (rc == 0) rc = f.upload(plan);
-  if (rc == 0) rc = f.run(plan);
+  if (rc == 0) rc = f.run();
   if (rc == 0) rc = f.lookup(spec_ids, cpacks, n, out);
   if (rc != 0) snprintf(err, err_len, "%s", f.error());
+  return rc;
+}
+
+int fill_static(int device, cudaStream_t stream, const OpTables& tab, const uint64_t* specs, const uint32_t* cpacks,
+                size_t n, MrlRow* out, char* err, size_t err_len) {
+  void* base = nullptr;
+  cudaError_t e = static_scratch_address(device, &base);
+  if (e == cudaSuccess) e = cudaSetDevice(device);
+  if (e != cudaSuccess) {
+    snprintf(err, err_len, "static scratch unavailable: %s", cudaGetErrorString(e));
+    return -1;
+  }
+  DeviceFill f;
+  f.attach_buffer(base, (size_t)MRL_STATIC_SCRATCH_BYTES, stream, device);
+  int rc = f.init_events();
+  if (rc == 0) rc = f.plan(tab);
+  if (rc == 0) rc = f.prepare_fill();
+  if (rc == 0) rc = f.run();
+  if (rc == -5) rc = 1;   // the plan's tables take a little room of their own: without them it may fit
+  if (rc == 0) rc = f.lookup_packed(specs, cpacks, n, out);
+  if (rc < 0) snprintf(err, err_len, "%s", f.error());
   return rc;
 }
 

@@ -2,6 +2,7 @@
 // stages. Callers hand in host data only.
 #pragma once
 #include "plan.hpp"
+#include "optable.hpp"
 #include <cuda_runtime.h>
 #include <atomic>
 #include <memory>
@@ -35,6 +36,7 @@ struct FillStats {
 
 class DeviceFill {
  public:
+  DeviceFill();
   ~DeviceFill();
   int init(int device);
   int init_events();   // the part of init a caller with its own stream and buffer needs
@@ -48,6 +50,22 @@ class DeviceFill {
   // skip_cands: the candidate records are not on this host; the caller fills device_cands()
   // itself (e.g. a broadcast from the rank that planned) and then calls cands_arrived().
   int upload(const Plan& plan, bool skip_cands = false);
+  // Plans the job on the device (devplan.cu): ids, headers and candidate records are worked out
+  // there from the factored tables. On return the plan's sizes are known; prepare_fill() then does
+  // for it what upload() does for a host plan. 1: not covered, or the fixed buffer is too small -
+  // plan on the host.
+  int plan(const OpTables& tab);
+  int prepare_fill();
+  struct StageIds { uint32_t lo, hi; uint64_t cand_end; };
+  const std::vector<StageIds>& stages() const { return stages_; }
+  uint64_t n_goals() const { return n_goals_; }
+  uint64_t n_cands() const { return n_cand_bytes_ / sizeof(CandRec); }
+  // Rows of Specs of a plan made on the device, by packed family and operands (OpTables::locate);
+  // a Spec that does not exist gets aux = 1.
+  int lookup_packed(const uint64_t* specs, const uint32_t* cpacks, size_t n, MrlRow* out);
+  // Packed family and operands of every Spec of a plan made on the device.
+  int read_specs(uint64_t* out);
+  int read_hdrs(SpecHdr* out);
   // Blocks until every candidate record is on the device.
   int wait_upload();
   void* device_cands() const { return d_cands_; }
@@ -56,20 +74,20 @@ class DeviceFill {
   // inside the plan, kinds and levels in range) and lets fills run.
   int cands_arrived();
   // Runs every stage: two launches per stage, no host synchronisation before the end.
-  int run(const Plan& plan);
+  int run();
   // The same one stage at a time, for callers that exchange tables between stages (multi-GPU):
   // begin_fill; per stage solve_stage, [exchange stage_masks], place_stage, [exchange rows];
   // end_fill. All work is enqueued on the stream; place_stage synchronises it once.
   int begin_fill();
-  int solve_stage(const Plan& plan, uint32_t stage);
-  int stage_masks(const Plan& plan, uint32_t stage, void** ptr, uint64_t* bytes);
-  int place_stage(const Plan& plan, uint32_t stage, void** rows_ptr, uint64_t* bytes);
+  int solve_stage(uint32_t stage);
+  int stage_masks(uint32_t stage, void** ptr, uint64_t* bytes);
+  int place_stage(uint32_t stage, void** rows_ptr, uint64_t* bytes);
   int end_fill();
   // Run on a caller-owned stream (e.g. the one a collective library orders against).
   int set_stream(cudaStream_t s);
   // Point lookups: rows of (Spec id, packed limit codes).
   int lookup(const uint32_t* spec_ids, const uint32_t* cpacks, size_t n, MrlRow* out);
-  int verify(const Plan& plan, uint64_t n_samples, uint64_t seed, uint64_t* checked, uint64_t* mismatches,
+  int verify(uint64_t n_samples, uint64_t seed, uint64_t* checked, uint64_t* mismatches,
              uint64_t* first_bad);
   // Order-independent 64-bit checksum of the logical table: per Spec its id, masks and rows in
   // cell order; where the rows lie in the table does not enter.
@@ -77,7 +95,7 @@ class DeviceFill {
   // The whole finished table in two copies: headers (masks, first row) and rows.
   int read_table(SpecHdr* hdrs_out, MrlRow* rows_out);
   // Replaces the table by a saved one (hdrs as read_table gave them).
-  int load_table(const Plan& plan, const SpecHdr* hdrs, const MrlRow* rows, uint64_t n_rows);
+  int load_table(const SpecHdr* hdrs, const MrlRow* rows, uint64_t n_rows);
   int read_hdr(uint32_t spec, SpecHdr* out);
   int read_rows(uint64_t first, uint64_t n, MrlRow* out);
   void release();
@@ -90,10 +108,16 @@ class DeviceFill {
   uint32_t n_specs() const { return n_specs_; }
 
  private:
+  // A device buffer that stays from one plan to the next while its size is of the right order.
+  struct DevBuf { void* p = nullptr; size_t cap = 0; };
+  int reserve_(DevBuf& b, size_t bytes, bool give_back = true);
+  void drop_(DevBuf& b);
   int alloc_(void** p, size_t bytes);
-  void free_(void* p);
-  int launch_solve_(const Plan& plan, uint32_t stage, bool place_too);
-  int launch_place_(const Plan& plan, uint32_t stage);
+  void begin_plan_();
+  int working_buffers_(bool sharded_mine, uint32_t world);
+  void stage_args_(void* args, uint32_t stage) const;
+  int launch_solve_(uint32_t stage, bool place_too);
+  int launch_place_(uint32_t stage);
   int read_ctl_();                       // device control block -> h_ctl_ (synchronises the stream)
   int grow_after_error_(uint32_t bits);  // enlarges the buffers a failed stage asked for
   int wait_cands_(uint64_t upto_bytes);  // until the candidate bytes [0, upto_bytes) are on the device
@@ -104,6 +128,9 @@ class DeviceFill {
   bool fixed_ = false;            // carved from an attached buffer: no growth
   unsigned char* buf_ = nullptr;  // attached buffer
   size_t buf_bytes_ = 0, buf_off_ = 0;
+  // buffers, and what lies in them
+  DevBuf b_ctl_, b_hdrs_, b_cands_, b_spec_, b_stage_specs_, b_mine_, b_chunks_, b_items_, b_temp_, b_rows_, b_lookup_;
+  DevBuf b_tables_, b_bits_, b_rank_, b_desc_, b_stage_lo_;   // of planning on the device
   SpecHdr* d_hdrs_ = nullptr;
   CandRec* d_cands_ = nullptr;
   uint4* d_rmask_ = nullptr;
@@ -120,8 +147,18 @@ class DeviceFill {
   uint32_t* d_fcount_ = nullptr;
   unsigned long long* d_block_sums_ = nullptr;
   FillCtl* d_ctl_ = nullptr;
-  void* d_stage_ = nullptr;      // lookup staging
-  size_t stage_bytes_ = 0;
+  std::vector<StageIds> stages_;
+  uint32_t top_pack_ = 0;
+  uint64_t n_goals_ = 0;
+  // the tables of a plan made on the device: what lookups address with
+  struct DevTables;
+  std::unique_ptr<DevTables> tab_;
+  void* h_stage_ = nullptr;      // pinned staging for tables, plan results and lookups
+  size_t h_stage_bytes_ = 0;
+  int reserve_host_(size_t bytes);
+  std::vector<unsigned char> h_pageable_;   // h_stage_ of a fixed buffer
+  template <class Fill, class Launch>
+  int lookup_batches_(size_t n, size_t query_bytes, MrlRow* out, Fill fill, Launch launch);
   FillCtl* h_ctl_ = nullptr;     // pinned, or &ctl_pageable_ when nothing may be allocated
   FillCtl ctl_pageable_;
   uint32_t n_specs_ = 0, max_stage_ = 1;
@@ -131,6 +168,7 @@ class DeviceFill {
   bool cands_present_ = false;   // the device candidate records are complete and checked
   bool filling_ = false;
   int coop_blocks_ = 0;          // co-resident blocks of the stage kernel on this device
+  int plan_blocks_ = 0;          // ... of the plan kernel, per SM
   int n_sm_ = 0;
   FillStats stats_;
   cudaStream_t stream_ = nullptr;
@@ -152,6 +190,9 @@ class DeviceFill {
 // One whole small fill inside the fixed device array: plan arrays, working buffers, row table
 // and lookup staging; no device allocation. See combine.cu.
 int fill_static(int device, cudaStream_t stream, const Plan& plan, const uint32_t* spec_ids, const uint32_t* cpacks,
+                size_t n, MrlRow* out, char* err, size_t err_len);
+// The same with the plan made on the device too; 1: plan on the host.
+int fill_static(int device, cudaStream_t stream, const OpTables& tab, const uint64_t* specs, const uint32_t* cpacks,
                 size_t n, MrlRow* out, char* err, size_t err_len);
 
 }  // namespace mrl

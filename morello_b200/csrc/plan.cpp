@@ -371,12 +371,11 @@ void Plan::adopt_done(u32 rank_, u32 world_, int n_threads_, bool have_cands) {
   assign_owners_();
 }
 
-u64 Plan::fingerprint(int n_threads_) const {
-  const size_t n = specs.size();
+u64 fingerprint_of(size_t n, const std::function<LogicalSpec(size_t)>& spec, const u32 top_code[NMEM], int n_threads) {
   std::vector<u64> hs(n);
-  parallel_for(n, n_threads_, [&](size_t i, int) {
+  parallel_for(n, n_threads, [&](size_t i, int) {
     char kb[LogicalSpec::MAX_KEY];
-    const int kl = specs[i].key_into(kb);
+    const int kl = spec(i).key_into(kb);
     hs[i] = hash_key(kb, kl) * (2 * (u64)i + 1);
   });
   u64 h = 0x243F6A8885A308D3ull ^ (u64)n;
@@ -385,17 +384,11 @@ u64 Plan::fingerprint(int n_threads_) const {
   return h ^ (h >> 31);
 }
 
-bool Plan::pack_limits(const u64 limits[NMEM], u32* out) const {
-  u32 pack = 0;
-  for (int k = 0; k < NMEM; k++) {
-    if (!mem_counts_registers((Mem)k) && limits[k] != 0 && !is_pow2(limits[k])) return false;
-    u32 code = limit_code(k, limits[k]);
-    if (code > top_code[k]) return false;  // beyond the limits this table was filled for
-    pack |= code << (8 * k);
-  }
-  *out = pack;
-  return true;
+u64 Plan::fingerprint(int n_threads_) const {
+  return fingerprint_of(specs.size(), [this](size_t i) { return specs[i]; }, top_code, n_threads_);
 }
+
+bool Plan::pack_limits(const u64 limits[NMEM], u32* out) const { return pack_limit_codes(limits, top_code, out); }
 
 namespace {
 

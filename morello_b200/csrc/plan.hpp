@@ -18,6 +18,7 @@
 #include "model/space.hpp"
 #include "device_types.h"
 #include <cstdlib>
+#include <functional>
 #include <new>
 #include <string>
 #include <memory>
@@ -181,6 +182,22 @@ std::vector<LogicalSpec> precompute_goals(u32 size, Through through, const std::
 
 // Lattice code <-> value helpers shared by planner and lookups.
 inline u32 limit_code(int mem, u64 value) { return mem_counts_registers((Mem)mem) ? (u32)value : bit_length(value); }
+// Limits as packed lattice codes (RF in byte 0 .. GL in byte 3); false when they are not lattice
+// points or exceed the top limits.
+inline bool pack_limit_codes(const u64 limits[NMEM], const u32 top_code[NMEM], u32* out) {
+  u32 pack = 0;
+  for (int k = 0; k < NMEM; k++) {
+    if (!mem_counts_registers((Mem)k) && limits[k] != 0 && !is_pow2(limits[k])) return false;
+    const u32 code = limit_code(k, limits[k]);
+    if (code > top_code[k]) return false;  // beyond the limits the table was filled for
+    pack |= code << (8 * k);
+  }
+  *out = pack;
+  return true;
+}
+
+// Fingerprint of a job by its Specs in id order and its top limits (Plan::fingerprint).
+u64 fingerprint_of(size_t n, const std::function<LogicalSpec(size_t)>& spec, const u32 top_code[NMEM], int n_threads);
 inline u64 limit_value(int mem, u32 code) { return mem_counts_registers((Mem)mem) ? code : bit_length_inverse(code); }
 
 }  // namespace mrl
