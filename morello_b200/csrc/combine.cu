@@ -62,8 +62,8 @@ static_assert(MRL_STATIC_SCRATCH_BYTES == MRL_NOALLOC_MAX_BYTES,
 
 namespace {
 
-constexpr int kBlock = 128;      // threads per block of every kernel here
-constexpr int kMinBlocks = 8;   // resident blocks per SM the stage kernel is compiled for
+constexpr int kBlock = 128;         // threads per block of the small kernels here
+constexpr int kStageBlock = 1024;   // ... of the stage kernel: one block per SM (64 registers), so few arrive at a barrier
 constexpr int kMaxPasses = 128;
 constexpr int kMaxSweeps = 256;   // per pass; a dependency chain is shorter than the 70 diagonals of the limits lattice
 
@@ -114,10 +114,9 @@ __device__ __forceinline__ uint32_t sel4(uint32_t a0, uint32_t a1, uint32_t a2, 
 }
 __device__ __forceinline__ uint32_t below(uint32_t code) { return (2u << code) - 1u; }   // codes <= code
 
-// The running optimum of a cell: the row's three key words and the index of the winning
-// candidate record within its Spec.
+// The running optimum of a cell: the row's three key words.
 struct Best {
-  uint32_t main, peaks, tail, ci;
+  uint32_t main, peaks, tail;
 };
 __device__ __forceinline__ bool key_less(uint32_t m, uint32_t p, uint32_t t, const Best& b) {
   if (m != b.main) return m < b.main;
@@ -165,7 +164,7 @@ __device__ __forceinline__ uint4 lookup(const SpecHdr* hdrs, const MrlRow* rows,
 // launch and may take the non-coherent load path.
 template <bool kFinished>
 __device__ __forceinline__ void eval_candidate(const SpecHdr* hdrs, const CandRec* __restrict__ cands, const MrlRow* rows,
-                                               const MrlRow* temp, uint32_t rec, const uint4 a, uint32_t ci, uint32_t cpack,
+                                               const MrlRow* temp, uint32_t rec, const uint4 a, uint32_t cpack,
                                                uint32_t bm0, uint32_t bm1, uint32_t bm2, uint32_t bm3, Best& best,
                                                Tally& tally) {
   const uint32_t action = a.x & 0xFFFFu, kind = (a.x >> 16) & 0xFFu, nchild = a.x >> 24;
@@ -242,7 +241,6 @@ __device__ __forceinline__ void eval_candidate(const SpecHdr* hdrs, const CandRe
     best.main = k_main;
     best.peaks = k_peaks;
     best.tail = k_tail;
-    best.ci = ci;
   }
 }
 
@@ -253,61 +251,15 @@ __device__ __forceinline__ Best solve_point(const SpecHdr* hdrs, const CandRec* 
   const uint32_t bm0 = below(code_of(cpack, 0)), bm1 = below(code_of(cpack, 1)), bm2 = below(code_of(cpack, 2)),
                  bm3 = below(code_of(cpack, 3));
   const uint2 cl = *reinterpret_cast<const uint2*>(&hdrs[spec].cand_off);
-  Best best = {MRL_UNSAT, MRL_UNSAT, MRL_UNSAT, MRL_UNSAT};
+  Best best = {MRL_UNSAT, MRL_UNSAT, MRL_UNSAT};
   for (uint32_t ci = 0; ci < cl.y; ci++) {
     const uint4 a = __ldg(reinterpret_cast<const uint4*>(&cands[cl.x + ci]));
-    eval_candidate<false>(hdrs, cands, rows, temp, cl.x + ci, a, ci, cpack, bm0, bm1, bm2, bm3, best, tally);
+    eval_candidate<false>(hdrs, cands, rows, temp, cl.x + ci, a, cpack, bm0, bm1, bm2, bm3, best, tally);
   }
   return best;
 }
 
 // ---- working grids ---------------------------------------------------------------------
-
-struct Grid {   // what a Spec's masks imply
-  uint32_t nn[4];
-  unsigned long long cells;
-  uint32_t F, cols, warps;
-};
-__device__ __forceinline__ Grid grid_of(const uint4 m) {
-  Grid g;
-  g.nn[0] = __popc(m.x); g.nn[1] = __popc(m.y); g.nn[2] = __popc(m.z); g.nn[3] = __popc(m.w);
-  g.cells = (unsigned long long)g.nn[0] * g.nn[1] * g.nn[2] * g.nn[3];
-  // The free memory is the one with the most slots (lowest index on ties): the longest columns,
-  // so the fewest chunks.
-  g.F = 0;
-  uint32_t best = g.nn[0];
-#pragma unroll
-  for (int k = 1; k < 4; k++)
-    if (g.nn[k] > best) { best = g.nn[k]; g.F = k; }
-  g.cols = (uint32_t)(g.cells / best);
-  g.warps = (g.cols + 31u) / 32u;
-  return g;
-}
-
-// Geometry of one thread's column. A column fixes the slot index in the three memories other
-// than the Spec's free memory F.
-struct Column {
-  uint32_t spec, F;
-  uint32_t mm[4], nn[4], idx[4];
-  bool valid;
-};
-__device__ __forceinline__ Column decode_column(const SpecHdr* hdrs, const Chunk ch, uint32_t lane) {
-  Column c;
-  c.spec = ch.spec;
-  c.F = ch.col_start >> 30;
-  const uint4 m = *reinterpret_cast<const uint4*>(&hdrs[ch.spec]);
-  c.mm[0] = m.x; c.mm[1] = m.y; c.mm[2] = m.z; c.mm[3] = m.w;
-  uint32_t rest = (ch.col_start & 0x3FFFFFFFu) + lane;
-#pragma unroll
-  for (int k = 0; k < 4; k++) {
-    c.nn[k] = (uint32_t)__popc(c.mm[k]);
-    const uint32_t nk = ((uint32_t)k == c.F) ? 1u : c.nn[k];
-    c.idx[k] = rest % nk;   // for F: slot 0
-    rest /= nk;
-  }
-  c.valid = rest == 0;  // false: column index beyond this Spec's grid
-  return c;
-}
 
 __device__ __forceinline__ void or_level(uint32_t& r0, uint32_t& r1, uint32_t& r2, uint32_t& r3, uint32_t level,
                                          uint32_t bits) {
@@ -335,142 +287,100 @@ __device__ __forceinline__ uint32_t shift_mask(uint32_t cm, uint32_t level, uint
   return out;
 }
 
-// Exclusive prefix of v over the block (kBlock threads); *total = the block's sum.
-__device__ __forceinline__ unsigned long long block_excl_scan(unsigned long long v, unsigned long long* total) {
-  __shared__ unsigned long long warp_sum[kBlock / 32];
-  __shared__ unsigned long long block_total;
-  const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  unsigned long long inc = v;
-  for (int o = 1; o < 32; o <<= 1) {
-    const unsigned long long t = __shfl_up_sync(0xFFFFFFFFu, inc, o);
-    if (lane >= (uint32_t)o) inc += t;
-  }
-  __syncthreads();   // protects the shared arrays across consecutive calls
-  if (lane == 31) warp_sum[w] = inc;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    unsigned long long run = 0;
-    for (int k = 0; k < kBlock / 32; k++) { const unsigned long long t = warp_sum[k]; warp_sum[k] = run; run += t; }
-    block_total = run;
-  }
-  __syncthreads();
-  *total = block_total;
-  return warp_sum[w] + inc - v;
-}
-
-// Everything a stage kernel needs; passed by value.
+// A run of stages, as one launch sees it; passed by value.
 struct StageArgs {
   SpecHdr* hdrs;
   const CandRec* cands;
   uint4* rmask;
   const uint8_t* mine;    // null: every Spec is computed here
-  uint8_t* dirty;         // by Spec id: 0 keep, 1 solve in the coming pass, 2 being solved in this pass
-  Chunk* chunks;
   WorkItem* items;
   MrlRow* rows;
-  MrlRow* temp;
-  MrlRow* base;                   // as many rows again: the grids of the unordered phase
-  SpecHdr* ehdr;                  // by position in the stage: masks and first row (in base) of the Spec's grid of the unordered phase
-  uint32_t* fcount;
+  MrlRow* temp;           // working rows; temp_cap rows further on, the grids of the unordered phase
+  uint32_t* minsat;       // by Spec id: lower corner of the satisfiable region (see phase_minsat)
+  StageSpec* sspec;       // by position in the stage
+  uint4* changed[3];      // by position in the stage, three sweeps in turn: codes of the slots a sweep changed
   unsigned long long* block_sums;
-  uint32_t* minsat;               // by Spec id: lower corner of the satisfiable region (see phase_minsat)
-  uint32_t* corner;               // by position in the stage: the corner its working grids are clipped at
-  uint32_t* stamp;                // by position in the stage: last relaxation sweep that improved a cell of the Spec
   FillCtl* ctl;
-  uint32_t lo, hi;                // the stage's Spec ids
-  uint32_t prev_lo, prev_hi;      // the stage before it
+  const uint2* stages;    // [first, end) Spec id of every stage
+  uint32_t stage_lo, stage_hi;   // the stages of this launch
   uint32_t top_pack;
-  uint32_t stage;
-  unsigned long long temp_cap, chunk_cap, item_cap, row_cap;
-  int solve, place;               // which halves to run
+  uint32_t team;          // TEAM_*: what a barrier spans
+  unsigned long long temp_cap, item_cap, row_cap;
+  int solve, place;       // which halves to run
 };
+enum { TEAM_BLOCK = 0, TEAM_CLUSTER = 1, TEAM_GRID = 2 };
 
 __device__ __forceinline__ bool computed_here(const StageArgs& a, uint32_t i) { return !a.mine || a.mine[i]; }
 
 // Lower corner of a Spec's satisfiable region: per memory the smallest limit code at which any
-// implementation exists at all, 5 bits each (RF in the low bits); 31 = none anywhere. More memory
+// implementation exists at all, one byte each (RF in the low byte); 31 = none anywhere. More memory
 // never loses an implementation, so every limits point with a coordinate below the corner is
 // unsatisfiable. For a finished Spec the corner is exact (read off its table); for a Spec of the
 // stage being solved it is a lower bound worked out from its candidates before anything is solved.
 #define MRL_NEVER 31u
-__device__ __forceinline__ uint32_t corner_of(uint32_t pack, uint32_t k) { return (pack >> (5 * k)) & 31u; }
+#define MRL_NEVER4 0x1F1F1F1Fu
+__device__ __forceinline__ uint32_t corner_of(uint32_t pack, uint32_t k) { return (pack >> (8 * k)) & 0xFFu; }
+// A cell with a limit below its Spec's corner has no implementation; no record needs to be read.
+__device__ __forceinline__ bool below_corner(uint32_t corner, uint32_t cpack) { return __vcmpltu4(cpack, corner) != 0; }
 
-// Exact corners of the Specs of the stage before this one (their rows are complete, also where
-// another rank computed them). Along memory k the cell with the top slot in every other memory is
-// satisfiable as soon as any cell with that slot in k is.
-__device__ __noinline__ void phase_minsat(const StageArgs& a, uint32_t gtid, uint32_t gthreads) {
-  for (uint32_t i = a.prev_lo + gtid; i < a.prev_hi; i += gthreads) {
-    const uint4 m = *reinterpret_cast<const uint4*>(&a.hdrs[i]);
-    const MrlRow* grid = a.rows + a.hdrs[i].row_base;
-    const uint32_t mm[4] = {m.x, m.y, m.z, m.w};
-    uint32_t nn[4], st[4];
+// Exact corner of a Spec from its finished rows. Along memory k the cell with the top slot in
+// every other memory is satisfiable as soon as any cell with that slot in k is.
+__device__ __forceinline__ uint32_t corner_from_rows(const uint4 m, const MrlRow* grid) {
+  const uint32_t mm[4] = {m.x, m.y, m.z, m.w};
+  uint32_t nn[4], st[4];
 #pragma unroll
-    for (int k = 0; k < 4; k++) nn[k] = __popc(mm[k]);
-    st[0] = 1; st[1] = nn[0]; st[2] = nn[0] * nn[1]; st[3] = nn[0] * nn[1] * nn[2];
-    uint32_t top = 0;
+  for (int k = 0; k < 4; k++) nn[k] = __popc(mm[k]);
+  st[0] = 1; st[1] = nn[0]; st[2] = nn[0] * nn[1]; st[3] = nn[0] * nn[1] * nn[2];
+  uint32_t top = 0;
 #pragma unroll
-    for (int k = 0; k < 4; k++) top += (nn[k] - 1) * st[k];
-    uint32_t pack = 0;
+  for (int k = 0; k < 4; k++) top += (nn[k] - 1) * st[k];
+  uint32_t pack = 0;
 #pragma unroll
-    for (int k = 0; k < 4; k++) {
-      uint32_t code = MRL_NEVER;
-      for (uint32_t sl = 0; sl < nn[k]; sl++) {
-        if (grid[top - (nn[k] - 1 - sl) * st[k]].tail != MRL_UNSAT) { code = nth_set_bit(mm[k], sl); break; }
-      }
-      pack |= code << (5 * k);
-    }
-    a.minsat[i] = pack;
+  for (int k = 0; k < 4; k++) {
+    uint32_t code = MRL_NEVER;
+    for (uint32_t sl = 0; sl < nn[k]; sl++)
+      if (grid[top - (nn[k] - 1 - sl) * st[k]].tail != MRL_UNSAT) { code = nth_set_bit(mm[k], sl); break; }
+    pack |= code << (8 * k);
   }
+  return pack;
 }
 
-// Step 0: the corner of every Spec of the stage, per memory the minimum over its candidates of
-// what each needs at least (its threshold; its children's corners, shifted by what a Move
-// takes). Two rounds: the first knows nothing about same-stage children (bound zero) and leaves
-// its result in minsat, the second reads those for same-stage children and writes the array the
-// grids are clipped with, so that no thread reads what another writes.
-__device__ __noinline__ void phase_corner(const StageArgs& a, uint32_t gtid, uint32_t gthreads, int round) {
-  for (uint32_t i = a.lo + gtid; i < a.hi; i += gthreads) {
-    if (!computed_here(a, i)) continue;
-    const uint2 cl = *reinterpret_cast<const uint2*>(&a.hdrs[i].cand_off);
-    uint32_t l0 = MRL_NEVER, l1 = MRL_NEVER, l2 = MRL_NEVER, l3 = MRL_NEVER;
-    for (uint32_t ci = 0; ci < cl.y; ci++) {
-      const uint4 c = __ldg(reinterpret_cast<const uint4*>(&a.cands[cl.x + ci]));
-      const uint32_t kind = (c.x >> 16) & 0xFFu, nchild = c.x >> 24;
-      const uint32_t level = c.z & 0xFFu, thr = (c.z >> 8) & 0xFFu, units = c.w;
-      uint32_t q0 = 0, q1 = 0, q2 = 0, q3 = 0;   // this candidate's corner
-      if (kind == MRL_CK_LEAF || kind == MRL_CK_MOVE) {
-        q0 = level == 0 ? thr : 0u; q1 = level == 1 ? thr : 0u; q2 = level == 2 ? thr : 0u; q3 = level == 3 ? thr : 0u;
+// Corners of the Specs of an earlier stage whose rows came from several ranks.
+__device__ __noinline__ void phase_minsat(const StageArgs& a, uint32_t lo, uint32_t hi, uint32_t gtid, uint32_t gthreads) {
+  for (uint32_t i = lo + gtid; i < hi; i += gthreads)
+    a.minsat[i] = corner_from_rows(*reinterpret_cast<const uint4*>(&a.hdrs[i]), a.rows + a.hdrs[i].row_base);
+}
+
+// What one record needs at least, per memory: its threshold; its children's corners, shifted by what
+// a Move takes. NEVER4: no limits inside the lattice satisfy it. Same-stage children: corner zero
+// (bounds = false), or what the round before worked out for them.
+__device__ __forceinline__ uint32_t record_corner(const StageArgs& a, uint32_t lo, const uint4 c, const uint4 b, bool bounds) {
+  const uint32_t kind = (c.x >> 16) & 0xFFu, nchild = c.x >> 24;
+  const uint32_t level = c.z & 0xFFu, thr = (c.z >> 8) & 0xFFu, units = c.w;
+  uint32_t q = (kind == MRL_CK_LEAF || kind == MRL_CK_MOVE) ? thr << (8 * level) : 0u;
+#pragma unroll
+  for (uint32_t j = 0; j < 3; j++) {
+    if (j >= nchild) break;
+    const uint32_t child = j == 0 ? b.x : (j == 1 ? b.y : b.z);
+    uint32_t e = (child < lo || bounds) ? a.minsat[child] : 0u;
+    if ((e & 0xFFu) == MRL_NEVER) return MRL_NEVER4;
+    if (kind == MRL_CK_MOVE) {
+      const uint32_t el = corner_of(e, level);
+      uint32_t sh = 0;
+      if (el) {
+        const uint32_t bit = shift_mask(1u << el, level, units, code_of(a.top_pack, level));
+        if (!bit) return MRL_NEVER4;
+        sh = __ffs(bit) - 1;
       }
-      bool never = false;
-      if (kind != MRL_CK_LEAF) {
-        const uint4 b = __ldg(reinterpret_cast<const uint4*>(&a.cands[cl.x + ci]) + 1);
-        for (uint32_t j = 0; j < nchild; j++) {
-          const uint32_t child = j == 0 ? b.x : (j == 1 ? b.y : b.z);
-          // a finished child's exact corner; a same-stage child's bound from the first round
-          const uint32_t cp = (child < a.lo || round) ? a.minsat[child] : 0u;
-          uint32_t e0 = corner_of(cp, 0), e1 = corner_of(cp, 1), e2 = corner_of(cp, 2), e3 = corner_of(cp, 3);
-          if (e0 == MRL_NEVER) { never = true; break; }
-          if (kind == MRL_CK_MOVE) {
-            const uint32_t e = sel4(e0, e1, e2, e3, level);
-            uint32_t sh = 0;
-            if (e) {
-              const uint32_t bit = shift_mask(1u << e, level, units, code_of(a.top_pack, level));
-              if (!bit) { never = true; break; }
-              sh = __ffs(bit) - 1;
-            }
-            e0 = level == 0 ? sh : e0; e1 = level == 1 ? sh : e1; e2 = level == 2 ? sh : e2; e3 = level == 3 ? sh : e3;
-          }
-          q0 = max(q0, e0); q1 = max(q1, e1); q2 = max(q2, e2); q3 = max(q3, e3);
-        }
-      }
-      if (!never) { l0 = min(l0, q0); l1 = min(l1, q1); l2 = min(l2, q2); l3 = min(l3, q3); }
+      e = (e & ~(0xFFu << (8 * level))) | (sh << (8 * level));
     }
-    const uint32_t t0 = code_of(a.top_pack, 0), t1 = code_of(a.top_pack, 1), t2 = code_of(a.top_pack, 2), t3 = code_of(a.top_pack, 3);
-    if (l0 > t0 || l1 > t1 || l2 > t2 || l3 > t3) l0 = l1 = l2 = l3 = MRL_NEVER;   // no limits inside the lattice reach it
-    const uint32_t corner = l0 | (l1 << 5) | (l2 << 10) | (l3 << 15);
-    if (round == 0) a.minsat[i] = corner;
-    a.corner[i - a.lo] = corner;
+    q = __vmaxu4(q, e);
   }
+  return q;
+}
+__device__ __forceinline__ uint32_t warp_min4(uint32_t v) {
+  for (int o = 16; o > 0; o >>= 1) v = __vminu4(v, __shfl_xor_sync(0xFFFFFFFFu, v, o));
+  return v;
 }
 
 // Clips a grid at the corner: below it everything is unsatisfiable, so one cell [0, corner) per
@@ -488,166 +398,260 @@ __device__ __forceinline__ uint4 clip_at_corner(uint4 nm, uint32_t corner) {
 // ORs into r the breakpoints one record puts into its Spec's grid: its own threshold, and its
 // children's breakpoints (for a Move, shifted in the memory it allocates in). Children of
 // finished stages contribute their final masks, same-stage children what rmask holds for them.
-__device__ __forceinline__ void record_breakpoints(const StageArgs& a, uint32_t rec, const uint4 c, uint32_t& r0, uint32_t& r1,
-                                                   uint32_t& r2, uint32_t& r3) {
+__device__ __forceinline__ void record_breakpoints(const StageArgs& a, uint32_t lo, const uint4 c, const uint4 b, uint4& r) {
   const uint32_t kind = (c.x >> 16) & 0xFFu, nchild = c.x >> 24;
   const uint32_t level = c.z & 0xFFu, thr = (c.z >> 8) & 0xFFu, units = c.w;
-  if (kind == MRL_CK_LEAF || kind == MRL_CK_MOVE) or_level(r0, r1, r2, r3, level, 1u << thr);
-  if (kind == MRL_CK_LEAF) return;
-  const uint4 b = __ldg(reinterpret_cast<const uint4*>(&a.cands[rec]) + 1);
-  for (uint32_t j = 0; j < nchild; j++) {
+  if (kind == MRL_CK_LEAF || kind == MRL_CK_MOVE) or_level(r.x, r.y, r.z, r.w, level, 1u << thr);
+#pragma unroll
+  for (uint32_t j = 0; j < 3; j++) {
+    if (j >= nchild) break;
     const uint32_t child = j == 0 ? b.x : (j == 1 ? b.y : b.z);
-    const uint4 cm = child < a.lo ? *reinterpret_cast<const uint4*>(&a.hdrs[child]) : a.rmask[child];
+    const uint4 cm = child < lo ? *reinterpret_cast<const uint4*>(&a.hdrs[child]) : a.rmask[child];
     if (kind == MRL_CK_MOVE) {
       const uint32_t s = shift_mask(sel4(cm.x, cm.y, cm.z, cm.w, level), level, units, code_of(a.top_pack, level));
-      r0 |= (level == 0) ? s : cm.x;
-      r1 |= (level == 1) ? s : cm.y;
-      r2 |= (level == 2) ? s : cm.z;
-      r3 |= (level == 3) ? s : cm.w;
+      r.x |= (level == 0) ? s : cm.x;
+      r.y |= (level == 1) ? s : cm.y;
+      r.z |= (level == 2) ? s : cm.z;
+      r.w |= (level == 3) ? s : cm.w;
     } else {
-      r0 |= cm.x; r1 |= cm.y; r2 |= cm.z; r3 |= cm.w;
+      r.x |= cm.x; r.y |= cm.y; r.z |= cm.z; r.w |= cm.w;
     }
   }
 }
-
-// Step 1: per Spec of the stage the grid of the unordered phase: the breakpoints of the records
-// whose children all lie in finished stages (they come first). Nothing of it depends on the
-// stage itself, so it is derived, and solved, once.
-__device__ __noinline__ void phase_derive_early(const StageArgs& a, uint32_t gtid, uint32_t gthreads) {
-  for (uint32_t i = a.lo + gtid; i < a.hi; i += gthreads) {
-    if (!computed_here(a, i)) continue;
-    const uint2 cl = *reinterpret_cast<const uint2*>(&a.hdrs[i].cand_off);
-    uint32_t r0 = 1, r1 = 1, r2 = 1, r3 = 1;
-    for (uint32_t ci = 0; ci < cl.y; ci++) {
-      const uint4 c = __ldg(reinterpret_cast<const uint4*>(&a.cands[cl.x + ci]));
-      if ((c.z >> 24) & 1u) break;   // records with a same-stage child come last
-      record_breakpoints(a, cl.x + ci, c, r0, r1, r2, r3);
-    }
-    *reinterpret_cast<uint4*>(&a.ehdr[i - a.lo]) = clip_at_corner(make_uint4(r0, r1, r2, r3), a.corner[i - a.lo]);
-  }
+__device__ __forceinline__ uint4 warp_or(uint4 r) {
+  r.x = __reduce_or_sync(0xFFFFFFFFu, r.x);
+  r.y = __reduce_or_sync(0xFFFFFFFFu, r.y);
+  r.z = __reduce_or_sync(0xFFFFFFFFu, r.z);
+  r.w = __reduce_or_sync(0xFFFFFFFFu, r.w);
+  return r;
 }
-
-// Pass step 1: per Spec of the stage the grid the records with a same-stage child are solved on:
-// the real breakpoints of what the unordered phase found (first pass: they are in rmask), the
-// breakpoints of those records, and for their same-stage children the breakpoints in rmask -
-// first pass: of what the unordered phase found for the child; later passes: found real by the
-// pass before. Grids only grow; a Spec whose masks grew is marked for solving.
-__device__ __noinline__ void phase_derive_late(const StageArgs& a, uint32_t gtid, uint32_t gthreads, int first) {
-  for (uint32_t i = a.lo + gtid; i < a.hi; i += gthreads) {
-    if (!computed_here(a, i)) continue;
-    const uint4 old = first ? a.rmask[i] : *reinterpret_cast<const uint4*>(&a.hdrs[i]);
-    const uint2 cl = *reinterpret_cast<const uint2*>(&a.hdrs[i].cand_off);
-    uint32_t r0 = old.x, r1 = old.y, r2 = old.z, r3 = old.w;
-    for (uint32_t back = 0; back < cl.y; back++) {
-      const uint32_t ci = cl.y - 1 - back;
-      const uint4 c = __ldg(reinterpret_cast<const uint4*>(&a.cands[cl.x + ci]));
-      if (!((c.z >> 24) & 1u)) break;
-      record_breakpoints(a, cl.x + ci, c, r0, r1, r2, r3);
-    }
-    const uint4 nm = clip_at_corner(make_uint4(r0, r1, r2, r3), a.corner[i - a.lo]);
-    if (first || nm.x != old.x || nm.y != old.y || nm.z != old.z || nm.w != old.w) {
-      *reinterpret_cast<uint4*>(&a.hdrs[i]) = nm;
-      a.dirty[i] = 1;
-    }
-  }
-}
-
-// A Spec with a marked same-stage child has to be solved again too (its lookups may change).
-// Monotone, so racing with other threads' marks is harmless; repeated until a round marks nothing.
-__device__ __noinline__ void phase_spread(const StageArgs& a, uint32_t gtid, uint32_t gthreads, uint32_t epoch) {
-  for (uint32_t i = a.lo + gtid; i < a.hi; i += gthreads) {
-    if (!computed_here(a, i) || a.dirty[i]) continue;
-    const uint2 cl = *reinterpret_cast<const uint2*>(&a.hdrs[i].cand_off);
-    bool hit = false;
-    for (uint32_t ci = 0; ci < cl.y && !hit; ci++) {
-      const uint4 c = __ldg(reinterpret_cast<const uint4*>(&a.cands[cl.x + ci]));
-      const uint32_t kind = (c.x >> 16) & 0xFFu, nchild = c.x >> 24;
-      if (kind != MRL_CK_MOVE) continue;   // only Moves have same-stage children
-      const uint4 b = __ldg(reinterpret_cast<const uint4*>(&a.cands[cl.x + ci]) + 1);
-      for (uint32_t j = 0; j < nchild; j++) {
-        const uint32_t child = j == 0 ? b.x : (j == 1 ? b.y : b.z);
-        if (child >= a.lo && a.dirty[child]) hit = true;
-      }
-    }
-    if (hit) {
-      a.dirty[i] = 1;
-      a.ctl->spread_epoch = epoch;   // every writer of a round stores the same value
-    }
-  }
-}
-
-// Totals of what the coming solve takes: the grids of the unordered phase of all the stage's
-// Specs (early), or the grids of the marked Specs (else).
-__device__ __noinline__ void phase_totals(const StageArgs& a, uint32_t gtid, uint32_t gthreads, bool early) {
-  unsigned long long cells = 0, warps = 0;
-  for (uint32_t i = a.lo + gtid; i < a.hi; i += gthreads) {
-    if (!computed_here(a, i) || !(early || a.dirty[i])) continue;
-    const Grid g = grid_of(*reinterpret_cast<const uint4*>(early ? &a.ehdr[i - a.lo] : &a.hdrs[i]));
-    cells += g.cells;
-    warps += g.warps;
-  }
-  for (int o = 16; o > 0; o >>= 1) {
-    cells += __shfl_xor_sync(0xFFFFFFFFu, cells, o);
-    warps += __shfl_xor_sync(0xFFFFFFFFu, warps, o);
-  }
-  if ((threadIdx.x & 31) == 0 && cells) {
-    atomicAdd(&a.ctl->cells, cells);
-    atomicAdd(&a.ctl->warps, warps);
-  }
-}
-
-// Gives every Spec of the stage the rows of its grid of the unordered phase (early: in the base
-// rows, from row 0), or every marked Spec fresh working rows (from temp_top up; Specs that are not
-// solved again keep theirs), with its work items and chunks, and resets its real-breakpoint
-// masks. Capacities were checked against the totals before.
-__device__ __noinline__ void phase_place(const StageArgs& a, unsigned long long temp_top, uint32_t item_cells, bool early) {
-  __shared__ unsigned long long row0, chunk0, item0;
-  for (uint32_t base = a.lo + blockIdx.x * kBlock; base < a.hi; base += gridDim.x * kBlock) {
-    const uint32_t i = base + threadIdx.x;
-    const bool active = i < a.hi && computed_here(a, i) && (early || a.dirty[i] == 1);
-    Grid g;
-    g.cells = 0; g.warps = 0; g.F = 0;
-    if (active) g = grid_of(*reinterpret_cast<const uint4*>(early ? &a.ehdr[i - a.lo] : &a.hdrs[i]));
-    const uint32_t n_items = (uint32_t)((g.cells + item_cells - 1) / item_cells);
-    unsigned long long tot_cells, tot_warps, tot_items;
-    const unsigned long long my_row = block_excl_scan(g.cells, &tot_cells);
-    const unsigned long long my_chunk = block_excl_scan(active ? g.warps : 0ull, &tot_warps);
-    const unsigned long long my_item = block_excl_scan(n_items, &tot_items);
-    if (threadIdx.x == 0) {
-      row0 = atomicAdd(&a.ctl->row_cursor, tot_cells);
-      chunk0 = atomicAdd(&a.ctl->chunk_cursor, (uint32_t)tot_warps);
-      item0 = atomicAdd(&a.ctl->item_cursor, (uint32_t)tot_items);
-    }
-    __syncthreads();
-    if (active) {
-      const unsigned long long cb = chunk0 + my_chunk;
-      for (uint32_t w = 0; w < n_items; w++) {
-        WorkItem it;
-        it.spec = i;
-        it.first_cell = w * item_cells;
-        a.items[item0 + my_item + w] = it;
-      }
-      if (early) {
-        a.ehdr[i - a.lo].row_base = row0 + my_row;
-      } else {
-        a.hdrs[i].row_base = (temp_top + row0 + my_row) | MRL_TEMP_FLAG;
-        a.dirty[i] = 2;   // solved by this pass
-      }
-      a.rmask[i] = make_uint4(1u, 1u, 1u, 1u);
-      for (uint32_t w = 0; w < g.warps; w++) {
-        Chunk c;
-        c.spec = i;
-        c.col_start = (w * 32u) | (g.F << 30);
-        a.chunks[cb + w] = c;
-      }
-    }
-    __syncthreads();   // row0 / chunk0 / item0 are rewritten by the next round
-  }
+__device__ __forceinline__ unsigned long long cells_of(const uint4 m) {
+  return (unsigned long long)__popc(m.x) * __popc(m.y) * __popc(m.z) * __popc(m.w);
 }
 
 // A candidate record whose body is a Spec of the same stage (a relayout Move): the planner flags
 // it and stores these records after all others, dearest first.
 __device__ __forceinline__ bool is_late(const uint4 a) { return (a.z >> 24) & 1u; }
+
+// The Specs a warp of a per-Spec phase takes at a time: as many as keep all warps busy, at most one
+// per lane.
+__device__ __forceinline__ uint32_t group_size(uint32_t n, uint32_t gwarps) { return max(1u, min(32u, (n + gwarps - 1) / gwarps)); }
+// Cells per work item: a work item's records are staged once, so long items where there are enough
+// of them; one step of the warp where Specs are few. Grids have 100 to 600 cells on average.
+__device__ __forceinline__ uint32_t item_size(uint32_t n, uint32_t gwarps) {
+  const unsigned long long want = (unsigned long long)n * 128u / gwarps;
+  return want >= MRL_ITEM_CELLS ? MRL_ITEM_CELLS : max(32u, (uint32_t)want & ~31u);
+}
+
+// Phase 1: one pass over the records of every Spec of the stage, a record per lane: the breakpoints of
+// the records whose children all lie in finished stages (they come first), and the corner with
+// nothing known about same-stage children.
+__device__ __noinline__ void phase_records(const StageArgs& a, uint32_t lo, uint32_t hi, uint32_t gwarp, uint32_t gwarps, uint32_t stage) {
+  const uint32_t lane = threadIdx.x & 31;
+  for (uint32_t i = lo + gwarp; i < hi; i += gwarps) {
+    if (!computed_here(a, i)) {
+      if (lane == 0) a.rmask[i] = make_uint4(0, 0, 0, 0);   // another rank's Spec: zero until the exchange
+      continue;
+    }
+    const uint2 cl = *reinterpret_cast<const uint2*>(&a.hdrs[i].cand_off);
+    uint4 r = make_uint4(1u, 1u, 1u, 1u);
+    uint32_t early = MRL_NEVER4, late = MRL_NEVER4, n_late = 0;
+    for (uint32_t c0 = 0; c0 < cl.y; c0 += 32) {
+      bool l = false;
+      if (c0 + lane < cl.y) {
+        const uint4* const rec = reinterpret_cast<const uint4*>(&a.cands[cl.x + c0 + lane]);
+        const uint4 c = __ldg(rec), b = __ldg(rec + 1);
+        l = is_late(c);
+        const uint32_t q = record_corner(a, lo, c, b, false);
+        if (l) late = __vminu4(late, q);
+        else {
+          early = __vminu4(early, q);
+          record_breakpoints(a, lo, c, b, r);
+        }
+      }
+      n_late += __popc(__ballot_sync(0xFFFFFFFFu, l));
+    }
+    r = warp_or(r);
+    early = warp_min4(early);
+    if (n_late) late = warp_min4(late);
+    if (lane == 0) {
+      StageSpec& s = a.sspec[i - lo];
+      s.emask = r;
+      s.corner = early;
+      s.n_late = n_late;
+      uint32_t bound = __vminu4(early, late);
+      if (__vcmpgtu4(bound, a.top_pack)) bound = MRL_NEVER4;   // no limits inside the lattice reach it
+      a.minsat[i] = bound;
+      if (n_late) a.ctl->any_late = stage + 1;   // every writer of a stage stores the same value
+    }
+  }
+}
+
+// Rows and work items for the grids of up to 32 Specs, one per lane (`cells` 0: none), by one warp:
+// the lane's first row, and items at the end of the list. What does not fit is counted and left out;
+// the totals are checked behind the next barrier.
+__device__ __forceinline__ unsigned long long place_grids(const StageArgs& a, unsigned long long* row_cursor, uint32_t spec, unsigned long long cells,
+                                                          unsigned long long item_cells_of, uint32_t item_cells, uint32_t flag, uint32_t lane) {
+  unsigned long long inc = cells;
+  uint32_t items = (uint32_t)((item_cells_of + item_cells - 1) / item_cells), iinc = items;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const unsigned long long t = __shfl_up_sync(0xFFFFFFFFu, inc, o);
+    const uint32_t u = __shfl_up_sync(0xFFFFFFFFu, iinc, o);
+    if (lane >= (uint32_t)o) { inc += t; iinc += u; }
+  }
+  unsigned long long row0 = 0;
+  uint32_t item0 = 0;
+  if (lane == 31) {
+    if (inc) row0 = atomicAdd(row_cursor, inc);
+    if (iinc) item0 = atomicAdd(&a.ctl->n_items, iinc);
+  }
+  row0 = __shfl_sync(0xFFFFFFFFu, row0, 31);
+  item0 = __shfl_sync(0xFFFFFFFFu, item0, 31);
+  uint32_t todo = __ballot_sync(0xFFFFFFFFu, items != 0);
+  while (todo) {
+    const uint32_t src = __ffs(todo) - 1;
+    todo &= todo - 1;
+    const uint32_t n = __shfl_sync(0xFFFFFFFFu, items, src), at = item0 + __shfl_sync(0xFFFFFFFFu, iinc, src) - n;
+    const uint32_t sp = __shfl_sync(0xFFFFFFFFu, spec, src), fl = __shfl_sync(0xFFFFFFFFu, flag, src);
+    for (uint32_t w = lane; w < n; w += 32)
+      if (at + w < a.item_cap) {
+        WorkItem it;
+        it.spec = sp;
+        it.first_cell = (w * item_cells) | fl;
+        a.items[at + w] = it;
+      }
+  }
+  return row0 + inc - cells;
+}
+
+// Phase 2: the final corner (records with a same-stage child again, with that child's bound), the grid
+// of the unordered phase, its rows and work items.
+__device__ __noinline__ void phase_place_early(const StageArgs& a, uint32_t lo, uint32_t hi, uint32_t gwarp, uint32_t gwarps, bool any_late) {
+  const uint32_t lane = threadIdx.x & 31;
+  const uint32_t G = group_size(hi - lo, gwarps), item_cells = item_size(hi - lo, gwarps);
+  for (uint32_t base = lo + gwarp * G; base < hi; base += gwarps * G) {
+    const uint32_t i = base + lane;
+    const bool mine = lane < G && i < hi && computed_here(a, i);
+    uint32_t corner = MRL_NEVER4, n_late = 0;
+    uint4 m = make_uint4(1u, 1u, 1u, 1u);
+    if (mine) {
+      const StageSpec& s = a.sspec[i - lo];
+      m = s.emask;
+      corner = s.corner;
+      n_late = s.n_late;
+    }
+    uint32_t todo = any_late ? __ballot_sync(0xFFFFFFFFu, n_late != 0) : 0u;
+    while (todo) {
+      const uint32_t src = __ffs(todo) - 1;
+      todo &= todo - 1;
+      const uint32_t n = __shfl_sync(0xFFFFFFFFu, n_late, src);
+      const uint2 cl = *reinterpret_cast<const uint2*>(&a.hdrs[base + src].cand_off);
+      uint32_t q = MRL_NEVER4;
+      for (uint32_t c = lane; c < n; c += 32) {
+        const uint4* const rec = reinterpret_cast<const uint4*>(&a.cands[cl.x + cl.y - 1 - c]);
+        q = __vminu4(q, record_corner(a, lo, __ldg(rec), __ldg(rec + 1), true));
+      }
+      q = warp_min4(q);
+      if (lane == src) corner = __vminu4(corner, q);
+    }
+    unsigned long long cells = 0;
+    if (mine) {
+      if (__vcmpgtu4(corner, a.top_pack)) corner = MRL_NEVER4;
+      m = clip_at_corner(m, corner);
+      cells = cells_of(m);
+    }
+    const unsigned long long row = place_grids(a, &a.ctl->rows_early, i, cells, cells, item_cells, 0, lane);
+    if (mine) {
+      StageSpec& s = a.sspec[i - lo];
+      s.emask = m;
+      s.corner = corner;
+      s.erow = row;
+      a.rmask[i] = make_uint4(1u, 1u, 1u, 1u);
+    }
+  }
+}
+
+// Phase 5 (and once more per further pass): the grid the records with a same-stage child are solved
+// on: the real breakpoints of what the unordered phase found (first pass: they are in rmask), the
+// breakpoints of those records, and for their same-stage children the breakpoints in rmask - first
+// pass: of what the unordered phase found for the child; later passes: found real by the pass
+// before. Grids only grow; one that grew gets new rows, and its old ones are remembered.
+// A Spec without such records is finished: its grid is that of the unordered phase.
+__device__ __noinline__ void phase_place_late(const StageArgs& a, uint32_t lo, uint32_t hi, uint32_t gwarp, uint32_t gwarps, uint32_t pass) {
+  const uint32_t lane = threadIdx.x & 31;
+  const uint32_t G = group_size(hi - lo, gwarps), item_cells = item_size(hi - lo, gwarps);
+  for (uint32_t base = lo + gwarp * G; base < hi; base += gwarps * G) {
+    const uint32_t i = base + lane;
+    const bool mine = lane < G && i < hi && computed_here(a, i);
+    uint32_t n_late = 0, corner = 0;
+    uint4 old = make_uint4(0, 0, 0, 0);
+    if (mine) {
+      const StageSpec& s = a.sspec[i - lo];
+      n_late = s.n_late;
+      corner = s.corner;
+      old = pass ? *reinterpret_cast<const uint4*>(&a.hdrs[i]) : a.rmask[i];
+      if (!pass) a.changed[0][i - lo] = a.changed[1][i - lo] = a.changed[2][i - lo] = make_uint4(0, 0, 0, 0);
+      if (!pass && !n_late) {
+        *reinterpret_cast<uint4*>(&a.hdrs[i]) = s.emask;
+        a.hdrs[i].row_base = (a.temp_cap + s.erow) | MRL_TEMP_FLAG;
+      }
+    }
+    uint4 nm = old;
+    uint32_t todo = __ballot_sync(0xFFFFFFFFu, n_late != 0);
+    while (todo) {
+      const uint32_t src = __ffs(todo) - 1;
+      todo &= todo - 1;
+      const uint32_t n = __shfl_sync(0xFFFFFFFFu, n_late, src);
+      const uint2 cl = *reinterpret_cast<const uint2*>(&a.hdrs[base + src].cand_off);
+      uint4 r = make_uint4(0, 0, 0, 0);
+      for (uint32_t c = lane; c < n; c += 32) {
+        const uint4* const rec = reinterpret_cast<const uint4*>(&a.cands[cl.x + cl.y - 1 - c]);
+        record_breakpoints(a, lo, __ldg(rec), __ldg(rec + 1), r);
+      }
+      r = warp_or(r);
+      if (lane == src) { nm.x |= r.x; nm.y |= r.y; nm.z |= r.z; nm.w |= r.w; }
+    }
+    bool fresh = false;
+    unsigned long long cells = 0;
+    if (n_late) {
+      nm = clip_at_corner(nm, corner);
+      fresh = !pass || nm.x != old.x || nm.y != old.y || nm.z != old.z || nm.w != old.w;
+      cells = cells_of(nm);
+    }
+    const unsigned long long row = place_grids(a, &a.ctl->rows_late, i, fresh ? cells : 0ull, cells, item_cells, fresh ? 1u : 0u, lane);
+    if (fresh) {
+      StageSpec& s = a.sspec[i - lo];
+      s.old_mask = old;
+      s.old_row = pass ? a.hdrs[i].row_base : 0ull;
+      *reinterpret_cast<uint4*>(&a.hdrs[i]) = nm;
+      a.hdrs[i].row_base = row | MRL_TEMP_FLAG;
+    }
+    if (pass && n_late) a.sspec[i - lo].dirty = fresh ? 1u : 0u;
+  }
+}
+
+// After a pass: does any grid lack a (shifted) real breakpoint of a same-stage child?
+__device__ __noinline__ void phase_check_grids(const StageArgs& a, uint32_t lo, uint32_t hi, uint32_t gwarp, uint32_t gwarps, uint32_t pass) {
+  const uint32_t lane = threadIdx.x & 31;
+  for (uint32_t i = lo + gwarp; i < hi; i += gwarps) {
+    if (!computed_here(a, i)) continue;
+    const uint32_t n = a.sspec[i - lo].n_late;
+    if (!n) continue;
+    const uint2 cl = *reinterpret_cast<const uint2*>(&a.hdrs[i].cand_off);
+    uint4 r = make_uint4(0, 0, 0, 0);
+    for (uint32_t c = lane; c < n; c += 32) {
+      const uint4* const rec = reinterpret_cast<const uint4*>(&a.cands[cl.x + cl.y - 1 - c]);
+      record_breakpoints(a, lo, __ldg(rec), __ldg(rec + 1), r);
+    }
+    const uint4 m = *reinterpret_cast<const uint4*>(&a.hdrs[i]);
+    const uint32_t corner = a.sspec[i - lo].corner;
+    // what the grid lacks above its corner (below it nothing is kept)
+    const uint32_t k0 = corner_of(corner, 0), k1 = corner_of(corner, 1), k2 = corner_of(corner, 2), k3 = corner_of(corner, 3);
+    const bool lacks = k0 != MRL_NEVER && (((r.x & ~m.x) >> k0) | ((r.y & ~m.y) >> k1) | ((r.z & ~m.z) >> k2) | ((r.w & ~m.w) >> k3));
+    if (lacks) a.ctl->grew = pass + 1;   // every writer of a pass stores the same value
+  }
+}
 
 // Step 2: the candidates whose children all lie in earlier stages, for every cell of every
 // Spec's grid of the unordered phase. No order is needed. A warp takes a work item (up to MRL_ITEM_CELLS cells of one
@@ -656,25 +660,17 @@ __device__ __forceinline__ bool is_late(const uint4 a) { return (a.z >> 24) & 1u
 // child header -> child row costs two round trips per batch of records instead of two per record;
 // then its lanes take 32 cells at a time and walk the staged records together, and the only
 // global loads left in that loop are the child rows.
-struct HotArgs {   // what the two solve phases read, by value: registers instead of the argument block in local memory
+struct HotArgs {   // what the solve phases read, by value: registers instead of the argument block
   const SpecHdr* hdrs;
   const CandRec* cands;
-  const MrlRow* rows;
+  MrlRow* rows;
   MrlRow* temp;
-  MrlRow* base;             // the grids of the unordered phase
-  const SpecHdr* ehdr;      // their masks and first rows; already offset: indexed by Spec id
-  const uint32_t* corner;   // already offset: indexed by Spec id
+  unsigned long long temp_cap;   // the grids of the unordered phase start here
+  StageSpec* sspec;              // already offset: indexed by Spec id
+  const WorkItem* items;
+  uint32_t n_items, item_cells;
+  uint32_t* next_item;
 };
-__device__ __forceinline__ HotArgs hot_args(const StageArgs& s) {
-  HotArgs h;
-  h.hdrs = s.hdrs; h.cands = s.cands; h.rows = s.rows; h.temp = s.temp; h.base = s.base; h.ehdr = s.ehdr - s.lo; h.corner = s.corner - s.lo;
-  return h;
-}
-// A cell with a limit below its Spec's corner has no implementation; no record needs to be read.
-__device__ __forceinline__ bool below_corner(uint32_t corner, uint32_t cpack) {
-  return code_of(cpack, 0) < corner_of(corner, 0) || code_of(cpack, 1) < corner_of(corner, 1) ||
-         code_of(cpack, 2) < corner_of(corner, 2) || code_of(cpack, 3) < corner_of(corner, 3);
-}
 
 constexpr int kBatch = 16;   // records staged at a time
 struct StagedRec {           // a record with what the row lookups of its children need
@@ -687,11 +683,10 @@ struct StagedRec {           // a record with what the row lookups of its childr
 static_assert(sizeof(StagedRec) == 128, "staged record");
 
 // What the lookups of one child need, into its slot of a staged record.
-__device__ __forceinline__ void stage_child(StagedRec& s, uint32_t j, const uint4 m, unsigned long long base, const MrlRow* rows,
-                                            const MrlRow* temp) {
+__device__ __forceinline__ void stage_child(StagedRec& s, uint32_t j, const uint4 m, const MrlRow* grid, bool in_temp) {
   s.mask[j] = m;
-  s.grid[j] = row_at(rows, temp, base);
-  s.in_temp[j] = (base & MRL_TEMP_FLAG) ? 1 : 0;
+  s.grid[j] = grid;
+  s.in_temp[j] = in_temp ? 1 : 0;
   const uint32_t n0 = __popc(m.x), n1 = __popc(m.y), n2 = __popc(m.z);
   s.stride[j][0] = n0;
   s.stride[j][1] = n0 * n1;
@@ -708,6 +703,16 @@ __device__ __forceinline__ const MrlRow* staged_row(const StagedRec& s, uint32_t
 // The lattice code of every slot of a grid, memory after memory, for the lanes of a warp to look
 // up instead of counting bits (a grid has at most 17 + 17 + 12 + 27 slots).
 constexpr int kMaxSlots = 80;
+constexpr int kMaxAffected = 16;
+struct WarpScratch {         // a warp's shared memory in the solve phases
+  StagedRec staged[kBatch];
+  uint4 affected[kMaxAffected];      // sweeps: per changed child the parent's codes that read a changed slot of it
+  uint32_t who[kMaxAffected];        // record (from the end) | child << 16
+  uint32_t queue[64];                // sweeps: cells to solve again, as packed slots
+  uint8_t codes[kMaxSlots];
+};
+static_assert(sizeof(WarpScratch) % 16 == 0, "warp scratch is made of 16-byte units");
+
 __device__ __forceinline__ void stage_slot_codes(uint8_t* codes, const uint4 m, uint32_t n0, uint32_t n1, uint32_t n2, uint32_t n3,
                                                  uint32_t lane) {
   __syncwarp();   // the previous item's codes have been read by every lane
@@ -719,10 +724,27 @@ __device__ __forceinline__ void stage_slot_codes(uint8_t* codes, const uint4 m, 
   __syncwarp();
 }
 
+// Whole-row accesses to working rows that other warps may be writing at the same time: one
+// 128-bit access each, so a reader sees a row either before or after an update, never a mix.
+__device__ __forceinline__ uint4 ld_row_shared(const MrlRow* p) {
+  unsigned long long lo, hi;
+  asm volatile("{\n\t.reg .b128 q;\n\tld.relaxed.gpu.global.b128 q, [%2];\n\tmov.b128 {%0, %1}, q;\n\t}"
+               : "=l"(lo), "=l"(hi) : "l"(p) : "memory");
+  return make_uint4((uint32_t)lo, (uint32_t)(lo >> 32), (uint32_t)hi, (uint32_t)(hi >> 32));
+}
+__device__ __forceinline__ void st_row_shared(MrlRow* p, const uint4 v) {
+  const unsigned long long lo = v.x | ((unsigned long long)v.y << 32), hi = v.z | ((unsigned long long)v.w << 32);
+  asm volatile("{\n\t.reg .b128 q;\n\tmov.b128 q, {%1, %2};\n\tst.relaxed.gpu.global.b128 [%0], q;\n\t}"
+               :: "l"(p), "l"(lo), "l"(hi) : "memory");
+}
+__device__ __forceinline__ uint4 ld_row(const MrlRow* p) { return *reinterpret_cast<const uint4*>(p); }
+
 // A staged record at one limits point; eval_candidate with the record and the child headers
-// already at hand. All children are finished, so the rows come from the table on the read-only path.
-__device__ __forceinline__ void eval_staged(const StagedRec& s, const MrlRow* __restrict__ rows, uint32_t ci,
-                                            uint32_t cpack, uint32_t bm0, uint32_t bm1, uint32_t bm2, uint32_t bm3,
+// already at hand. kMoving: a child's rows may change while this runs. Rows are read with plain
+// loads even where they are final: a launch may hold several stages, so they may have been written
+// earlier in it, and the read-only path does not see that.
+template <bool kMoving>
+__device__ __forceinline__ void eval_staged(const StagedRec& s, uint32_t cpack, uint32_t bm0, uint32_t bm1, uint32_t bm2, uint32_t bm3,
                                             Best& best, Tally& tally) {
   const uint4 a = s.rec;
   const uint32_t action = a.x & 0xFFFFu, kind = (a.x >> 16) & 0xFFu, nchild = a.x >> 24;   // the same in all lanes
@@ -749,29 +771,35 @@ __device__ __forceinline__ void eval_staged(const StagedRec& s, const MrlRow* __
       c2 = (level == 2) ? cb : c2;
       c3 = (level == 3) ? cb : c3;
     }
-    const uint4 r0 = __ldg(reinterpret_cast<const uint4*>(staged_row(s, 0, c0, c1, c2, c3)));
-    uint4 r1 = r0, r2 = r0;
-    if (nchild > 1) r1 = __ldg(reinterpret_cast<const uint4*>(staged_row(s, 1, c0, c1, c2, c3)));
-    if (nchild > 2) r2 = __ldg(reinterpret_cast<const uint4*>(staged_row(s, 2, c0, c1, c2, c3)));
+    uint4 r[3];
+#pragma unroll
+    for (int j = 0; j < 3; j++) {
+      if ((uint32_t)j < nchild) {
+        const MrlRow* const p = staged_row(s, j, c0, c1, c2, c3);
+        r[j] = (kMoving && s.in_temp[j]) ? ld_row_shared(p) : ld_row(p);
+      } else {
+        r[j] = r[0];
+      }
+    }
     tally.lookups += nchild;
-    if (r0.z == MRL_UNSAT || r1.z == MRL_UNSAT || r2.z == MRL_UNSAT) return;
+    if (r[0].z == MRL_UNSAT || r[1].z == MRL_UNSAT || r[2].z == MRL_UNSAT) return;
     uint32_t depth;
     if (kind == MRL_CK_LOOP) {
-      k_main = sat_mul(r0.x, imm);
-      k_peaks = r0.y;
+      k_main = sat_mul(r[0].x, imm);
+      k_peaks = r[0].y;
       depth = 1u;
     } else {
-      k_main = (kind == MRL_CK_MOVE) ? sat_add(imm, r0.x) : r0.x;
-      if (nchild > 1) k_main = sat_add(k_main, r1.x);
-      if (nchild > 2) k_main = sat_add(k_main, r2.x);
+      k_main = (kind == MRL_CK_MOVE) ? sat_add(imm, r[0].x) : r[0].x;
+      if (nchild > 1) k_main = sat_add(k_main, r[1].x);
+      if (nchild > 2) k_main = sat_add(k_main, r[2].x);
       if (k_main > best.main) return;
-      k_peaks = __vmaxu4(__vmaxu4(r0.y, r1.y), r2.y);
+      k_peaks = __vmaxu4(__vmaxu4(r[0].y, r[1].y), r[2].y);
       if (kind == MRL_CK_MOVE) {
         const uint32_t cc = (k_peaks >> sh) & 0xFFu;
         const uint32_t ncode = level < 2 ? units + cc : cache_code_ceil(units + cache_value(cc));
         k_peaks = (k_peaks & ~(0xFFu << sh)) | (ncode << sh);
       }
-      depth = min(max(max(r0.z >> 16, r1.z >> 16), r2.z >> 16) + 1u, 255u);
+      depth = min(max(max(r[0].z >> 16, r[1].z >> 16), r[2].z >> 16) + 1u, 255u);
     }
     k_tail = (depth << 16) | action;
   }
@@ -779,52 +807,63 @@ __device__ __forceinline__ void eval_staged(const StagedRec& s, const MrlRow* __
     best.main = k_main;
     best.peaks = k_peaks;
     best.tail = k_tail;
-    best.ci = ci;
   }
 }
 
-__device__ __noinline__ void phase_early(const HotArgs a, const WorkItem* items, uint32_t n_items, uint32_t item_cells,
-                                         uint32_t* next_item, unsigned long long* block_stats) {
+__device__ __forceinline__ WarpScratch& warp_scratch() {
+  extern __shared__ uint4 dyn_smem[];
+  return reinterpret_cast<WarpScratch*>(dyn_smem)[threadIdx.x >> 5];
+}
+__device__ __forceinline__ uint32_t warp_number() { return blockIdx.x * (kStageBlock / 32) + (threadIdx.x >> 5); }
+__device__ __forceinline__ uint32_t warp_count() { return gridDim.x * (kStageBlock / 32); }
+// Every warp starts with the item of its own number; further items are handed out by a counter (no
+// atomics at all when there are fewer items than warps).
+__device__ __forceinline__ bool next_item(const HotArgs& a, uint32_t& w, uint32_t lane) {
+  const uint32_t gwarps = warp_count();
+  if (a.n_items <= gwarps) return false;
+  if (lane == 0) w = gwarps + atomicAdd(a.next_item, 1u);
+  w = __shfl_sync(0xFFFFFFFFu, w, 0);
+  return w < a.n_items;
+}
+__device__ __forceinline__ void add_tally(const Tally& tally, unsigned long long* cands, unsigned long long* lookups, uint32_t lane) {
+  const uint32_t tc = __reduce_add_sync(0xFFFFFFFFu, tally.cands), tl = __reduce_add_sync(0xFFFFFFFFu, tally.lookups);
+  if (lane == 0 && (tc | tl)) {
+    atomicAdd(cands, (unsigned long long)tc);
+    atomicAdd(lookups, (unsigned long long)tl);
+  }
+}
+
+__device__ __noinline__ void phase_early(const HotArgs a, unsigned long long* block_stats) {
   const uint32_t lane = threadIdx.x & 31;
-  const uint32_t gwarps = gridDim.x * (kBlock / 32);
-  __shared__ StagedRec staged_all[kBlock / 32][kBatch];
-  __shared__ uint8_t codes_all[kBlock / 32][kMaxSlots];
-  StagedRec* const staged = staged_all[threadIdx.x >> 5];   // this warp's
-  uint8_t* const codes = codes_all[threadIdx.x >> 5];
+  WarpScratch& ws = warp_scratch();
+  StagedRec* const staged = ws.staged;
+  const uint8_t* const codes = ws.codes;
   Tally tally = {0, 0};
-  // every warp starts with the item of its own number; further items are handed out by a counter
-  // (no atomics at all when there are fewer items than warps)
-  for (uint32_t w = blockIdx.x * (kBlock / 32) + (threadIdx.x >> 5); w < n_items;) {
-    const WorkItem it = items[w];
+  uint32_t w = warp_number();
+  if (w < a.n_items) do {
+    const WorkItem it = a.items[w];
     const uint32_t i = it.spec;
-    const uint4 m = *reinterpret_cast<const uint4*>(&a.ehdr[i]);
+    const uint4 m = a.sspec[i].emask;
+    const uint32_t corner = a.sspec[i].corner;
     const uint2 cl = *reinterpret_cast<const uint2*>(&a.hdrs[i].cand_off);
-    MrlRow* const grid = a.base + a.ehdr[i].row_base;
+    MrlRow* const grid = a.temp + a.temp_cap + a.sspec[i].erow;
+    const uint32_t n_early = cl.y - a.sspec[i].n_late;   // records with a same-stage child come last
     const uint32_t n0 = __popc(m.x), n1 = __popc(m.y), n2 = __popc(m.z), n3 = __popc(m.w);
     const uint32_t cells = n0 * n1 * n2 * n3;
-    const uint32_t c_end = min(cells, it.first_cell + item_cells);
-    const uint32_t corner = a.corner[i];
-    stage_slot_codes(codes, m, n0, n1, n2, n3, lane);
+    const uint32_t c_end = min(cells, it.first_cell + a.item_cells);
+    stage_slot_codes(ws.codes, m, n0, n1, n2, n3, lane);
     uint32_t b0 = 0;
     do {
-      // stage the next records (those with a same-stage child come last and end the walk) ...
-      const uint32_t nb = min((uint32_t)kBatch, cl.y - b0);
+      // stage the next records, and the headers of their children, one (record, child) per lane
+      const uint32_t n_here = min((uint32_t)kBatch, n_early - b0);
       __syncwarp();   // the previous batch has been read by every lane
-      bool late = false;
-      if (lane < nb) {
-        const uint4 c = __ldg(reinterpret_cast<const uint4*>(&a.cands[cl.x + b0 + lane]));
-        staged[lane].rec = c;
-        late = is_late(c);
-      }
-      const uint32_t late_lanes = __ballot_sync(0xFFFFFFFFu, late);
-      const uint32_t n_here = late_lanes ? (uint32_t)__ffs(late_lanes) - 1u : nb;
+      if (lane < n_here) staged[lane].rec = __ldg(reinterpret_cast<const uint4*>(&a.cands[cl.x + b0 + lane]));
       __syncwarp();
-      // ... and the headers of their children, one (record, child) per lane
       for (uint32_t t = lane; t < n_here * 3u; t += 32) {
         const uint32_t r = t / 3u, j = t - r * 3u;
         if (j < (staged[r].rec.x >> 24)) {
           const uint32_t child = __ldg(&a.cands[cl.x + b0 + r].child[j]);
-          stage_child(staged[r], j, __ldg(reinterpret_cast<const uint4*>(&a.hdrs[child])), __ldg(&a.hdrs[child].row_base), a.rows, a.rows);
+          stage_child(staged[r], j, *reinterpret_cast<const uint4*>(&a.hdrs[child]), a.rows + a.hdrs[child].row_base, false);
         }
       }
       __syncwarp();
@@ -838,131 +877,53 @@ __device__ __noinline__ void phase_early(const HotArgs a, const WorkItem* items,
         const uint32_t k3 = codes[n0 + n1 + n2 + rest];
         const uint32_t cpack = k0 | (k1 << 8) | (k2 << 16) | (k3 << 24);
         const bool live = valid && !below_corner(corner, cpack);
-        Best best = {MRL_UNSAT, MRL_UNSAT, MRL_UNSAT, MRL_UNSAT};
+        Best best = {MRL_UNSAT, MRL_UNSAT, MRL_UNSAT};
         if (!__any_sync(0xFFFFFFFFu, live)) {
-          if (valid && b0 == 0) *reinterpret_cast<uint4*>(grid + cell) = make_uint4(best.main, best.peaks, best.tail, best.ci);
+          if (valid && b0 == 0) *reinterpret_cast<uint4*>(grid + cell) = make_uint4(best.main, best.peaks, best.tail, 0u);
           continue;
         }
         if (b0 && live) {   // what the earlier batches found
-          const uint4 r = *reinterpret_cast<const uint4*>(grid + cell);
-          best.main = r.x; best.peaks = r.y; best.tail = r.z; best.ci = r.w;
+          const uint4 r = ld_row(grid + cell);
+          best.main = r.x; best.peaks = r.y; best.tail = r.z;
         }
         const uint32_t bm0 = below(k0), bm1 = below(k1), bm2 = below(k2), bm3 = below(k3);
         if (live) {
-          for (uint32_t r = 0; r < n_here; r++) eval_staged(staged[r], a.rows, b0 + r, cpack, bm0, bm1, bm2, bm3, best, tally);
+          for (uint32_t r = 0; r < n_here; r++) eval_staged<false>(staged[r], cpack, bm0, bm1, bm2, bm3, best, tally);
         }
-        if (valid && (b0 == 0 || live))
-          *reinterpret_cast<uint4*>(grid + cell) = make_uint4(best.main, best.peaks, best.tail, best.ci);
+        if (valid && (b0 == 0 || live)) *reinterpret_cast<uint4*>(grid + cell) = make_uint4(best.main, best.peaks, best.tail, 0u);
       }
-      if (late_lanes) break;
-      b0 += nb;
-    } while (b0 < cl.y);
-    if (n_items <= gwarps) break;
-    if (lane == 0) w = gwarps + atomicAdd(next_item, 1u);
-    w = __shfl_sync(0xFFFFFFFFu, w, 0);
-  }
-  uint32_t tc = tally.cands, tl = tally.lookups;
-  for (int o = 16; o > 0; o >>= 1) {
-    tc += __shfl_xor_sync(0xFFFFFFFFu, tc, o);
-    tl += __shfl_xor_sync(0xFFFFFFFFu, tl, o);
-  }
-  if (lane == 0 && (tc | tl)) {
-    atomicAdd(&block_stats[0], (unsigned long long)tc);
-    atomicAdd(&block_stats[1], (unsigned long long)tl);
-  }
+      b0 += n_here;
+    } while (b0 < n_early);
+  } while (next_item(a, w, lane));
+  add_tally(tally, &block_stats[0], &block_stats[1], lane);
 }
 
-// Whole-row accesses to working rows that other warps may be writing at the same time: one
-// 128-bit access each, so a reader sees a row either before or after an update, never a mix.
-__device__ __forceinline__ uint4 ld_row_shared(const MrlRow* p) {
-  unsigned long long lo, hi;
-  asm volatile("{\n\t.reg .b128 q;\n\tld.relaxed.gpu.global.b128 q, [%2];\n\tmov.b128 {%0, %1}, q;\n\t}"
-               : "=l"(lo), "=l"(hi) : "l"(p) : "memory");
-  return make_uint4((uint32_t)lo, (uint32_t)(lo >> 32), (uint32_t)hi, (uint32_t)(hi >> 32));
-}
-__device__ __forceinline__ void st_row_shared(MrlRow* p, const uint4 v) {
-  const unsigned long long lo = v.x | ((unsigned long long)v.y << 32), hi = v.z | ((unsigned long long)v.w << 32);
-  asm volatile("{\n\t.reg .b128 q;\n\tmov.b128 q, {%1, %2};\n\tst.relaxed.gpu.global.b128 [%0], q;\n\t}"
-               :: "l"(p), "l"(lo), "l"(hi) : "memory");
-}
-
-// A staged record with a same-stage child at one limits point. Children of the stage being solved
-// live in the working rows and may improve while this runs; finished children are read-only.
-__device__ __forceinline__ void eval_staged_late(const StagedRec& s, const MrlRow* __restrict__ rows, const MrlRow* temp,
-                                                 uint32_t ci, uint32_t cpack, uint32_t bm0, uint32_t bm1, uint32_t bm2,
-                                                 uint32_t bm3, Best& best, Tally& tally) {
-  const uint4 a = s.rec;
-  const uint32_t action = a.x & 0xFFFFu, kind = (a.x >> 16) & 0xFFu, nchild = a.x >> 24;   // the same in all lanes
-  const uint32_t imm = a.y;
-  const uint32_t level = a.z & 0xFFu, thr = (a.z >> 8) & 0xFFu;
-  const uint32_t units = a.w;
-  const uint32_t lv = code_of(cpack, level);
-  tally.cands++;
-  uint32_t c0 = bm0, c1 = bm1, c2 = bm2, c3 = bm3;
-  const uint32_t sh = peak_shift(level);
-  if (kind == MRL_CK_MOVE) {
-    if (lv < thr) return;
-    if (imm > best.main) return;   // a Move costs at least its own base cost
-    const uint32_t cb = below(child_code(level, lv, units));
-    c0 = (level == 0) ? cb : c0;
-    c1 = (level == 1) ? cb : c1;
-    c2 = (level == 2) ? cb : c2;
-    c3 = (level == 3) ? cb : c3;
-  }
-  uint4 r[3];
-#pragma unroll
-  for (int j = 0; j < 3; j++) {
-    if ((uint32_t)j < nchild) {
-      const MrlRow* const p = staged_row(s, j, c0, c1, c2, c3);
-      r[j] = s.in_temp[j] ? ld_row_shared(p) : __ldg(reinterpret_cast<const uint4*>(p));
-    } else {
-      r[j] = r[0];
-    }
-  }
-  tally.lookups += nchild;
-  if (r[0].z == MRL_UNSAT || r[1].z == MRL_UNSAT || r[2].z == MRL_UNSAT) return;
-  uint32_t k_main, k_peaks, depth;
-  if (kind == MRL_CK_LOOP) {
-    k_main = sat_mul(r[0].x, imm);
-    k_peaks = r[0].y;
-    depth = 1u;
-  } else {
-    k_main = (kind == MRL_CK_MOVE) ? sat_add(imm, r[0].x) : r[0].x;
-    if (nchild > 1) k_main = sat_add(k_main, r[1].x);
-    if (nchild > 2) k_main = sat_add(k_main, r[2].x);
-    if (k_main > best.main) return;
-    k_peaks = __vmaxu4(__vmaxu4(r[0].y, r[1].y), r[2].y);
-    if (kind == MRL_CK_MOVE) {
-      const uint32_t cc = (k_peaks >> sh) & 0xFFu;
-      const uint32_t ncode = level < 2 ? units + cc : cache_code_ceil(units + cache_value(cc));
-      k_peaks = (k_peaks & ~(0xFFu << sh)) | (ncode << sh);
-    }
-    depth = min(max(max(r[0].z >> 16, r[1].z >> 16), r[2].z >> 16) + 1u, 255u);
-  }
-  const uint32_t k_tail = (depth << 16) | action;
-  if (key_less(k_main, k_peaks, k_tail, best)) {
-    best.main = k_main;
-    best.peaks = k_peaks;
-    best.tail = k_tail;
-    best.ci = ci;
-  }
-}
-
-// Pass step 4b, one relaxation sweep: the candidates with a child in the Spec's own stage (relayout
-// Moves). Such a child is read at limits reduced by what the Move allocates, so the dependencies
-// between cells form no cycle and the system "cell = best of its candidates at its children's
-// values" has exactly one solution. A sweep recomputes every cell from what phase_early found at
-// its limits (in the base rows) and all its same-stage records at the children's current values, in
-// place, while other warps read and write their own cells; a cell whose children all hold their
-// final values gets its final value, so every sweep settles at least one more level of the
-// dependency order, and the pass is finished after a sweep that changed nothing anywhere. (Keeping
-// the better of the old and the new value instead of recomputing would be wrong: a child that
-// improves can make the parent's peaks or depth worse.) From the second sweep on a Spec is looked
-// at again only if one of its same-stage children changed since the sweep before last began
-// (stamp = number of the last sweep that changed any cell of a Spec).
+// Step 4, relaxation sweeps: the records with a child in the Spec's own stage (relayout Moves). Such
+// a child is read at limits reduced by what the Move allocates, so the dependencies between cells
+// form no cycle and the system "cell = best of its candidates at its children's values" has exactly
+// one solution. A sweep recomputes cells from what the unordered phase found at their limits and all
+// their same-stage records at the children's current values, in place, while other warps read and
+// write their own cells. (Keeping the better of the old and the new value instead of recomputing
+// would be wrong: a child that improves can make the parent's peaks or depth worse.) Which cells:
+//   first pass, first sweep   all of them, their same-stage children at what the unordered phase
+//                             found for those - tables that do not change during the sweep, so the
+//                             working rows need no initial values
+//   later pass, first sweep   of the grids that grew (their cells hold the old grid's values, copied
+//                             at their limits), those that start at a new breakpoint in some memory:
+//                             the others read the same children at the same limits as before
+//   every other sweep         those that read a slot of a child which the sweep before changed. A
+//                             sweep leaves, per Spec and memory, the codes of the slots it changed a
+//                             cell of; a cell is solved again when its limits at some child fall into
+//                             such slots in all four memories.
+// Every cell is thus consistent with its children when a sweep changes nothing anywhere: it was
+// solved after its children last changed, or nothing it reads has changed. At size 8 this took the
+// sweeps after the first from 459 ms (whole Specs solved again when a child changed anywhere) to a
+// small part of that.
 // The records come dearest first and are staged from the end, so the cheapest Move is tried first.
-__device__ __forceinline__ void stage_late_batch(const HotArgs& a, StagedRec* staged, uint32_t last_rec, uint32_t n_here,
-                                                 uint32_t lane) {
+enum { SWEEP_ALL = 0, SWEEP_NEW = 1, SWEEP_CHANGED = 2 };
+
+template <int kMode>
+__device__ __forceinline__ void stage_late_batch(const HotArgs& a, uint32_t lo, StagedRec* staged, uint32_t last_rec, uint32_t n_here, uint32_t lane) {
   __syncwarp();   // the previous batch has been read by every lane
   if (lane < n_here) staged[lane].rec = __ldg(reinterpret_cast<const uint4*>(&a.cands[last_rec - lane]));
   __syncwarp();
@@ -970,484 +931,641 @@ __device__ __forceinline__ void stage_late_batch(const HotArgs& a, StagedRec* st
     const uint32_t r = t / 3u, j = t - r * 3u;
     if (j < (staged[r].rec.x >> 24)) {
       const uint32_t child = __ldg(&a.cands[last_rec - r].child[j]);
-      stage_child(staged[r], j, *reinterpret_cast<const uint4*>(&a.hdrs[child]), a.hdrs[child].row_base, a.rows, a.temp);   // same-stage headers: written earlier in this launch
+      if (kMode == SWEEP_ALL && child >= lo) {
+        stage_child(staged[r], j, a.sspec[child].emask, a.temp + a.temp_cap + a.sspec[child].erow, false);
+      } else {
+        const unsigned long long base = a.hdrs[child].row_base;
+        stage_child(staged[r], j, *reinterpret_cast<const uint4*>(&a.hdrs[child]), row_at(a.rows, a.temp, base), (base & MRL_TEMP_FLAG) != 0);
+      }
     }
   }
   __syncwarp();
 }
 
-// Pass step 3: every cell of the grids placed by this pass starts from what the unordered phase
-// found at the cell's limits. For a Spec without same-stage records that is its final value.
-__device__ __noinline__ void phase_late_init(const HotArgs a, const WorkItem* items, uint32_t n_items, uint32_t item_cells,
-                                             uint32_t* next_item) {
+// The parent's codes in memory k whose lookups of a child end in one of the child's slots `changed`
+// (a mask of the slots' codes). parent, child: masks of the two grids.
+__device__ __forceinline__ uint32_t codes_reading(uint32_t parent, uint32_t child, uint32_t changed, bool shifted, uint32_t level, uint32_t thr,
+                                                  uint32_t units) {
+  uint32_t out = 0;
+  while (parent) {
+    const uint32_t p = __ffs(parent) - 1;
+    parent &= parent - 1;
+    if (shifted && p < thr) continue;   // the Move does not fit
+    const uint32_t q = shifted ? child_code(level, p, units) : p;
+    const uint32_t slot = 31 - __clz(child & below(q));   // bit 0 is always set
+    if ((changed >> slot) & 1u) out |= 1u << p;
+  }
+  return out;
+}
+
+template <int kMode>
+__device__ __noinline__ void phase_sweep(const HotArgs a, uint32_t lo, const uint4* changed_before, uint4* changed_now, uint32_t sweep, uint32_t* any_changed,
+                                         unsigned long long* block_stats) {
   const uint32_t lane = threadIdx.x & 31;
-  const uint32_t gwarps = gridDim.x * (kBlock / 32);
-  for (uint32_t w = blockIdx.x * (kBlock / 32) + (threadIdx.x >> 5); w < n_items;) {
-    const WorkItem it = items[w];
-    const uint32_t i = it.spec;
+  WarpScratch& ws = warp_scratch();
+  StagedRec* const staged = ws.staged;
+  const uint8_t* const codes = ws.codes;
+  Tally tally = {0, 0};
+  uint32_t w = warp_number();
+  if (w < a.n_items) do {
+    const WorkItem it = a.items[w];
+    const uint32_t i = it.spec, first_cell = it.first_cell & ~31u;
+    if (kMode == SWEEP_NEW && !(it.first_cell & 1u)) continue;   // the grid did not grow
+    const uint2 cl = *reinterpret_cast<const uint2*>(&a.hdrs[i].cand_off);
+    const uint32_t n_late = a.sspec[i].n_late, last = cl.x + cl.y - 1;   // the records with a same-stage child are the last ones
+    const uint4 m = *reinterpret_cast<const uint4*>(&a.hdrs[i]);
+    uint32_t n_aff = 0;
+    if (kMode == SWEEP_NEW) {
+      if (lane == 0) {
+        const uint4 om = a.sspec[i].old_mask;
+        ws.affected[0] = make_uint4(m.x & ~om.x, m.y & ~om.y, m.z & ~om.z, m.w & ~om.w);
+      }
+      __syncwarp();
+    }
+    if (kMode == SWEEP_CHANGED) {
+      // children that the sweep before changed
+      __syncwarp();   // the previous item's list has been read by every lane
+      for (uint32_t t0 = 0; t0 < n_late * 3u; t0 += 32) {
+        const uint32_t t = t0 + lane, r = t / 3u, j = t - r * 3u;
+        bool hit = false;
+        if (r < n_late) {
+          const CandRec* const rec = &a.cands[last - r];
+          if (j < (__ldg(reinterpret_cast<const uint32_t*>(rec)) >> 24)) {
+            const uint32_t child = __ldg(&rec->child[j]);
+            hit = child >= lo && changed_before[child - lo].x != 0;
+          }
+        }
+        const uint32_t hits = __ballot_sync(0xFFFFFFFFu, hit);
+        const uint32_t at = n_aff + __popc(hits & ((1u << lane) - 1u));
+        if (hit && at < kMaxAffected) ws.who[at] = r | (j << 16);
+        n_aff += __popc(hits);
+      }
+      if (!n_aff) continue;
+      __syncwarp();
+      // per such child and memory, the codes of this grid that read one of its changed slots
+      if (n_aff <= kMaxAffected) {
+        for (uint32_t t = lane; t < n_aff * 4u; t += 32) {
+          const uint32_t k = t & 3u, r = ws.who[t >> 2] & 0xFFFFu, j = ws.who[t >> 2] >> 16;
+          const CandRec* const rec = &a.cands[last - r];
+          const uint4 c = __ldg(reinterpret_cast<const uint4*>(rec));
+          const uint32_t child = __ldg(&rec->child[j]), level = c.z & 0xFFu;
+          const uint4 cm = *reinterpret_cast<const uint4*>(&a.hdrs[child]);
+          const uint4 ch = changed_before[child - lo];
+          reinterpret_cast<uint32_t*>(&ws.affected[t >> 2])[k] =
+              codes_reading(sel4(m.x, m.y, m.z, m.w, k), sel4(cm.x, cm.y, cm.z, cm.w, k), sel4(ch.x, ch.y, ch.z, ch.w, k), k == level, level,
+                            (c.z >> 8) & 0xFFu, c.w);
+        }
+      }
+      __syncwarp();
+    }
+    if (lane == 0) atomicAdd(&block_stats[4], 1ull);
+    MrlRow* const grid = a.temp + (a.hdrs[i].row_base & ~MRL_TEMP_FLAG);
+    const uint4 em = a.sspec[i].emask;   // where the unordered phase left its result
+    const MrlRow* const egrid = a.temp + a.temp_cap + a.sspec[i].erow;
+    const uint32_t n0 = __popc(m.x), n1 = __popc(m.y), n2 = __popc(m.z), n3 = __popc(m.w);
+    const uint32_t cells = n0 * n1 * n2 * n3;
+    const uint32_t corner = a.sspec[i].corner;
+    // Grids are clipped at the corner, so the cells below it are exactly those in slot 0 of a
+    // clipped memory; they stay unsatisfiable and are left out: the lanes walk the live cells
+    // only. The item's share of them: its range of all cells, scaled (the items of a Spec tile
+    // its cells, so the scaled ranges tile the live ones).
+    const bool none = corner_of(corner, 0) == MRL_NEVER;
+    const uint32_t z0 = corner_of(corner, 0) ? 1u : 0u, z1 = corner_of(corner, 1) ? 1u : 0u, z2 = corner_of(corner, 2) ? 1u : 0u,
+                   z3 = corner_of(corner, 3) ? 1u : 0u;
+    const uint32_t v0 = n0 - z0, v1 = n1 - z1, v2 = n2 - z2, v3 = n3 - z3;
+    const unsigned long long live_cells = none ? 0ull : (unsigned long long)v0 * v1 * v2 * v3;
+    const uint32_t c_hi = min(cells, first_cell + a.item_cells);
+    const uint32_t l_begin = (uint32_t)(live_cells * first_cell / cells), l_end = (uint32_t)(live_cells * c_hi / cells);
+    if (kMode == SWEEP_ALL) {   // the cells below the corner
+      for (uint32_t cell = first_cell + lane; cell < c_hi; cell += 32) {
+        uint32_t rest = cell;
+        const bool d0 = rest % n0 < z0; rest /= n0;
+        const bool d1 = rest % n1 < z1; rest /= n1;
+        const bool d2 = rest % n2 < z2; rest /= n2;
+        if (none || d0 || d1 || d2 || rest < z3) *reinterpret_cast<uint4*>(grid + cell) = make_uint4(MRL_UNSAT, MRL_UNSAT, MRL_UNSAT, 0u);
+      }
+    }
+    if (l_begin == l_end) continue;
+    const bool single = n_late <= (uint32_t)kBatch;   // all records staged once for the whole item
+    stage_slot_codes(ws.codes, m, n0, n1, n2, n3, lane);
+    bool staged_yet = false;
+    uint4 ch = make_uint4(0, 0, 0, 0);   // codes of the slots of the cells that change
+    auto solve = [&](bool live, uint32_t slots) {   // packed slots, one cell per lane
+      if (single && !staged_yet) {
+        stage_late_batch<kMode>(a, lo, staged, last, n_late, lane);
+        staged_yet = true;
+      }
+      const uint32_t s0 = slots & 0xFFu, s1 = (slots >> 8) & 0xFFu, s2 = (slots >> 16) & 0xFFu, s3 = slots >> 24;
+      const uint32_t k0 = codes[s0], k1 = codes[n0 + s1], k2 = codes[n0 + n1 + s2], k3 = codes[n0 + n1 + n2 + s3];
+      const uint32_t cpack = k0 | (k1 << 8) | (k2 << 16) | (k3 << 24);
+      const uint32_t bm0 = below(k0), bm1 = below(k1), bm2 = below(k2), bm3 = below(k3);
+      MrlRow* const at = grid + (((s3 * n2 + s2) * n1 + s1) * n0 + s0);
+      Best best = {MRL_UNSAT, MRL_UNSAT, MRL_UNSAT};
+      uint4 was = make_uint4(MRL_UNSAT, MRL_UNSAT, MRL_UNSAT, 0u);
+      if (live) {
+        const uint32_t i0 = __popc(em.x & bm0) - 1, i1 = __popc(em.y & bm1) - 1, i2 = __popc(em.z & bm2) - 1, i3 = __popc(em.w & bm3) - 1;
+        const uint4 f = ld_row(egrid + (((i3 * __popc(em.z) + i2) * __popc(em.y) + i1) * __popc(em.x) + i0));
+        best.main = f.x; best.peaks = f.y; best.tail = f.z;
+        was = kMode == SWEEP_ALL ? f : ld_row(at);   // only this warp writes the cell in this sweep
+      }
+      for (uint32_t b = 0; b < n_late; b += kBatch) {
+        const uint32_t n_here = min((uint32_t)kBatch, n_late - b);
+        if (!single) stage_late_batch<kMode>(a, lo, staged, last - b, n_here, lane);
+        if (live)
+          for (uint32_t r = 0; r < n_here; r++) eval_staged<kMode != SWEEP_ALL>(staged[r], cpack, bm0, bm1, bm2, bm3, best, tally);
+      }
+      if (live) {
+        const bool differs = best.main != was.x || best.peaks != was.y || best.tail != was.z;
+        if (kMode == SWEEP_ALL) *reinterpret_cast<uint4*>(at) = make_uint4(best.main, best.peaks, best.tail, 0u);
+        else if (differs) st_row_shared(at, make_uint4(best.main, best.peaks, best.tail, 0u));
+        if (differs) { ch.x |= 1u << k0; ch.y |= 1u << k1; ch.z |= 1u << k2; ch.w |= 1u << k3; }
+      }
+    };
+    uint32_t queued = 0;
+    for (uint32_t c0 = l_begin; c0 < l_end; c0 += 32) {
+      const bool live = c0 + lane < l_end;
+      uint32_t rest = live ? c0 + lane : l_begin;
+      const uint32_t s0 = rest % v0 + z0; rest /= v0;
+      const uint32_t s1 = rest % v1 + z1; rest /= v1;
+      const uint32_t s2 = rest % v2 + z2;
+      const uint32_t s3 = rest / v2 + z3;
+      const uint32_t slots = s0 | (s1 << 8) | (s2 << 16) | (s3 << 24);
+      if (kMode == SWEEP_ALL) {
+        solve(live, slots);
+        continue;
+      }
+      bool again = false;
+      const uint32_t k0 = codes[s0], k1 = codes[n0 + s1], k2 = codes[n0 + n1 + s2], k3 = codes[n0 + n1 + n2 + s3];
+      if (kMode == SWEEP_NEW) {
+        const uint4 f = ws.affected[0];
+        again = ((f.x >> k0) | (f.y >> k1) | (f.z >> k2) | (f.w >> k3)) & 1u;
+      } else if (n_aff > (uint32_t)kMaxAffected) {
+        again = true;
+      } else {
+        uint32_t hit = 0;
+        for (uint32_t e = 0; e < n_aff; e++) {
+          const uint4 f = ws.affected[e];
+          hit |= (f.x >> k0) & (f.y >> k1) & (f.z >> k2) & (f.w >> k3);
+        }
+        again = hit & 1u;
+      }
+      again = again && live;
+      // the cells to solve are collected until there is one per lane
+      const uint32_t who = __ballot_sync(0xFFFFFFFFu, again);
+      if (again) ws.queue[queued + __popc(who & ((1u << lane) - 1u))] = slots;
+      queued += __popc(who);
+      __syncwarp();
+      if (queued >= 32) {
+        const uint32_t mine = ws.queue[lane], rest_of = ws.queue[32 + lane];
+        __syncwarp();
+        solve(true, mine);
+        queued -= 32;
+        if (lane < queued) ws.queue[lane] = rest_of;
+        __syncwarp();
+      }
+    }
+    if (queued) {
+      const uint32_t mine = lane < queued ? ws.queue[lane] : (z0 | (z1 << 8) | (z2 << 16) | (z3 << 24));
+      __syncwarp();
+      solve(lane < queued, mine);
+    }
+    ch = warp_or(ch);
+    if (ch.x && lane == 0) {
+      uint32_t* const out = reinterpret_cast<uint32_t*>(&changed_now[i - lo]);
+      atomicOr(out, ch.x); atomicOr(out + 1, ch.y); atomicOr(out + 2, ch.z); atomicOr(out + 3, ch.w);
+      a.sspec[i].dirty = 1;
+      *any_changed = sweep;
+    }
+  } while (next_item(a, w, lane));
+  add_tally(tally, &block_stats[2], &block_stats[3], lane);
+}
+
+// A further pass: the cells of the grids that grew start from the old grid's values at their limits.
+__device__ __noinline__ void phase_refine(const HotArgs a) {
+  const uint32_t lane = threadIdx.x & 31;
+  uint32_t w = warp_number();
+  if (w < a.n_items) do {
+    const WorkItem it = a.items[w];
+    if (!(it.first_cell & 1u)) continue;
+    const uint32_t i = it.spec, first_cell = it.first_cell & ~31u;
     const uint4 m = *reinterpret_cast<const uint4*>(&a.hdrs[i]);
     MrlRow* const grid = a.temp + (a.hdrs[i].row_base & ~MRL_TEMP_FLAG);
-    const uint4 em = *reinterpret_cast<const uint4*>(&a.ehdr[i]);
-    const unsigned long long ebase = a.ehdr[i].row_base;
+    const uint4 om = a.sspec[i].old_mask;
+    const unsigned long long obase = a.sspec[i].old_row;
     const uint32_t n0 = __popc(m.x), n1 = __popc(m.y), n2 = __popc(m.z), n3 = __popc(m.w);
-    const uint32_t c_end = min(n0 * n1 * n2 * n3, it.first_cell + item_cells);
-    for (uint32_t cell = it.first_cell + lane; cell < c_end; cell += 32) {
+    const uint32_t c_end = min(n0 * n1 * n2 * n3, first_cell + a.item_cells);
+    for (uint32_t cell = first_cell + lane; cell < c_end; cell += 32) {
       uint32_t rest = cell;
       const uint32_t k0 = nth_set_bit(m.x, rest % n0); rest /= n0;
       const uint32_t k1 = nth_set_bit(m.y, rest % n1); rest /= n1;
       const uint32_t k2 = nth_set_bit(m.z, rest % n2); rest /= n2;
       const uint32_t k3 = nth_set_bit(m.w, rest);
-      *reinterpret_cast<uint4*>(grid + cell) =
-          *reinterpret_cast<const uint4*>(row_of(a.base, a.base, em, ebase, below(k0), below(k1), below(k2), below(k3)));
+      *reinterpret_cast<uint4*>(grid + cell) = ld_row(row_of(a.rows, a.temp, om, obase, below(k0), below(k1), below(k2), below(k3)));
     }
-    if (n_items <= gwarps) break;
-    if (lane == 0) w = gwarps + atomicAdd(next_item, 1u);
-    w = __shfl_sync(0xFFFFFFFFu, w, 0);
-  }
+  } while (next_item(a, w, lane));
 }
 
-__device__ __noinline__ void phase_late(const HotArgs a, const WorkItem* items, uint32_t n_items, uint32_t item_cells,
-                                        uint32_t* next_item, uint32_t lo, uint32_t* stamp /* by position in the stage */,
-                                        uint32_t sweep, bool first_sweep, uint32_t* changed,
-                                        unsigned long long* block_stats) {
-  __shared__ StagedRec staged_all[kBlock / 32][kBatch];
-  __shared__ uint8_t codes_all[kBlock / 32][kMaxSlots];
-  StagedRec* const staged = staged_all[threadIdx.x >> 5];   // this warp's
-  uint8_t* const codes = codes_all[threadIdx.x >> 5];
+// Which breakpoints of the grids are real: a breakpoint (memory k, code c) is real when some cell
+// starting at c differs from its neighbour one slot lower in k. kEarly: of the grids of the
+// unordered phase, else of the working grids (only_dirty: of those that grew or changed). A warp
+// stops comparing in a memory at codes it knows to be real.
+template <bool kEarly>
+__device__ __noinline__ void phase_real_masks(const HotArgs a, uint4* rmask, bool only_dirty) {
   const uint32_t lane = threadIdx.x & 31;
-  const uint32_t gwarps = gridDim.x * (kBlock / 32);
-  Tally tally = {0, 0};
-  for (uint32_t w = blockIdx.x * (kBlock / 32) + (threadIdx.x >> 5); w < n_items;) {
-    const WorkItem it = items[w];
-    const uint32_t i = it.spec;
-    const uint2 cl = *reinterpret_cast<const uint2*>(&a.hdrs[i].cand_off);
-    // the records with a same-stage child are the last ones
-    uint32_t n_late = 0;
-    for (uint32_t k = 0; k < cl.y; k += 32) {
-      const bool late = k + lane < cl.y && ((__ldg(&reinterpret_cast<const uint32_t*>(&a.cands[cl.x + cl.y - 1 - k - lane])[2]) >> 24) & 1u);
-      const uint32_t not_late = ~__ballot_sync(0xFFFFFFFFu, late);
-      const uint32_t run = not_late ? (uint32_t)__ffs(not_late) - 1u : 32u;
-      n_late += run;
-      if (run < 32) break;
+  WarpScratch& ws = warp_scratch();
+  const uint8_t* const codes = ws.codes;
+  uint32_t w = warp_number();
+  if (w < a.n_items) do {
+    const WorkItem it = a.items[w];
+    const uint32_t i = it.spec, first_cell = it.first_cell & ~31u;
+    if (only_dirty && !a.sspec[i].dirty) continue;
+    const uint4 m = kEarly ? a.sspec[i].emask : *reinterpret_cast<const uint4*>(&a.hdrs[i]);
+    const MrlRow* const grid = kEarly ? a.temp + a.temp_cap + a.sspec[i].erow : a.temp + (a.hdrs[i].row_base & ~MRL_TEMP_FLAG);
+    const uint32_t n0 = __popc(m.x), n1 = __popc(m.y), n2 = __popc(m.z), n3 = __popc(m.w);
+    const uint32_t c_end = min(n0 * n1 * n2 * n3, first_cell + a.item_cells);
+    const uint32_t st1 = n0, st2 = n0 * n1, st3 = st2 * n2;
+    stage_slot_codes(ws.codes, m, n0, n1, n2, n3, lane);
+    uint4 real = make_uint4(1u, 1u, 1u, 1u);   // the same in all lanes
+    for (uint32_t c0 = first_cell; c0 < c_end; c0 += 32) {
+      const uint32_t cell = c0 + lane;
+      uint4 bits = make_uint4(0, 0, 0, 0);
+      if (cell < c_end) {
+        uint32_t rest = cell;
+        const uint32_t s0 = rest % n0; rest /= n0;
+        const uint32_t s1 = rest % n1; rest /= n1;
+        const uint32_t s2 = rest % n2, s3 = rest / n2;
+        const MrlRow* const p = grid + cell;
+        const uint32_t q0 = 1u << codes[s0], q1 = 1u << codes[n0 + s1], q2 = 1u << codes[n0 + n1 + s2], q3 = 1u << codes[n0 + n1 + n2 + s3];
+        const bool w0 = s0 && !(real.x & q0), w1 = s1 && !(real.y & q1), w2 = s2 && !(real.z & q2), w3 = s3 && !(real.w & q3);
+        if (w0 || w1 || w2 || w3) {
+          const uint4 r = ld_row(p);
+          uint4 x0 = r, x1 = r, x2 = r, x3 = r;
+          if (w0) x0 = ld_row(p - 1);
+          if (w1) x1 = ld_row(p - st1);
+          if (w2) x2 = ld_row(p - st2);
+          if (w3) x3 = ld_row(p - st3);
+          if (x0.x != r.x || x0.y != r.y || x0.z != r.z) bits.x = q0;
+          if (x1.x != r.x || x1.y != r.y || x1.z != r.z) bits.y = q1;
+          if (x2.x != r.x || x2.y != r.y || x2.z != r.z) bits.z = q2;
+          if (x3.x != r.x || x3.y != r.y || x3.z != r.z) bits.w = q3;
+        }
+      }
+      bits = warp_or(bits);
+      real.x |= bits.x; real.y |= bits.y; real.z |= bits.z; real.w |= bits.w;
     }
-    bool fresh = first_sweep && n_late;   // some same-stage child changed lately
-    if (n_late && !first_sweep) {
-      for (uint32_t t = lane; t < n_late * 3u; t += 32) {
-        const uint32_t r = t / 3u, j = t - r * 3u;
-        const CandRec* const rec = &a.cands[cl.x + cl.y - 1 - r];
-        if (j < (__ldg(reinterpret_cast<const uint32_t*>(rec)) >> 24)) {
-          const uint32_t child = __ldg(&rec->child[j]);
-          if (child >= lo && stamp[child - lo] + 1u >= sweep) fresh = true;
-        }
-      }
-      fresh = __any_sync(0xFFFFFFFFu, fresh);
-    }
-    if (fresh) {
-      if (lane == 0) atomicAdd(&block_stats[4], 1ull);
-      const uint4 m = *reinterpret_cast<const uint4*>(&a.hdrs[i]);
-      MrlRow* const grid = a.temp + (a.hdrs[i].row_base & ~MRL_TEMP_FLAG);
-      const uint4 em = *reinterpret_cast<const uint4*>(&a.ehdr[i]);   // where the unordered phase left its result
-      const unsigned long long ebase = a.ehdr[i].row_base;
-      const uint32_t n0 = __popc(m.x), n1 = __popc(m.y), n2 = __popc(m.z), n3 = __popc(m.w);
-      const uint32_t cells = n0 * n1 * n2 * n3;
-      const uint32_t corner = a.corner[i];
-      // Grids are clipped at the corner, so the cells below it are exactly those in slot 0 of a
-      // clipped memory; they stay unsatisfiable and are left out: the lanes walk the live cells
-      // only. The item's share of them: its range of all cells, scaled (the items of a Spec tile
-      // its cells, so the scaled ranges tile the live ones).
-      const uint32_t z0 = corner_of(corner, 0) ? 1u : 0u, z1 = corner_of(corner, 1) ? 1u : 0u, z2 = corner_of(corner, 2) ? 1u : 0u,
-                     z3 = corner_of(corner, 3) ? 1u : 0u;
-      const uint32_t v0 = n0 - z0, v1 = n1 - z1, v2 = n2 - z2, v3 = n3 - z3;
-      const unsigned long long live_cells = (corner_of(corner, 0) == MRL_NEVER) ? 0ull : (unsigned long long)v0 * v1 * v2 * v3;
-      const uint32_t c_hi = min(cells, it.first_cell + item_cells);
-      const uint32_t l_begin = (uint32_t)(live_cells * it.first_cell / cells), l_end = (uint32_t)(live_cells * c_hi / cells);
-      const bool single = n_late <= (uint32_t)kBatch;   // all records staged once for the whole item
-      stage_slot_codes(codes, m, n0, n1, n2, n3, lane);
-      if (single) stage_late_batch(a, staged, cl.x + cl.y - 1, n_late, lane);
-      bool changed_any = false;
-      for (uint32_t c0 = l_begin; c0 < l_end; c0 += 32) {
-        const bool live = c0 + lane < l_end;
-        uint32_t rest = live ? c0 + lane : l_begin;
-        const uint32_t s0 = rest % v0 + z0; rest /= v0;
-        const uint32_t s1 = rest % v1 + z1; rest /= v1;
-        const uint32_t s2 = rest % v2 + z2;
-        const uint32_t s3 = rest / v2 + z3;
-        const uint32_t cell = ((s3 * n2 + s2) * n1 + s1) * n0 + s0;
-        const uint32_t k0 = codes[s0], k1 = codes[n0 + s1], k2 = codes[n0 + n1 + s2], k3 = codes[n0 + n1 + n2 + s3];
-        const uint32_t cpack = k0 | (k1 << 8) | (k2 << 16) | (k3 << 24);
-        Best best = {MRL_UNSAT, MRL_UNSAT, MRL_UNSAT, MRL_UNSAT};
-        const uint32_t bm0 = below(k0), bm1 = below(k1), bm2 = below(k2), bm3 = below(k3);
-        if (live) {
-          const uint4 f = *reinterpret_cast<const uint4*>(row_of(a.base, a.base, em, ebase, bm0, bm1, bm2, bm3));
-          best.main = f.x; best.peaks = f.y; best.tail = f.z; best.ci = f.w;
-        }
-        for (uint32_t b = 0; b < n_late; b += kBatch) {
-          const uint32_t n_here = min((uint32_t)kBatch, n_late - b);
-          if (!single) stage_late_batch(a, staged, cl.x + cl.y - 1 - b, n_here, lane);
-          if (live)
-            for (uint32_t r = 0; r < n_here; r++)
-              eval_staged_late(staged[r], a.rows, a.temp, cl.y - 1 - b - r, cpack, bm0, bm1, bm2, bm3, best, tally);
-        }
-        if (live) {
-          const uint4 was = *reinterpret_cast<const uint4*>(grid + cell);   // only this warp writes the cell in this sweep
-          if (best.main != was.x || best.peaks != was.y || best.tail != was.z) {
-            st_row_shared(grid + cell, make_uint4(best.main, best.peaks, best.tail, best.ci));
-            changed_any = true;
-          }
-        }
-      }
-      if (__any_sync(0xFFFFFFFFu, changed_any) && lane == 0) {
-        stamp[i - lo] = sweep;
-        *changed = sweep;
-      }
-    }
-    if (n_items <= gwarps) break;
-    if (lane == 0) w = gwarps + atomicAdd(next_item, 1u);
-    w = __shfl_sync(0xFFFFFFFFu, w, 0);
-  }
-  uint32_t tc = tally.cands, tl = tally.lookups;
-  for (int o = 16; o > 0; o >>= 1) {
-    tc += __shfl_xor_sync(0xFFFFFFFFu, tc, o);
-    tl += __shfl_xor_sync(0xFFFFFFFFu, tl, o);
-  }
-  if (lane == 0 && (tc | tl)) {
-    atomicAdd(&block_stats[2], (unsigned long long)tc);
-    atomicAdd(&block_stats[3], (unsigned long long)tl);
-  }
-}
-
-// Pass step 5: which breakpoints of the working grids are real. A breakpoint (memory k, code c)
-// is real when some cell starting at c differs from its neighbour one slot lower in k.
-// early: of the grids of the unordered phase (in the base rows), else of the working grids.
-__device__ __noinline__ void phase_real_masks(const StageArgs& a, uint32_t n_chunks, bool early) {
-  const uint32_t lane = threadIdx.x & 31;
-  const uint32_t gwarps = gridDim.x * (kBlock / 32);
-  const SpecHdr* const H = early ? a.ehdr - a.lo : a.hdrs;
-  const MrlRow* const R = early ? a.base : a.temp;
-  for (uint32_t w = blockIdx.x * (kBlock / 32) + (threadIdx.x >> 5); w < n_chunks; w += gwarps) {
-    const Chunk ch = a.chunks[w];
-    const Column c = decode_column(H, ch, lane);
-    uint32_t bits[4] = {0, 0, 0, 0};
-    if (c.valid) {
-      const unsigned long long base = H[ch.spec].row_base & ~MRL_TEMP_FLAG;
-      const uint32_t st[4] = {1u, c.nn[0], c.nn[0] * c.nn[1], c.nn[0] * c.nn[1] * c.nn[2]};
-      const uint32_t mF = sel4(c.mm[0], c.mm[1], c.mm[2], c.mm[3], c.F);
-      const uint32_t nF = sel4(c.nn[0], c.nn[1], c.nn[2], c.nn[3], c.F);
-      const uint32_t stF = sel4(st[0], st[1], st[2], st[3], c.F);
-      uint32_t off0 = 0;
-#pragma unroll
-      for (int k = 0; k < 4; k++) off0 += c.idx[k] * st[k];   // idx[F] is 0
-      uint4 prev = make_uint4(0, 0, 0, 0);
-      uint32_t fbits = 0, mrest = mF, differs = 0;   // differs: memories in which some cell of the column differs from its lower neighbour
-      for (uint32_t s = 0; s < nF; s++) {
-        const uint32_t codeF = __ffs(mrest) - 1;
-        mrest &= mrest - 1;
-        const unsigned long long r_at = base + off0 + (unsigned long long)s * stF;
-        const uint4 r = *reinterpret_cast<const uint4*>(R + r_at);
-#pragma unroll
-        for (int k = 0; k < 4; k++) {
-          if ((uint32_t)k == c.F || c.idx[k] == 0) continue;
-          const uint4 nb = *reinterpret_cast<const uint4*>(R + r_at - st[k]);
-          if (nb.x != r.x || nb.y != r.y || nb.z != r.z) differs |= 1u << k;
-        }
-        if (s > 0 && (prev.x != r.x || prev.y != r.y || prev.z != r.z)) fbits |= 1u << codeF;
-        prev = r;
-      }
-#pragma unroll
-      for (int k = 0; k < 4; k++) {
-        if ((uint32_t)k == c.F) bits[k] = fbits;
-        else if ((differs >> k) & 1u) bits[k] = 1u << nth_set_bit(c.mm[k], c.idx[k]);   // the column's slot in that memory starts at a real breakpoint
-      }
-    }
-#pragma unroll
-    for (int k = 0; k < 4; k++) bits[k] = __reduce_or_sync(0xFFFFFFFFu, bits[k]);
     if (lane == 0) {
-      uint32_t* out = reinterpret_cast<uint32_t*>(&a.rmask[ch.spec]);
-#pragma unroll
-      for (int k = 0; k < 4; k++)
-        if (bits[k]) atomicOr(out + k, bits[k]);
+      uint32_t* const out = reinterpret_cast<uint32_t*>(&rmask[i]);
+      if (real.x & ~1u) atomicOr(out, real.x);
+      if (real.y & ~1u) atomicOr(out + 1, real.y);
+      if (real.z & ~1u) atomicOr(out + 2, real.z);
+      if (real.w & ~1u) atomicOr(out + 3, real.w);
     }
-  }
+  } while (next_item(a, w, lane));
 }
 
 // ---- compaction: working grids -> final table ---------------------------------------------
 
-// Final cell count per Spec of the stage, the sum per run of kBlock Specs, and the algorithmic
-// bytes of the stage's final rows.
-__device__ __noinline__ void phase_final_count(const StageArgs& a) {
+// The Specs a block counts and compacts: a contiguous part of the stage, so that the places of its
+// rows follow from the sums of the blocks before it.
+__device__ __forceinline__ void block_specs(uint32_t lo, uint32_t hi, uint32_t& b_lo, uint32_t& b_hi) {
+  const uint32_t per = (hi - lo + gridDim.x - 1) / gridDim.x;
+  b_lo = min(hi, lo + blockIdx.x * per);
+  b_hi = min(hi, b_lo + per);
+}
+
+__device__ __forceinline__ unsigned long long block_sum(unsigned long long v) {
+  __shared__ unsigned long long part[kStageBlock / 32];
+  __shared__ unsigned long long all;
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xFFFFFFFFu, v, o);
+  __syncthreads();   // protects the shared values across consecutive calls
+  if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = v;
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    unsigned long long s = threadIdx.x < kStageBlock / 32 ? part[threadIdx.x] : 0ull;
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xFFFFFFFFu, s, o);
+    if (threadIdx.x == 0) all = s;
+  }
+  __syncthreads();
+  return all;
+}
+
+// Final cells of this block's Specs, by their real breakpoints.
+__device__ __noinline__ void phase_count(const StageArgs& a, uint32_t lo, uint32_t hi) {
+  uint32_t b_lo, b_hi;
+  block_specs(lo, hi, b_lo, b_hi);
+  unsigned long long n = 0;
+  for (uint32_t i = b_lo + threadIdx.x; i < b_hi; i += kStageBlock) n += cells_of(a.rmask[i]);
+  n = block_sum(n);
+  if (threadIdx.x == 0) a.block_sums[blockIdx.x] = n;
+}
+
+// Copies each Spec's real cells from its grid to its final rows and repoints the header, a warp per
+// Spec. Specs computed by another rank get zero rows (the exchange adds the owner's rows onto
+// them). Returns the bytes of records and rows the final rows are the combination of.
+__device__ __noinline__ void phase_compact(const StageArgs& a, uint32_t lo, uint32_t hi, unsigned long long first_row) {
+  __shared__ unsigned long long off[kStageBlock];
+  __shared__ unsigned long long warp_base[kStageBlock / 32];
+  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  uint32_t b_lo, b_hi;
+  block_specs(lo, hi, b_lo, b_hi);
   unsigned long long bytes = 0;
-  for (uint32_t base = a.lo + blockIdx.x * kBlock; base < a.hi; base += gridDim.x * kBlock) {
-    const uint32_t i = base + threadIdx.x;
-    unsigned long long n = 0;
-    if (i < a.hi) {
-      const uint4 m = a.rmask[i];
-      n = (unsigned long long)__popc(m.x) * __popc(m.y) * __popc(m.z) * __popc(m.w);
-      a.fcount[i - a.lo] = (uint32_t)n;
+  for (uint32_t base = b_lo; base < b_hi; base += kStageBlock) {
+    // places of the next kStageBlock Specs
+    const uint32_t own = base + threadIdx.x;
+    const unsigned long long n_own = own < b_hi ? cells_of(a.rmask[own]) : 0ull;
+    unsigned long long inc = n_own;
+    for (int o = 1; o < 32; o <<= 1) {
+      const unsigned long long t = __shfl_up_sync(0xFFFFFFFFu, inc, o);
+      if (lane >= (uint32_t)o) inc += t;
+    }
+    __syncthreads();
+    off[threadIdx.x] = inc - n_own;
+    if (lane == 31) warp_base[warp] = inc;
+    __syncthreads();
+    if (warp == 0) {
+      const unsigned long long v = lane < kStageBlock / 32 ? warp_base[lane] : 0ull;
+      unsigned long long s = v;
+      for (int o = 1; o < 32; o <<= 1) {
+        const unsigned long long t = __shfl_up_sync(0xFFFFFFFFu, s, o);
+        if (lane >= (uint32_t)o) s += t;
+      }
+      if (lane < kStageBlock / 32) warp_base[lane] = s - v;
+    }
+    __syncthreads();
+    const uint32_t here = min((uint32_t)kStageBlock, b_hi - base);
+    unsigned long long last = 0;
+    for (uint32_t k = warp; k < here; k += kStageBlock / 32) {
+      const uint32_t i = base + k;
+      const unsigned long long fbase = first_row + warp_base[k >> 5] + off[k];
+      const uint4 fm = a.rmask[i];
+      const uint32_t f0 = __popc(fm.x), f1 = __popc(fm.y), f2 = __popc(fm.z), f3 = __popc(fm.w), n = f0 * f1 * f2 * f3;
+      MrlRow* const to = a.rows + fbase;
       if (computed_here(a, i)) {
+        const uint4 tm = *reinterpret_cast<const uint4*>(&a.hdrs[i]);
+        const MrlRow* const from = row_at(a.rows, a.temp, a.hdrs[i].row_base);
+        const uint32_t t0 = __popc(tm.x), t1 = __popc(tm.y), t2 = __popc(tm.z);
+        const bool same = tm.x == fm.x && tm.y == fm.y && tm.z == fm.z && tm.w == fm.w;
+        for (uint32_t j = lane; j < n; j += 32) {
+          uint32_t toff = j;
+          if (!same) {
+            uint32_t rest = j;
+            const uint32_t j0 = rest % f0; rest /= f0;
+            const uint32_t j1 = rest % f1; rest /= f1;
+            const uint32_t j2 = rest % f2, j3 = rest / f2;
+            const uint32_t i0 = __popc(tm.x & below(nth_set_bit(fm.x, j0))) - 1;
+            const uint32_t i1 = __popc(tm.y & below(nth_set_bit(fm.y, j1))) - 1;
+            const uint32_t i2 = __popc(tm.z & below(nth_set_bit(fm.z, j2))) - 1;
+            const uint32_t i3 = __popc(tm.w & below(nth_set_bit(fm.w, j3))) - 1;
+            toff = ((i3 * t2 + i2) * t1 + i1) * t0 + i0;
+          }
+          uint4 r = ld_row(from + toff);
+          r.w = 0;
+          *reinterpret_cast<uint4*>(to + j) = r;
+        }
+        // statistics: 12 bytes per row, 16 per record, 16 per child of every record that fits the row's limits
         const uint2 cl = *reinterpret_cast<const uint2*>(&a.hdrs[i].cand_off);
-        bytes += n * (12ull + 16ull * cl.y);
-        for (uint32_t ci = 0; ci < cl.y; ci++) {
-          const uint4 c = __ldg(reinterpret_cast<const uint4*>(&a.cands[cl.x + ci]));
-          const uint32_t kind = (c.x >> 16) & 0xFFu, nchild = c.x >> 24;
-          if (!nchild) continue;
+        if (lane == 0) bytes += n * (12ull + 16ull * cl.y);
+        for (uint32_t c = lane; c < cl.y; c += 32) {
+          const uint4 rec = __ldg(reinterpret_cast<const uint4*>(&a.cands[cl.x + c]));
+          const uint32_t kind = (rec.x >> 16) & 0xFFu, nchild = rec.x >> 24;
           unsigned long long feasible = n;
           if (kind == MRL_CK_MOVE) {
-            const uint32_t ml = sel4(m.x, m.y, m.z, m.w, c.z & 0xFFu), thr = (c.z >> 8) & 0xFFu;
+            const uint32_t ml = sel4(fm.x, fm.y, fm.z, fm.w, rec.z & 0xFFu), thr = (rec.z >> 8) & 0xFFu;
             feasible = n / (uint32_t)__popc(ml) * (uint32_t)__popc(ml >> thr);   // final cells at or above the threshold
           }
           bytes += feasible * nchild * 16ull;
         }
+      } else {
+        for (uint32_t j = lane; j < n; j += 32) *reinterpret_cast<uint4*>(to + j) = make_uint4(0, 0, 0, 0);
+      }
+      __syncwarp();   // the header is repointed when every lane has read it, and the corner read off rows that are written
+      if (lane == 0) {
+        *reinterpret_cast<uint4*>(&a.hdrs[i]) = fm;
+        a.hdrs[i].row_base = fbase;
+        if (!a.mine) a.minsat[i] = corner_from_rows(fm, to);
       }
     }
-    unsigned long long total;
-    block_excl_scan(n, &total);
-    if (threadIdx.x == 0) a.block_sums[(base - a.lo) / kBlock] = total;
+    last = warp_base[kStageBlock / 32 - 1] + off[kStageBlock - 1];
+    {
+      // the last Spec's cells end the run
+      const uint32_t q = base + kStageBlock - 1;
+      if (q < b_hi) last += cells_of(a.rmask[q]);
+    }
+    first_row += last;   // only used when another run follows, and then this one is full
   }
   for (int o = 16; o > 0; o >>= 1) bytes += __shfl_xor_sync(0xFFFFFFFFu, bytes, o);
-  if ((threadIdx.x & 31) == 0 && bytes) atomicAdd(&a.ctl->st_final_bytes, bytes);
+  if (lane == 0 && bytes) atomicAdd(&a.ctl->st_final_bytes, bytes);
 }
 
-// Exclusive scan of the run sums (one block), and the stage's place in the table.
-__device__ __noinline__ void phase_scan_sums(const StageArgs& a) {
-  const uint32_t n_runs = (a.hi - a.lo + kBlock - 1) / kBlock;
-  unsigned long long carry = 0;
-  for (uint32_t b0 = 0; b0 < n_runs; b0 += kBlock) {
-    const uint32_t b = b0 + threadIdx.x;
-    const unsigned long long v = b < n_runs ? a.block_sums[b] : 0ull;
-    unsigned long long total;
-    const unsigned long long ex = block_excl_scan(v, &total);
-    if (b < n_runs) a.block_sums[b] = carry + ex;
-    carry += total;
-  }
-  if (threadIdx.x == 0) {
-    FillCtl* ctl = a.ctl;
-    ctl->stage_first_row = ctl->final_top;
-    ctl->stage_rows = carry;
-    if (ctl->final_top + carry > a.row_cap) {
-      if (!ctl->error) ctl->failed_stage = a.stage;
-      ctl->error |= MRL_ERR_TABLE;
-      ctl->need_rows = ctl->final_top + carry;
-    } else {
-      ctl->final_top += carry;
-    }
-  }
+// What the phases of a stage count and hand out; zero at its start.
+__device__ __forceinline__ void reset_stage_ctl(FillCtl* ctl) {
+  ctl->rows_early = ctl->rows_late = 0;
+  ctl->n_items = 0;
+  ctl->any_changed = ctl->grew = 0;
+#pragma unroll
+  for (int k = 0; k < 8; k++) ctl->next_item[k] = 0;
 }
 
-// Copies each Spec's real cells from its working grid to its final rows and repoints the header.
-// Specs computed by another rank get zero rows (the exchange adds the owner's rows onto them).
-__device__ __noinline__ void phase_compact(const StageArgs& a) {
-  const unsigned long long first_row = a.ctl->stage_first_row;
-  for (uint32_t base = a.lo + blockIdx.x * kBlock; base < a.hi; base += gridDim.x * kBlock) {
-    const uint32_t i = base + threadIdx.x;
-    const unsigned long long n = i < a.hi ? a.fcount[i - a.lo] : 0u;
-    unsigned long long total;
-    const unsigned long long ex = block_excl_scan(n, &total);
-    if (i >= a.hi) continue;
-    const unsigned long long fbase = first_row + a.block_sums[(base - a.lo) / kBlock] + ex;
-    const uint4 fm = a.rmask[i];
-    if (computed_here(a, i)) {
-      const uint4 tm = *reinterpret_cast<const uint4*>(&a.hdrs[i]);
-      const unsigned long long tbase = a.hdrs[i].row_base & ~MRL_TEMP_FLAG;
-      const uint32_t f0 = __popc(fm.x), f1 = __popc(fm.y), f2 = __popc(fm.z);
-      const uint32_t t0 = __popc(tm.x), t1 = __popc(tm.y), t2 = __popc(tm.z);
-      for (uint32_t j = 0; j < (uint32_t)n; j++) {
-        uint32_t rest = j;
-        const uint32_t j0 = rest % f0; rest /= f0;
-        const uint32_t j1 = rest % f1; rest /= f1;
-        const uint32_t j2 = rest % f2; rest /= f2;
-        const uint32_t j3 = rest;
-        const uint32_t i0 = __popc(tm.x & below(nth_set_bit(fm.x, j0))) - 1;
-        const uint32_t i1 = __popc(tm.y & below(nth_set_bit(fm.y, j1))) - 1;
-        const uint32_t i2 = __popc(tm.z & below(nth_set_bit(fm.z, j2))) - 1;
-        const uint32_t i3 = __popc(tm.w & below(nth_set_bit(fm.w, j3))) - 1;
-        const uint32_t toff = ((i3 * t2 + i2) * t1 + i1) * t0 + i0;
-        uint4 r = *reinterpret_cast<const uint4*>(a.temp + tbase + toff);
-        r.w = 0;
-        *reinterpret_cast<uint4*>(a.rows + fbase + j) = r;
-      }
-    } else {
-      for (uint32_t j = 0; j < (uint32_t)n; j++) *reinterpret_cast<uint4*>(a.rows + fbase + j) = make_uint4(0, 0, 0, 0);
-    }
-    *reinterpret_cast<uint4*>(&a.hdrs[i]) = fm;
-    a.hdrs[i].row_base = fbase;
-  }
-}
-
-// One stage, start to finish, in one cooperative launch. Every thread of the grid reaches every
-// barrier: what decides the control flow (totals, the closure epoch, the sweep that last changed
-// a cell, the error word) is read from device memory after a barrier and written again only
-// after a later one, so all threads take the same branches.
-__global__ void __launch_bounds__(kBlock, kMinBlocks) stage_kernel(const StageArgs a) {
-  cg::grid_group grid = cg::this_grid();
-  const uint32_t gtid = blockIdx.x * kBlock + threadIdx.x;
-  const uint32_t gthreads = gridDim.x * kBlock;
+// A run of stages, each start to finish, by one team of blocks: the grid (cooperative launch), one
+// cluster, or one block. Every thread of the team reaches every barrier: what decides the control
+// flow (totals, the sweep that last changed a cell, the error word) is read from device memory after
+// a barrier and written again only after a later one, so all threads take the same branches.
+//
+// What bounds a small stage is the number of barriers: a grid-wide one takes 2 us and more, and a
+// 2x2x2 Matmul search has 86 stages of 9 Specs on average. So the team fits the stage - a cluster's
+// barrier takes a fraction of that and a block's next to nothing - and a stage makes as few as its
+// phases depend on each other: 5 without same-stage children, 10 with them and one pass.
+__global__ void __launch_bounds__(kStageBlock, 1) stage_kernel(const __grid_constant__ StageArgs a) {
+  const uint32_t gtid = blockIdx.x * kStageBlock + threadIdx.x;
+  const uint32_t gthreads = gridDim.x * kStageBlock;
+  const uint32_t gwarp = gtid >> 5, gwarps = gthreads >> 5;
   FillCtl* const ctl = a.ctl;
   uint32_t syncs = 0;
-#define GRID_SYNC() do { grid.sync(); syncs++; } while (0)
+  auto team_sync = [&]() {
+    syncs++;
+    if (a.team == TEAM_GRID) {
+      cg::this_grid().sync();
+    } else if (a.team == TEAM_CLUSTER) {
+      asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+    } else {
+      __syncthreads();
+    }
+  };
   if (ctl->error) return;   // an earlier stage failed: the host repairs and resumes (uniform: nothing writes it before the first barrier)
-  __shared__ unsigned long long block_stats[5];   // candidates evaluated and rows gathered by the unordered phase; by the sweeps; items the sweeps evaluated
+  __shared__ unsigned long long block_stats[5];   // candidates evaluated and rows gathered by the unordered phase; by the sweeps; items the sweeps solved cells of
   if (threadIdx.x < 5) block_stats[threadIdx.x] = 0;
   __syncthreads();
-  if (a.solve) {
-    if (gtid == 0) {
-      ctl->cells = ctl->warps = ctl->row_cursor = 0;
-      ctl->chunk_cursor = ctl->item_cursor = ctl->item_next = 0;
-      ctl->spread_epoch = 0;
-      ctl->temp_top = 0;
-      ctl->sweep_next[0] = ctl->sweep_next[1] = 0;
-      ctl->late_changed = 0;
-    }
-    for (uint32_t i = gtid; i < a.hi - a.lo; i += gthreads) a.stamp[i] = 0;
-    if (a.mine)
-      for (uint32_t i = a.lo + gtid; i < a.hi; i += gthreads) a.rmask[i] = make_uint4(0, 0, 0, 0);   // other ranks' Specs: zero until the exchange
-    for (uint32_t i = a.lo + gtid; i < a.hi; i += gthreads) a.dirty[i] = 0;
-    phase_minsat(a, gtid, gthreads);
-    GRID_SYNC();
-    uint32_t epoch = 0, sweep = 0, sweep_before = 0;
-    unsigned long long n_sweeps = 0, t_last = 0;
-    if (gtid == 0) asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t_last));
-    // device time since the last mark goes to part ph (thread 0 only; after a barrier)
+  unsigned long long final_top = ctl->final_top;   // rows of the table; written below behind a barrier
+  unsigned long long t_last = 0, st_cells = 0, st_early = 0;
+  uint32_t n_sweeps = 0, n_passes = 0;
+  if (gtid == 0) asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t_last));
+  // device time since the last mark goes to part ph (thread 0 only; after a barrier)
 #define MARK(ph) do { if (gtid == 0) { unsigned long long t_now; asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t_now)); \
                                        ctl->st_phase_ns[ph] += t_now - t_last; t_last = t_now; } } while (0)
+  for (uint32_t st = a.stage_lo; st < a.stage_hi; st++) {
+    const uint2 ids = __ldg(&a.stages[st]);
+    const uint32_t lo = ids.x, hi = ids.y;
     bool failed = false;
-    const uint32_t gwarps = gridDim.x * (kBlock / 32);
-    // ---- once per stage: the corners, then the candidates whose children are all finished, on grids of their own
-    phase_corner(a, gtid, gthreads, 0);
-    GRID_SYNC();
-    phase_corner(a, gtid, gthreads, 1);
-    GRID_SYNC();
-    phase_derive_early(a, gtid, gthreads);
-    GRID_SYNC();
-    phase_totals(a, gtid, gthreads, true);
-    GRID_SYNC();
-    {
-      const unsigned long long cells = ctl->cells, warps = ctl->warps;
-      // Work items: an even share of the cells per warp, in whole warp-wide steps, at most
-      // MRL_ITEM_CELLS; every Spec adds at most one partial item.
-      const uint32_t item_cells = (uint32_t)min((unsigned long long)MRL_ITEM_CELLS, max(32ull, ((cells + gwarps - 1) / gwarps + 31ull) & ~31ull));
-      const unsigned long long max_items = cells / item_cells + (a.hi - a.lo);
-      if (cells > a.temp_cap || warps > a.chunk_cap || max_items > a.item_cap || cells >= 0xFFFFFFF0ull || warps >= 0xFFFFFFF0ull) {
-        failed = true;
+    if (a.solve) {
+      uint32_t ph = 0;   // phases that hand out items take the counters in turn; one is cleared four phases ahead
+      HotArgs h;
+      h.hdrs = a.hdrs; h.cands = a.cands; h.rows = a.rows; h.temp = a.temp; h.temp_cap = a.temp_cap; h.sspec = a.sspec - lo;
+      h.items = a.items; h.item_cells = item_size(hi - lo, gwarps); h.n_items = 0; h.next_item = nullptr;
+      auto hand_out = [&](uint32_t n_items) {
+        h.n_items = n_items;
+        h.next_item = &ctl->next_item[ph & 7];
+        if (gtid == 0) ctl->next_item[(ph + 4) & 7] = 0;
+        ph++;
+      };
+      auto too_small = [&](unsigned long long rows_early, unsigned long long rows_late, unsigned long long items) {
+        if (rows_early <= a.temp_cap && rows_late <= a.temp_cap && items <= a.item_cap) return false;
         if (gtid == 0) {
-          ctl->failed_stage = a.stage;
+          ctl->failed_stage = st;
           ctl->error |= MRL_ERR_WORKING;
-          ctl->need_temp = cells;
-          ctl->need_chunks = warps;
-          ctl->need_items = max_items;
+          ctl->need_temp = max(rows_early, rows_late);
+          ctl->need_items = items;
         }
-      } else if (cells) {
-        phase_place(a, 0, item_cells, true);
-        GRID_SYNC();
+        return true;
+      };
+      if (a.mine && st) {
+        phase_minsat(a, __ldg(&a.stages[st - 1]).x, __ldg(&a.stages[st - 1]).y, gtid, gthreads);
+        team_sync();
+      }
+      phase_records(a, lo, hi, gwarp, gwarps, st);
+      team_sync();
+      const bool any_late = __ldcg(&ctl->any_late) == st + 1;
+      phase_place_early(a, lo, hi, gwarp, gwarps, any_late);
+      team_sync();
+      const unsigned long long cells = __ldcg(&ctl->rows_early);
+      const uint32_t n_early_items = __ldcg(&ctl->n_items);
+      failed = too_small(cells, 0, n_early_items);
+      if (!failed && cells) {
         MARK(MRL_PH_SETUP);
-        const uint32_t n_items = ctl->item_cursor;
-        phase_early(hot_args(a), a.items, n_items, item_cells, &ctl->item_next, block_stats);
-        GRID_SYNC();
+        hand_out(n_early_items);
+        phase_early(h, block_stats);
+        st_cells += cells;
+        st_early += cells;
+        team_sync();
         MARK(MRL_PH_EARLY);
-        phase_real_masks(a, (uint32_t)warps, true);   // into rmask: what the first pass seeds the working grids with
-        if (gtid == 0) {
-          ctl->st_cells += cells;
-          ctl->st_early_cells += cells;
-          ctl->cells = ctl->warps = ctl->row_cursor = 0;
-          ctl->chunk_cursor = ctl->item_cursor = ctl->item_next = 0;
-        }
-        GRID_SYNC();
+        if (gtid == 0) ctl->n_items = 0;   // read above, behind a barrier; used again from phase_place_late on
+        hand_out(n_early_items);
+        phase_real_masks<true>(h, a.rmask, false);
+        team_sync();
         MARK(MRL_PH_EARLY_MASKS);
-      }
-    }
-    // ---- passes: the candidates with a same-stage child, until every working grid is consistent
-    for (int pass = 0; !failed; pass++) {
-      if (pass >= kMaxPasses) { failed = true; if (gtid == 0) { ctl->failed_stage = a.stage; ctl->error |= MRL_ERR_PASSES; } break; }
-      phase_derive_late(a, gtid, gthreads, pass == 0);
-      GRID_SYNC();
-      if (pass > 0) {
-        // close the marks under "has a marked same-stage child"
-        for (;;) {
-          epoch++;
-          phase_spread(a, gtid, gthreads, epoch);
-          GRID_SYNC();
-          if (ctl->spread_epoch != epoch) break;
+        uint32_t sweep = 0;
+        unsigned long long rows_before = 0;
+        if (!any_late) phase_place_late(a, lo, hi, gwarp, gwarps, 0);   // headers only; the places of the rows need no barrier behind it
+        for (uint32_t pass = 0; any_late; pass++) {
+          if (pass >= (uint32_t)kMaxPasses) { failed = true; if (gtid == 0) { ctl->failed_stage = st; ctl->error |= MRL_ERR_PASSES; } break; }
+          phase_place_late(a, lo, hi, gwarp, gwarps, pass);
+          team_sync();
+          const unsigned long long rows = __ldcg(&ctl->rows_late);
+          const uint32_t n_items = __ldcg(&ctl->n_items);
+          if ((failed = too_small(0, rows, n_items))) break;
+          MARK(MRL_PH_PASS_SETUP);
+          if (pass) {
+            hand_out(n_items);
+            phase_refine(h);
+            team_sync();
+            MARK(MRL_PH_INIT);
+          } else {
+            for (uint32_t i = lo + gtid; i < hi; i += gthreads)   // what the unordered phase found real has been used
+              if (computed_here(a, i) && a.sspec[i - lo].n_late) a.rmask[i] = make_uint4(1u, 1u, 1u, 1u);
+          }
+          st_cells += rows - rows_before;
+          rows_before = rows;
+          const uint32_t sweep_before = sweep;
+          for (bool first = true;; first = false) {
+            sweep++;
+            uint4* const now = a.changed[sweep % 3], *const idle = a.changed[(sweep + 1) % 3];
+            const uint4* const before = a.changed[(sweep + 2) % 3];
+            if (sweep > 1)   // the first sweeps' are zero from phase_place_late
+              for (uint32_t i = gtid; i < hi - lo; i += gthreads) idle[i] = make_uint4(0, 0, 0, 0);
+            hand_out(n_items);
+            if (!first) phase_sweep<SWEEP_CHANGED>(h, lo, before, now, sweep, &ctl->any_changed, block_stats);
+            else if (pass) phase_sweep<SWEEP_NEW>(h, lo, before, now, sweep, &ctl->any_changed, block_stats);
+            else phase_sweep<SWEEP_ALL>(h, lo, before, now, sweep, &ctl->any_changed, block_stats);
+            team_sync();
+            MARK(first ? MRL_PH_SWEEP_FIRST : MRL_PH_SWEEP_MORE);
+            if (__ldcg(&ctl->any_changed) != sweep) break;   // nothing changed anywhere: the stage's cells are consistent
+            if (sweep - sweep_before >= (uint32_t)kMaxSweeps) {   // more sweeps than the limits lattice has diagonals: give up rather than spin
+              failed = true;
+              if (gtid == 0) { ctl->failed_stage = st; ctl->error |= MRL_ERR_PASSES; }
+              break;
+            }
+          }
+          if (failed) break;
+          n_sweeps += sweep - sweep_before;
+          n_passes++;
+          if (pass) {
+            for (uint32_t i = lo + gtid; i < hi; i += gthreads)
+              if (computed_here(a, i) && a.sspec[i - lo].n_late && a.sspec[i - lo].dirty) a.rmask[i] = make_uint4(1u, 1u, 1u, 1u);
+            team_sync();
+          }
+          if (gtid == 0) ctl->n_items = 0;
+          hand_out(n_items);
+          phase_real_masks<false>(h, a.rmask, pass != 0);
+          team_sync();
+          phase_check_grids(a, lo, hi, gwarp, gwarps, pass);
+          if (a.place) phase_count(a, lo, hi);   // for when no grid grows
+          team_sync();
+          MARK(MRL_PH_PASS_MASKS);
+          if (__ldcg(&ctl->grew) != pass + 1) break;   // every working grid is consistent
+        }
+        if (!any_late && !failed) {
+          if (a.place) phase_count(a, lo, hi);
+          team_sync();
         }
       }
-      phase_totals(a, gtid, gthreads, false);
-      GRID_SYNC();
-      const unsigned long long cells = ctl->cells, warps = ctl->warps, temp_top = ctl->temp_top;
-      const uint32_t item_cells = (uint32_t)min((unsigned long long)MRL_ITEM_CELLS, max(32ull, ((cells + gwarps - 1) / gwarps + 31ull) & ~31ull));
-      const unsigned long long max_items = cells / item_cells + (a.hi - a.lo);
-      if (cells == 0) break;   // nothing left to solve: every working grid is consistent
-      if (temp_top + cells > a.temp_cap || warps > a.chunk_cap || max_items > a.item_cap ||
-          cells >= 0xFFFFFFF0ull || warps >= 0xFFFFFFF0ull) {
+    } else {
+      phase_count(a, lo, hi);
+      team_sync();
+    }
+    if (!failed && a.place) {
+      unsigned long long before = 0, total = 0;
+      for (uint32_t b = threadIdx.x; b < gridDim.x; b += kStageBlock) {
+        const unsigned long long v = __ldcg(&a.block_sums[b]);
+        total += v;
+        if (b < blockIdx.x) before += v;
+      }
+      before = block_sum(before);
+      total = block_sum(total);
+      if (final_top + total > a.row_cap) {   // uniform
         failed = true;
         if (gtid == 0) {
-          ctl->failed_stage = a.stage;
-          ctl->error |= MRL_ERR_WORKING;
-          ctl->need_temp = temp_top + cells;
-          ctl->need_chunks = warps;
-          ctl->need_items = max_items;
+          ctl->failed_stage = st;
+          ctl->error |= MRL_ERR_TABLE;
+          ctl->need_rows = final_top + total;
         }
-        break;
-      }
-      phase_place(a, temp_top, item_cells, false);
-      GRID_SYNC();
-      MARK(MRL_PH_PASS_SETUP);
-      const uint32_t n_chunks = (uint32_t)warps;
-      const uint32_t n_items = ctl->item_cursor;
-      phase_late_init(hot_args(a), a.items, n_items, item_cells, &ctl->item_next);
-      GRID_SYNC();
-      MARK(MRL_PH_INIT);
-      for (bool first_sweep = true;; first_sweep = false) {
-        sweep++;
-        if (gtid == 0) ctl->sweep_next[(sweep + 1) & 1] = 0;   // the other counter is idle during this sweep
-        phase_late(hot_args(a), a.items, n_items, item_cells, &ctl->sweep_next[sweep & 1], a.lo, a.stamp, sweep, first_sweep,
-                   &ctl->late_changed, block_stats);
-        GRID_SYNC();
-        MARK(first_sweep ? MRL_PH_SWEEP_FIRST : MRL_PH_SWEEP_MORE);
-        if (ctl->late_changed != sweep) break;   // nothing changed anywhere: the stage's cells are consistent
-        if (sweep - sweep_before >= (uint32_t)kMaxSweeps) {   // more sweeps than the limits lattice has diagonals: give up rather than spin
-          failed = true;
-          if (gtid == 0) { ctl->failed_stage = a.stage; ctl->error |= MRL_ERR_PASSES; }
-          break;
+      } else {
+        phase_compact(a, lo, hi, final_top + before);
+        if (gtid == 0) {
+          ctl->stage_first_row = final_top;
+          ctl->stage_rows = total;
+          reset_stage_ctl(ctl);
         }
+        final_top += total;
+        if (gtid == 0) ctl->final_top = final_top;
+        if (st + 1 < a.stage_hi) team_sync();
       }
-      if (failed) break;
-      n_sweeps += sweep - sweep_before;
-      sweep_before = sweep;
-      phase_real_masks(a, n_chunks, false);
-      for (uint32_t i = a.lo + gtid; i < a.hi; i += gthreads)
-        if (a.dirty[i] == 2) a.dirty[i] = 0;
-      if (gtid == 0) {
-        ctl->temp_top = temp_top + cells;
-        ctl->st_cells += cells;
-        ctl->st_passes += 1;
-        ctl->cells = ctl->warps = ctl->row_cursor = 0;
-        ctl->chunk_cursor = ctl->item_cursor = ctl->item_next = 0;
-      }
-      GRID_SYNC();
-      MARK(MRL_PH_PASS_MASKS);
     }
-    MARK(MRL_PH_PASS_SETUP);   // of a pass that found nothing left to solve
+    if (failed) break;   // uniform
+  }
 #undef MARK
-    __syncthreads();
-    if (threadIdx.x == 0 && (block_stats[0] | block_stats[1] | block_stats[2] | block_stats[4])) {
-      atomicAdd(&ctl->st_cands, block_stats[0] + block_stats[2]);
-      atomicAdd(&ctl->st_lookups, block_stats[1] + block_stats[3]);
-      atomicAdd(&ctl->st_late_cands, block_stats[2]);
-      atomicAdd(&ctl->st_late_items, block_stats[4]);
-    }
-    if (gtid == 0) ctl->st_sweeps += n_sweeps;
-    if (failed) {
-      if (gtid == 0) ctl->st_syncs += syncs;
-      return;   // uniform
-    }
+  __syncthreads();
+  if (threadIdx.x == 0 && (block_stats[0] | block_stats[1] | block_stats[2] | block_stats[4])) {
+    atomicAdd(&ctl->st_cands, block_stats[0] + block_stats[2]);
+    atomicAdd(&ctl->st_lookups, block_stats[1] + block_stats[3]);
+    atomicAdd(&ctl->st_late_cands, block_stats[2]);
+    atomicAdd(&ctl->st_late_items, block_stats[4]);
   }
-  if (a.place) {
-    phase_final_count(a);
-    GRID_SYNC();
-    if (blockIdx.x == 0) phase_scan_sums(a);
-    GRID_SYNC();
-    if (!(ctl->error & MRL_ERR_TABLE)) phase_compact(a);   // uniform: set by phase_scan_sums only
+  if (gtid == 0) {
+    ctl->st_sweeps += n_sweeps;
+    ctl->st_passes += n_passes;
+    ctl->st_cells += st_cells;
+    ctl->st_early_cells += st_early;
+    ctl->st_syncs += syncs;
   }
-  if (gtid == 0) ctl->st_syncs += syncs;
-#undef GRID_SYNC
 }
 
 // Consistency check of a finished table: at sampled (or all) points of the limits lattice, for
@@ -1582,6 +1700,8 @@ namespace mrl {
     }                                                                                      \
   } while (0)
 
+constexpr size_t kStageSmem = (kStageBlock / 32) * sizeof(WarpScratch);
+
 static size_t align256(size_t x) { return (x + 255) & ~size_t(255); }
 
 struct DeviceFill::DevTables {
@@ -1658,7 +1778,7 @@ int DeviceFill::reserve_host_(size_t bytes) {
 
 void DeviceFill::release() {
   wait_upload();
-  for (DevBuf* b : {&b_ctl_, &b_hdrs_, &b_cands_, &b_spec_, &b_stage_specs_, &b_mine_, &b_chunks_, &b_items_, &b_temp_, &b_rows_,
+  for (DevBuf* b : {&b_ctl_, &b_hdrs_, &b_cands_, &b_spec_, &b_stage_specs_, &b_mine_, &b_stages_, &b_items_, &b_temp_, &b_rows_,
                     &b_lookup_, &b_tables_, &b_bits_, &b_rank_, &b_desc_, &b_stage_lo_})
     drop_(*b);
   tab_.reset();
@@ -1694,7 +1814,8 @@ int DeviceFill::init_events() {
   CK(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device_));
   CK(cudaDeviceGetAttribute(&n_sm_, cudaDevAttrMultiProcessorCount, device_));
   if (!coop) { snprintf(err_, sizeof(err_), "the device does not support cooperative launches"); return -1; }
-  CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, stage_kernel, kBlock, 0));
+  CK(cudaFuncSetAttribute(stage_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kStageSmem));
+  CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, stage_kernel, kStageBlock, kStageSmem));
   if (per_sm < 1) { snprintf(err_, sizeof(err_), "the stage kernel does not fit an SM"); return -1; }
   coop_blocks_ = per_sm * n_sm_;
   plan_blocks_ = plan_kernel_blocks_per_sm();
@@ -1745,7 +1866,7 @@ int DeviceFill::wait_upload() { return wait_cands_(~uint64_t(0) >> 1); }
 void DeviceFill::begin_plan_() {
   wait_upload();   // of an earlier plan
   if (fixed_) {    // carved afresh by every plan
-    for (DevBuf* b : {&b_ctl_, &b_hdrs_, &b_cands_, &b_spec_, &b_stage_specs_, &b_mine_, &b_chunks_, &b_items_, &b_temp_, &b_rows_,
+    for (DevBuf* b : {&b_ctl_, &b_hdrs_, &b_cands_, &b_spec_, &b_stage_specs_, &b_mine_, &b_stages_, &b_items_, &b_temp_, &b_rows_,
                       &b_lookup_, &b_tables_, &b_bits_, &b_rank_, &b_desc_, &b_stage_lo_})
       drop_(*b);
     buf_off_ = 0;
@@ -1764,39 +1885,39 @@ int DeviceFill::working_buffers_(bool with_mine, uint32_t world) {
   max_stage_ = 1;
   for (const StageIds& st : stages_) max_stage_ = std::max(max_stage_, st.hi - st.lo);
   const size_t n = std::max<uint32_t>(n_specs_, 1), ms = max_stage_;
-  // per Spec: real-breakpoint masks, corner, marks; per Spec of a stage: grid of the unordered phase, corner, stamp, final cells
-  const size_t o_minsat = align256(n * sizeof(uint4)), o_dirty = o_minsat + align256(n * sizeof(uint32_t));
-  if ((rc = reserve_(b_spec_, o_dirty + align256(n)))) return rc;
+  // per Spec: real-breakpoint masks, corner; per Spec of a stage: what the stage kernel keeps, and three
+  // sweeps' changes
+  const size_t o_minsat = align256(n * sizeof(uint4));
+  if ((rc = reserve_(b_spec_, o_minsat + n * sizeof(uint32_t)))) return rc;
   unsigned char* p = static_cast<unsigned char*>(b_spec_.p);
   d_rmask_ = reinterpret_cast<uint4*>(p);
   d_minsat_ = reinterpret_cast<uint32_t*>(p + o_minsat);
-  d_dirty_ = p + o_dirty;
-  const size_t o_corner = align256(ms * sizeof(SpecHdr)), o_stamp = o_corner + align256(ms * sizeof(uint32_t)),
-               o_fcount = o_stamp + align256(ms * sizeof(uint32_t)), o_sums = o_fcount + align256(ms * sizeof(uint32_t));
-  if ((rc = reserve_(b_stage_specs_, o_sums + (ms / kBlock + 1) * sizeof(unsigned long long)))) return rc;
+  const size_t o_changed = align256(ms * sizeof(StageSpec)), o_sums = o_changed + 3 * align256(ms * sizeof(uint4));
+  if ((rc = reserve_(b_stage_specs_, o_sums + (size_t)coop_blocks_ * sizeof(unsigned long long)))) return rc;
   p = static_cast<unsigned char*>(b_stage_specs_.p);
-  d_ehdr_ = reinterpret_cast<SpecHdr*>(p);
-  d_corner_ = reinterpret_cast<uint32_t*>(p + o_corner);
-  d_stamp_ = reinterpret_cast<uint32_t*>(p + o_stamp);
-  d_fcount_ = reinterpret_cast<uint32_t*>(p + o_fcount);
+  d_sspec_ = p;
+  for (int k = 0; k < 3; k++) d_changed_[k] = reinterpret_cast<uint4*>(p + o_changed + k * align256(ms * sizeof(uint4)));
   d_block_sums_ = reinterpret_cast<unsigned long long*>(p + o_sums);
+  std::vector<uint2> ids(stages_.size());
+  for (size_t k = 0; k < ids.size(); k++) ids[k] = make_uint2(stages_[k].lo, stages_[k].hi);
+  if ((rc = reserve_(b_stages_, ids.size() * sizeof(uint2)))) return rc;
+  if (!ids.empty()) CK(cudaMemcpyAsync(b_stages_.p, ids.data(), ids.size() * sizeof(uint2), cudaMemcpyHostToDevice, stream_));
   d_mine_ = nullptr;
   if (with_mine) {
     if ((rc = reserve_(b_mine_, n))) return rc;
     d_mine_ = static_cast<uint8_t*>(b_mine_.p);
   }
   if (fixed_) {
-    // Everything left is split once: lookup staging, chunks, work items, working rows and final rows.
+    // Everything left is split once: lookup staging, work items, working rows and final rows.
     if ((rc = reserve_(b_lookup_, 64 << 10))) return rc;
     const size_t left = buf_bytes_ > align256(buf_off_) + 2048 ? buf_bytes_ - align256(buf_off_) - 2048 : 0;
     // per working cell: two rows of 16 bytes (the cell and what the unordered phase found for it),
-    // under 1 byte of chunks and work items; the rest is the table
-    chunk_cap_ = left / 64 / sizeof(Chunk);
+    // under 1 byte of work items; the rest is the table
     item_cap_ = left / 64 / sizeof(WorkItem);
     temp_cap_ = left * 10 / 32 / (2 * sizeof(MrlRow));
-    row_cap_ = (left - 2 * (left / 64) - left * 10 / 32) / sizeof(MrlRow);
+    row_cap_ = (left - left / 64 - left * 10 / 32) / sizeof(MrlRow);
     if (item_cap_ < temp_cap_ / 32 + max_stage_ + 1) return too_large_();
-    if (chunk_cap_ == 0 || row_cap_ == 0) return too_large_();
+    if (row_cap_ == 0) return too_large_();
     h_ctl_ = &ctl_pageable_;
   } else {
     // Starting sizes from what fills of this kind ended with (about 45 table rows per Spec; 1000
@@ -1817,19 +1938,14 @@ int DeviceFill::working_buffers_(bool with_mine, uint32_t world) {
     if ((rc = reserve_(b_temp_, temp * 2 * sizeof(MrlRow))) || (rc = reserve_(b_rows_, rows * sizeof(MrlRow)))) return rc;
     temp_cap_ = b_temp_.cap / (2 * sizeof(MrlRow));
     row_cap_ = b_rows_.cap / sizeof(MrlRow);
-    chunk_cap_ = std::max<uint64_t>(1u << 16, stage_part * 32);
     item_cap_ = temp_cap_ / 32 + max_stage_ + 1;   // a work item holds at least 32 cells, and every Spec at most one partial item
     if (!h_ctl_) CK(cudaHostAlloc((void**)&h_ctl_, sizeof(FillCtl), cudaHostAllocDefault));
   }
-  if ((rc = reserve_(b_chunks_, chunk_cap_ * sizeof(Chunk)))) return rc;
   if ((rc = reserve_(b_items_, item_cap_ * sizeof(WorkItem)))) return rc;
   if (fixed_) {
     if ((rc = reserve_(b_temp_, temp_cap_ * 2 * sizeof(MrlRow)))) return rc;   // the cells, then what the unordered phase found for them
     if ((rc = reserve_(b_rows_, row_cap_ * sizeof(MrlRow)))) return rc;
-  } else {
-    chunk_cap_ = b_chunks_.cap / sizeof(Chunk);
   }
-  d_chunks_ = static_cast<Chunk*>(b_chunks_.p);
   d_items_ = static_cast<WorkItem*>(b_items_.p);
   d_temp_ = static_cast<MrlRow*>(b_temp_.p);
   d_rows_ = static_cast<MrlRow*>(b_rows_.p);
@@ -2062,7 +2178,7 @@ int DeviceFill::cands_arrived() {
   }
   if (read_ctl_() != 0) return -1;
   if (h_ctl_->error) {
-    CK(cudaMemsetAsync(&d_ctl_->error, 0, sizeof(uint32_t), stream_));
+    CK(cudaMemsetAsync(d_ctl_, 0, offsetof(FillCtl, failed_stage), stream_));   // the error, and what its stage had counted
     snprintf(err_, sizeof(err_), "the candidate records on the device do not describe this plan (a field is out of range)");
     return -2;
   }
@@ -2087,13 +2203,11 @@ int DeviceFill::grow_after_error_(uint32_t bits) {
   };
   int rc = 0;
   if (bits & MRL_ERR_WORKING) {
-    if ((rc = regrow(b_temp_, h_ctl_->need_temp, 2 * sizeof(MrlRow))) == 0 && (rc = regrow(b_chunks_, h_ctl_->need_chunks, sizeof(Chunk))) == 0)
+    if ((rc = regrow(b_temp_, h_ctl_->need_temp, 2 * sizeof(MrlRow))) == 0)
       rc = regrow(b_items_, h_ctl_->need_items, sizeof(WorkItem));
     temp_cap_ = b_temp_.cap / (2 * sizeof(MrlRow));
-    chunk_cap_ = b_chunks_.cap / sizeof(Chunk);
     item_cap_ = b_items_.cap / sizeof(WorkItem);
     d_temp_ = static_cast<MrlRow*>(b_temp_.p);
-    d_chunks_ = static_cast<Chunk*>(b_chunks_.p);
     d_items_ = static_cast<WorkItem*>(b_items_.p);
     if (rc) return rc;
   }
@@ -2132,52 +2246,69 @@ int DeviceFill::begin_fill() {
   return 0;
 }
 
-void DeviceFill::stage_args_(void* args, uint32_t si) const {
-  StageArgs& a = *static_cast<StageArgs*>(args);
-  const StageIds& st = stages_[si];
-  a.hdrs = d_hdrs_; a.cands = d_cands_; a.rmask = d_rmask_; a.mine = d_mine_; a.dirty = d_dirty_;
-  a.chunks = d_chunks_; a.items = d_items_; a.rows = d_rows_; a.temp = d_temp_; a.base = d_temp_ + temp_cap_; a.ehdr = d_ehdr_;
-  a.fcount = d_fcount_; a.block_sums = d_block_sums_; a.minsat = d_minsat_; a.corner = d_corner_; a.stamp = d_stamp_; a.ctl = d_ctl_;
-  a.lo = st.lo; a.hi = st.hi; a.top_pack = top_pack_; a.stage = si;
-  a.prev_lo = si ? stages_[si - 1].lo : 0; a.prev_hi = si ? stages_[si - 1].hi : 0;
-  a.temp_cap = temp_cap_; a.chunk_cap = chunk_cap_; a.item_cap = item_cap_; a.row_cap = row_cap_;
+// One launch of the stage kernel for the stages [from, to), by a team that fits them (see the
+// thresholds in run).
+int DeviceFill::launch_stages_(uint32_t from, uint32_t to, int team, int blocks, bool solve, bool place) {
+  StageArgs a;
+  a.hdrs = d_hdrs_; a.cands = d_cands_; a.rmask = d_rmask_; a.mine = d_mine_; a.items = d_items_; a.rows = d_rows_; a.temp = d_temp_;
+  a.minsat = d_minsat_; a.sspec = static_cast<StageSpec*>(d_sspec_);
+  for (int k = 0; k < 3; k++) a.changed[k] = d_changed_[k];
+  a.block_sums = d_block_sums_; a.ctl = d_ctl_; a.stages = static_cast<const uint2*>(b_stages_.p);
+  a.stage_lo = from; a.stage_hi = to; a.top_pack = top_pack_; a.team = team;
+  a.temp_cap = temp_cap_; a.item_cap = item_cap_; a.row_cap = row_cap_;
+  a.solve = solve ? 1 : 0;
+  a.place = place ? 1 : 0;
+  cudaLaunchConfig_t cfg;
+  memset(&cfg, 0, sizeof(cfg));
+  cfg.gridDim = dim3(blocks);
+  cfg.blockDim = dim3(kStageBlock);
+  cfg.dynamicSmemBytes = kStageSmem;
+  cfg.stream = stream_;
+  cudaLaunchAttribute attr[1];
+  if (team == TEAM_GRID) {
+    attr[0].id = cudaLaunchAttributeCooperative;
+    attr[0].val.cooperative = 1;
+  } else {
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = blocks;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  }
+  cfg.attrs = attr;
+  cfg.numAttrs = team == TEAM_BLOCK ? 0 : 1;
+  CK(cudaLaunchKernelEx(&cfg, stage_kernel, a));
+  stats_.launches++;
+  return 0;
+}
+
+// The team for a stage of n Specs. A grid-wide barrier takes 2 us and a stage has 5 to 20 of them, a
+// cluster's a fraction of that, a block's less still; a Spec is 100 to 600 cells of some 30 records.
+// Measured over fills of 60 to 640 k Specs: a block up to 24 Specs, a cluster of 8 up to 256 (an 8x8x8
+// Matmul fill takes 81 ms with the cluster's limit at 256, 124 ms at 1024; a 2x2x2 one 6.4 ms with the grid
+// for every stage, 2.5 ms so).
+void DeviceFill::team_for_(uint32_t n, int* team, int* blocks) const {
+  if (n <= 24) { *team = TEAM_BLOCK; *blocks = 1; }
+  else if (n <= 256) { *team = TEAM_CLUSTER; *blocks = 8; }
+  else { *team = TEAM_GRID; *blocks = coop_blocks_; }
 }
 
 int DeviceFill::launch_solve_(uint32_t si, bool place_too) {
   const StageIds& st = stages_[si];
-  const uint32_t n = st.hi - st.lo;
-  if (n == 0) return 0;
+  if (st.hi == st.lo) return 0;
   // the stage reads its own Specs' candidate records (ids, and with them the records, are in
   // stage order): wait for that much of a background upload
   int rc = wait_cands_(st.cand_end * sizeof(CandRec));
   if (rc) return rc;
-  StageArgs a;
-  stage_args_(&a, si);
-  a.solve = 1;
-  a.place = place_too ? 1 : 0;
-  // Small stages run on fewer blocks: a grid-wide barrier costs less, and there is no work for more.
-  const uint64_t want = ((uint64_t)n * 24 + kBlock - 1) / kBlock;
-  const int blocks = (int)std::min<uint64_t>((uint64_t)coop_blocks_, std::max<uint64_t>((uint64_t)n_sm_, want));
-  void* args[] = {&a};
-  CK(cudaLaunchCooperativeKernel((const void*)stage_kernel, dim3(blocks), dim3(kBlock), args, 0, stream_));
-  stats_.launches++;
-  return 0;
+  int team, blocks;
+  team_for_(st.hi - st.lo, &team, &blocks);
+  return launch_stages_(si, si + 1, team, blocks, true, place_too);
 }
 
 int DeviceFill::launch_place_(uint32_t si) {
   const StageIds& st = stages_[si];
-  const uint32_t n = st.hi - st.lo;
-  if (n == 0) return 0;
-  StageArgs a;
-  stage_args_(&a, si);
-  a.solve = 0;
-  a.place = 1;
-  const uint64_t want = ((uint64_t)n + kBlock - 1) / kBlock;
-  const int blocks = (int)std::min<uint64_t>((uint64_t)coop_blocks_, std::max<uint64_t>(1, want));
-  void* args[] = {&a};
-  CK(cudaLaunchCooperativeKernel((const void*)stage_kernel, dim3(blocks), dim3(kBlock), args, 0, stream_));
-  stats_.launches++;
-  return 0;
+  if (st.hi == st.lo) return 0;
+  int team, blocks;
+  team_for_(st.hi - st.lo, &team, &blocks);
+  return launch_stages_(si, si + 1, team, blocks, false, true);
 }
 
 int DeviceFill::solve_stage(uint32_t si) {
@@ -2206,7 +2337,7 @@ int DeviceFill::stage_masks(uint32_t si, void** ptr, uint64_t* bytes) {
         return -2;
       }
       if ((rc = grow_after_error_(MRL_ERR_WORKING))) return rc;
-      CK(cudaMemsetAsync(&d_ctl_->error, 0, sizeof(uint32_t), stream_));
+      CK(cudaMemsetAsync(d_ctl_, 0, offsetof(FillCtl, failed_stage), stream_));   // the error, and what its stage had counted
       if ((rc = launch_solve_(si, false))) return rc;
       if (read_ctl_() != 0) return -1;
       if (h_ctl_->error) {
@@ -2246,7 +2377,7 @@ int DeviceFill::place_stage(uint32_t si, void** rows_ptr, uint64_t* bytes) {
       return -2;
     }
     if ((rc = grow_after_error_(bits))) return rc;
-    CK(cudaMemsetAsync(&d_ctl_->error, 0, sizeof(uint32_t), stream_));
+    CK(cudaMemsetAsync(d_ctl_, 0, offsetof(FillCtl, failed_stage), stream_));   // the error, and what its stage had counted
     if ((rc = launch_place_(si))) return rc;
     if (read_ctl_() != 0) return -1;
     if (h_ctl_->error) { snprintf(err_, sizeof(err_), "stage %u failed again after its buffers were enlarged (0x%x)", si, h_ctl_->error); return -2; }
@@ -2295,9 +2426,20 @@ int DeviceFill::run() {
   int rc;
   if ((rc = begin_fill())) return rc;
   uint32_t from = 0;
+  int team_max, blocks_max;
+  team_for_(max_stage_, &team_max, &blocks_max);
+  const bool one_launch = team_max != TEAM_GRID && !stages_.empty();
   for (int attempt = 0;; attempt++) {
-    for (uint32_t s = from; s < stages_.size(); s++)
-      if ((rc = launch_solve_(s, true))) return rc;
+    // A plan whose stages are all small runs as one launch; otherwise every stage has its own, with
+    // the team that fits it.
+    if (one_launch) {
+      int team, blocks;
+      team_for_(max_stage_, &team, &blocks);
+      if ((rc = wait_upload()) || (rc = launch_stages_(from, (uint32_t)stages_.size(), team, blocks, true, true))) return rc;
+    } else {
+      for (uint32_t s = from; s < stages_.size(); s++)
+        if ((rc = launch_solve_(s, true))) return rc;
+    }
     CK(cudaEventRecord(ev1_, stream_));
     if (read_ctl_() != 0) return -1;
     const uint32_t bits = h_ctl_->error;
@@ -2310,7 +2452,7 @@ int DeviceFill::run() {
     }
     from = h_ctl_->failed_stage;
     if ((rc = grow_after_error_(bits))) { filling_ = false; return rc; }
-    CK(cudaMemsetAsync(&d_ctl_->error, 0, sizeof(uint32_t), stream_));
+    CK(cudaMemsetAsync(d_ctl_, 0, offsetof(FillCtl, failed_stage), stream_));   // the error, and what its stage had counted
   }
   filling_ = false;
   CK(cudaEventElapsedTime(&stats_.fill_ms, ev0_, ev1_));

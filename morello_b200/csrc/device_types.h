@@ -52,22 +52,29 @@ struct CandRec {
   uint32_t pad1;
 };
 
-// A warp-sized slice of one Spec's "columns": cells with the slot of one memory (the Spec's
-// free memory F, the one with the most slots) left open; the column index runs over the other
-// three memories, lowest first. col_start = first column | F << 30.
-struct Chunk {
-  uint32_t spec;
-  uint32_t col_start;
-};
-
 // A piece of one Spec's grid for a solve phase: consecutive cells from
-// first_cell on, at most MRL_ITEM_CELLS of them (a pass picks the size). Warps take items as they
-// finish others.
+// first_cell on, at most MRL_ITEM_CELLS of them (the stage kernel picks the size, a multiple of 32;
+// bit 0 of first_cell: the grid is new in this pass). Warps take items as they finish others.
 #define MRL_ITEM_CELLS 1024u
 struct WorkItem {
   uint32_t spec;
   uint32_t first_cell;
 };
+
+// What the stage kernel keeps per Spec of the stage being solved.
+#ifdef __CUDACC__
+struct __align__(16) StageSpec {
+  uint4 emask;         // grid of the unordered phase
+  uint4 old_mask;      // working grid before it last grew, and its rows
+  unsigned long long erow;      // first row of the grid of the unordered phase
+  unsigned long long old_row;
+  uint32_t corner;     // where its grids are clipped
+  uint32_t n_late;     // records with a same-stage child
+  uint32_t dirty;      // its working grid grew or changed in this pass
+  uint32_t pad;
+};
+#endif
+#define MRL_STAGE_SPEC_BYTES 64u
 
 // Error bits a fill kernel can raise (sticky until the host clears them).
 enum {
@@ -93,23 +100,18 @@ enum {
 // here and leave the host nothing to decide between launches; the host reads it once per fill
 // (once per stage when the fill is sharded).
 struct FillCtl {
-  // -- one solve pass (zeroed by the kernel before every pass)
-  unsigned long long cells;          // working cells of the Specs solved in this pass
-  unsigned long long warps;          // chunks those cells need
-  unsigned long long row_cursor;     // placement cursors of the pass
-  uint32_t chunk_cursor;
-  uint32_t item_cursor;
-  uint32_t item_next;                // next work item to hand out
-  uint32_t spread_epoch;             // closure of the re-solve marks: last round that marked a Spec
-  uint32_t sweep_next[2];            // work hand-out of the relaxation sweeps, alternating
-  uint32_t late_changed;             // last relaxation sweep that improved a cell
-  uint32_t pad0;
-  // -- one stage
-  unsigned long long temp_top;       // working rows handed out so far in this stage
+  // -- one stage (zero at its start)
+  unsigned long long rows_early;     // rows handed out to the grids of the unordered phase
+  unsigned long long rows_late;      // working rows handed out
+  uint32_t n_items;                  // work items listed
+  uint32_t any_late;                 // stage + 1 when some Spec of it has a record with a same-stage child
+  uint32_t any_changed;              // last relaxation sweep that changed a cell
+  uint32_t grew;                     // pass + 1 when a grid has to grow after it
+  uint32_t next_item[8];             // item hand-out of a phase; the phases take turns
   // -- sticky over a fill
   uint32_t error;                    // MRL_ERR_* bits
   uint32_t failed_stage;             // first stage that raised one
-  unsigned long long need_temp, need_chunks, need_items, need_rows;   // what it would have taken
+  unsigned long long need_temp, need_items, need_rows;   // what it would have taken
   unsigned long long final_top;      // rows of the finished table
   unsigned long long stage_first_row, stage_rows;   // the last placed stage's slice of the table
   // -- statistics of a fill

@@ -73,7 +73,7 @@ class DeviceFill {
   // After the caller has written device_cands(): checks every record on the device (child ids
   // inside the plan, kinds and levels in range) and lets fills run.
   int cands_arrived();
-  // Runs every stage: two launches per stage, no host synchronisation before the end.
+  // Runs every stage: at most one launch per stage, no host synchronisation before the end.
   int run();
   // The same one stage at a time, for callers that exchange tables between stages (multi-GPU):
   // begin_fill; per stage solve_stage, [exchange stage_masks], place_stage, [exchange rows];
@@ -115,7 +115,8 @@ class DeviceFill {
   int alloc_(void** p, size_t bytes);
   void begin_plan_();
   int working_buffers_(bool sharded_mine, uint32_t world);
-  void stage_args_(void* args, uint32_t stage) const;
+  int launch_stages_(uint32_t from, uint32_t to, int team, int blocks, bool solve, bool place);
+  void team_for_(uint32_t n_specs, int* team, int* blocks) const;
   int launch_solve_(uint32_t stage, bool place_too);
   int launch_place_(uint32_t stage);
   int read_ctl_();                       // device control block -> h_ctl_ (synchronises the stream)
@@ -129,22 +130,18 @@ class DeviceFill {
   unsigned char* buf_ = nullptr;  // attached buffer
   size_t buf_bytes_ = 0, buf_off_ = 0;
   // buffers, and what lies in them
-  DevBuf b_ctl_, b_hdrs_, b_cands_, b_spec_, b_stage_specs_, b_mine_, b_chunks_, b_items_, b_temp_, b_rows_, b_lookup_;
+  DevBuf b_ctl_, b_hdrs_, b_cands_, b_spec_, b_stage_specs_, b_mine_, b_stages_, b_items_, b_temp_, b_rows_, b_lookup_;
   DevBuf b_tables_, b_bits_, b_rank_, b_desc_, b_stage_lo_;   // of planning on the device
   SpecHdr* d_hdrs_ = nullptr;
   CandRec* d_cands_ = nullptr;
   uint4* d_rmask_ = nullptr;
   uint8_t* d_mine_ = nullptr;
-  uint8_t* d_dirty_ = nullptr;   // by Spec id: to be solved (again) in the coming pass
   uint32_t* d_minsat_ = nullptr; // by Spec id: lower corner of the satisfiable region
-  SpecHdr* d_ehdr_ = nullptr;    // by position in the stage being solved: the Spec's grid of the unordered phase
-  uint32_t* d_stamp_ = nullptr;  // by position in the stage being solved: last relaxation sweep that improved the Spec
-  uint32_t* d_corner_ = nullptr; // by position in the stage being solved: where its working grids are clipped
-  Chunk* d_chunks_ = nullptr;
+  void* d_sspec_ = nullptr;      // by position in the stage being solved: StageSpec
+  uint4* d_changed_[3] = {};     // by position in the stage being solved: what a relaxation sweep changed
   WorkItem* d_items_ = nullptr;  // pieces of grids, handed out to warps by the solve phases
   MrlRow* d_rows_ = nullptr;     // the table
   MrlRow* d_temp_ = nullptr;     // working grids of the stage being solved (temp_cap_ rows), then as many rows for the grids of the unordered phase
-  uint32_t* d_fcount_ = nullptr;
   unsigned long long* d_block_sums_ = nullptr;
   FillCtl* d_ctl_ = nullptr;
   std::vector<StageIds> stages_;
@@ -162,7 +159,7 @@ class DeviceFill {
   FillCtl* h_ctl_ = nullptr;     // pinned, or &ctl_pageable_ when nothing may be allocated
   FillCtl ctl_pageable_;
   uint32_t n_specs_ = 0, max_stage_ = 1;
-  uint64_t row_cap_ = 0, temp_cap_ = 0, chunk_cap_ = 0, item_cap_ = 0;
+  uint64_t row_cap_ = 0, temp_cap_ = 0, item_cap_ = 0;
   uint64_t h2d_bytes_ = 0;
   uint64_t n_cand_bytes_ = 0;
   bool cands_present_ = false;   // the device candidate records are complete and checked
