@@ -1,8 +1,10 @@
 """ctypes binding of the C ABI declared in include/morello_b200.h."""
 import ctypes as C
+import importlib.machinery
+import importlib.util
 import os
 
-from .build import LIB_PATH
+from .build import LIB_PATH, PYHOST_PATH
 
 
 class Decision(C.Structure):
@@ -87,6 +89,20 @@ EXPORTS = {
 }
 
 _lib = None
+_pyhost = None
+
+
+def pyhost():
+    """The compiled helper of the query calls (csrc/pyhost.cpp); like the library, it has to be built."""
+    global _pyhost
+    if _pyhost is None:
+        if not os.path.exists(PYHOST_PATH):
+            raise RuntimeError(f"{PYHOST_PATH} is missing: build the extension first (python -c 'import __graft_entry__ as g; g.build()')")
+        loader = importlib.machinery.ExtensionFileLoader("_pyhost", PYHOST_PATH)
+        spec = importlib.util.spec_from_file_location("_pyhost", PYHOST_PATH, loader=loader)
+        _pyhost = importlib.util.module_from_spec(spec)
+        loader.exec_module(_pyhost)
+    return _pyhost
 
 
 def load():

@@ -2,12 +2,15 @@
 import os
 import shutil
 import subprocess
+import sysconfig
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB_DIR = os.path.join(HERE, "_lib")
 LIB_PATH = os.path.join(LIB_DIR, "libmorello_b200.so")
 SOURCES = ["combine.cu", "devplan.cu", "plan.cpp", "optable.cpp", "capi.cpp"]
+# the Python mirror's query calls (CPython C API); loaded as morello_b200._lib's helper, not as a package
+PYHOST_PATH = os.path.join(LIB_DIR, "_pyhost.so")
 
 
 def _nvcc():
@@ -18,9 +21,9 @@ def _nvcc():
 
 
 def needs_build():
-    if not os.path.exists(LIB_PATH):
+    if not os.path.exists(LIB_PATH) or not os.path.exists(PYHOST_PATH):
         return True
-    built = os.path.getmtime(LIB_PATH)
+    built = min(os.path.getmtime(LIB_PATH), os.path.getmtime(PYHOST_PATH))
     deps = []
     for root, _dirs, files in os.walk(CSRC):
         deps += [os.path.join(root, f) for f in files]
@@ -43,4 +46,8 @@ def build(force=False, verbose=False):
     res = subprocess.run(cmd, capture_output=True, text=True)
     if res.returncode != 0:
         raise RuntimeError("nvcc failed:\n" + res.stdout + res.stderr)
+    res = subprocess.run(["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-I" + sysconfig.get_paths()["include"],
+                          os.path.join(CSRC, "pyhost.cpp"), "-o", PYHOST_PATH], capture_output=True, text=True)
+    if res.returncode != 0:
+        raise RuntimeError("g++ failed:\n" + res.stdout + res.stderr)
     return LIB_PATH

@@ -730,6 +730,26 @@ void reconstruct(mrl_ctx* ctx, const LogicalSpec& ls, const u64 limits[4], int l
 }
 }  // namespace
 
+namespace {
+// The same from the nodes the device walked.
+void write_nodes(mrl_ctx* ctx, const std::vector<WalkNode>& nodes, uint32_t k, int level, std::string& out) {
+  const WalkNode& w = nodes[k];
+  if (w.status == WALK_NO_SPEC) throw ModelError("not in the tables");
+  const LogicalSpec ls = ctx->on_device ? ctx->tab.spec_of(w.spec) : ctx->plan.specs[w.id];
+  if (w.status == WALK_UNSAT) throw ModelError("no implementation for " + ls.str());
+  MrlRow row;
+  row.main = w.main; row.peaks = w.peaks; row.tail = w.tail; row.aux = 0;
+  mrl_decision d;
+  decode_row(row, &d);
+  Candidate c;
+  if (w.status != WALK_OK || !action_of(ls, d.action, c)) throw ModelError("stored action is not among the Spec's actions: " + ls.str());
+  u64 limits[4];
+  for (int m = 0; m < 4; m++) limits[m] = limit_value(m, (w.cpack >> (8 * m)) & 0xFF);
+  out += impl_line(level, ls, limits, d.action, action_text(c), d.main_cost, d.peaks, d.depth);
+  for (uint32_t j = 0; j < w.n_child; j++) write_nodes(ctx, nodes, w.first_child + j, level + 1, out);
+}
+}  // namespace
+
 long mrl_get_impl(mrl_ctx* ctx, const uint8_t* blob, size_t len, const uint64_t limits[4], char* out, size_t cap) {
   if (!ctx) return -1;
   if (!ctx->filled) return fail(ctx, -1, "tables are not filled");
@@ -737,7 +757,31 @@ long mrl_get_impl(mrl_ctx* ctx, const uint8_t* blob, size_t len, const uint64_t 
     LogicalSpec ls = LogicalSpec::from_key(std::string((const char*)blob, len));
     if (logicalspec_canonicalize(ls) != CANON_OK) return fail(ctx, -4, "Spec is not canonicalizable");
     std::string text;
-    reconstruct(ctx, ls, limits, 0, text);
+    bool done = false;
+    if (!ctx->table_only && !ctx->cands_elsewhere) {   // the records are on the device: one walk there
+      uint64_t root = 0;
+      uint32_t pack = 0;
+      bool known;
+      if (ctx->on_device) {
+        known = ctx->tab.locate(ls, &root);
+      } else {
+        const long id = ctx->plan.find(ls);
+        known = id >= 0;
+        root = (uint64_t)id;
+      }
+      uint32_t top[4];
+      for (int k = 0; k < 4; k++) top[k] = top_code_of(ctx, k);
+      if (!known || !pack_limit_codes(limits, top, &pack)) throw ModelError("not in the tables: " + ls.str());
+      std::vector<WalkNode> nodes;
+      const int rc = ctx->dev.walk(root, ctx->on_device, pack, nodes);
+      if (rc < 0) throw ModelError(ctx->dev.error());
+      if (rc == 0) {
+        if (nodes[0].status == WALK_NO_SPEC) throw ModelError("not in the tables: " + ls.str());
+        write_nodes(ctx, nodes, 0, 0, text);
+        done = true;
+      }
+    }
+    if (!done) reconstruct(ctx, ls, limits, 0, text);
     if (text.size() + 1 > cap) return fail(ctx, -3, "implementation text needs " + std::to_string(text.size() + 1) + " bytes");
     memcpy(out, text.c_str(), text.size() + 1);
     return (long)text.size();
@@ -820,12 +864,7 @@ int mrl_export_all(mrl_ctx* ctx, uint32_t* masks, uint64_t* first_row, mrl_row* 
   try {
     const uint64_t n = spec_count(ctx), n_rows = ctx->dev.stats().n_rows;
     if (rows_cap < n_rows) return fail(ctx, -3, "export buffer too small");
-    std::vector<SpecHdr> h(n);
-    if (ctx->dev.read_table(h.data(), reinterpret_cast<MrlRow*>(rows)) != 0) return fail(ctx, -2, ctx->dev.error());
-    for (uint64_t i = 0; i < n; i++) {
-      for (int k = 0; k < 4; k++) masks[4 * i + k] = h[i].mask[k];
-      first_row[i] = h[i].row_base;
-    }
+    if (ctx->dev.export_table(masks, first_row, reinterpret_cast<MrlRow*>(rows)) != 0) return fail(ctx, -2, ctx->dev.error());
     first_row[n] = n_rows;
     ctx->stats.d2h_bytes = n * sizeof(SpecHdr) + n_rows * sizeof(MrlRow);
     return 0;

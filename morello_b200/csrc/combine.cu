@@ -54,6 +54,7 @@
 #include <chrono>
 #include <mutex>
 #include <thread>
+#include <type_traits>
 
 namespace cg = cooperative_groups;
 
@@ -113,6 +114,29 @@ __device__ __forceinline__ uint32_t sel4(uint32_t a0, uint32_t a1, uint32_t a2, 
   return k == 0 ? a0 : (k == 1 ? a1 : (k == 2 ? a2 : a3));
 }
 __device__ __forceinline__ uint32_t below(uint32_t code) { return (2u << code) - 1u; }   // codes <= code
+
+// Slot indices come out of cell numbers by division by slot counts (1 to 31). x / n = the high word of x *
+// ceil(2^32 / n) while x * n < 2^32 (cells of a Spec < 2^20), three instructions instead of twenty.
+__constant__ uint32_t kReciprocal[32] = {
+#define MRL_R(n) (n) < 2 ? 0u : 0xFFFFFFFFu / ((n) < 2 ? 2u : (n)) + 1u
+    MRL_R(0), MRL_R(1), MRL_R(2), MRL_R(3), MRL_R(4), MRL_R(5), MRL_R(6), MRL_R(7), MRL_R(8), MRL_R(9), MRL_R(10),
+    MRL_R(11), MRL_R(12), MRL_R(13), MRL_R(14), MRL_R(15), MRL_R(16), MRL_R(17), MRL_R(18), MRL_R(19), MRL_R(20), MRL_R(21),
+    MRL_R(22), MRL_R(23), MRL_R(24), MRL_R(25), MRL_R(26), MRL_R(27), MRL_R(28), MRL_R(29), MRL_R(30), MRL_R(31)
+#undef MRL_R
+};
+// x / n, and x becomes x % n.
+__device__ __forceinline__ uint32_t div_slots(uint32_t& x, uint32_t n) {
+  const uint32_t q = n == 1 ? x : __umulhi(x, kReciprocal[n]);
+  x -= q * n;
+  return q;
+}
+// Slots of a cell (RF fastest) in a grid of n0 * n1 * n2 * .. slots.
+__device__ __forceinline__ void cell_slots(uint32_t cell, uint32_t n0, uint32_t n1, uint32_t n2, uint32_t& s0, uint32_t& s1, uint32_t& s2, uint32_t& s3) {
+  s0 = cell;
+  s1 = div_slots(s0, n0);
+  s2 = div_slots(s1, n1);
+  s3 = div_slots(s2, n2);
+}
 
 // The running optimum of a cell: the row's three key words.
 struct Best {
@@ -276,6 +300,7 @@ __device__ __forceinline__ uint32_t shift_mask(uint32_t cm, uint32_t level, uint
   const uint32_t keep = (2u << top) - 1u;   // top <= 30
   if (level < 2) return units >= 32 ? 0u : (uint32_t)(((unsigned long long)cm << units) & keep);
   uint32_t out = 0;
+#pragma unroll 1
   while (cm) {
     const uint32_t b = __ffs(cm) - 1;
     cm &= cm - 1;
@@ -287,7 +312,8 @@ __device__ __forceinline__ uint32_t shift_mask(uint32_t cm, uint32_t level, uint
   return out;
 }
 
-// A run of stages, as one launch sees it; passed by value.
+// A run of stages, as one launch sees it; passed by value. The stage's counters (StageCtl) lie in the
+// control block, or in shared memory when the team is one block.
 struct StageArgs {
   SpecHdr* hdrs;
   const CandRec* cands;
@@ -323,9 +349,9 @@ __device__ __forceinline__ uint32_t corner_of(uint32_t pack, uint32_t k) { retur
 // A cell with a limit below its Spec's corner has no implementation; no record needs to be read.
 __device__ __forceinline__ bool below_corner(uint32_t corner, uint32_t cpack) { return __vcmpltu4(cpack, corner) != 0; }
 
-// Exact corner of a Spec from its finished rows. Along memory k the cell with the top slot in
-// every other memory is satisfiable as soon as any cell with that slot in k is.
-__device__ __forceinline__ uint32_t corner_from_rows(const uint4 m, const MrlRow* grid) {
+// Exact corner of a Spec from its finished rows, by a warp. Along memory k the cell with the top slot
+// in every other memory is satisfiable as soon as any cell with that slot in k is.
+__device__ __forceinline__ uint32_t corner_from_rows(const uint4 m, const MrlRow* grid, uint32_t lane) {
   const uint32_t mm[4] = {m.x, m.y, m.z, m.w};
   uint32_t nn[4], st[4];
 #pragma unroll
@@ -334,21 +360,26 @@ __device__ __forceinline__ uint32_t corner_from_rows(const uint4 m, const MrlRow
   uint32_t top = 0;
 #pragma unroll
   for (int k = 0; k < 4; k++) top += (nn[k] - 1) * st[k];
+  uint32_t tail[4];
+#pragma unroll
+  for (int k = 0; k < 4; k++) tail[k] = lane < nn[k] ? grid[top - (nn[k] - 1 - lane) * st[k]].tail : MRL_UNSAT;   // at most 31 slots
   uint32_t pack = 0;
 #pragma unroll
   for (int k = 0; k < 4; k++) {
-    uint32_t code = MRL_NEVER;
-    for (uint32_t sl = 0; sl < nn[k]; sl++)
-      if (grid[top - (nn[k] - 1 - sl) * st[k]].tail != MRL_UNSAT) { code = nth_set_bit(mm[k], sl); break; }
-    pack |= code << (8 * k);
+    const uint32_t sat = __ballot_sync(0xFFFFFFFFu, tail[k] != MRL_UNSAT);
+    pack |= (sat ? nth_set_bit(mm[k], __ffs(sat) - 1) : MRL_NEVER) << (8 * k);
   }
   return pack;
 }
 
 // Corners of the Specs of an earlier stage whose rows came from several ranks.
-__device__ __noinline__ void phase_minsat(const StageArgs& a, uint32_t lo, uint32_t hi, uint32_t gtid, uint32_t gthreads) {
-  for (uint32_t i = lo + gtid; i < hi; i += gthreads)
-    a.minsat[i] = corner_from_rows(*reinterpret_cast<const uint4*>(&a.hdrs[i]), a.rows + a.hdrs[i].row_base);
+__device__ __noinline__ void phase_minsat(const StageArgs& a, uint32_t lo, uint32_t hi, uint32_t gwarp, uint32_t gwarps) {
+  const uint32_t lane = threadIdx.x & 31;
+  #pragma unroll 1
+  for (uint32_t i = lo + gwarp; i < hi; i += gwarps) {
+    const uint32_t corner = corner_from_rows(*reinterpret_cast<const uint4*>(&a.hdrs[i]), a.rows + a.hdrs[i].row_base, lane);
+    if (lane == 0) a.minsat[i] = corner;
+  }
 }
 
 // What one record needs at least, per memory: its threshold; its children's corners, shifted by what
@@ -358,20 +389,16 @@ __device__ __forceinline__ uint32_t record_corner(const StageArgs& a, uint32_t l
   const uint32_t kind = (c.x >> 16) & 0xFFu, nchild = c.x >> 24;
   const uint32_t level = c.z & 0xFFu, thr = (c.z >> 8) & 0xFFu, units = c.w;
   uint32_t q = (kind == MRL_CK_LEAF || kind == MRL_CK_MOVE) ? thr << (8 * level) : 0u;
-#pragma unroll
-  for (uint32_t j = 0; j < 3; j++) {
-    if (j >= nchild) break;
+#pragma unroll 1
+  for (uint32_t j = 0; j < nchild; j++) {
     const uint32_t child = j == 0 ? b.x : (j == 1 ? b.y : b.z);
     uint32_t e = (child < lo || bounds) ? a.minsat[child] : 0u;
     if ((e & 0xFFu) == MRL_NEVER) return MRL_NEVER4;
     if (kind == MRL_CK_MOVE) {
       const uint32_t el = corner_of(e, level);
-      uint32_t sh = 0;
-      if (el) {
-        const uint32_t bit = shift_mask(1u << el, level, units, code_of(a.top_pack, level));
-        if (!bit) return MRL_NEVER4;
-        sh = __ffs(bit) - 1;
-      }
+      // the smallest code whose child code reaches el
+      const uint32_t sh = el == 0 ? 0u : (level < 2 ? el + units : cache_code_ceil(cache_value(el) + units));
+      if (sh > code_of(a.top_pack, level)) return MRL_NEVER4;
       e = (e & ~(0xFFu << (8 * level))) | (sh << (8 * level));
     }
     q = __vmaxu4(q, e);
@@ -402,9 +429,8 @@ __device__ __forceinline__ void record_breakpoints(const StageArgs& a, uint32_t 
   const uint32_t kind = (c.x >> 16) & 0xFFu, nchild = c.x >> 24;
   const uint32_t level = c.z & 0xFFu, thr = (c.z >> 8) & 0xFFu, units = c.w;
   if (kind == MRL_CK_LEAF || kind == MRL_CK_MOVE) or_level(r.x, r.y, r.z, r.w, level, 1u << thr);
-#pragma unroll
-  for (uint32_t j = 0; j < 3; j++) {
-    if (j >= nchild) break;
+#pragma unroll 1
+  for (uint32_t j = 0; j < nchild; j++) {
     const uint32_t child = j == 0 ? b.x : (j == 1 ? b.y : b.z);
     const uint4 cm = child < lo ? *reinterpret_cast<const uint4*>(&a.hdrs[child]) : a.rmask[child];
     if (kind == MRL_CK_MOVE) {
@@ -439,41 +465,50 @@ __device__ __forceinline__ uint32_t group_size(uint32_t n, uint32_t gwarps) { re
 // Cells per work item: a work item's records are staged once, so long items where there are enough
 // of them; one step of the warp where Specs are few. Grids have 100 to 600 cells on average.
 __device__ __forceinline__ uint32_t item_size(uint32_t n, uint32_t gwarps) {
-  const unsigned long long want = (unsigned long long)n * 128u / gwarps;
-  return want >= MRL_ITEM_CELLS ? MRL_ITEM_CELLS : max(32u, (uint32_t)want & ~31u);
+  if (n >= gwarps * (MRL_ITEM_CELLS / 128u)) return MRL_ITEM_CELLS;
+  return max(32u, n * 128u / gwarps & ~31u);
 }
 
-// Phase 1: one pass over the records of every Spec of the stage, a record per lane: the breakpoints of
-// the records whose children all lie in finished stages (they come first), and the corner with
-// nothing known about same-stage children.
-__device__ __noinline__ void phase_records(const StageArgs& a, uint32_t lo, uint32_t hi, uint32_t gwarp, uint32_t gwarps, uint32_t stage) {
+// One pass over the records of a Spec, a record per lane: the breakpoints of the records whose children
+// all lie in finished stages (they come first), the corner of those, and of the others with nothing
+// known about same-stage children.
+__device__ __noinline__ uint4 scan_records(const StageArgs& a, uint32_t lo, const uint2 cl, uint32_t& early, uint32_t& late, uint32_t& n_late,
+                                              uint32_t lane) {
+  uint4 r = make_uint4(1u, 1u, 1u, 1u);
+  early = late = MRL_NEVER4;
+  n_late = 0;
+  #pragma unroll 1
+  for (uint32_t c0 = 0; c0 < cl.y; c0 += 32) {
+    bool l = false;
+    if (c0 + lane < cl.y) {
+      const uint4* const rec = reinterpret_cast<const uint4*>(&a.cands[cl.x + c0 + lane]);
+      const uint4 c = __ldg(rec), b = __ldg(rec + 1);
+      l = is_late(c);
+      const uint32_t q = record_corner(a, lo, c, b, false);
+      if (l) late = __vminu4(late, q);
+      else {
+        early = __vminu4(early, q);
+        record_breakpoints(a, lo, c, b, r);
+      }
+    }
+    n_late += __popc(__ballot_sync(0xFFFFFFFFu, l));
+  }
+  early = warp_min4(early);
+  if (n_late) late = warp_min4(late);
+  return warp_or(r);
+}
+
+// Phase 1.
+__device__ __noinline__ void phase_records(const StageArgs& a, StageCtl* sc, uint32_t lo, uint32_t hi, uint32_t gwarp, uint32_t gwarps, uint32_t stage) {
   const uint32_t lane = threadIdx.x & 31;
+  #pragma unroll 1
   for (uint32_t i = lo + gwarp; i < hi; i += gwarps) {
     if (!computed_here(a, i)) {
       if (lane == 0) a.rmask[i] = make_uint4(0, 0, 0, 0);   // another rank's Spec: zero until the exchange
       continue;
     }
-    const uint2 cl = *reinterpret_cast<const uint2*>(&a.hdrs[i].cand_off);
-    uint4 r = make_uint4(1u, 1u, 1u, 1u);
-    uint32_t early = MRL_NEVER4, late = MRL_NEVER4, n_late = 0;
-    for (uint32_t c0 = 0; c0 < cl.y; c0 += 32) {
-      bool l = false;
-      if (c0 + lane < cl.y) {
-        const uint4* const rec = reinterpret_cast<const uint4*>(&a.cands[cl.x + c0 + lane]);
-        const uint4 c = __ldg(rec), b = __ldg(rec + 1);
-        l = is_late(c);
-        const uint32_t q = record_corner(a, lo, c, b, false);
-        if (l) late = __vminu4(late, q);
-        else {
-          early = __vminu4(early, q);
-          record_breakpoints(a, lo, c, b, r);
-        }
-      }
-      n_late += __popc(__ballot_sync(0xFFFFFFFFu, l));
-    }
-    r = warp_or(r);
-    early = warp_min4(early);
-    if (n_late) late = warp_min4(late);
+    uint32_t early, late, n_late;
+    const uint4 r = scan_records(a, lo, *reinterpret_cast<const uint2*>(&a.hdrs[i].cand_off), early, late, n_late, lane);
     if (lane == 0) {
       StageSpec& s = a.sspec[i - lo];
       s.emask = r;
@@ -482,7 +517,7 @@ __device__ __noinline__ void phase_records(const StageArgs& a, uint32_t lo, uint
       uint32_t bound = __vminu4(early, late);
       if (__vcmpgtu4(bound, a.top_pack)) bound = MRL_NEVER4;   // no limits inside the lattice reach it
       a.minsat[i] = bound;
-      if (n_late) a.ctl->any_late = stage + 1;   // every writer of a stage stores the same value
+      if (n_late) sc->any_late = stage + 1;   // every writer of a stage stores the same value
     }
   }
 }
@@ -490,7 +525,7 @@ __device__ __noinline__ void phase_records(const StageArgs& a, uint32_t lo, uint
 // Rows and work items for the grids of up to 32 Specs, one per lane (`cells` 0: none), by one warp:
 // the lane's first row, and items at the end of the list. What does not fit is counted and left out;
 // the totals are checked behind the next barrier.
-__device__ __forceinline__ unsigned long long place_grids(const StageArgs& a, unsigned long long* row_cursor, uint32_t spec, unsigned long long cells,
+__device__ __forceinline__ unsigned long long place_grids(const StageArgs& a, StageCtl* sc, unsigned long long* row_cursor, uint32_t spec, unsigned long long cells,
                                                           unsigned long long item_cells_of, uint32_t item_cells, uint32_t flag, uint32_t lane) {
   unsigned long long inc = cells;
   uint32_t items = (uint32_t)((item_cells_of + item_cells - 1) / item_cells), iinc = items;
@@ -504,16 +539,18 @@ __device__ __forceinline__ unsigned long long place_grids(const StageArgs& a, un
   uint32_t item0 = 0;
   if (lane == 31) {
     if (inc) row0 = atomicAdd(row_cursor, inc);
-    if (iinc) item0 = atomicAdd(&a.ctl->n_items, iinc);
+    if (iinc) item0 = atomicAdd(&sc->n_items, iinc);
   }
   row0 = __shfl_sync(0xFFFFFFFFu, row0, 31);
   item0 = __shfl_sync(0xFFFFFFFFu, item0, 31);
   uint32_t todo = __ballot_sync(0xFFFFFFFFu, items != 0);
+  #pragma unroll 1
   while (todo) {
     const uint32_t src = __ffs(todo) - 1;
     todo &= todo - 1;
     const uint32_t n = __shfl_sync(0xFFFFFFFFu, items, src), at = item0 + __shfl_sync(0xFFFFFFFFu, iinc, src) - n;
     const uint32_t sp = __shfl_sync(0xFFFFFFFFu, spec, src), fl = __shfl_sync(0xFFFFFFFFu, flag, src);
+    #pragma unroll 1
     for (uint32_t w = lane; w < n; w += 32)
       if (at + w < a.item_cap) {
         WorkItem it;
@@ -527,9 +564,10 @@ __device__ __forceinline__ unsigned long long place_grids(const StageArgs& a, un
 
 // Phase 2: the final corner (records with a same-stage child again, with that child's bound), the grid
 // of the unordered phase, its rows and work items.
-__device__ __noinline__ void phase_place_early(const StageArgs& a, uint32_t lo, uint32_t hi, uint32_t gwarp, uint32_t gwarps, bool any_late) {
+__device__ __noinline__ void phase_place_early(const StageArgs& a, StageCtl* sc, uint32_t lo, uint32_t hi, uint32_t gwarp, uint32_t gwarps, bool any_late) {
   const uint32_t lane = threadIdx.x & 31;
   const uint32_t G = group_size(hi - lo, gwarps), item_cells = item_size(hi - lo, gwarps);
+  #pragma unroll 1
   for (uint32_t base = lo + gwarp * G; base < hi; base += gwarps * G) {
     const uint32_t i = base + lane;
     const bool mine = lane < G && i < hi && computed_here(a, i);
@@ -542,12 +580,14 @@ __device__ __noinline__ void phase_place_early(const StageArgs& a, uint32_t lo, 
       n_late = s.n_late;
     }
     uint32_t todo = any_late ? __ballot_sync(0xFFFFFFFFu, n_late != 0) : 0u;
+    #pragma unroll 1
     while (todo) {
       const uint32_t src = __ffs(todo) - 1;
       todo &= todo - 1;
       const uint32_t n = __shfl_sync(0xFFFFFFFFu, n_late, src);
       const uint2 cl = *reinterpret_cast<const uint2*>(&a.hdrs[base + src].cand_off);
       uint32_t q = MRL_NEVER4;
+      #pragma unroll 1
       for (uint32_t c = lane; c < n; c += 32) {
         const uint4* const rec = reinterpret_cast<const uint4*>(&a.cands[cl.x + cl.y - 1 - c]);
         q = __vminu4(q, record_corner(a, lo, __ldg(rec), __ldg(rec + 1), true));
@@ -561,7 +601,7 @@ __device__ __noinline__ void phase_place_early(const StageArgs& a, uint32_t lo, 
       m = clip_at_corner(m, corner);
       cells = cells_of(m);
     }
-    const unsigned long long row = place_grids(a, &a.ctl->rows_early, i, cells, cells, item_cells, 0, lane);
+    const unsigned long long row = place_grids(a, sc, &sc->rows_early, i, cells, cells, item_cells, 0, lane);
     if (mine) {
       StageSpec& s = a.sspec[i - lo];
       s.emask = m;
@@ -578,9 +618,10 @@ __device__ __noinline__ void phase_place_early(const StageArgs& a, uint32_t lo, 
 // pass: of what the unordered phase found for the child; later passes: found real by the pass
 // before. Grids only grow; one that grew gets new rows, and its old ones are remembered.
 // A Spec without such records is finished: its grid is that of the unordered phase.
-__device__ __noinline__ void phase_place_late(const StageArgs& a, uint32_t lo, uint32_t hi, uint32_t gwarp, uint32_t gwarps, uint32_t pass) {
+__device__ __noinline__ void phase_place_late(const StageArgs& a, StageCtl* sc, uint32_t lo, uint32_t hi, uint32_t gwarp, uint32_t gwarps, uint32_t pass) {
   const uint32_t lane = threadIdx.x & 31;
   const uint32_t G = group_size(hi - lo, gwarps), item_cells = item_size(hi - lo, gwarps);
+  #pragma unroll 1
   for (uint32_t base = lo + gwarp * G; base < hi; base += gwarps * G) {
     const uint32_t i = base + lane;
     const bool mine = lane < G && i < hi && computed_here(a, i);
@@ -599,12 +640,14 @@ __device__ __noinline__ void phase_place_late(const StageArgs& a, uint32_t lo, u
     }
     uint4 nm = old;
     uint32_t todo = __ballot_sync(0xFFFFFFFFu, n_late != 0);
+    #pragma unroll 1
     while (todo) {
       const uint32_t src = __ffs(todo) - 1;
       todo &= todo - 1;
       const uint32_t n = __shfl_sync(0xFFFFFFFFu, n_late, src);
       const uint2 cl = *reinterpret_cast<const uint2*>(&a.hdrs[base + src].cand_off);
       uint4 r = make_uint4(0, 0, 0, 0);
+      #pragma unroll 1
       for (uint32_t c = lane; c < n; c += 32) {
         const uint4* const rec = reinterpret_cast<const uint4*>(&a.cands[cl.x + cl.y - 1 - c]);
         record_breakpoints(a, lo, __ldg(rec), __ldg(rec + 1), r);
@@ -619,7 +662,7 @@ __device__ __noinline__ void phase_place_late(const StageArgs& a, uint32_t lo, u
       fresh = !pass || nm.x != old.x || nm.y != old.y || nm.z != old.z || nm.w != old.w;
       cells = cells_of(nm);
     }
-    const unsigned long long row = place_grids(a, &a.ctl->rows_late, i, fresh ? cells : 0ull, cells, item_cells, fresh ? 1u : 0u, lane);
+    const unsigned long long row = place_grids(a, sc, &sc->rows_late, i, fresh ? cells : 0ull, cells, item_cells, fresh ? 1u : 0u, lane);
     if (fresh) {
       StageSpec& s = a.sspec[i - lo];
       s.old_mask = old;
@@ -632,14 +675,16 @@ __device__ __noinline__ void phase_place_late(const StageArgs& a, uint32_t lo, u
 }
 
 // After a pass: does any grid lack a (shifted) real breakpoint of a same-stage child?
-__device__ __noinline__ void phase_check_grids(const StageArgs& a, uint32_t lo, uint32_t hi, uint32_t gwarp, uint32_t gwarps, uint32_t pass) {
+__device__ __noinline__ void phase_check_grids(const StageArgs& a, StageCtl* sc, uint32_t lo, uint32_t hi, uint32_t gwarp, uint32_t gwarps, uint32_t pass) {
   const uint32_t lane = threadIdx.x & 31;
+  #pragma unroll 1
   for (uint32_t i = lo + gwarp; i < hi; i += gwarps) {
     if (!computed_here(a, i)) continue;
     const uint32_t n = a.sspec[i - lo].n_late;
     if (!n) continue;
     const uint2 cl = *reinterpret_cast<const uint2*>(&a.hdrs[i].cand_off);
     uint4 r = make_uint4(0, 0, 0, 0);
+    #pragma unroll 1
     for (uint32_t c = lane; c < n; c += 32) {
       const uint4* const rec = reinterpret_cast<const uint4*>(&a.cands[cl.x + cl.y - 1 - c]);
       record_breakpoints(a, lo, __ldg(rec), __ldg(rec + 1), r);
@@ -649,7 +694,7 @@ __device__ __noinline__ void phase_check_grids(const StageArgs& a, uint32_t lo, 
     // what the grid lacks above its corner (below it nothing is kept)
     const uint32_t k0 = corner_of(corner, 0), k1 = corner_of(corner, 1), k2 = corner_of(corner, 2), k3 = corner_of(corner, 3);
     const bool lacks = k0 != MRL_NEVER && (((r.x & ~m.x) >> k0) | ((r.y & ~m.y) >> k1) | ((r.z & ~m.z) >> k2) | ((r.w & ~m.w) >> k3));
-    if (lacks) a.ctl->grew = pass + 1;   // every writer of a pass stores the same value
+    if (lacks) sc->grew = pass + 1;   // every writer of a pass stores the same value
   }
 }
 
@@ -703,7 +748,7 @@ __device__ __forceinline__ const MrlRow* staged_row(const StagedRec& s, uint32_t
 // The lattice code of every slot of a grid, memory after memory, for the lanes of a warp to look
 // up instead of counting bits (a grid has at most 17 + 17 + 12 + 27 slots).
 constexpr int kMaxSlots = 80;
-constexpr int kMaxAffected = 16;
+constexpr int kMaxAffected = 32;
 struct WarpScratch {         // a warp's shared memory in the solve phases
   StagedRec staged[kBatch];
   uint4 affected[kMaxAffected];      // sweeps: per changed child the parent's codes that read a changed slot of it
@@ -716,6 +761,7 @@ static_assert(sizeof(WarpScratch) % 16 == 0, "warp scratch is made of 16-byte un
 __device__ __forceinline__ void stage_slot_codes(uint8_t* codes, const uint4 m, uint32_t n0, uint32_t n1, uint32_t n2, uint32_t n3,
                                                  uint32_t lane) {
   __syncwarp();   // the previous item's codes have been read by every lane
+  #pragma unroll 1
   for (uint32_t t = lane; t < n0 + n1 + n2 + n3; t += 32) {
     uint32_t mk = m.x, slot = t;
     if (slot >= n0) { slot -= n0; mk = m.y; if (slot >= n1) { slot -= n1; mk = m.z; if (slot >= n2) { slot -= n2; mk = m.w; } } }
@@ -833,67 +879,73 @@ __device__ __forceinline__ void add_tally(const Tally& tally, unsigned long long
   }
 }
 
+// The records of a Spec whose children all lie in finished stages, for the cells [first, end) of its
+// grid of the unordered phase, by a warp. The grid's slot codes are staged.
+__device__ __noinline__ void solve_early_cells(const HotArgs a, WarpScratch& ws, uint32_t cand_off, uint32_t n_early, const uint4 m, uint32_t corner,
+                                                  MrlRow* grid, uint32_t first, uint32_t end, Tally& tally, uint32_t lane) {
+  StagedRec* const staged = ws.staged;
+  const uint8_t* const codes = ws.codes;
+  const uint32_t n0 = __popc(m.x), n1 = __popc(m.y), n2 = __popc(m.z);
+  uint32_t b0 = 0;
+  do {
+    // stage the next records, and the headers of their children, one (record, child) per lane
+    const uint32_t n_here = min((uint32_t)kBatch, n_early - b0);
+    __syncwarp();   // the previous batch has been read by every lane
+    if (lane < n_here) staged[lane].rec = __ldg(reinterpret_cast<const uint4*>(&a.cands[cand_off + b0 + lane]));
+    __syncwarp();
+    #pragma unroll 1
+    for (uint32_t t = lane; t < n_here * 3u; t += 32) {
+      const uint32_t r = t / 3u, j = t - r * 3u;
+      if (j < (staged[r].rec.x >> 24)) {
+        const uint32_t child = __ldg(&a.cands[cand_off + b0 + r].child[j]);
+        stage_child(staged[r], j, *reinterpret_cast<const uint4*>(&a.hdrs[child]), a.rows + a.hdrs[child].row_base, false);
+      }
+    }
+    __syncwarp();
+    #pragma unroll 1
+    for (uint32_t c0 = first; c0 < end; c0 += 32) {
+      const uint32_t cell = c0 + lane;
+      const bool valid = cell < end;
+      uint32_t s0, s1, s2, s3;
+      cell_slots(valid ? cell : 0u, n0, n1, n2, s0, s1, s2, s3);
+      const uint32_t k0 = codes[s0], k1 = codes[n0 + s1], k2 = codes[n0 + n1 + s2], k3 = codes[n0 + n1 + n2 + s3];
+      const uint32_t cpack = k0 | (k1 << 8) | (k2 << 16) | (k3 << 24);
+      const bool live = valid && !below_corner(corner, cpack);
+      Best best = {MRL_UNSAT, MRL_UNSAT, MRL_UNSAT};
+      if (!__any_sync(0xFFFFFFFFu, live)) {
+        if (valid && b0 == 0) *reinterpret_cast<uint4*>(grid + cell) = make_uint4(best.main, best.peaks, best.tail, 0u);
+        continue;
+      }
+      if (b0 && live) {   // what the earlier batches found
+        const uint4 r = ld_row(grid + cell);
+        best.main = r.x; best.peaks = r.y; best.tail = r.z;
+      }
+      const uint32_t bm0 = below(k0), bm1 = below(k1), bm2 = below(k2), bm3 = below(k3);
+      if (live) {
+        #pragma unroll 1
+        for (uint32_t r = 0; r < n_here; r++) eval_staged<false>(staged[r], cpack, bm0, bm1, bm2, bm3, best, tally);
+      }
+      if (valid && (b0 == 0 || live)) *reinterpret_cast<uint4*>(grid + cell) = make_uint4(best.main, best.peaks, best.tail, 0u);
+    }
+    b0 += n_here;
+  } while (b0 < n_early);
+}
+
 __device__ __noinline__ void phase_early(const HotArgs a, unsigned long long* block_stats) {
   const uint32_t lane = threadIdx.x & 31;
   WarpScratch& ws = warp_scratch();
-  StagedRec* const staged = ws.staged;
-  const uint8_t* const codes = ws.codes;
   Tally tally = {0, 0};
   uint32_t w = warp_number();
-  if (w < a.n_items) do {
+  if (w < a.n_items)
+#pragma unroll 1
+  do {
     const WorkItem it = a.items[w];
-    const uint32_t i = it.spec;
-    const uint4 m = a.sspec[i].emask;
-    const uint32_t corner = a.sspec[i].corner;
-    const uint2 cl = *reinterpret_cast<const uint2*>(&a.hdrs[i].cand_off);
-    MrlRow* const grid = a.temp + a.temp_cap + a.sspec[i].erow;
-    const uint32_t n_early = cl.y - a.sspec[i].n_late;   // records with a same-stage child come last
-    const uint32_t n0 = __popc(m.x), n1 = __popc(m.y), n2 = __popc(m.z), n3 = __popc(m.w);
-    const uint32_t cells = n0 * n1 * n2 * n3;
-    const uint32_t c_end = min(cells, it.first_cell + a.item_cells);
-    stage_slot_codes(ws.codes, m, n0, n1, n2, n3, lane);
-    uint32_t b0 = 0;
-    do {
-      // stage the next records, and the headers of their children, one (record, child) per lane
-      const uint32_t n_here = min((uint32_t)kBatch, n_early - b0);
-      __syncwarp();   // the previous batch has been read by every lane
-      if (lane < n_here) staged[lane].rec = __ldg(reinterpret_cast<const uint4*>(&a.cands[cl.x + b0 + lane]));
-      __syncwarp();
-      for (uint32_t t = lane; t < n_here * 3u; t += 32) {
-        const uint32_t r = t / 3u, j = t - r * 3u;
-        if (j < (staged[r].rec.x >> 24)) {
-          const uint32_t child = __ldg(&a.cands[cl.x + b0 + r].child[j]);
-          stage_child(staged[r], j, *reinterpret_cast<const uint4*>(&a.hdrs[child]), a.rows + a.hdrs[child].row_base, false);
-        }
-      }
-      __syncwarp();
-      for (uint32_t c0 = it.first_cell; c0 < c_end; c0 += 32) {
-        const uint32_t cell = c0 + lane;
-        const bool valid = cell < c_end;
-        uint32_t rest = valid ? cell : 0u;
-        const uint32_t k0 = codes[rest % n0]; rest /= n0;
-        const uint32_t k1 = codes[n0 + rest % n1]; rest /= n1;
-        const uint32_t k2 = codes[n0 + n1 + rest % n2]; rest /= n2;
-        const uint32_t k3 = codes[n0 + n1 + n2 + rest];
-        const uint32_t cpack = k0 | (k1 << 8) | (k2 << 16) | (k3 << 24);
-        const bool live = valid && !below_corner(corner, cpack);
-        Best best = {MRL_UNSAT, MRL_UNSAT, MRL_UNSAT};
-        if (!__any_sync(0xFFFFFFFFu, live)) {
-          if (valid && b0 == 0) *reinterpret_cast<uint4*>(grid + cell) = make_uint4(best.main, best.peaks, best.tail, 0u);
-          continue;
-        }
-        if (b0 && live) {   // what the earlier batches found
-          const uint4 r = ld_row(grid + cell);
-          best.main = r.x; best.peaks = r.y; best.tail = r.z;
-        }
-        const uint32_t bm0 = below(k0), bm1 = below(k1), bm2 = below(k2), bm3 = below(k3);
-        if (live) {
-          for (uint32_t r = 0; r < n_here; r++) eval_staged<false>(staged[r], cpack, bm0, bm1, bm2, bm3, best, tally);
-        }
-        if (valid && (b0 == 0 || live)) *reinterpret_cast<uint4*>(grid + cell) = make_uint4(best.main, best.peaks, best.tail, 0u);
-      }
-      b0 += n_here;
-    } while (b0 < n_early);
+    const StageSpec& sp = a.sspec[it.spec];
+    const uint4 m = sp.emask;
+    const uint2 cl = *reinterpret_cast<const uint2*>(&a.hdrs[it.spec].cand_off);
+    stage_slot_codes(ws.codes, m, __popc(m.x), __popc(m.y), __popc(m.z), __popc(m.w), lane);
+    solve_early_cells(a, ws, cl.x, cl.y - sp.n_late, m, sp.corner, a.temp + a.temp_cap + sp.erow, it.first_cell,
+                      min((uint32_t)cells_of(m), it.first_cell + a.item_cells), tally, lane);
   } while (next_item(a, w, lane));
   add_tally(tally, &block_stats[0], &block_stats[1], lane);
 }
@@ -922,16 +974,17 @@ __device__ __noinline__ void phase_early(const HotArgs a, unsigned long long* bl
 // The records come dearest first and are staged from the end, so the cheapest Move is tried first.
 enum { SWEEP_ALL = 0, SWEEP_NEW = 1, SWEEP_CHANGED = 2 };
 
-template <int kMode>
+template <bool kAll>
 __device__ __forceinline__ void stage_late_batch(const HotArgs& a, uint32_t lo, StagedRec* staged, uint32_t last_rec, uint32_t n_here, uint32_t lane) {
   __syncwarp();   // the previous batch has been read by every lane
   if (lane < n_here) staged[lane].rec = __ldg(reinterpret_cast<const uint4*>(&a.cands[last_rec - lane]));
   __syncwarp();
+  #pragma unroll 1
   for (uint32_t t = lane; t < n_here * 3u; t += 32) {
     const uint32_t r = t / 3u, j = t - r * 3u;
     if (j < (staged[r].rec.x >> 24)) {
       const uint32_t child = __ldg(&a.cands[last_rec - r].child[j]);
-      if (kMode == SWEEP_ALL && child >= lo) {
+      if (kAll && child >= lo) {
         stage_child(staged[r], j, a.sspec[child].emask, a.temp + a.temp_cap + a.sspec[child].erow, false);
       } else {
         const unsigned long long base = a.hdrs[child].row_base;
@@ -947,6 +1000,7 @@ __device__ __forceinline__ void stage_late_batch(const HotArgs& a, uint32_t lo, 
 __device__ __forceinline__ uint32_t codes_reading(uint32_t parent, uint32_t child, uint32_t changed, bool shifted, uint32_t level, uint32_t thr,
                                                   uint32_t units) {
   uint32_t out = 0;
+  #pragma unroll 1
   while (parent) {
     const uint32_t p = __ffs(parent) - 1;
     parent &= parent - 1;
@@ -958,8 +1012,8 @@ __device__ __forceinline__ uint32_t codes_reading(uint32_t parent, uint32_t chil
   return out;
 }
 
-template <int kMode>
-__device__ __noinline__ void phase_sweep(const HotArgs a, uint32_t lo, const uint4* changed_before, uint4* changed_now, uint32_t sweep, uint32_t* any_changed,
+template <bool kAll>
+__device__ __noinline__ void phase_sweep(const HotArgs a, int mode, uint32_t lo, const uint4* changed_before, uint4* changed_now, uint32_t sweep, uint32_t* any_changed,
                                          unsigned long long* block_stats) {
   const uint32_t lane = threadIdx.x & 31;
   WarpScratch& ws = warp_scratch();
@@ -967,24 +1021,27 @@ __device__ __noinline__ void phase_sweep(const HotArgs a, uint32_t lo, const uin
   const uint8_t* const codes = ws.codes;
   Tally tally = {0, 0};
   uint32_t w = warp_number();
-  if (w < a.n_items) do {
+  if (w < a.n_items)
+#pragma unroll 1
+  do {
     const WorkItem it = a.items[w];
     const uint32_t i = it.spec, first_cell = it.first_cell & ~31u;
-    if (kMode == SWEEP_NEW && !(it.first_cell & 1u)) continue;   // the grid did not grow
+    if (!kAll && mode == SWEEP_NEW && !(it.first_cell & 1u)) continue;   // the grid did not grow
     const uint2 cl = *reinterpret_cast<const uint2*>(&a.hdrs[i].cand_off);
     const uint32_t n_late = a.sspec[i].n_late, last = cl.x + cl.y - 1;   // the records with a same-stage child are the last ones
     const uint4 m = *reinterpret_cast<const uint4*>(&a.hdrs[i]);
     uint32_t n_aff = 0;
-    if (kMode == SWEEP_NEW) {
+    if (!kAll && mode == SWEEP_NEW) {
       if (lane == 0) {
         const uint4 om = a.sspec[i].old_mask;
         ws.affected[0] = make_uint4(m.x & ~om.x, m.y & ~om.y, m.z & ~om.z, m.w & ~om.w);
       }
       __syncwarp();
     }
-    if (kMode == SWEEP_CHANGED) {
+    if (!kAll && mode == SWEEP_CHANGED) {
       // children that the sweep before changed
       __syncwarp();   // the previous item's list has been read by every lane
+      #pragma unroll 1
       for (uint32_t t0 = 0; t0 < n_late * 3u; t0 += 32) {
         const uint32_t t = t0 + lane, r = t / 3u, j = t - r * 3u;
         bool hit = false;
@@ -1004,6 +1061,7 @@ __device__ __noinline__ void phase_sweep(const HotArgs a, uint32_t lo, const uin
       __syncwarp();
       // per such child and memory, the codes of this grid that read one of its changed slots
       if (n_aff <= kMaxAffected) {
+        #pragma unroll 1
         for (uint32_t t = lane; t < n_aff * 4u; t += 32) {
           const uint32_t k = t & 3u, r = ws.who[t >> 2] & 0xFFFFu, j = ws.who[t >> 2] >> 16;
           const CandRec* const rec = &a.cands[last - r];
@@ -1033,16 +1091,19 @@ __device__ __noinline__ void phase_sweep(const HotArgs a, uint32_t lo, const uin
     const uint32_t z0 = corner_of(corner, 0) ? 1u : 0u, z1 = corner_of(corner, 1) ? 1u : 0u, z2 = corner_of(corner, 2) ? 1u : 0u,
                    z3 = corner_of(corner, 3) ? 1u : 0u;
     const uint32_t v0 = n0 - z0, v1 = n1 - z1, v2 = n2 - z2, v3 = n3 - z3;
-    const unsigned long long live_cells = none ? 0ull : (unsigned long long)v0 * v1 * v2 * v3;
+    const uint32_t live_cells = none ? 0u : v0 * v1 * v2 * v3;
     const uint32_t c_hi = min(cells, first_cell + a.item_cells);
-    const uint32_t l_begin = (uint32_t)(live_cells * first_cell / cells), l_end = (uint32_t)(live_cells * c_hi / cells);
-    if (kMode == SWEEP_ALL) {   // the cells below the corner
+    uint32_t l_begin = 0, l_end = live_cells;
+    if (cells > a.item_cells) {   // several items
+      l_begin = (uint32_t)((unsigned long long)live_cells * first_cell / cells);
+      l_end = (uint32_t)((unsigned long long)live_cells * c_hi / cells);
+    }
+    if (kAll) {   // the cells below the corner
+      #pragma unroll 1
       for (uint32_t cell = first_cell + lane; cell < c_hi; cell += 32) {
-        uint32_t rest = cell;
-        const bool d0 = rest % n0 < z0; rest /= n0;
-        const bool d1 = rest % n1 < z1; rest /= n1;
-        const bool d2 = rest % n2 < z2; rest /= n2;
-        if (none || d0 || d1 || d2 || rest < z3) *reinterpret_cast<uint4*>(grid + cell) = make_uint4(MRL_UNSAT, MRL_UNSAT, MRL_UNSAT, 0u);
+        uint32_t s0, s1, s2, s3;
+        cell_slots(cell, n0, n1, n2, s0, s1, s2, s3);
+        if (none || s0 < z0 || s1 < z1 || s2 < z2 || s3 < z3) *reinterpret_cast<uint4*>(grid + cell) = make_uint4(MRL_UNSAT, MRL_UNSAT, MRL_UNSAT, 0u);
       }
     }
     if (l_begin == l_end) continue;
@@ -1050,9 +1111,57 @@ __device__ __noinline__ void phase_sweep(const HotArgs a, uint32_t lo, const uin
     stage_slot_codes(ws.codes, m, n0, n1, n2, n3, lane);
     bool staged_yet = false;
     uint4 ch = make_uint4(0, 0, 0, 0);   // codes of the slots of the cells that change
-    auto solve = [&](bool live, uint32_t slots) {   // packed slots, one cell per lane
+    uint32_t c0 = l_begin, queued = 0;
+#pragma unroll 1
+    for (;;) {
+      // the next cells to solve, one per lane: all of them in order, or collected from those that qualify
+      bool live;
+      uint32_t slots;
+      if (kAll) {
+        if (c0 >= l_end) break;
+        live = c0 + lane < l_end;
+        uint32_t s0, s1, s2, s3;
+        cell_slots(live ? c0 + lane : l_begin, v0, v1, v2, s0, s1, s2, s3);
+        slots = (s0 + z0) | ((s1 + z1) << 8) | ((s2 + z2) << 16) | ((s3 + z3) << 24);
+        c0 += 32;
+      } else {
+#pragma unroll 1
+        while (queued < 32 && c0 < l_end) {
+          const bool in = c0 + lane < l_end;
+          uint32_t s0, s1, s2, s3;
+          cell_slots(in ? c0 + lane : l_begin, v0, v1, v2, s0, s1, s2, s3);
+          s0 += z0; s1 += z1; s2 += z2; s3 += z3;
+          const uint32_t k0 = codes[s0], k1 = codes[n0 + s1], k2 = codes[n0 + n1 + s2], k3 = codes[n0 + n1 + n2 + s3];
+          uint32_t hit = 0;
+          if (mode == SWEEP_NEW) {
+            const uint4 f = ws.affected[0];
+            hit = (f.x >> k0) | (f.y >> k1) | (f.z >> k2) | (f.w >> k3);
+          } else if (n_aff > (uint32_t)kMaxAffected) {
+            hit = 1;
+          } else {
+#pragma unroll 1
+            for (uint32_t e = 0; e < n_aff; e++) {
+              const uint4 f = ws.affected[e];
+              hit |= (f.x >> k0) & (f.y >> k1) & (f.z >> k2) & (f.w >> k3);
+            }
+          }
+          const bool again = in && (hit & 1u);
+          const uint32_t who = __ballot_sync(0xFFFFFFFFu, again);
+          if (again) ws.queue[queued + __popc(who & ((1u << lane) - 1u))] = s0 | (s1 << 8) | (s2 << 16) | (s3 << 24);
+          queued += __popc(who);
+          c0 += 32;
+        }
+        if (!queued) break;
+        __syncwarp();
+        live = lane < queued;
+        slots = live ? ws.queue[lane] : (z0 | (z1 << 8) | (z2 << 16) | (z3 << 24));
+        const uint32_t rest_of = ws.queue[32 + lane];
+        __syncwarp();
+        queued = queued > 32 ? queued - 32 : 0;
+        if (lane < queued) ws.queue[lane] = rest_of;
+      }
       if (single && !staged_yet) {
-        stage_late_batch<kMode>(a, lo, staged, last, n_late, lane);
+        stage_late_batch<kAll>(a, lo, staged, last, n_late, lane);
         staged_yet = true;
       }
       const uint32_t s0 = slots & 0xFFu, s1 = (slots >> 8) & 0xFFu, s2 = (slots >> 16) & 0xFFu, s3 = slots >> 24;
@@ -1066,68 +1175,22 @@ __device__ __noinline__ void phase_sweep(const HotArgs a, uint32_t lo, const uin
         const uint32_t i0 = __popc(em.x & bm0) - 1, i1 = __popc(em.y & bm1) - 1, i2 = __popc(em.z & bm2) - 1, i3 = __popc(em.w & bm3) - 1;
         const uint4 f = ld_row(egrid + (((i3 * __popc(em.z) + i2) * __popc(em.y) + i1) * __popc(em.x) + i0));
         best.main = f.x; best.peaks = f.y; best.tail = f.z;
-        was = kMode == SWEEP_ALL ? f : ld_row(at);   // only this warp writes the cell in this sweep
+        was = kAll ? f : ld_row(at);   // only this warp writes the cell in this sweep
       }
+#pragma unroll 1
       for (uint32_t b = 0; b < n_late; b += kBatch) {
         const uint32_t n_here = min((uint32_t)kBatch, n_late - b);
-        if (!single) stage_late_batch<kMode>(a, lo, staged, last - b, n_here, lane);
+        if (!single) stage_late_batch<kAll>(a, lo, staged, last - b, n_here, lane);
         if (live)
-          for (uint32_t r = 0; r < n_here; r++) eval_staged<kMode != SWEEP_ALL>(staged[r], cpack, bm0, bm1, bm2, bm3, best, tally);
+#pragma unroll 1
+          for (uint32_t r = 0; r < n_here; r++) eval_staged<!kAll>(staged[r], cpack, bm0, bm1, bm2, bm3, best, tally);
       }
       if (live) {
         const bool differs = best.main != was.x || best.peaks != was.y || best.tail != was.z;
-        if (kMode == SWEEP_ALL) *reinterpret_cast<uint4*>(at) = make_uint4(best.main, best.peaks, best.tail, 0u);
+        if (kAll) *reinterpret_cast<uint4*>(at) = make_uint4(best.main, best.peaks, best.tail, 0u);
         else if (differs) st_row_shared(at, make_uint4(best.main, best.peaks, best.tail, 0u));
         if (differs) { ch.x |= 1u << k0; ch.y |= 1u << k1; ch.z |= 1u << k2; ch.w |= 1u << k3; }
       }
-    };
-    uint32_t queued = 0;
-    for (uint32_t c0 = l_begin; c0 < l_end; c0 += 32) {
-      const bool live = c0 + lane < l_end;
-      uint32_t rest = live ? c0 + lane : l_begin;
-      const uint32_t s0 = rest % v0 + z0; rest /= v0;
-      const uint32_t s1 = rest % v1 + z1; rest /= v1;
-      const uint32_t s2 = rest % v2 + z2;
-      const uint32_t s3 = rest / v2 + z3;
-      const uint32_t slots = s0 | (s1 << 8) | (s2 << 16) | (s3 << 24);
-      if (kMode == SWEEP_ALL) {
-        solve(live, slots);
-        continue;
-      }
-      bool again = false;
-      const uint32_t k0 = codes[s0], k1 = codes[n0 + s1], k2 = codes[n0 + n1 + s2], k3 = codes[n0 + n1 + n2 + s3];
-      if (kMode == SWEEP_NEW) {
-        const uint4 f = ws.affected[0];
-        again = ((f.x >> k0) | (f.y >> k1) | (f.z >> k2) | (f.w >> k3)) & 1u;
-      } else if (n_aff > (uint32_t)kMaxAffected) {
-        again = true;
-      } else {
-        uint32_t hit = 0;
-        for (uint32_t e = 0; e < n_aff; e++) {
-          const uint4 f = ws.affected[e];
-          hit |= (f.x >> k0) & (f.y >> k1) & (f.z >> k2) & (f.w >> k3);
-        }
-        again = hit & 1u;
-      }
-      again = again && live;
-      // the cells to solve are collected until there is one per lane
-      const uint32_t who = __ballot_sync(0xFFFFFFFFu, again);
-      if (again) ws.queue[queued + __popc(who & ((1u << lane) - 1u))] = slots;
-      queued += __popc(who);
-      __syncwarp();
-      if (queued >= 32) {
-        const uint32_t mine = ws.queue[lane], rest_of = ws.queue[32 + lane];
-        __syncwarp();
-        solve(true, mine);
-        queued -= 32;
-        if (lane < queued) ws.queue[lane] = rest_of;
-        __syncwarp();
-      }
-    }
-    if (queued) {
-      const uint32_t mine = lane < queued ? ws.queue[lane] : (z0 | (z1 << 8) | (z2 << 16) | (z3 << 24));
-      __syncwarp();
-      solve(lane < queued, mine);
     }
     ch = warp_or(ch);
     if (ch.x && lane == 0) {
@@ -1144,7 +1207,9 @@ __device__ __noinline__ void phase_sweep(const HotArgs a, uint32_t lo, const uin
 __device__ __noinline__ void phase_refine(const HotArgs a) {
   const uint32_t lane = threadIdx.x & 31;
   uint32_t w = warp_number();
-  if (w < a.n_items) do {
+  if (w < a.n_items)
+#pragma unroll 1
+  do {
     const WorkItem it = a.items[w];
     if (!(it.first_cell & 1u)) continue;
     const uint32_t i = it.spec, first_cell = it.first_cell & ~31u;
@@ -1154,65 +1219,69 @@ __device__ __noinline__ void phase_refine(const HotArgs a) {
     const unsigned long long obase = a.sspec[i].old_row;
     const uint32_t n0 = __popc(m.x), n1 = __popc(m.y), n2 = __popc(m.z), n3 = __popc(m.w);
     const uint32_t c_end = min(n0 * n1 * n2 * n3, first_cell + a.item_cells);
+    #pragma unroll 1
     for (uint32_t cell = first_cell + lane; cell < c_end; cell += 32) {
-      uint32_t rest = cell;
-      const uint32_t k0 = nth_set_bit(m.x, rest % n0); rest /= n0;
-      const uint32_t k1 = nth_set_bit(m.y, rest % n1); rest /= n1;
-      const uint32_t k2 = nth_set_bit(m.z, rest % n2); rest /= n2;
-      const uint32_t k3 = nth_set_bit(m.w, rest);
+      uint32_t s0, s1, s2, s3;
+      cell_slots(cell, n0, n1, n2, s0, s1, s2, s3);
+      const uint32_t k0 = nth_set_bit(m.x, s0), k1 = nth_set_bit(m.y, s1), k2 = nth_set_bit(m.z, s2), k3 = nth_set_bit(m.w, s3);
       *reinterpret_cast<uint4*>(grid + cell) = ld_row(row_of(a.rows, a.temp, om, obase, below(k0), below(k1), below(k2), below(k3)));
     }
   } while (next_item(a, w, lane));
 }
 
-// Which breakpoints of the grids are real: a breakpoint (memory k, code c) is real when some cell
-// starting at c differs from its neighbour one slot lower in k. kEarly: of the grids of the
-// unordered phase, else of the working grids (only_dirty: of those that grew or changed). A warp
-// stops comparing in a memory at codes it knows to be real.
+// Which breakpoints of a grid are real, from its cells [first, end), by a warp: a breakpoint (memory k,
+// code c) is real when some cell starting at c differs from its neighbour one slot lower in k. The
+// comparing stops in a memory at codes known to be real. The grid's slot codes are staged.
+__device__ __noinline__ uint4 real_breakpoints(const uint8_t* codes, const uint4 m, const MrlRow* grid, uint32_t first, uint32_t end, uint32_t lane) {
+  const uint32_t n0 = __popc(m.x), n1 = __popc(m.y), n2 = __popc(m.z);
+  const uint32_t st1 = n0, st2 = n0 * n1, st3 = st2 * n2;
+  uint4 real = make_uint4(1u, 1u, 1u, 1u);   // the same in all lanes
+  #pragma unroll 1
+  for (uint32_t c0 = first; c0 < end; c0 += 32) {
+    const uint32_t cell = c0 + lane;
+    uint4 bits = make_uint4(0, 0, 0, 0);
+    if (cell < end) {
+      uint32_t s0, s1, s2, s3;
+      cell_slots(cell, n0, n1, n2, s0, s1, s2, s3);
+      const MrlRow* const p = grid + cell;
+      const uint32_t q0 = 1u << codes[s0], q1 = 1u << codes[n0 + s1], q2 = 1u << codes[n0 + n1 + s2], q3 = 1u << codes[n0 + n1 + n2 + s3];
+      const bool w0 = s0 && !(real.x & q0), w1 = s1 && !(real.y & q1), w2 = s2 && !(real.z & q2), w3 = s3 && !(real.w & q3);
+      if (w0 || w1 || w2 || w3) {
+        const uint4 r = ld_row(p);
+        uint4 x0 = r, x1 = r, x2 = r, x3 = r;
+        if (w0) x0 = ld_row(p - 1);
+        if (w1) x1 = ld_row(p - st1);
+        if (w2) x2 = ld_row(p - st2);
+        if (w3) x3 = ld_row(p - st3);
+        if (x0.x != r.x || x0.y != r.y || x0.z != r.z) bits.x = q0;
+        if (x1.x != r.x || x1.y != r.y || x1.z != r.z) bits.y = q1;
+        if (x2.x != r.x || x2.y != r.y || x2.z != r.z) bits.z = q2;
+        if (x3.x != r.x || x3.y != r.y || x3.z != r.z) bits.w = q3;
+      }
+    }
+    bits = warp_or(bits);
+    real.x |= bits.x; real.y |= bits.y; real.z |= bits.z; real.w |= bits.w;
+  }
+  return real;
+}
+
+// kEarly: of the grids of the unordered phase, else of the working grids (only_dirty: of those that
+// grew or changed).
 template <bool kEarly>
 __device__ __noinline__ void phase_real_masks(const HotArgs a, uint4* rmask, bool only_dirty) {
   const uint32_t lane = threadIdx.x & 31;
   WarpScratch& ws = warp_scratch();
-  const uint8_t* const codes = ws.codes;
   uint32_t w = warp_number();
-  if (w < a.n_items) do {
+  if (w < a.n_items)
+#pragma unroll 1
+  do {
     const WorkItem it = a.items[w];
     const uint32_t i = it.spec, first_cell = it.first_cell & ~31u;
     if (only_dirty && !a.sspec[i].dirty) continue;
     const uint4 m = kEarly ? a.sspec[i].emask : *reinterpret_cast<const uint4*>(&a.hdrs[i]);
     const MrlRow* const grid = kEarly ? a.temp + a.temp_cap + a.sspec[i].erow : a.temp + (a.hdrs[i].row_base & ~MRL_TEMP_FLAG);
-    const uint32_t n0 = __popc(m.x), n1 = __popc(m.y), n2 = __popc(m.z), n3 = __popc(m.w);
-    const uint32_t c_end = min(n0 * n1 * n2 * n3, first_cell + a.item_cells);
-    const uint32_t st1 = n0, st2 = n0 * n1, st3 = st2 * n2;
-    stage_slot_codes(ws.codes, m, n0, n1, n2, n3, lane);
-    uint4 real = make_uint4(1u, 1u, 1u, 1u);   // the same in all lanes
-    for (uint32_t c0 = first_cell; c0 < c_end; c0 += 32) {
-      const uint32_t cell = c0 + lane;
-      uint4 bits = make_uint4(0, 0, 0, 0);
-      if (cell < c_end) {
-        uint32_t rest = cell;
-        const uint32_t s0 = rest % n0; rest /= n0;
-        const uint32_t s1 = rest % n1; rest /= n1;
-        const uint32_t s2 = rest % n2, s3 = rest / n2;
-        const MrlRow* const p = grid + cell;
-        const uint32_t q0 = 1u << codes[s0], q1 = 1u << codes[n0 + s1], q2 = 1u << codes[n0 + n1 + s2], q3 = 1u << codes[n0 + n1 + n2 + s3];
-        const bool w0 = s0 && !(real.x & q0), w1 = s1 && !(real.y & q1), w2 = s2 && !(real.z & q2), w3 = s3 && !(real.w & q3);
-        if (w0 || w1 || w2 || w3) {
-          const uint4 r = ld_row(p);
-          uint4 x0 = r, x1 = r, x2 = r, x3 = r;
-          if (w0) x0 = ld_row(p - 1);
-          if (w1) x1 = ld_row(p - st1);
-          if (w2) x2 = ld_row(p - st2);
-          if (w3) x3 = ld_row(p - st3);
-          if (x0.x != r.x || x0.y != r.y || x0.z != r.z) bits.x = q0;
-          if (x1.x != r.x || x1.y != r.y || x1.z != r.z) bits.y = q1;
-          if (x2.x != r.x || x2.y != r.y || x2.z != r.z) bits.z = q2;
-          if (x3.x != r.x || x3.y != r.y || x3.z != r.z) bits.w = q3;
-        }
-      }
-      bits = warp_or(bits);
-      real.x |= bits.x; real.y |= bits.y; real.z |= bits.z; real.w |= bits.w;
-    }
+    stage_slot_codes(ws.codes, m, __popc(m.x), __popc(m.y), __popc(m.z), __popc(m.w), lane);
+    const uint4 real = real_breakpoints(ws.codes, m, grid, first_cell, min((uint32_t)cells_of(m), first_cell + a.item_cells), lane);
     if (lane == 0) {
       uint32_t* const out = reinterpret_cast<uint32_t*>(&rmask[i]);
       if (real.x & ~1u) atomicOr(out, real.x);
@@ -1221,6 +1290,80 @@ __device__ __noinline__ void phase_real_masks(const HotArgs a, uint4* rmask, boo
       if (real.w & ~1u) atomicOr(out + 3, real.w);
     }
   } while (next_item(a, w, lane));
+}
+
+// Phases 1 to 4 in one, for the small teams: a warp takes a Spec from its records to the real
+// breakpoints of its grid of the unordered phase, without a barrier between. Grids of more than
+// kInlineCells cells become work items for the phases proper. The corner is the first round's: a
+// weaker bound makes more cells, not other rows.
+constexpr uint32_t kInlineCells = 128;
+constexpr uint32_t kWarmLines = 960;   // 120 KB
+__device__ __noinline__ void phase_early_fused(const StageArgs& a, const HotArgs h, StageCtl* sc, uint32_t lo, uint32_t hi, uint32_t gwarp, uint32_t gwarps,
+                                               uint32_t stage, unsigned long long* block_stats) {
+  const uint32_t lane = threadIdx.x & 31;
+  WarpScratch& ws = warp_scratch();
+  Tally tally = {0, 0};
+  #pragma unroll 1
+  for (uint32_t i = lo + gwarp; i < hi; i += gwarps) {
+    if (!computed_here(a, i)) {
+      if (lane == 0) a.rmask[i] = make_uint4(0, 0, 0, 0);   // another rank's Spec: zero until the exchange
+      continue;
+    }
+    uint32_t corner, n_late;
+    const uint2 cl = *reinterpret_cast<const uint2*>(&a.hdrs[i].cand_off);
+    uint4 m;
+    {
+      uint32_t early, late;
+      m = scan_records(a, lo, cl, early, late, n_late, lane);
+      corner = __vminu4(early, late);
+      if (__vcmpgtu4(corner, a.top_pack)) corner = MRL_NEVER4;   // no limits inside the lattice reach it
+    }
+    m = clip_at_corner(m, corner);
+    const unsigned long long cells = cells_of(m);
+    const bool here = cells <= kInlineCells;
+    const uint32_t n_items = here ? 0u : (uint32_t)((cells + h.item_cells - 1) / h.item_cells);
+    unsigned long long row = 0;
+    uint32_t item0 = 0;
+    if (lane == 0) {
+      row = atomicAdd(&sc->rows_early, cells);
+      if (n_items) item0 = atomicAdd(&sc->n_items, n_items);
+    }
+    row = __shfl_sync(0xFFFFFFFFu, row, 0);
+    item0 = __shfl_sync(0xFFFFFFFFu, item0, 0);
+    #pragma unroll 1
+    for (uint32_t w = lane; w < n_items; w += 32) {
+      const uint32_t at = item0 + w;
+      if (at < a.item_cap) {
+        WorkItem it;
+        it.spec = i;
+        it.first_cell = w * h.item_cells;
+        a.items[at] = it;
+      }
+    }
+    uint4 real = make_uint4(1u, 1u, 1u, 1u);
+    if (here && row + cells <= a.temp_cap) {   // (the total is checked behind the barrier)
+      MrlRow* const grid = a.temp + a.temp_cap + row;
+      stage_slot_codes(ws.codes, m, __popc(m.x), __popc(m.y), __popc(m.z), __popc(m.w), lane);
+      solve_early_cells(h, ws, cl.x, cl.y - n_late, m, corner, grid, 0, (uint32_t)cells, tally, lane);
+      __syncwarp();   // the lanes' rows, for the others to compare with
+      real = real_breakpoints(ws.codes, m, grid, 0, (uint32_t)cells, lane);
+    }
+    if (lane == 0) {
+      StageSpec& s = a.sspec[i - lo];
+      s.emask = m;
+      s.erow = row;
+      s.corner = corner;
+      s.n_late = n_late;
+      a.rmask[i] = real;
+      if (n_late) {
+        sc->any_late = stage + 1;   // every writer of a stage stores the same value
+      } else {                      // finished: its grid is that of the unordered phase
+        *reinterpret_cast<uint4*>(&a.hdrs[i]) = m;
+        a.hdrs[i].row_base = (a.temp_cap + row) | MRL_TEMP_FLAG;
+      }
+    }
+  }
+  add_tally(tally, &block_stats[0], &block_stats[1], lane);
 }
 
 // ---- compaction: working grids -> final table ---------------------------------------------
@@ -1254,116 +1397,156 @@ __device__ __noinline__ void phase_count(const StageArgs& a, uint32_t lo, uint32
   uint32_t b_lo, b_hi;
   block_specs(lo, hi, b_lo, b_hi);
   unsigned long long n = 0;
+  #pragma unroll 1
   for (uint32_t i = b_lo + threadIdx.x; i < b_hi; i += kStageBlock) n += cells_of(a.rmask[i]);
   n = block_sum(n);
   if (threadIdx.x == 0) a.block_sums[blockIdx.x] = n;
 }
 
-// Copies each Spec's real cells from its grid to its final rows and repoints the header, a warp per
-// Spec. Specs computed by another rank get zero rows (the exchange adds the owner's rows onto
-// them). Returns the bytes of records and rows the final rows are the combination of.
-__device__ __noinline__ void phase_compact(const StageArgs& a, uint32_t lo, uint32_t hi, unsigned long long first_row) {
-  __shared__ unsigned long long off[kStageBlock];
-  __shared__ unsigned long long warp_base[kStageBlock / 32];
+// Copies each Spec's real cells from its grid to its final rows (from first_row on) and repoints the
+// header, a warp per Spec. Specs computed by another rank get zero rows (the exchange adds the
+// owner's rows onto them). Returns the rows that this block's Specs take.
+__device__ __noinline__ unsigned long long phase_compact(const StageArgs& a, uint32_t lo, uint32_t hi, unsigned long long first_row,
+                                                         unsigned long long* block_bytes) {
+  __shared__ uint32_t off[kStageBlock];
+  __shared__ uint32_t warp_base[kStageBlock / 32 + 1];
   const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  WarpScratch& ws = warp_scratch();
   uint32_t b_lo, b_hi;
   block_specs(lo, hi, b_lo, b_hi);
-  unsigned long long bytes = 0;
+  const bool few = b_hi - b_lo <= 32;   // then every warp works the places out by itself
+  unsigned long long bytes = 0, taken = 0;
+#pragma unroll 1
   for (uint32_t base = b_lo; base < b_hi; base += kStageBlock) {
     // places of the next kStageBlock Specs
-    const uint32_t own = base + threadIdx.x;
-    const unsigned long long n_own = own < b_hi ? cells_of(a.rmask[own]) : 0ull;
-    unsigned long long inc = n_own;
+    const uint32_t own = base + (few ? lane : threadIdx.x);
+    const uint32_t n_own = own < b_hi ? (uint32_t)cells_of(a.rmask[own]) : 0u;
+    uint32_t inc = n_own;
     for (int o = 1; o < 32; o <<= 1) {
-      const unsigned long long t = __shfl_up_sync(0xFFFFFFFFu, inc, o);
+      const uint32_t t = __shfl_up_sync(0xFFFFFFFFu, inc, o);
       if (lane >= (uint32_t)o) inc += t;
     }
-    __syncthreads();
-    off[threadIdx.x] = inc - n_own;
-    if (lane == 31) warp_base[warp] = inc;
-    __syncthreads();
-    if (warp == 0) {
-      const unsigned long long v = lane < kStageBlock / 32 ? warp_base[lane] : 0ull;
-      unsigned long long s = v;
-      for (int o = 1; o < 32; o <<= 1) {
-        const unsigned long long t = __shfl_up_sync(0xFFFFFFFFu, s, o);
-        if (lane >= (uint32_t)o) s += t;
+    if (!few) {
+      __syncthreads();   // the run before has been read
+      off[threadIdx.x] = inc - n_own;
+      if (lane == 31) warp_base[warp] = inc;
+      __syncthreads();
+      if (warp == 0) {
+        const uint32_t v = warp_base[lane];
+        uint32_t s = v;
+        for (int o = 1; o < 32; o <<= 1) {
+          const uint32_t t = __shfl_up_sync(0xFFFFFFFFu, s, o);
+          if (lane >= (uint32_t)o) s += t;
+        }
+        warp_base[lane] = s - v;
+        if (lane == 31) warp_base[32] = s;
       }
-      if (lane < kStageBlock / 32) warp_base[lane] = s - v;
+      __syncthreads();
     }
-    __syncthreads();
     const uint32_t here = min((uint32_t)kStageBlock, b_hi - base);
-    unsigned long long last = 0;
+#pragma unroll 1
     for (uint32_t k = warp; k < here; k += kStageBlock / 32) {
       const uint32_t i = base + k;
-      const unsigned long long fbase = first_row + warp_base[k >> 5] + off[k];
-      const uint4 fm = a.rmask[i];
+      const uint32_t place = few ? __shfl_sync(0xFFFFFFFFu, inc - n_own, k) : warp_base[k >> 5] + off[k];
+      const unsigned long long fbase = first_row + taken + place;
+      const uint4 fm = a.rmask[i], tm = *reinterpret_cast<const uint4*>(&a.hdrs[i]);
+      const unsigned long long tbase = a.hdrs[i].row_base;
+      const uint2 cl = *reinterpret_cast<const uint2*>(&a.hdrs[i].cand_off);
       const uint32_t f0 = __popc(fm.x), f1 = __popc(fm.y), f2 = __popc(fm.z), f3 = __popc(fm.w), n = f0 * f1 * f2 * f3;
       MrlRow* const to = a.rows + fbase;
       if (computed_here(a, i)) {
-        const uint4 tm = *reinterpret_cast<const uint4*>(&a.hdrs[i]);
-        const MrlRow* const from = row_at(a.rows, a.temp, a.hdrs[i].row_base);
-        const uint32_t t0 = __popc(tm.x), t1 = __popc(tm.y), t2 = __popc(tm.z);
+        // (for the statistics below)
+        const uint4 rec0 = lane < cl.y ? __ldg(reinterpret_cast<const uint4*>(&a.cands[cl.x + lane])) : make_uint4(0, 0, 0, 0);
+        const MrlRow* const from = row_at(a.rows, a.temp, tbase);
         const bool same = tm.x == fm.x && tm.y == fm.y && tm.z == fm.z && tm.w == fm.w;
+        if (!same) {   // the grid's slot of every final slot, memory after memory
+          __syncwarp();   // the Spec before has been read by every lane
+#pragma unroll 1
+          for (uint32_t t = lane; t < f0 + f1 + f2 + f3; t += 32) {
+            uint32_t mk = fm.x, tk = tm.x, slot = t;
+            if (slot >= f0) { slot -= f0; mk = fm.y; tk = tm.y; if (slot >= f1) { slot -= f1; mk = fm.z; tk = tm.z; if (slot >= f2) { slot -= f2; mk = fm.w; tk = tm.w; } } }
+            ws.codes[t] = (uint8_t)(__popc(tk & below(nth_set_bit(mk, slot))) - 1);
+          }
+          __syncwarp();
+        }
+        const uint32_t t0 = __popc(tm.x), t1 = __popc(tm.y), t2 = __popc(tm.z);
+#pragma unroll 1
         for (uint32_t j = lane; j < n; j += 32) {
           uint32_t toff = j;
           if (!same) {
-            uint32_t rest = j;
-            const uint32_t j0 = rest % f0; rest /= f0;
-            const uint32_t j1 = rest % f1; rest /= f1;
-            const uint32_t j2 = rest % f2, j3 = rest / f2;
-            const uint32_t i0 = __popc(tm.x & below(nth_set_bit(fm.x, j0))) - 1;
-            const uint32_t i1 = __popc(tm.y & below(nth_set_bit(fm.y, j1))) - 1;
-            const uint32_t i2 = __popc(tm.z & below(nth_set_bit(fm.z, j2))) - 1;
-            const uint32_t i3 = __popc(tm.w & below(nth_set_bit(fm.w, j3))) - 1;
-            toff = ((i3 * t2 + i2) * t1 + i1) * t0 + i0;
+            uint32_t j0, j1, j2, j3;
+            cell_slots(j, f0, f1, f2, j0, j1, j2, j3);
+            toff = ((ws.codes[f0 + f1 + f2 + j3] * t2 + ws.codes[f0 + f1 + j2]) * t1 + ws.codes[f0 + j1]) * t0 + ws.codes[j0];
           }
           uint4 r = ld_row(from + toff);
           r.w = 0;
           *reinterpret_cast<uint4*>(to + j) = r;
         }
         // statistics: 12 bytes per row, 16 per record, 16 per child of every record that fits the row's limits
-        const uint2 cl = *reinterpret_cast<const uint2*>(&a.hdrs[i].cand_off);
         if (lane == 0) bytes += n * (12ull + 16ull * cl.y);
+        #pragma unroll 1
         for (uint32_t c = lane; c < cl.y; c += 32) {
-          const uint4 rec = __ldg(reinterpret_cast<const uint4*>(&a.cands[cl.x + c]));
+          const uint4 rec = c < 32 ? rec0 : __ldg(reinterpret_cast<const uint4*>(&a.cands[cl.x + c]));
           const uint32_t kind = (rec.x >> 16) & 0xFFu, nchild = rec.x >> 24;
-          unsigned long long feasible = n;
+          uint32_t feasible = n;
           if (kind == MRL_CK_MOVE) {
             const uint32_t ml = sel4(fm.x, fm.y, fm.z, fm.w, rec.z & 0xFFu), thr = (rec.z >> 8) & 0xFFu;
             feasible = n / (uint32_t)__popc(ml) * (uint32_t)__popc(ml >> thr);   // final cells at or above the threshold
           }
-          bytes += feasible * nchild * 16ull;
+          bytes += (unsigned long long)feasible * nchild * 16ull;
         }
       } else {
+        #pragma unroll 1
         for (uint32_t j = lane; j < n; j += 32) *reinterpret_cast<uint4*>(to + j) = make_uint4(0, 0, 0, 0);
       }
-      __syncwarp();   // the header is repointed when every lane has read it, and the corner read off rows that are written
+      __syncwarp();   // the header has been read by every lane, and the rows are there for the corner
+      uint32_t corner = 0;
+      if (!a.mine) corner = corner_from_rows(fm, to, lane);
       if (lane == 0) {
         *reinterpret_cast<uint4*>(&a.hdrs[i]) = fm;
         a.hdrs[i].row_base = fbase;
-        if (!a.mine) a.minsat[i] = corner_from_rows(fm, to);
+        if (!a.mine) a.minsat[i] = corner;
       }
     }
-    last = warp_base[kStageBlock / 32 - 1] + off[kStageBlock - 1];
-    {
-      // the last Spec's cells end the run
-      const uint32_t q = base + kStageBlock - 1;
-      if (q < b_hi) last += cells_of(a.rmask[q]);
-    }
-    first_row += last;   // only used when another run follows, and then this one is full
+    taken += few ? __shfl_sync(0xFFFFFFFFu, inc, 31) : warp_base[32];
   }
   for (int o = 16; o > 0; o >>= 1) bytes += __shfl_xor_sync(0xFFFFFFFFu, bytes, o);
-  if (lane == 0 && bytes) atomicAdd(&a.ctl->st_final_bytes, bytes);
+  if (lane == 0 && bytes) atomicAdd(block_bytes, bytes);
+  return taken;
 }
 
-// What the phases of a stage count and hand out; zero at its start.
-__device__ __forceinline__ void reset_stage_ctl(FillCtl* ctl) {
-  ctl->rows_early = ctl->rows_late = 0;
-  ctl->n_items = 0;
-  ctl->any_changed = ctl->grew = 0;
-#pragma unroll
-  for (int k = 0; k < 8; k++) ctl->next_item[k] = 0;
+// Out of line: a grid-wide barrier is a hundred instructions, a stage has a dozen of them, and what a small
+// stage waits for is instructions.
+__device__ __noinline__ void team_barrier(uint32_t team) {
+  if (team == TEAM_GRID) {
+    cg::this_grid().sync();
+  } else if (team == TEAM_CLUSTER) {
+    asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+  } else {
+    __syncthreads();
+  }
+}
+
+// A block alone reads and writes everything through its own L1, where a hit takes a tenth of the 700
+// cycles that a dependent read from L2 was measured to take here, and a small plan is nothing but chains
+// of such reads. So what the run touches is brought in at its start, as far as L1 reaches; stores
+// update what they hit.
+__device__ __noinline__ void warm_l1(const StageArgs& a) {
+  const uint32_t lo = __ldg(&a.stages[a.stage_lo]).x, hi = __ldg(&a.stages[a.stage_hi - 1]).y, n = hi - lo;
+  uint32_t acc = 0, left = kWarmLines;
+  auto touch = [&](const void* p, size_t bytes) {
+    const uint32_t lines = (uint32_t)min((size_t)left, (bytes + 127) / 128);
+    #pragma unroll 1
+    for (uint32_t k = threadIdx.x; k < lines; k += kStageBlock) acc ^= *reinterpret_cast<const uint32_t*>(static_cast<const char*>(p) + k * 128u);
+    left -= lines;
+  };
+  const SpecHdr* const h = a.hdrs + lo;
+  touch(h, n * sizeof(SpecHdr));
+  const uint32_t c_lo = h[0].cand_off, c_hi = h[n - 1].cand_off + h[n - 1].ncand;
+  touch(a.rmask + lo, n * sizeof(uint4));
+  touch(a.minsat + lo, n * sizeof(uint32_t));
+  touch(a.cands + c_lo, (size_t)(c_hi - c_lo) * sizeof(CandRec));
+  if (acc == 0x9E3779B9u && left > kWarmLines) a.ctl->scratch[0] = acc;   // (never: the loads are to be made)
 }
 
 // A run of stages, each start to finish, by one team of blocks: the grid (cooperative launch), one
@@ -1383,25 +1566,28 @@ __global__ void __launch_bounds__(kStageBlock, 1) stage_kernel(const __grid_cons
   uint32_t syncs = 0;
   auto team_sync = [&]() {
     syncs++;
-    if (a.team == TEAM_GRID) {
-      cg::this_grid().sync();
-    } else if (a.team == TEAM_CLUSTER) {
-      asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
-    } else {
-      __syncthreads();
-    }
+    team_barrier(a.team);
   };
   if (ctl->error) return;   // an earlier stage failed: the host repairs and resumes (uniform: nothing writes it before the first barrier)
-  __shared__ unsigned long long block_stats[5];   // candidates evaluated and rows gathered by the unordered phase; by the sweeps; items the sweeps solved cells of
-  if (threadIdx.x < 5) block_stats[threadIdx.x] = 0;
+  // statistics of the block: candidates evaluated and rows gathered by the unordered phase; by the
+  // sweeps; items the sweeps solved cells of; bytes of the finished rows
+  __shared__ unsigned long long block_stats[6], phase_ns[8];
+  __shared__ StageCtl own_ctl;
+  StageCtl* const sc = a.team == TEAM_BLOCK ? &own_ctl : &ctl->stage;
+  if (threadIdx.x < 6) block_stats[threadIdx.x] = 0;
+  if (threadIdx.x < 8) phase_ns[threadIdx.x] = 0;
+  if (threadIdx.x < sizeof(StageCtl) / 4) reinterpret_cast<uint32_t*>(&own_ctl)[threadIdx.x] = 0;
   __syncthreads();
+  auto get = [](const auto* p) { return *reinterpret_cast<const volatile std::remove_const_t<std::remove_pointer_t<decltype(p)>>*>(p); };   // past L1: others write it
   unsigned long long final_top = ctl->final_top;   // rows of the table; written below behind a barrier
   unsigned long long t_last = 0, st_cells = 0, st_early = 0;
   uint32_t n_sweeps = 0, n_passes = 0;
   if (gtid == 0) asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t_last));
   // device time since the last mark goes to part ph (thread 0 only; after a barrier)
 #define MARK(ph) do { if (gtid == 0) { unsigned long long t_now; asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t_now)); \
-                                       ctl->st_phase_ns[ph] += t_now - t_last; t_last = t_now; } } while (0)
+                                       phase_ns[ph] += t_now - t_last; t_last = t_now; } } while (0)
+  if (a.team == TEAM_BLOCK) warm_l1(a);
+  #pragma unroll 1
   for (uint32_t st = a.stage_lo; st < a.stage_hi; st++) {
     const uint2 ids = __ldg(&a.stages[st]);
     const uint32_t lo = ids.x, hi = ids.y;
@@ -1413,8 +1599,8 @@ __global__ void __launch_bounds__(kStageBlock, 1) stage_kernel(const __grid_cons
       h.items = a.items; h.item_cells = item_size(hi - lo, gwarps); h.n_items = 0; h.next_item = nullptr;
       auto hand_out = [&](uint32_t n_items) {
         h.n_items = n_items;
-        h.next_item = &ctl->next_item[ph & 7];
-        if (gtid == 0) ctl->next_item[(ph + 4) & 7] = 0;
+        h.next_item = &sc->next_item[ph & 7];
+        if (gtid == 0) sc->next_item[(ph + 4) & 7] = 0;
         ph++;
       };
       auto too_small = [&](unsigned long long rows_early, unsigned long long rows_late, unsigned long long items) {
@@ -1428,39 +1614,51 @@ __global__ void __launch_bounds__(kStageBlock, 1) stage_kernel(const __grid_cons
         return true;
       };
       if (a.mine && st) {
-        phase_minsat(a, __ldg(&a.stages[st - 1]).x, __ldg(&a.stages[st - 1]).y, gtid, gthreads);
+        phase_minsat(a, __ldg(&a.stages[st - 1]).x, __ldg(&a.stages[st - 1]).y, gwarp, gwarps);
         team_sync();
       }
-      phase_records(a, lo, hi, gwarp, gwarps, st);
-      team_sync();
-      const bool any_late = __ldcg(&ctl->any_late) == st + 1;
-      phase_place_early(a, lo, hi, gwarp, gwarps, any_late);
-      team_sync();
-      const unsigned long long cells = __ldcg(&ctl->rows_early);
-      const uint32_t n_early_items = __ldcg(&ctl->n_items);
+      const bool fused = a.team != TEAM_GRID;
+      bool any_late;
+      if (fused) {
+        phase_early_fused(a, h, sc, lo, hi, gwarp, gwarps, st, block_stats);
+        team_sync();
+        any_late = get(&sc->any_late) == st + 1;
+        MARK(MRL_PH_EARLY);
+      } else {
+        phase_records(a, sc, lo, hi, gwarp, gwarps, st);
+        team_sync();
+        any_late = get(&sc->any_late) == st + 1;
+        phase_place_early(a, sc, lo, hi, gwarp, gwarps, any_late);
+        team_sync();
+        MARK(MRL_PH_SETUP);
+      }
+      const unsigned long long cells = get(&sc->rows_early);
+      const uint32_t n_early_items = get(&sc->n_items);
       failed = too_small(cells, 0, n_early_items);
       if (!failed && cells) {
-        MARK(MRL_PH_SETUP);
-        hand_out(n_early_items);
-        phase_early(h, block_stats);
         st_cells += cells;
         st_early += cells;
-        team_sync();
-        MARK(MRL_PH_EARLY);
-        if (gtid == 0) ctl->n_items = 0;   // read above, behind a barrier; used again from phase_place_late on
-        hand_out(n_early_items);
-        phase_real_masks<true>(h, a.rmask, false);
-        team_sync();
-        MARK(MRL_PH_EARLY_MASKS);
+        if (n_early_items) {
+          hand_out(n_early_items);
+          phase_early(h, block_stats);
+          team_sync();
+          MARK(MRL_PH_EARLY);
+          if (gtid == 0) sc->n_items = 0;   // read above, behind a barrier; used again from phase_place_late on
+          hand_out(n_early_items);
+          phase_real_masks<true>(h, a.rmask, false);
+          team_sync();
+          MARK(MRL_PH_EARLY_MASKS);
+        }
         uint32_t sweep = 0;
         unsigned long long rows_before = 0;
-        if (!any_late) phase_place_late(a, lo, hi, gwarp, gwarps, 0);   // headers only; the places of the rows need no barrier behind it
+        if (!any_late && !fused) phase_place_late(a, sc, lo, hi, gwarp, gwarps, 0);   // headers only; the places of the rows need no barrier behind it
+        #pragma unroll 1
         for (uint32_t pass = 0; any_late; pass++) {
           if (pass >= (uint32_t)kMaxPasses) { failed = true; if (gtid == 0) { ctl->failed_stage = st; ctl->error |= MRL_ERR_PASSES; } break; }
-          phase_place_late(a, lo, hi, gwarp, gwarps, pass);
+          phase_place_late(a, sc, lo, hi, gwarp, gwarps, pass);
           team_sync();
-          const unsigned long long rows = __ldcg(&ctl->rows_late);
-          const uint32_t n_items = __ldcg(&ctl->n_items);
+          const unsigned long long rows = get(&sc->rows_late);
+          const uint32_t n_items = get(&sc->n_items);
           if ((failed = too_small(0, rows, n_items))) break;
           MARK(MRL_PH_PASS_SETUP);
           if (pass) {
@@ -1469,25 +1667,27 @@ __global__ void __launch_bounds__(kStageBlock, 1) stage_kernel(const __grid_cons
             team_sync();
             MARK(MRL_PH_INIT);
           } else {
+            #pragma unroll 1
             for (uint32_t i = lo + gtid; i < hi; i += gthreads)   // what the unordered phase found real has been used
               if (computed_here(a, i) && a.sspec[i - lo].n_late) a.rmask[i] = make_uint4(1u, 1u, 1u, 1u);
           }
           st_cells += rows - rows_before;
           rows_before = rows;
           const uint32_t sweep_before = sweep;
+          #pragma unroll 1
           for (bool first = true;; first = false) {
             sweep++;
             uint4* const now = a.changed[sweep % 3], *const idle = a.changed[(sweep + 1) % 3];
             const uint4* const before = a.changed[(sweep + 2) % 3];
             if (sweep > 1)   // the first sweeps' are zero from phase_place_late
+              #pragma unroll 1
               for (uint32_t i = gtid; i < hi - lo; i += gthreads) idle[i] = make_uint4(0, 0, 0, 0);
             hand_out(n_items);
-            if (!first) phase_sweep<SWEEP_CHANGED>(h, lo, before, now, sweep, &ctl->any_changed, block_stats);
-            else if (pass) phase_sweep<SWEEP_NEW>(h, lo, before, now, sweep, &ctl->any_changed, block_stats);
-            else phase_sweep<SWEEP_ALL>(h, lo, before, now, sweep, &ctl->any_changed, block_stats);
+            if (first && !pass) phase_sweep<true>(h, SWEEP_ALL, lo, before, now, sweep, &sc->any_changed, block_stats);
+            else phase_sweep<false>(h, first ? SWEEP_NEW : SWEEP_CHANGED, lo, before, now, sweep, &sc->any_changed, block_stats);
             team_sync();
             MARK(first ? MRL_PH_SWEEP_FIRST : MRL_PH_SWEEP_MORE);
-            if (__ldcg(&ctl->any_changed) != sweep) break;   // nothing changed anywhere: the stage's cells are consistent
+            if (get(&sc->any_changed) != sweep) break;   // nothing changed anywhere: the stage's cells are consistent
             if (sweep - sweep_before >= (uint32_t)kMaxSweeps) {   // more sweeps than the limits lattice has diagonals: give up rather than spin
               failed = true;
               if (gtid == 0) { ctl->failed_stage = st; ctl->error |= MRL_ERR_PASSES; }
@@ -1498,39 +1698,51 @@ __global__ void __launch_bounds__(kStageBlock, 1) stage_kernel(const __grid_cons
           n_sweeps += sweep - sweep_before;
           n_passes++;
           if (pass) {
+            #pragma unroll 1
             for (uint32_t i = lo + gtid; i < hi; i += gthreads)
               if (computed_here(a, i) && a.sspec[i - lo].n_late && a.sspec[i - lo].dirty) a.rmask[i] = make_uint4(1u, 1u, 1u, 1u);
             team_sync();
           }
-          if (gtid == 0) ctl->n_items = 0;
+          if (gtid == 0) sc->n_items = 0;
           hand_out(n_items);
           phase_real_masks<false>(h, a.rmask, pass != 0);
           team_sync();
-          phase_check_grids(a, lo, hi, gwarp, gwarps, pass);
-          if (a.place) phase_count(a, lo, hi);   // for when no grid grows
+          phase_check_grids(a, sc, lo, hi, gwarp, gwarps, pass);
+          if (a.place && gridDim.x > 1) phase_count(a, lo, hi);   // for when no grid grows
           team_sync();
           MARK(MRL_PH_PASS_MASKS);
-          if (__ldcg(&ctl->grew) != pass + 1) break;   // every working grid is consistent
+          if (get(&sc->grew) != pass + 1) break;   // every working grid is consistent
         }
-        if (!any_late && !failed) {
+        if (!any_late && !failed && gridDim.x > 1) {
           if (a.place) phase_count(a, lo, hi);
           team_sync();
         }
       }
-    } else {
+    } else if (gridDim.x > 1) {
       phase_count(a, lo, hi);
       team_sync();
     }
     if (!failed && a.place) {
       unsigned long long before = 0, total = 0;
-      for (uint32_t b = threadIdx.x; b < gridDim.x; b += kStageBlock) {
-        const unsigned long long v = __ldcg(&a.block_sums[b]);
-        total += v;
-        if (b < blockIdx.x) before += v;
+      bool fits = false;
+      if (gridDim.x > 1) {
+        #pragma unroll 1
+        for (uint32_t b = threadIdx.x; b < gridDim.x; b += kStageBlock) {
+          const unsigned long long v = get(&a.block_sums[b]);
+          total += v;
+          if (b < blockIdx.x) before += v;
+        }
+        before = block_sum(before);
+        total = block_sum(total);
+      } else {   // a block alone learns its total from the compaction, where no total could be too large
+        fits = a.solve && final_top + get(&sc->rows_early) + get(&sc->rows_late) <= a.row_cap;
+        if (!fits) {
+          #pragma unroll 1
+          for (uint32_t i = lo + threadIdx.x; i < hi; i += kStageBlock) total += cells_of(a.rmask[i]);
+          total = block_sum(total);
+        }
       }
-      before = block_sum(before);
-      total = block_sum(total);
-      if (final_top + total > a.row_cap) {   // uniform
+      if (!fits && final_top + total > a.row_cap) {   // uniform
         failed = true;
         if (gtid == 0) {
           ctl->failed_stage = st;
@@ -1538,26 +1750,33 @@ __global__ void __launch_bounds__(kStageBlock, 1) stage_kernel(const __grid_cons
           ctl->need_rows = final_top + total;
         }
       } else {
-        phase_compact(a, lo, hi, final_top + before);
+        const unsigned long long taken = phase_compact(a, lo, hi, final_top + before, &block_stats[5]);
+        if (gridDim.x == 1) total = taken;
+        __syncthreads();   // the counters read above are cleared below
         if (gtid == 0) {
           ctl->stage_first_row = final_top;
           ctl->stage_rows = total;
-          reset_stage_ctl(ctl);
+          sc->rows_early = sc->rows_late = 0;
+          sc->n_items = sc->any_changed = sc->grew = 0;
+#pragma unroll
+          for (int k = 0; k < 8; k++) sc->next_item[k] = 0;
         }
         final_top += total;
         if (gtid == 0) ctl->final_top = final_top;
         if (st + 1 < a.stage_hi) team_sync();
+        MARK(MRL_PH_SETUP);
       }
     }
     if (failed) break;   // uniform
   }
 #undef MARK
   __syncthreads();
-  if (threadIdx.x == 0 && (block_stats[0] | block_stats[1] | block_stats[2] | block_stats[4])) {
+  if (threadIdx.x == 0 && (block_stats[0] | block_stats[1] | block_stats[2] | block_stats[4] | block_stats[5])) {
     atomicAdd(&ctl->st_cands, block_stats[0] + block_stats[2]);
     atomicAdd(&ctl->st_lookups, block_stats[1] + block_stats[3]);
     atomicAdd(&ctl->st_late_cands, block_stats[2]);
     atomicAdd(&ctl->st_late_items, block_stats[4]);
+    atomicAdd(&ctl->st_final_bytes, block_stats[5]);
   }
   if (gtid == 0) {
     ctl->st_sweeps += n_sweeps;
@@ -1565,6 +1784,7 @@ __global__ void __launch_bounds__(kStageBlock, 1) stage_kernel(const __grid_cons
     ctl->st_cells += st_cells;
     ctl->st_early_cells += st_early;
     ctl->st_syncs += syncs;
+    for (int k = 0; k < 8; k++) ctl->st_phase_ns[k] += phase_ns[k];
   }
 }
 
@@ -1637,6 +1857,86 @@ lookup_packed_kernel(const mrl::DpTables t, const SpecHdr* hdrs, const MrlRow* r
     r.w = 0;
   }
   *reinterpret_cast<uint4*>(out + i) = r;
+}
+
+// The implementation tree of one Spec: from its row, the record with the stored action, that record's
+// sub-Specs at the limits the action leaves them, and so on, level by level; a node per warp, its
+// records over the lanes. The host turns the nodes into text. One block: a tree has tens of nodes, and a
+// level costs four dependent reads.
+constexpr uint32_t kWalkMost = 2048;
+__global__ void __launch_bounds__(kBlock)
+walk_kernel(const mrl::DpTables t, const unsigned long long* desc, const SpecHdr* hdrs, const CandRec* __restrict__ cands, const MrlRow* rows,
+            uint32_t n_specs, unsigned long long root, uint32_t root_is_packed, uint32_t cpack, mrl::WalkNode* nodes, uint32_t* count) {
+  __shared__ uint32_t n, level_end;
+  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (threadIdx.x == 0) {
+    mrl::WalkNode r;
+    memset(&r, 0, sizeof(r));
+    r.cpack = cpack;
+    r.id = (uint32_t)root;
+    if (root_is_packed) {
+      const uint32_t pos = mrl::dp_pos(t, t.fams[root >> 48], (uint32_t)(root >> 32) & 0xFFFFu, (uint32_t)(root >> 16) & 0xFFFFu, (uint32_t)root & 0xFFFFu);
+      r.id = (t.rank[pos >> 5].x >> (pos & 31u)) & 1u ? mrl::dp_id(t, pos) : 0xFFFFFFFFu;
+    }
+    nodes[0] = r;
+    n = level_end = 1;
+  }
+  __syncthreads();
+  uint32_t lo = 0;
+  for (uint32_t depth = 0; depth < 512 && lo < level_end; depth++) {
+    const uint32_t hi = level_end;
+    for (uint32_t k = lo + warp; k < hi; k += kBlock / 32) {
+      const uint32_t id = nodes[k].id, cp = nodes[k].cpack;
+      if (id >= n_specs) { if (lane == 0) nodes[k].status = mrl::WALK_NO_SPEC; continue; }
+      const uint4 r = lookup(hdrs, rows, rows, id, below(code_of(cp, 0)), below(code_of(cp, 1)), below(code_of(cp, 2)), below(code_of(cp, 3)));
+      if (lane == 0) {
+        nodes[k].spec = desc ? desc[id] : 0ull;
+        nodes[k].main = r.x; nodes[k].peaks = r.y; nodes[k].tail = r.z;
+      }
+      if (r.z == MRL_UNSAT) { if (lane == 0) nodes[k].status = mrl::WALK_UNSAT; continue; }
+      const uint2 cl = *reinterpret_cast<const uint2*>(&hdrs[id].cand_off);
+      bool found = false;
+      for (uint32_t c0 = 0; c0 < cl.y && !found; c0 += 32) {
+        const uint32_t c = c0 + lane;
+        const uint32_t head = c < cl.y ? __ldg(reinterpret_cast<const uint32_t*>(&cands[cl.x + c])) : 0u;
+        const bool hit = c < cl.y && (head & 0xFFFFu) == (r.z & 0xFFFFu);
+        found = __any_sync(0xFFFFFFFFu, hit);
+        if (!hit) continue;
+        const CandRec rec = cands[cl.x + c];
+        uint32_t child_cp = cp;
+        if (rec.kind == MRL_CK_MOVE) {
+          const uint32_t lv = code_of(cp, rec.level), q = lv >= rec.thr_code ? child_code(rec.level, lv, rec.units) : 0u;
+          child_cp = (cp & ~(0xFFu << (8 * rec.level))) | (q << (8 * rec.level));
+          if (lv < rec.thr_code) nodes[k].status = mrl::WALK_BAD;
+        }
+        const uint32_t at = atomicAdd(&n, (uint32_t)rec.nchild);
+        nodes[k].first_child = at;
+        nodes[k].n_child = rec.nchild;
+        for (uint32_t j = 0; j < rec.nchild; j++)
+          if (at + j < kWalkMost) {
+            mrl::WalkNode q;
+            memset(&q, 0, sizeof(q));
+            q.id = rec.child[j];
+            q.cpack = child_cp;
+            nodes[at + j] = q;
+          }
+      }
+      if (!found && lane == 0) nodes[k].status = mrl::WALK_BAD;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) level_end = min(n, kWalkMost);
+    lo = hi;
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) *count = n;
+}
+
+// The finished table's headers as the two arrays a bulk export hands out.
+__global__ void __launch_bounds__(kBlock) export_headers_kernel(const SpecHdr* hdrs, uint32_t n_specs, uint4* masks, unsigned long long* first_row) {
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n_specs) return;
+  masks[i] = *reinterpret_cast<const uint4*>(&hdrs[i]);
+  first_row[i] = hdrs[i].row_base;
 }
 
 __device__ __forceinline__ unsigned long long mix64(unsigned long long z) {
@@ -2072,7 +2372,7 @@ int DeviceFill::plan(const OpTables& tab) {
   for (const Part& q : parts) if (q.bytes) memcpy(static_cast<unsigned char*>(h_stage_) + q.off, q.src, q.bytes);
   const size_t word_bytes = align256((size_t)n_words * sizeof(u32));
   if ((rc = reserve_(b_ctl_, 512)) || (rc = reserve_(b_tables_, bytes)) || (rc = reserve_(b_bits_, word_bytes + (size_t)tab.n_positions * sizeof(u64))) ||
-      (rc = reserve_(b_rank_, (size_t)n_words * sizeof(uint2))) || (rc = reserve_(b_stage_lo_, back + (size_t)coop_blocks_ * 16)))
+      (rc = reserve_(b_rank_, (size_t)n_words * sizeof(uint2))) || (rc = reserve_(b_stage_lo_, back + (size_t)plan_blocks_ * n_sm_ * sizeof(unsigned long long))))
     return rc == -5 ? 1 : rc;
   d_ctl_ = static_cast<FillCtl*>(b_ctl_.p);
   CK(cudaMemcpyAsync(b_tables_.p, h_stage_, bytes, cudaMemcpyHostToDevice, stream_));
@@ -2109,7 +2409,7 @@ int DeviceFill::plan(const OpTables& tab) {
   // A warp per Spec: the grid follows the positions, up to what is co-resident. While positions are
   // few, headers and records for all of them are reserved ahead and one launch does everything;
   // otherwise the sizes come back after the closure, and again after the records are counted.
-  const u32 max_blocks = (u32)std::min(plan_blocks_ * n_sm_, coop_blocks_);
+  const u32 max_blocks = (u32)(plan_blocks_ * n_sm_);
   auto blocks = [&](uint64_t specs) { return (int)std::min<uint64_t>(max_blocks, std::max<uint64_t>(8, (specs + 7) / 8)); };
   uint64_t want_specs = 0, want_cands = 0;
   if (!fixed_) {
@@ -2519,6 +2819,109 @@ int DeviceFill::lookup_packed(const uint64_t* specs, const uint32_t* cpacks, siz
                            lookup_packed_kernel<<<(unsigned)((m + kBlock - 1) / kBlock), kBlock, 0, stream_>>>(
                                tab_->t, d_hdrs_, d_rows_, static_cast<const PackedQuery*>(q), m, d_out);
                          });
+}
+
+int DeviceFill::walk(uint64_t root, bool packed, uint32_t cpack, std::vector<WalkNode>& out) {
+  std::lock_guard<std::mutex> guard(lookup_mu_);
+  CK(cudaSetDevice(device_));
+  if (packed && !tab_) { snprintf(err_, sizeof(err_), "no plan made on the device"); return -3; }
+  const size_t head = align256(sizeof(uint32_t)), bytes = head + kWalkMost * sizeof(WalkNode), first = head + 96 * sizeof(WalkNode);
+  int rc;
+  if ((rc = reserve_(b_lookup_, bytes, false)) || (rc = reserve_host_(bytes))) return rc;
+  unsigned char* const d = static_cast<unsigned char*>(b_lookup_.p);
+  DpTables t;
+  memset(&t, 0, sizeof(t));
+  if (tab_) t = tab_->t;
+  walk_kernel<<<1, kBlock, 0, stream_>>>(t, tab_ ? static_cast<const unsigned long long*>(b_desc_.p) : nullptr, d_hdrs_, d_cands_, d_rows_, n_specs_,
+                                         root, packed ? 1u : 0u, cpack, reinterpret_cast<WalkNode*>(d + head), reinterpret_cast<uint32_t*>(d));
+  CK(cudaGetLastError());
+  unsigned char* const h = static_cast<unsigned char*>(h_stage_);
+  CK(cudaMemcpyAsync(h, d, first, cudaMemcpyDeviceToHost, stream_));   // most trees are smaller than this
+  CK(cudaStreamSynchronize(stream_));
+  const uint32_t n = *reinterpret_cast<const uint32_t*>(h);
+  if (n > kWalkMost) return 1;
+  if (head + n * sizeof(WalkNode) > first) {
+    CK(cudaMemcpyAsync(h + first, d + first, head + n * sizeof(WalkNode) - first, cudaMemcpyDeviceToHost, stream_));
+    CK(cudaStreamSynchronize(stream_));
+  }
+  const WalkNode* const nodes = reinterpret_cast<const WalkNode*>(h + head);
+  out.assign(nodes, nodes + n);
+  return 0;
+}
+
+// Device memory into pageable memory of the caller's, which is often fresh: the driver's own staging
+// runs on one thread, and half of its time goes into page faults. Large parts are brought over in
+// pieces by a few threads, each through two pinned buffers of its own.
+int DeviceFill::read_bulk_(void* out, const void* src, size_t bytes) {
+  const size_t piece = size_t(2) << 20;
+  if (bytes < 4 * piece || fixed_) {
+    if (bytes) CK(cudaMemcpyAsync(out, src, bytes, cudaMemcpyDeviceToHost, stream_));
+    CK(cudaStreamSynchronize(stream_));
+    return 0;
+  }
+  CK(cudaStreamSynchronize(stream_));
+  const int n_threads = 4;
+  int rc = reserve_host_(n_threads * 2 * piece);
+  if (rc) return rc;
+  std::atomic<size_t> next{0};
+  std::atomic<int> error{0};
+  const size_t pieces = (bytes + piece - 1) / piece;
+  auto work = [&](int t) {
+    unsigned char* const pin = static_cast<unsigned char*>(h_stage_) + (size_t)t * 2 * piece;
+    cudaStream_t st = nullptr;
+    cudaEvent_t ev[2] = {nullptr, nullptr};
+    cudaError_t e = cudaSetDevice(device_);
+    if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking);
+    for (int b = 0; b < 2 && e == cudaSuccess; b++) e = cudaEventCreateWithFlags(&ev[b], cudaEventDisableTiming);
+    size_t at[2] = {pieces, pieces};   // piece under way in each buffer
+    for (int b = 0; e == cudaSuccess; b ^= 1) {
+      if (at[b] < pieces) {
+        e = cudaEventSynchronize(ev[b]);
+        if (e != cudaSuccess) break;
+        memcpy(static_cast<unsigned char*>(out) + at[b] * piece, pin + b * piece, std::min(piece, bytes - at[b] * piece));
+        at[b] = pieces;
+      }
+      const size_t k = next.fetch_add(1);
+      if (k < pieces) {
+        at[b] = k;
+        e = cudaMemcpyAsync(pin + b * piece, static_cast<const unsigned char*>(src) + k * piece, std::min(piece, bytes - k * piece),
+                            cudaMemcpyDeviceToHost, st);
+        if (e == cudaSuccess) e = cudaEventRecord(ev[b], st);
+      } else if (at[b ^ 1] >= pieces) {
+        break;
+      }
+    }
+    if (st) { cudaStreamSynchronize(st); cudaStreamDestroy(st); }
+    for (cudaEvent_t v : ev) if (v) cudaEventDestroy(v);
+    if (e != cudaSuccess) error.store((int)e);
+  };
+  std::vector<std::thread> pool;
+  for (int t = 1; t < n_threads; t++) pool.emplace_back(work, t);
+  work(0);
+  for (auto& th : pool) th.join();
+  CK((cudaError_t)error.load());
+  return 0;
+}
+
+int DeviceFill::export_table(uint32_t* masks, uint64_t* first_row, MrlRow* rows) {
+  std::lock_guard<std::mutex> guard(lookup_mu_);   // the pinned staging is the lookups'
+  CK(cudaSetDevice(device_));
+  if (n_specs_) {
+    const size_t o_first = align256((size_t)n_specs_ * sizeof(uint4)), need = o_first + (size_t)n_specs_ * sizeof(uint64_t);
+    // the working rows are idle between fills
+    if (b_temp_.cap < need) {
+      int rc = reserve_(b_lookup_, need, false);
+      if (rc) return rc;
+    }
+    unsigned char* const d = static_cast<unsigned char*>(b_temp_.cap >= need ? b_temp_.p : b_lookup_.p);
+    export_headers_kernel<<<(n_specs_ + kBlock - 1) / kBlock, kBlock, 0, stream_>>>(d_hdrs_, n_specs_, reinterpret_cast<uint4*>(d),
+                                                                                    reinterpret_cast<unsigned long long*>(d + o_first));
+    CK(cudaGetLastError());
+    int rc;
+    if ((rc = read_bulk_(masks, d, (size_t)n_specs_ * sizeof(uint4))) || (rc = read_bulk_(first_row, d + o_first, (size_t)n_specs_ * sizeof(uint64_t))))
+      return rc;
+  }
+  return read_bulk_(rows, d_rows_, stats_.n_rows * sizeof(MrlRow));
 }
 
 int DeviceFill::read_specs(uint64_t* out) {

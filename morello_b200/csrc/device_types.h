@@ -99,8 +99,7 @@ enum {
 // Control block of a fill, in device memory. The stage kernels read their sizes and cursors
 // here and leave the host nothing to decide between launches; the host reads it once per fill
 // (once per stage when the fill is sharded).
-struct FillCtl {
-  // -- one stage (zero at its start)
+struct StageCtl {                    // of one stage; zero at its start
   unsigned long long rows_early;     // rows handed out to the grids of the unordered phase
   unsigned long long rows_late;      // working rows handed out
   uint32_t n_items;                  // work items listed
@@ -108,6 +107,9 @@ struct FillCtl {
   uint32_t any_changed;              // last relaxation sweep that changed a cell
   uint32_t grew;                     // pass + 1 when a grid has to grow after it
   uint32_t next_item[8];             // item hand-out of a phase; the phases take turns
+};
+struct FillCtl {
+  StageCtl stage;
   // -- sticky over a fill
   uint32_t error;                    // MRL_ERR_* bits
   uint32_t failed_stage;             // first stage that raised one

@@ -11,6 +11,17 @@
 
 namespace mrl {
 
+// A node of an implementation tree as the device walks it.
+struct WalkNode {
+  uint64_t spec;          // packed family and operands (plans made on the device)
+  uint32_t id, cpack;     // Spec and limits
+  uint32_t main, peaks, tail;
+  uint32_t first_child;
+  uint16_t n_child, status;
+  uint32_t pad;
+};
+enum { WALK_OK = 0, WALK_NO_SPEC = 1, WALK_UNSAT = 2, WALK_BAD = 3 };
+
 struct FillStats {
   uint64_t n_rows = 0;          // final table rows
   uint64_t cells_solved = 0;    // working-grid cells solved, all passes
@@ -63,6 +74,12 @@ class DeviceFill {
   // Rows of Specs of a plan made on the device, by packed family and operands (OpTables::locate);
   // a Spec that does not exist gets aux = 1.
   int lookup_packed(const uint64_t* specs, const uint32_t* cpacks, size_t n, MrlRow* out);
+  // The implementation tree of a Spec at given limits, nodes in breadth-first order, from the tables
+  // and records on the device. root: a Spec id, or packed family and operands. 1: more nodes than the
+  // walk holds.
+  int walk(uint64_t root, bool packed, uint32_t cpack, std::vector<WalkNode>& out);
+  // The finished table as masks (4 words per Spec), first rows and rows.
+  int export_table(uint32_t* masks, uint64_t* first_row, MrlRow* rows);
   // Packed family and operands of every Spec of a plan made on the device.
   int read_specs(uint64_t* out);
   int read_hdrs(SpecHdr* out);
@@ -153,6 +170,7 @@ class DeviceFill {
   void* h_stage_ = nullptr;      // pinned staging for tables, plan results and lookups
   size_t h_stage_bytes_ = 0;
   int reserve_host_(size_t bytes);
+  int read_bulk_(void* out, const void* src, size_t bytes);
   std::vector<unsigned char> h_pageable_;   // h_stage_ of a fixed buffer
   template <class Fill, class Launch>
   int lookup_batches_(size_t n, size_t query_bytes, MrlRow* out, Fill fill, Launch launch);

@@ -31,6 +31,74 @@ inline std::string action_text(const Candidate& c) {
   }
 }
 
+// The action with a given number, as text needs it (what, operand or dimension, destination or size):
+// found by the enumeration's counts (tabulate_candidates), without working out any other action.
+// False: the Spec has no such action.
+inline bool action_of(const LogicalSpec& spec, u32 action, Candidate& c) {
+  c.action = (u16)action;
+  u32 at = 0;
+  for (int i = 0; i < spec.nops(); i++) {
+    const TensorSpec op = spec.operand(i);
+    bool contains_source = false;
+    auto take = [&](Mem mem, const Layout& layout, u32 vs) {
+      if (at++ != action) return false;
+      c.what = ACT_MOVE;
+      c.kind = CK_MOVE;
+      c.arg0 = (u8)i;
+      c.arg1 = (u8)mem;
+      c.arg2 = vs;
+      c.lay = layout;
+      return true;
+    };
+    const std::vector<Mem> mems = possible_destination_memories(op.aux.mem);
+    for (const Layout& layout : move_destination_layouts(op.shape, op.dtype)) {
+      contains_source = contains_source || layout == op.aux.layout;
+      for (Mem mem : mems) {
+        const std::vector<u32>& vb = mem_vector_bytes(mem);
+        if (vb.empty()) { if (take(mem, layout, 0)) return true; }
+        else for (u32 b : vb) if (take(mem, layout, b / dtype_size(op.dtype))) return true;
+      }
+    }
+    if (!contains_source)
+      for (Mem mem : mems)
+        if (!mem_is_addressed(mem) && take(mem, op.aux.layout, 0)) return true;
+  }
+  const Shape out = spec.operand_shape(kind_output_index(spec.kind));
+  u32 max_dim = 0;
+  for (int d = 0; d < out.n; d++) if (out[d] > max_dim) max_dim = out[d];
+  for (u32 size : dim_range_pow2(max_dim, true))
+    for (int dim = 0; dim < out.n; dim++)
+      if (at++ == action) {
+        c.what = ACT_TILE_OUT;
+        c.kind = CK_LOOP;
+        c.arg0 = (u8)dim;
+        c.arg2 = size;
+        return true;
+      }
+  std::vector<Candidate> leaves;
+  at = tabulate_leaves(spec, at, leaves);
+  for (const Candidate& l : leaves) if (l.action == action) { c = l; return true; }
+  if (spec.kind == K_MATMUL && at == action) {
+    c.what = ACT_TO_ACCUM;
+    c.kind = CK_BLOCK;
+    return true;
+  }
+  if (spec.kind == K_MATMUL_ACCUM) {
+    const TensorSpec a = spec.operand(0), b = spec.operand(1);
+    const u32 bt = spec.spec_shape[0], m = spec.spec_shape[1], n = spec.spec_shape[3];
+    for (u32 k : dim_range_pow2(spec.spec_shape[2], false)) {
+      if (!tensorspec_valid_tile_shape(a, Shape{bt, m, k}) || !tensorspec_valid_tile_shape(b, Shape{bt, k, n})) continue;
+      if (at++ == action) {
+        c.what = ACT_SPLIT;
+        c.kind = CK_LOOP;
+        c.arg2 = k;
+        return true;
+      }
+    }
+  }
+  return false;
+}
+
 inline std::string limits_text(const u64 v[NMEM]) {
   std::string s = "[";
   for (int i = 0; i < NMEM; i++) { if (i) s += ", "; s += std::to_string(v[i]); }

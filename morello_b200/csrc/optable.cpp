@@ -95,30 +95,33 @@ u32 OpTables::layout_id_(const Layout& l) {
   return (u32)layouts_.size() - 1;
 }
 
-u32 OpTables::op_id_(u32 shape, const Aux& a) {
-  auto hash = [&](u32 sh, const Aux& x) { return mix(layout_hash(x.layout), (u64)sh << 16 | (u64)x.mem << 8 | x.vector_size); };
-  const size_t at = probe(op_tab_, tops_.size(), hash(shape, a), [&](u32 i) { return tops_[i].shape == shape && tops_[i].aux == a; },
-                          [&](u32 i) { return hash(tops_[i].shape, tops_[i].aux); });
+u32 OpTables::op_id_(u32 shape, Mem mem, u8 vs, u32 layout) {
+  auto hash = [](u32 sh, u32 m, u32 v, u32 l) { return mix(mix(3, (u64)sh << 32 | l), (u64)m << 8 | v); };
+  const size_t at = probe(op_tab_, tops_.size(), hash(shape, mem, vs, layout),
+                          [&](u32 i) { const TmpOp& t = tops_[i]; return t.shape == shape && t.layout_id == layout && t.aux.mem == mem && t.aux.vector_size == vs; },
+                          [&](u32 i) { const TmpOp& t = tops_[i]; return hash(t.shape, t.aux.mem, t.aux.vector_size, t.layout_id); });
   if (op_tab_[at]) return op_tab_[at] - 1;
   const u32 id = (u32)tops_.size();
   op_tab_[at] = id + 1;
   tops_.emplace_back();
   TmpOp& t = tops_[id];
-  t.aux = a;
+  t.aux.mem = mem;
+  t.aux.vector_size = vs;
+  t.aux.layout = layouts_[layout];
   t.shape = shape;
-  t.layout_id = layout_id_(a.layout);
+  t.layout_id = layout;
   TensorSpec ts;
   ts.shape = tshapes_[shape].s;
   ts.dtype = dt_;
-  ts.aux = a;
+  ts.aux = t.aux;
   t.cost = move_cost(ts);
   const u64 units = tensorspec_memory_units(ts);
   t.units = (u32)units;
-  const u32 thr = code_of_units(a.mem, (u32)units);
-  t.fits = thr <= top_code[a.mem];
+  const u32 thr = code_of_units(mem, (u32)units);
+  t.fits = thr <= top_code[mem];
   t.thr = t.fits ? (u8)thr : 0;
-  t.flags = (a.layout.fully_contiguous() ? DPO_CONTIG : 0) | (a.layout.is_row_major() ? DPO_ROW_MAJOR : 0) |
-            (a.layout.is_col_major() ? DPO_COL_MAJOR : 0);
+  t.flags = (t.aux.layout.fully_contiguous() ? DPO_CONTIG : 0) | (t.aux.layout.is_row_major() ? DPO_ROW_MAJOR : 0) |
+            (t.aux.layout.is_col_major() ? DPO_COL_MAJOR : 0);
   tshapes_[shape].ops.push_back(id);
   return id;
 }
@@ -135,7 +138,7 @@ int OpTables::dest_op_(u32 shape, u32 d, Mem mem, int v) {
   t.aux.mem = mem;
   t.aux.vector_size = mem == VRF ? (u8)(mem_vector_bytes(VRF)[v] / dtype_size(dt_)) : 0;
   if (mem_has_layout(mem)) {
-    t.aux.layout = mem == L1 ? e.l1_lay : e.lay;
+    t.aux.layout = layouts_[mem == L1 ? e.l1_lay : e.lay];
     t.aux.layout.contig = t.aux.layout.n;
   }
   int to = -1;
@@ -144,15 +147,54 @@ int OpTables::dest_op_(u32 shape, u32 d, Mem mem, int v) {
   return to;
 }
 
+// What tiling does to a layout (tile_operand, the part that an operand's memory has no say in), for
+// every dimension and tile size of the shape: layout id | DPT_OK | DPT_APPLIES. Operands in several
+// memories share layouts, so this is worked out once per shape and layout: it is most of the cost of
+// an operand.
+u32 OpTables::tiled_layouts_(u32 shape, u32 layout) {
+  const u64 key = (u64)shape << 32 | layout;
+  const size_t at = probe(tiled_tab_, tiled_keys_.size(), mix(4, key), [&](u32 i) { return tiled_keys_[i] == key; },
+                          [&](u32 i) { return mix(4, tiled_keys_[i]); });
+  if (tiled_tab_[at]) return tiled_at_[tiled_tab_[at] - 1];
+  tiled_keys_.push_back(key);
+  tiled_at_.push_back((u32)tiled_.size());
+  tiled_tab_[at] = (u32)tiled_keys_.size();
+  const Shape s = tshapes_[shape].s;
+  const Layout own = layouts_[layout];
+  Layout nl, canon;
+  for (int d = 0; d < s.n; d++)
+    for (u32 e = 1; e < s[d]; e *= 2) {
+      Shape tile = s;
+      tile[d] = e;
+      u32 entry = 0;
+      if (layout_update_for_tiling(own, s, tile, nl)) {
+        entry = DPT_APPLIES;
+        if (layout_update_for_tiling(nl, tile, tile, canon)) {
+          const u32 id = layout_id_(canon);
+          if (id > 0x3FFFFFFFu) throw ModelError("too many layouts");
+          entry |= DPT_OK | id;
+        }
+      }
+      tiled_.push_back(entry);
+    }
+  if (!layout_update_for_tiling(own, s, s, nl) || nl != own) throw ModelError("an operand is not canonical");
+  return tiled_at_.back();
+}
+
 // Moves and tiles of one operand (operand_moves and tile_operand of model/actions.hpp, with what
 // they share between operands of one shape worked out once).
 void OpTables::tabulate_op_(u32 o) {
   const u32 sh = tops_[o].shape;
-  const Aux aux = tops_[o].aux;
+  const Mem mem = tops_[o].aux.mem;
+  const u8 vs = tops_[o].aux.vector_size;
+  const u32 lay = tops_[o].layout_id;
+  const bool contig = (tops_[o].flags & DPO_CONTIG) != 0;
+  const Shape shape = tshapes_[sh].s;
   if (!tshapes_[sh].ready) {
-    for (const Layout& l : move_destination_layouts(tshapes_[sh].s, dt_)) {
+    for (const Layout& l : move_destination_layouts(shape, dt_)) {
       Dest e;
-      e.lay = l;
+      e.lay = layout_id_(l);
+      e.l1_lay = 0;
       e.l1_ready = false;
       for (int& x : e.to) x = -2;
       for (int& x : e.vrf) x = -2;
@@ -160,7 +202,6 @@ void OpTables::tabulate_op_(u32 o) {
     }
     tshapes_[sh].ready = true;
   }
-  const Shape shape = tshapes_[sh].s;
   const u32 src_cost = tops_[o].cost;
   u32 n_actions = 0;
   const u32 moves_off = (u32)tmoves_.size();
@@ -170,32 +211,34 @@ void OpTables::tabulate_op_(u32 o) {
     const TmpOp& t = tops_[to];
     tmoves_.push_back(TmpMove{src_cost + t.cost, t.units, (u32)to, (u16)rel, (u8)t.aux.mem, t.thr, (u8)miss});
   };
-  auto same_layout_in_l1 = [&]() { Aux a; a.mem = L1; a.layout = aux.layout; return (int)op_id_(sh, a); };
+  auto same_layout_in_l1 = [&]() { return (int)op_id_(sh, L1, 0, lay); };
   bool contains_source = false;
   const size_t n_dests = tshapes_[sh].dests.size();
-  const bool from_l1 = aux.mem == L1, from_gl = aux.mem == GL;
+  const bool from_l1 = mem == L1, from_gl = mem == GL;
   for (u32 d = 0; d < n_dests; d++) {
-    contains_source |= tshapes_[sh].dests[d].lay == aux.layout;
+    contains_source |= tshapes_[sh].dests[d].lay == lay;
     // possible_destination_memories, in its order
-    if (aux.mem == RF) emit(dest_op_(sh, d, RF, 0), false);
+    if (mem == RF) emit(dest_op_(sh, d, RF, 0), false);
     if (from_gl) emit(dest_op_(sh, d, GL, 0), false);
     if (from_l1 || from_gl) {
-      Dest& e = tshapes_[sh].dests[d];
-      if (!e.l1_ready) {
-        if (!layout_canonicalize(e.lay, shape, e.l1_lay)) throw ModelError("destination layout does not apply to the moved tensor");
-        e.l1_ready = true;
+      if (!tshapes_[sh].dests[d].l1_ready) {
+        Layout l1;
+        if (!layout_canonicalize(layouts_[tshapes_[sh].dests[d].lay], shape, l1)) throw ModelError("destination layout does not apply to the moved tensor");
+        const u32 id = layout_id_(l1);
+        tshapes_[sh].dests[d].l1_lay = id;
+        tshapes_[sh].dests[d].l1_ready = true;
       }
-      const bool miss = e.l1_lay == aux.layout;
+      const bool miss = tshapes_[sh].dests[d].l1_lay == lay;
       emit(miss ? same_layout_in_l1() : dest_op_(sh, d, L1, 0), miss);
     }
     if (from_l1) emit(dest_op_(sh, d, RF, 0), false);
-    if (from_l1 || aux.mem == VRF)
+    if (from_l1 || mem == VRF)
       for (int v = 0; v < 2; v++) emit(dest_op_(sh, d, VRF, v), false);
   }
   if (!contains_source && (from_l1 || from_gl)) {
-    Layout lay;
-    if (!layout_canonicalize(aux.layout, shape, lay)) throw ModelError("destination layout does not apply to the moved tensor");
-    if (lay != aux.layout) throw ModelError("an operand's layout is not canonical");
+    Layout l;
+    if (!layout_canonicalize(layouts_[lay], shape, l)) throw ModelError("destination layout does not apply to the moved tensor");
+    if (l != layouts_[lay]) throw ModelError("an operand's layout is not canonical");
     emit(same_layout_in_l1(), true);
   }
   TmpOp& t = tops_[o];
@@ -204,35 +247,28 @@ void OpTables::tabulate_op_(u32 o) {
   t.n_actions = n_actions;
   // row-major in the same memory: what the matching-layouts rule of Move Specs turns the operand into
   u32 rm = o;
-  if (mem_has_layout(aux.mem) && aux.layout.fully_contiguous()) {
-    Aux a = aux;
-    a.layout = layout_row_major(shape);
-    rm = op_id_(sh, a);
-  }
+  if (mem_has_layout(mem) && contig) rm = op_id_(sh, mem, vs, layout_id_(layout_row_major(shape)));
   tops_[o].rm = rm;
   // tiles
   tops_[o].tile_off = (u32)ttiles_.size();
-  TensorSpec ts;
-  ts.shape = shape;
-  ts.dtype = dt_;
-  ts.aux = aux;
+  if (check_tensor_vector_size(shape, dt_, mem, vs) != CANON_OK) throw ModelError("an operand is not canonical");
+  const u32 from = mem_has_layout(mem) ? tiled_layouts_(sh, lay) : 0;
   u32 c = 0;
   for (int d = 0; d < shape.n; d++)
     for (u32 e = 1; e < shape[d]; e *= 2, c++) {
       Shape tile = shape;
       tile[d] = e;
-      const TileResult r = tile_operand(ts, tile);
-      u32 entry = 0;
-      if (r.applies) entry |= DPT_APPLIES;
-      if (r.ok) {
-        const u32 to = op_id_(tshapes_[sh].child[c], r.aux);
+      u32 entry = mem_has_layout(mem) ? tiled_[from + c] : (DPT_APPLIES | DPT_OK | lay);   // RF: no layout to change
+      if ((entry & DPT_OK) && check_tensor_vector_size(tile, dt_, mem, vs) != CANON_OK) entry &= DPT_APPLIES;
+      if (entry & DPT_OK) {
+        const u32 to = op_id_(tshapes_[sh].child[c], mem, vs, entry & 0x3FFFFFFFu);
         if (to > 0x3FFFFFFFu) throw ModelError("too many operands");
-        entry |= DPT_OK | to;
+        entry = (entry & (DPT_OK | DPT_APPLIES)) | to;
+      } else {
+        entry &= DPT_APPLIES;
       }
       ttiles_.push_back(entry);
     }
-  const TileResult self = tile_operand(ts, shape);
-  if (!self.ok || self.aux != aux) throw ModelError("an operand is not canonical");
 }
 
 void OpTables::close_operands_() {
@@ -317,11 +353,24 @@ void OpTables::build_precompute(u32 size, Through through, const std::vector<Dty
     for (int j = 0; j < fams[f].nops; j++) {
       const u32 sh = fams[f].shape[j];
       if (!goal_lists_[sh].empty()) continue;
+      // (what aux_variants lists per memory: the layouts are the same in every memory that has any)
       const Shape shape = tshapes_[sh].s;
-      for (int mem = 0; mem < NMEM; mem++)
-        for (const Aux& a : aux_variants(shape, dt_, (Mem)mem))
-          if (check_tensor_vector_size(shape, dt_, a.mem, a.vector_size) == CANON_OK && aux_is_canonical(a, shape))
-            goal_lists_[sh].push_back(op_id_(sh, a));
+      goal_lists_[sh].push_back(op_id_(sh, RF, 0, layout_id_(Layout())));
+      std::vector<u32> vs;
+      for (u32 b : mem_vector_bytes(VRF))
+        if (check_tensor_vector_size(shape, dt_, VRF, b / dtype_size(dt_)) == CANON_OK) vs.push_back(b / dtype_size(dt_));
+      for (const Layout& l : all_layouts_for_shape(shape, dt_))
+        for (int contig = 0; contig <= l.n; contig++) {
+          Aux a;
+          a.mem = GL;
+          a.layout = l;
+          a.layout.contig = (u8)contig;
+          if (!aux_is_canonical(a, shape)) continue;
+          const u32 id = layout_id_(a.layout);
+          goal_lists_[sh].push_back(op_id_(sh, GL, 0, id));
+          goal_lists_[sh].push_back(op_id_(sh, L1, 0, id));
+          for (u32 v : vs) goal_lists_[sh].push_back(op_id_(sh, VRF, (u8)v, id));
+        }
     }
   close_operands_();
   finish_();

@@ -100,7 +100,7 @@ class OpTables {
     u8 thr, flags;
     bool fits;
   };
-  struct Dest { Layout lay, l1_lay; int to[4]; int vrf[2]; bool l1_ready; };   // -2: not worked out yet, -1: does not apply
+  struct Dest { u32 lay, l1_lay; int to[4]; int vrf[2]; bool l1_ready; };   // layout ids; operands: -2 not worked out yet, -1 does not apply
   struct TmpShape {
     Shape s;
     std::vector<Dest> dests;
@@ -110,7 +110,9 @@ class OpTables {
   };
   struct TmpMove { u32 imm, units, to; u16 rel; u8 mem, thr, miss; };
   u32 shape_id_(const Shape& s);
-  u32 op_id_(u32 shape, const Aux& a);
+  u32 op_id_(u32 shape, const Aux& a) { return op_id_(shape, a.mem, a.vector_size, layout_id_(a.layout)); }
+  u32 op_id_(u32 shape, Mem mem, u8 vs, u32 layout);
+  u32 tiled_layouts_(u32 shape, u32 layout);
   u32 layout_id_(const Layout& l);
   u32 fam_id_(u8 kind, u8 dtype, const Shape& s);
   void close_operands_();
@@ -126,7 +128,9 @@ class OpTables {
   std::vector<TmpMove> tmoves_;
   std::vector<u32> ttiles_;      // temporary id | flags, as in tiles
   std::vector<Layout> layouts_;
-  std::vector<u32> op_tab_, lay_tab_, fam_tab_, shape_tab_;   // open addressing, ids + 1
+  std::vector<u32> op_tab_, lay_tab_, fam_tab_, shape_tab_, tiled_tab_;   // open addressing, ids + 1
+  std::vector<u64> tiled_keys_;                // shape << 32 | layout
+  std::vector<u32> tiled_at_, tiled_;          // its entries: the layout after each tiling, as in ttiles_
   std::vector<u64> fam_keys_, shape_keys_;
   std::vector<u32> loc_;         // temporary id -> local index
   std::vector<u32> find_tab_;    // final: operand index + 1 by hash of (shape, key bytes)

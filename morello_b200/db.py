@@ -75,21 +75,14 @@ def tabulate(blob: bytes):
     return out
 
 
-def _pack(blobs: Sequence[bytes], limits: Optional[Sequence[Sequence[int]]]):
+def _pack(blobs: Sequence[bytes]):
     off = (C.c_uint64 * (len(blobs) + 1))()
     pos = 0
     for i, b in enumerate(blobs):
         off[i] = pos
         pos += len(b)
     off[len(blobs)] = pos
-    data = b"".join(blobs)
-    lim = None
-    if limits is not None:
-        lim = (C.c_uint64 * (4 * len(blobs)))()
-        for i, l in enumerate(limits):
-            for k in range(4):
-                lim[4 * i + k] = l[k]
-    return data, off, lim
+    return b"".join(blobs), off
 
 
 class SynthesisDatabase:
@@ -103,6 +96,9 @@ class SynthesisDatabase:
 
     def __init__(self, device: int = 0, threads: int = 0):
         self._lib = L.load()
+        self._call_many = L.pyhost().call_many
+        self._fn = {name: C.cast(getattr(self._lib, name), C.c_void_p).value
+                    for name in ("mrl_top_down_many", "mrl_top_down_many_noalloc", "mrl_get_many")}
         self._ctx = C.c_void_p()
         rc = self._lib.mrl_ctx_create(device, threads, C.byref(self._ctx))
         if rc != 0:
@@ -123,6 +119,11 @@ class SynthesisDatabase:
         except Exception:
             pass
 
+    def _many(self, name, specs, limits) -> List[Decision]:
+        rc, out = self._call_many(self._fn[name], self._ctx.value if self._ctx else 0, specs, limits, Decision)
+        self._check(rc)
+        return out
+
     def _check(self, rc):
         if rc != 0:
             err = RuntimeError(self._lib.mrl_last_error(self._ctx).decode() or f"status {rc}")
@@ -137,10 +138,7 @@ class SynthesisDatabase:
     def top_down_many(self, goals: Sequence[bytes], limits: Optional[Sequence[Sequence[int]]] = None) -> List[Decision]:
         if limits is None:
             limits = [MAX_MEM] * len(goals)
-        data, off, lim = _pack(goals, limits)
-        out = (L.Decision * len(goals))()
-        self._check(self._lib.mrl_top_down_many(self._ctx, data, off, len(goals), lim, out))
-        return [Decision.from_c(d) for d in out]
+        return self._many("mrl_top_down_many", goals, limits)
 
     def top_down_many_noalloc(self, goals: Sequence[bytes],
                               limits: Optional[Sequence[Sequence[int]]] = None) -> List[Decision]:
@@ -149,10 +147,7 @@ class SynthesisDatabase:
         time per GPU; make the first call before any stream capture."""
         if limits is None:
             limits = [MAX_MEM] * len(goals)
-        data, off, lim = _pack(goals, limits)
-        out = (L.Decision * len(goals))()
-        self._check(self._lib.mrl_top_down_many_noalloc(self._ctx, data, off, len(goals), lim, out))
-        return [Decision.from_c(d) for d in out]
+        return self._many("mrl_top_down_many_noalloc", goals, limits)
 
     def top_down(self, goal: bytes, limits: Sequence[int] = MAX_MEM) -> Decision:
         return self.top_down_many([goal], [limits])[0]
@@ -167,7 +162,7 @@ class SynthesisDatabase:
         self._check(self._lib.mrl_plan_precompute(self._ctx, size, through, self._dtype_mask(dtypes)))
 
     def plan_goals(self, goals: Sequence[bytes]):
-        data, off, _ = _pack(goals, None)
+        data, off = _pack(goals)
         self._check(self._lib.mrl_plan_goals(self._ctx, data, off, len(goals)))
 
     def upload(self):
@@ -178,10 +173,7 @@ class SynthesisDatabase:
 
     # --- FilesDatabase::get ---
     def get_many(self, specs: Sequence[bytes], limits: Sequence[Sequence[int]]) -> List[Decision]:
-        data, off, lim = _pack(specs, limits)
-        out = (L.Decision * len(specs))()
-        self._check(self._lib.mrl_get_many(self._ctx, data, off, len(specs), lim, out))
-        return [Decision.from_c(d) for d in out]
+        return self._many("mrl_get_many", specs, limits)
 
     def get(self, spec: bytes, limits: Sequence[int] = MAX_MEM) -> Decision:
         return self.get_many([spec], [limits])[0]
@@ -280,11 +272,14 @@ class SynthesisDatabase:
     def get_impl(self, spec: bytes, limits: Sequence[int] = MAX_MEM) -> str:
         """The optimal implementation of (Spec, limits) reconstructed from the tables, as text."""
         lim = (C.c_uint64 * 4)(*limits)
-        buf = C.create_string_buffer(1 << 20)
-        n = self._lib.mrl_get_impl(self._ctx, spec, len(spec), lim, buf, len(buf))
+        for cap in (1 << 14, 1 << 20):   # most trees are a few kilobytes of text
+            buf = C.create_string_buffer(cap)
+            n = self._lib.mrl_get_impl(self._ctx, spec, len(spec), lim, buf, cap)
+            if n != -3:
+                break
         if n < 0:
             self._check(int(n))
-        return buf.raw[:n].decode()
+        return C.string_at(buf, n).decode()
 
     def verify(self, n_samples: int = 0, seed: int = 1):
         """(points checked, mismatches): recomputes the decision from the children's tables at
@@ -337,9 +332,9 @@ class SynthesisDatabase:
         first_row[n_specs + 1] uint64, rows[n_rows, 4] uint32 = main, peak codes, depth << 16 | action, 0)."""
         import numpy as np
         n, n_rows = self.num_specs(), int(self.stats()["n_rows"])
-        masks = np.zeros((n, 4), dtype=np.uint32)
-        first = np.zeros(n + 1, dtype=np.uint64)
-        rows = np.zeros((max(n_rows, 1), 4), dtype=np.uint32)
+        masks = np.empty((n, 4), dtype=np.uint32)   # all of it is written below
+        first = np.empty(n + 1, dtype=np.uint64)
+        rows = np.empty((max(n_rows, 1), 4), dtype=np.uint32)
         self._check(self._lib.mrl_export_all(self._ctx, masks.ctypes.data, first.ctypes.data, rows.ctypes.data, n_rows))
         return masks, first, rows[:n_rows]
 
