@@ -2353,6 +2353,16 @@ int DeviceFill::upload(const Plan& plan, bool skip_cands) {
 
 int DeviceFill::plan(const OpTables& tab) {
   CK(cudaSetDevice(device_));
+  int rc = plan_(tab);
+  if (rc == -6) rc = 1;   // no room for the planning buffers: the host planner needs none of them
+  if (rc == 1 && !fixed_) {
+    CK(cudaStreamSynchronize(stream_));
+    for (DevBuf* b : {&b_tables_, &b_bits_, &b_rank_, &b_desc_, &b_stage_lo_}) drop_(*b);
+  }
+  return rc;
+}
+
+int DeviceFill::plan_(const OpTables& tab) {
   if (tab.max_records > DP_MAX_RECORDS || tab.n_positions == 0) return 1;
   begin_plan_();
   int rc;
@@ -2371,7 +2381,11 @@ int DeviceFill::plan(const OpTables& tab) {
   if ((rc = reserve_host_(std::max(bytes, back)))) return rc;
   for (const Part& q : parts) if (q.bytes) memcpy(static_cast<unsigned char*>(h_stage_) + q.off, q.src, q.bytes);
   const size_t word_bytes = align256((size_t)n_words * sizeof(u32));
-  if ((rc = reserve_(b_ctl_, 512)) || (rc = reserve_(b_tables_, bytes)) || (rc = reserve_(b_bits_, word_bytes + (size_t)tab.n_positions * sizeof(u64))) ||
+  // The closure's queue has room for every position (size 8 in one dtype: 1.9 GB), so it lies in the
+  // working rows, which are idle until the fill; a fixed buffer carves those last.
+  const size_t queue_bytes = (size_t)tab.n_positions * sizeof(u64);
+  if (!fixed_ && (rc = reserve_(b_temp_, queue_bytes, false))) return rc;
+  if ((rc = reserve_(b_ctl_, 512)) || (rc = reserve_(b_tables_, bytes)) || (rc = reserve_(b_bits_, word_bytes + (fixed_ ? queue_bytes : 0))) ||
       (rc = reserve_(b_rank_, (size_t)n_words * sizeof(uint2))) || (rc = reserve_(b_stage_lo_, back + (size_t)plan_blocks_ * n_sm_ * sizeof(unsigned long long))))
     return rc == -5 ? 1 : rc;
   d_ctl_ = static_cast<FillCtl*>(b_ctl_.p);
@@ -2397,7 +2411,7 @@ int DeviceFill::plan(const OpTables& tab) {
   a.n_seeds = (u32)tab.seeds.size();
   a.n_words = n_words;
   a.found = static_cast<u32*>(b_bits_.p);
-  a.queue = reinterpret_cast<u64*>(static_cast<unsigned char*>(b_bits_.p) + word_bytes);
+  a.queue = fixed_ ? reinterpret_cast<u64*>(static_cast<unsigned char*>(b_bits_.p) + word_bytes) : static_cast<u64*>(b_temp_.p);
   a.rank = static_cast<uint2*>(b_rank_.p);
   a.t.rank = a.rank;
   unsigned char* const res = static_cast<unsigned char*>(b_stage_lo_.p);

@@ -131,6 +131,7 @@ class DeviceFill {
   void drop_(DevBuf& b);
   int alloc_(void** p, size_t bytes);
   void begin_plan_();
+  int plan_(const OpTables& tab);
   int working_buffers_(bool sharded_mine, uint32_t world);
   int launch_stages_(uint32_t from, uint32_t to, int team, int blocks, bool solve, bool place);
   void team_for_(uint32_t n_specs, int* team, int* blocks) const;
