@@ -754,6 +754,8 @@ struct WarpScratch {         // a warp's shared memory in the solve phases
   uint4 affected[kMaxAffected];      // sweeps: per changed child the parent's codes that read a changed slot of it
   uint32_t who[kMaxAffected];        // record (from the end) | child << 16
   uint32_t queue[64];                // sweeps: cells to solve again, as packed slots
+  uint32_t bound[kBatch];            // per staged record: no cell of the item gets a main cost below this from it
+  uint8_t order[kBatch];             // the staged records that can apply, by that bound
   uint8_t codes[kMaxSlots];
 };
 static_assert(sizeof(WarpScratch) % 16 == 0, "warp scratch is made of 16-byte units");
@@ -879,6 +881,93 @@ __device__ __forceinline__ void add_tally(const Tally& tally, unsigned long long
   }
 }
 
+// Limit codes that no cell of [first, end) exceeds: per memory the largest among them. n: slots per
+// memory; z: slots left out at the bottom of each (cells are numbered without them).
+__device__ __forceinline__ uint32_t top_codes(const uint8_t* codes, uint32_t first, uint32_t end, uint32_t n0, uint32_t n1, uint32_t n2, uint32_t z0,
+                                              uint32_t z1, uint32_t z2, uint32_t z3) {
+  uint32_t f0, f1, f2, f3, l0, l1, l2, l3;
+  cell_slots(first, n0 - z0, n1 - z1, n2 - z2, f0, f1, f2, f3);
+  cell_slots(end - 1, n0 - z0, n1 - z1, n2 - z2, l0, l1, l2, l3);
+  const bool same3 = f3 == l3, same2 = same3 && f2 == l2, same1 = same2 && f1 == l1;
+  const uint32_t t0 = same1 ? l0 + z0 : n0 - 1, t1 = same2 ? l1 + z1 : n1 - 1, t2 = same3 ? l2 + z2 : n2 - 1, t3 = l3 + z3;
+  return codes[t0] | (codes[n0 + t1] << 8) | (codes[n0 + n1 + t2] << 16) | ((uint32_t)codes[n0 + n1 + n2 + t3] << 24);
+}
+
+// Lower bounds of the staged records over a run of cells, and the order to try them in. More memory
+// never makes an optimum's main cost larger nor loses an implementation, so what a record costs with
+// its children read at the run's largest limits bounds it from below at every cell of the run, and one
+// whose child has no implementation there, or that does not fit, applies nowhere in it. Cells then
+// take the records cheapest bound first and stop where no lane's optimum so far is above the bound
+// (ties are evaluated: peaks, depth and action number decide those). kMoving: tables that may change
+// while this runs bound nothing. Returns the number of records that can apply.
+// Evaluating a record at 32 cells is a hundred instructions and 1.4 gathered rows a lane; of the 59 G
+// evaluations of the size-8 u32 fill 22 G are left, and the fill takes 490 ms instead of 639.
+template <bool kMoving>
+__device__ __noinline__ uint32_t stage_bounds(WarpScratch& ws, uint32_t n_here, uint32_t cmax, uint32_t lane) {
+  #pragma unroll 1
+  for (uint32_t t = lane; t < kBatch * 4u; t += 32) {   // four lanes per record, one per child and one idle
+    const uint32_t r = t >> 2, j = t & 3u;
+    uint32_t part = 0, kind = MRL_CK_LEAF, imm = 0;
+    bool dead = r >= n_here;
+    if (!dead) {
+      const StagedRec& s = ws.staged[r];
+      const uint4 a = s.rec;
+      kind = (a.x >> 16) & 0xFFu;
+      imm = a.y;
+      const uint32_t nchild = a.x >> 24, level = a.z & 0xFFu, lv = code_of(cmax, level);
+      if ((kind == MRL_CK_LEAF || kind == MRL_CK_MOVE) && lv < ((a.z >> 8) & 0xFFu)) {
+        dead = true;
+      } else if (j < nchild && !(kMoving && s.in_temp[j])) {
+        uint32_t c = cmax;
+        if (kind == MRL_CK_MOVE) c = (c & ~(0xFFu << (8 * level))) | (child_code(level, lv, a.w) << (8 * level));
+        const uint4 row = ld_row(staged_row(s, j, below(code_of(c, 0)), below(code_of(c, 1)), below(code_of(c, 2)), below(code_of(c, 3))));
+        dead = row.z == MRL_UNSAT;
+        part = row.x;
+      }
+    }
+    part = sat_add(part, __shfl_xor_sync(0xFFFFFFFFu, part, 1));
+    part = sat_add(part, __shfl_xor_sync(0xFFFFFFFFu, part, 2));
+    const uint32_t any_dead = (__ballot_sync(0xFFFFFFFFu, dead) >> (lane & ~3u)) & 0xFu;
+    if (j == 0) {
+      ws.bound[r] = kind == MRL_CK_LEAF ? imm : (kind == MRL_CK_LOOP ? sat_mul(part, imm) : (kind == MRL_CK_MOVE ? sat_add(part, imm) : part));
+      ws.order[r] = any_dead ? 1 : 0;
+    }
+  }
+  __syncwarp();
+  const uint32_t own = lane < kBatch ? ws.bound[lane] : 0u;
+  const uint32_t alive = __ballot_sync(0xFFFFFFFFu, lane < kBatch && !ws.order[lane & (kBatch - 1)]);
+  uint32_t at = 0;
+  #pragma unroll 1
+  for (uint32_t rest = alive; rest; rest &= rest - 1) {
+    const uint32_t k = __ffs(rest) - 1, b = __shfl_sync(0xFFFFFFFFu, own, k);
+    at += b < own || (b == own && k < lane);
+  }
+  __syncwarp();
+  if ((alive >> lane) & 1u) ws.order[at] = (uint8_t)lane;
+  __syncwarp();
+  return __popc(alive);
+}
+// From this many cells on the bounds of a run of them are worth their reads (one more dependent read per
+// record, against one evaluation per record and 32 cells).
+constexpr uint32_t kBoundCells = 64;
+
+// The staged records at the lanes' cells. n: what stage_bounds left of them, or all (bounded = false).
+template <bool kMoving>
+__device__ __forceinline__ void eval_batch(const WarpScratch& ws, uint32_t n, bool bounded, bool live, uint32_t cpack, uint32_t bm0, uint32_t bm1,
+                                           uint32_t bm2, uint32_t bm3, Best& best, Tally& tally) {
+  #pragma unroll 1
+  for (uint32_t q = 0; q < n; q++) {
+    uint32_t r = q;
+    bool go = live;
+    if (bounded) {
+      r = ws.order[q];
+      go = live && ws.bound[r] <= best.main;
+      if (!__any_sync(0xFFFFFFFFu, go)) break;
+    }
+    if (go) eval_staged<kMoving>(ws.staged[r], cpack, bm0, bm1, bm2, bm3, best, tally);
+  }
+}
+
 // The records of a Spec whose children all lie in finished stages, for the cells [first, end) of its
 // grid of the unordered phase, by a warp. The grid's slot codes are staged.
 __device__ __noinline__ void solve_early_cells(const HotArgs a, WarpScratch& ws, uint32_t cand_off, uint32_t n_early, const uint4 m, uint32_t corner,
@@ -886,6 +975,8 @@ __device__ __noinline__ void solve_early_cells(const HotArgs a, WarpScratch& ws,
   StagedRec* const staged = ws.staged;
   const uint8_t* const codes = ws.codes;
   const uint32_t n0 = __popc(m.x), n1 = __popc(m.y), n2 = __popc(m.z);
+  const bool bounded = end - first > kBoundCells;
+  const uint32_t cmax = bounded ? top_codes(codes, first, end, n0, n1, n2, 0, 0, 0, 0) : 0u;
   uint32_t b0 = 0;
   do {
     // stage the next records, and the headers of their children, one (record, child) per lane
@@ -902,6 +993,7 @@ __device__ __noinline__ void solve_early_cells(const HotArgs a, WarpScratch& ws,
       }
     }
     __syncwarp();
+    const uint32_t n_apply = bounded ? stage_bounds<false>(ws, n_here, cmax, lane) : n_here;
     #pragma unroll 1
     for (uint32_t c0 = first; c0 < end; c0 += 32) {
       const uint32_t cell = c0 + lane;
@@ -920,11 +1012,7 @@ __device__ __noinline__ void solve_early_cells(const HotArgs a, WarpScratch& ws,
         const uint4 r = ld_row(grid + cell);
         best.main = r.x; best.peaks = r.y; best.tail = r.z;
       }
-      const uint32_t bm0 = below(k0), bm1 = below(k1), bm2 = below(k2), bm3 = below(k3);
-      if (live) {
-        #pragma unroll 1
-        for (uint32_t r = 0; r < n_here; r++) eval_staged<false>(staged[r], cpack, bm0, bm1, bm2, bm3, best, tally);
-      }
+      eval_batch<false>(ws, n_apply, bounded, live, cpack, below(k0), below(k1), below(k2), below(k3), best, tally);
       if (valid && (b0 == 0 || live)) *reinterpret_cast<uint4*>(grid + cell) = make_uint4(best.main, best.peaks, best.tail, 0u);
     }
     b0 += n_here;
@@ -1109,22 +1197,47 @@ __device__ __noinline__ void phase_sweep(const HotArgs a, int mode, uint32_t lo,
     if (l_begin == l_end) continue;
     const bool single = n_late <= (uint32_t)kBatch;   // all records staged once for the whole item
     stage_slot_codes(ws.codes, m, n0, n1, n2, n3, lane);
-    bool staged_yet = false;
+    const bool bounded = l_end - l_begin > kBoundCells && (kAll || single);
+    const uint32_t cmax = bounded ? top_codes(codes, l_begin, l_end, n0, n1, n2, z0, z1, z2, z3) : 0u;
     uint4 ch = make_uint4(0, 0, 0, 0);   // codes of the slots of the cells that change
+    if (kAll) {
+      // every cell, one batch of records after the other: nothing reads the working rows meanwhile, so
+      // they hold what the batches so far have found
+#pragma unroll 1
+      for (uint32_t b = 0; b < n_late; b += kBatch) {
+        const uint32_t n_here = min((uint32_t)kBatch, n_late - b);
+        stage_late_batch<true>(a, lo, staged, last - b, n_here, lane);
+        const uint32_t n_apply = bounded ? stage_bounds<false>(ws, n_here, cmax, lane) : n_here;
+#pragma unroll 1
+        for (uint32_t c0 = l_begin; c0 < l_end; c0 += 32) {
+          const bool live = c0 + lane < l_end;
+          uint32_t s0, s1, s2, s3;
+          cell_slots(live ? c0 + lane : l_begin, v0, v1, v2, s0, s1, s2, s3);
+          s0 += z0; s1 += z1; s2 += z2; s3 += z3;
+          const uint32_t k0 = codes[s0], k1 = codes[n0 + s1], k2 = codes[n0 + n1 + s2], k3 = codes[n0 + n1 + n2 + s3];
+          const uint32_t bm0 = below(k0), bm1 = below(k1), bm2 = below(k2), bm3 = below(k3);
+          MrlRow* const at = grid + (((s3 * n2 + s2) * n1 + s1) * n0 + s0);
+          const uint32_t i0 = __popc(em.x & bm0) - 1, i1 = __popc(em.y & bm1) - 1, i2 = __popc(em.z & bm2) - 1, i3 = __popc(em.w & bm3) - 1;
+          const uint4 f = ld_row(egrid + (((i3 * __popc(em.z) + i2) * __popc(em.y) + i1) * __popc(em.x) + i0));
+          const uint4 was = b ? ld_row(at) : f;
+          Best best = {was.x, was.y, was.z};
+          eval_batch<false>(ws, n_apply, bounded, live, k0 | (k1 << 8) | (k2 << 16) | (k3 << 24), bm0, bm1, bm2, bm3, best, tally);
+          if (live) {
+            *reinterpret_cast<uint4*>(at) = make_uint4(best.main, best.peaks, best.tail, 0u);
+            if (best.main != f.x || best.peaks != f.y || best.tail != f.z) { ch.x |= 1u << k0; ch.y |= 1u << k1; ch.z |= 1u << k2; ch.w |= 1u << k3; }
+          }
+        }
+      }
+    } else {
+    bool staged_yet = false;
+    uint32_t n_apply = n_late;
     uint32_t c0 = l_begin, queued = 0;
 #pragma unroll 1
     for (;;) {
-      // the next cells to solve, one per lane: all of them in order, or collected from those that qualify
+      // the next cells to solve, one per lane, collected from those that qualify
       bool live;
       uint32_t slots;
-      if (kAll) {
-        if (c0 >= l_end) break;
-        live = c0 + lane < l_end;
-        uint32_t s0, s1, s2, s3;
-        cell_slots(live ? c0 + lane : l_begin, v0, v1, v2, s0, s1, s2, s3);
-        slots = (s0 + z0) | ((s1 + z1) << 8) | ((s2 + z2) << 16) | ((s3 + z3) << 24);
-        c0 += 32;
-      } else {
+      {
 #pragma unroll 1
         while (queued < 32 && c0 < l_end) {
           const bool in = c0 + lane < l_end;
@@ -1161,7 +1274,8 @@ __device__ __noinline__ void phase_sweep(const HotArgs a, int mode, uint32_t lo,
         if (lane < queued) ws.queue[lane] = rest_of;
       }
       if (single && !staged_yet) {
-        stage_late_batch<kAll>(a, lo, staged, last, n_late, lane);
+        stage_late_batch<false>(a, lo, staged, last, n_late, lane);
+        if (bounded) n_apply = stage_bounds<true>(ws, n_late, cmax, lane);
         staged_yet = true;
       }
       const uint32_t s0 = slots & 0xFFu, s1 = (slots >> 8) & 0xFFu, s2 = (slots >> 16) & 0xFFu, s3 = slots >> 24;
@@ -1175,22 +1289,19 @@ __device__ __noinline__ void phase_sweep(const HotArgs a, int mode, uint32_t lo,
         const uint32_t i0 = __popc(em.x & bm0) - 1, i1 = __popc(em.y & bm1) - 1, i2 = __popc(em.z & bm2) - 1, i3 = __popc(em.w & bm3) - 1;
         const uint4 f = ld_row(egrid + (((i3 * __popc(em.z) + i2) * __popc(em.y) + i1) * __popc(em.x) + i0));
         best.main = f.x; best.peaks = f.y; best.tail = f.z;
-        was = kAll ? f : ld_row(at);   // only this warp writes the cell in this sweep
+        was = ld_row(at);   // only this warp writes the cell in this sweep
       }
 #pragma unroll 1
       for (uint32_t b = 0; b < n_late; b += kBatch) {
         const uint32_t n_here = min((uint32_t)kBatch, n_late - b);
-        if (!single) stage_late_batch<kAll>(a, lo, staged, last - b, n_here, lane);
-        if (live)
-#pragma unroll 1
-          for (uint32_t r = 0; r < n_here; r++) eval_staged<!kAll>(staged[r], cpack, bm0, bm1, bm2, bm3, best, tally);
+        if (!single) stage_late_batch<false>(a, lo, staged, last - b, n_here, lane);
+        eval_batch<true>(ws, single ? n_apply : n_here, bounded, live, cpack, bm0, bm1, bm2, bm3, best, tally);
       }
-      if (live) {
-        const bool differs = best.main != was.x || best.peaks != was.y || best.tail != was.z;
-        if (kAll) *reinterpret_cast<uint4*>(at) = make_uint4(best.main, best.peaks, best.tail, 0u);
-        else if (differs) st_row_shared(at, make_uint4(best.main, best.peaks, best.tail, 0u));
-        if (differs) { ch.x |= 1u << k0; ch.y |= 1u << k1; ch.z |= 1u << k2; ch.w |= 1u << k3; }
+      if (live && (best.main != was.x || best.peaks != was.y || best.tail != was.z)) {
+        st_row_shared(at, make_uint4(best.main, best.peaks, best.tail, 0u));
+        ch.x |= 1u << k0; ch.y |= 1u << k1; ch.z |= 1u << k2; ch.w |= 1u << k3;
       }
+    }
     }
     ch = warp_or(ch);
     if (ch.x && lane == 0) {
