@@ -46,7 +46,7 @@ typedef struct mrl_stats {
   uint64_t n_candidates_evaluated; /* candidate records evaluated by those solves */
   uint64_t n_rows_gathered;    /* child rows they read */
   uint64_t n_passes;           /* solve passes of the last fill, summed over stages */
-  uint64_t n_launches;         /* kernel launches of the last fill (one cooperative launch per stage) */
+  uint64_t n_launches;         /* kernel launches of the last fill (one per stage; in small plans one per run of stages) */
   uint64_t n_grid_syncs;       /* grid-wide barriers inside those launches */
   uint64_t algorithmic_bytes;  /* of the finished table: per final row 12 bytes out, 16 per candidate record of
                                 * its Spec, 16 per child of each candidate that fits the row's limits */

@@ -2115,6 +2115,22 @@ constexpr size_t kStageSmem = (kStageBlock / 32) * sizeof(WarpScratch);
 
 static size_t align256(size_t x) { return (x + 255) & ~size_t(255); }
 
+// The team for a stage of n Specs of one kind, log-shape sum and level rank. A grid-wide barrier takes
+// 2 us and a stage has 5 to 20 of them, a cluster's a fraction of that, a block's less still; against
+// that stands the work, and Specs differ in it by orders of magnitude: their grids grow with the
+// operands' volume, and with how many of the operands are still in the slowest memory (the finished
+// rows of a Matmul stage: 2 per Spec at 1x1x2, 200 at 2x8x4, 1 900 at 8x8x8 with all operands there, a
+// tenth of that with all in the others).
+constexpr uint32_t kMergeSpecs = 1u << 18;
+constexpr uint32_t kBlockSpecs = 24, kBlockWork = 3000, kClusterSpecs = 256, kClusterWork = 20000;
+static uint32_t team_of_stage(uint32_t n, uint32_t kind, uint32_t shape_sum, uint32_t level_rank) {
+  const int below_top = (kind == K_MOVE || kind == K_FILL_ZERO ? (int)GL : 3 * (int)GL) - (int)level_rank;
+  const uint32_t shift = shape_sum + (uint32_t)std::min(3, std::max(0, 4 - below_top));
+  const uint64_t work = shift < 32 ? (uint64_t)n << shift : ~uint64_t(0);
+  if (n <= kBlockSpecs && work <= kBlockWork) return TEAM_BLOCK;
+  return n <= kClusterSpecs && work <= kClusterWork ? TEAM_CLUSTER : TEAM_GRID;
+}
+
 struct DeviceFill::DevTables {
   DpTables t;
 };
@@ -2370,7 +2386,7 @@ int DeviceFill::upload(const Plan& plan, bool skip_cands) {
   top_pack_ = plan.top_pack();
   n_goals_ = plan.stats.n_goal_specs;
   for (const Stage& st : plan.stages) {
-    StageIds s = {st.spec_lo, st.spec_hi, 0};
+    StageIds s = {st.spec_lo, st.spec_hi, 0, team_of_stage(st.spec_hi - st.spec_lo, st.phase, st.shape_sum, st.level_rank)};
     if (st.spec_hi > st.spec_lo) s.cand_end = (uint64_t)plan.hdrs[st.spec_hi - 1].cand_off + plan.hdrs[st.spec_hi - 1].ncand;
     stages_.push_back(s);
   }
@@ -2573,7 +2589,10 @@ int DeviceFill::plan_(const OpTables& tab) {
   n_goals_ = ctl->n_goals;
   n_cand_bytes_ = ctl->n_cands * sizeof(CandRec);
   for (u32 g = 0; g < n_stages; g++)
-    if (lo[g + 1] > lo[g]) stages_.push_back(StageIds{lo[g], lo[g + 1], 0});
+    if (lo[g + 1] > lo[g]) {
+      const u32 key = tab.stage_key[g];
+      stages_.push_back(StageIds{lo[g], lo[g + 1], 0, team_of_stage(lo[g + 1] - lo[g], key >> 16, (key >> 8) & 0xFFu, key & 0xFFu)});
+    }
   top_pack_ = 0;
   for (int k = 0; k < NMEM; k++) top_pack_ |= tab.top_code[k] << (8 * k);
   h2d_bytes_ = bytes;
@@ -2705,16 +2724,7 @@ int DeviceFill::launch_stages_(uint32_t from, uint32_t to, int team, int blocks,
   return 0;
 }
 
-// The team for a stage of n Specs. A grid-wide barrier takes 2 us and a stage has 5 to 20 of them, a
-// cluster's a fraction of that, a block's less still; a Spec is 100 to 600 cells of some 30 records.
-// Measured over fills of 60 to 640 k Specs: a block up to 24 Specs, a cluster of 8 up to 256 (an 8x8x8
-// Matmul fill takes 81 ms with the cluster's limit at 256, 124 ms at 1024; a 2x2x2 one 6.4 ms with the grid
-// for every stage, 2.5 ms so).
-void DeviceFill::team_for_(uint32_t n, int* team, int* blocks) const {
-  if (n <= 24) { *team = TEAM_BLOCK; *blocks = 1; }
-  else if (n <= 256) { *team = TEAM_CLUSTER; *blocks = 8; }
-  else { *team = TEAM_GRID; *blocks = coop_blocks_; }
-}
+int DeviceFill::blocks_of_(int team) const { return team == TEAM_BLOCK ? 1 : (team == TEAM_CLUSTER ? 8 : coop_blocks_); }
 
 int DeviceFill::launch_solve_(uint32_t si, bool place_too) {
   const StageIds& st = stages_[si];
@@ -2723,17 +2733,13 @@ int DeviceFill::launch_solve_(uint32_t si, bool place_too) {
   // stage order): wait for that much of a background upload
   int rc = wait_cands_(st.cand_end * sizeof(CandRec));
   if (rc) return rc;
-  int team, blocks;
-  team_for_(st.hi - st.lo, &team, &blocks);
-  return launch_stages_(si, si + 1, team, blocks, true, place_too);
+  return launch_stages_(si, si + 1, st.team, blocks_of_(st.team), true, place_too);
 }
 
 int DeviceFill::launch_place_(uint32_t si) {
   const StageIds& st = stages_[si];
   if (st.hi == st.lo) return 0;
-  int team, blocks;
-  team_for_(st.hi - st.lo, &team, &blocks);
-  return launch_stages_(si, si + 1, team, blocks, false, true);
+  return launch_stages_(si, si + 1, st.team, blocks_of_(st.team), false, true);
 }
 
 int DeviceFill::solve_stage(uint32_t si) {
@@ -2851,19 +2857,20 @@ int DeviceFill::run() {
   int rc;
   if ((rc = begin_fill())) return rc;
   uint32_t from = 0;
-  int team_max, blocks_max;
-  team_for_(max_stage_, &team_max, &blocks_max);
-  const bool one_launch = team_max != TEAM_GRID && !stages_.empty();
   for (int attempt = 0;; attempt++) {
-    // A plan whose stages are all small runs as one launch; otherwise every stage has its own, with
-    // the team that fits it.
-    if (one_launch) {
-      int team, blocks;
-      team_for_(max_stage_, &team, &blocks);
-      if ((rc = wait_upload()) || (rc = launch_stages_(from, (uint32_t)stages_.size(), team, blocks, true, true))) return rc;
-    } else {
-      for (uint32_t s = from; s < stages_.size(); s++)
-        if ((rc = launch_solve_(s, true))) return rc;
+    // Consecutive stages with the same team run as one launch: a launch of its own costs a stage 20 us
+    // (gap, cold instruction and data caches) where a small one takes 15 (2x8x4 Matmul in both dtypes,
+    // 40 k Specs in 141 stages: 14.8 -> 12.3 ms together with the teams). In plans of more than
+    // kMergeSpecs that is 2 % or less (precompute 4, 642 k Specs: 28.3 -> 27.7 ms), and a launch per stage
+    // is what their statistics and profiles are read by. While candidate records are still on their way
+    // up, every stage waits for its own.
+    for (uint32_t s = from, e; s < stages_.size(); s = e) {
+      e = s + 1;
+      if (n_specs_ <= kMergeSpecs && up_threads_.empty())
+        while (e < stages_.size() && stages_[e].team == stages_[s].team) e++;
+      if (e == s + 1) rc = launch_solve_(s, true);
+      else rc = launch_stages_(s, e, stages_[s].team, blocks_of_(stages_[s].team), true, true);
+      if (rc) return rc;
     }
     CK(cudaEventRecord(ev1_, stream_));
     if (read_ctl_() != 0) return -1;

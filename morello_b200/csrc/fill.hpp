@@ -67,7 +67,7 @@ class DeviceFill {
   // plan on the host.
   int plan(const OpTables& tab);
   int prepare_fill();
-  struct StageIds { uint32_t lo, hi; uint64_t cand_end; };
+  struct StageIds { uint32_t lo, hi; uint64_t cand_end; uint32_t team; };
   const std::vector<StageIds>& stages() const { return stages_; }
   uint64_t n_goals() const { return n_goals_; }
   uint64_t n_cands() const { return n_cand_bytes_ / sizeof(CandRec); }
@@ -134,7 +134,7 @@ class DeviceFill {
   int plan_(const OpTables& tab);
   int working_buffers_(bool sharded_mine, uint32_t world);
   int launch_stages_(uint32_t from, uint32_t to, int team, int blocks, bool solve, bool place);
-  void team_for_(uint32_t n_specs, int* team, int* blocks) const;
+  int blocks_of_(int team) const;
   int launch_solve_(uint32_t stage, bool place_too);
   int launch_place_(uint32_t stage);
   int read_ctl_();                       // device control block -> h_ctl_ (synchronises the stream)
