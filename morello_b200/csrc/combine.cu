@@ -748,17 +748,23 @@ __device__ __forceinline__ const MrlRow* staged_row(const StagedRec& s, uint32_t
 // The lattice code of every slot of a grid, memory after memory, for the lanes of a warp to look
 // up instead of counting bits (a grid has at most 17 + 17 + 12 + 27 slots).
 constexpr int kMaxSlots = 80;
-constexpr int kMaxAffected = 32;
+constexpr int kMaxAffected = 26;   // more: every cell is solved again
 struct WarpScratch {         // a warp's shared memory in the solve phases
   StagedRec staged[kBatch];
   uint4 affected[kMaxAffected];      // sweeps: per changed child the parent's codes that read a changed slot of it
-  uint32_t who[kMaxAffected];        // record (from the end) | child << 16
+  uint32_t who[32];                  // record (from the end) | child << 16 | position among such records << 20
   uint32_t queue[64];                // sweeps: cells to solve again, as packed slots
-  uint32_t bound[kBatch];            // per staged record: no cell of the item gets a main cost below this from it
+  uint16_t reads[64];                // ... and which of the staged records read something that changed there
+  union {
+    uint32_t bound[kBatch];          // per staged record: no cell of the item gets a main cost below this from it
+    uint32_t listed[kBatch];         // or, in later sweeps, the records (from the end) with a changed child
+  };
   uint8_t order[kBatch];             // the staged records that can apply, by that bound
   uint8_t codes[kMaxSlots];
 };
-static_assert(sizeof(WarpScratch) % 16 == 0, "warp scratch is made of 16-byte units");
+// With the static shared memory 100 KB a block, which leaves L1 156 KB of an SM; 132 KB is the next step
+// (size 8 u32: 2 % slower).
+static_assert(sizeof(WarpScratch) == 3136, "warp scratch");
 
 __device__ __forceinline__ void stage_slot_codes(uint8_t* codes, const uint4 m, uint32_t n0, uint32_t n1, uint32_t n2, uint32_t n3,
                                                  uint32_t lane) {
@@ -1054,7 +1060,9 @@ __device__ __noinline__ void phase_early(const HotArgs a, unsigned long long* bl
 //   every other sweep         those that read a slot of a child which the sweep before changed. A
 //                             sweep leaves, per Spec and memory, the codes of the slots it changed a
 //                             cell of; a cell is solved again when its limits at some child fall into
-//                             such slots in all four memories.
+//                             such slots in all four memories - from the records with such children
+//                             alone, where a batch holds them (the size-8 u32 fill's sweeps after the
+//                             first: 120 ms with all records, 80 so).
 // Every cell is thus consistent with its children when a sweep changes nothing anywhere: it was
 // solved after its children last changed, or nothing it reads has changed. At size 8 this took the
 // sweeps after the first from 459 ms (whole Specs solved again when a child changed anywhere) to a
@@ -1063,15 +1071,16 @@ __device__ __noinline__ void phase_early(const HotArgs a, unsigned long long* bl
 enum { SWEEP_ALL = 0, SWEEP_NEW = 1, SWEEP_CHANGED = 2 };
 
 template <bool kAll>
-__device__ __forceinline__ void stage_late_batch(const HotArgs& a, uint32_t lo, StagedRec* staged, uint32_t last_rec, uint32_t n_here, uint32_t lane) {
+__device__ __forceinline__ void stage_late_batch(const HotArgs& a, uint32_t lo, StagedRec* staged, uint32_t last_rec, uint32_t n_here, uint32_t lane,
+                                                 const uint32_t* listed = nullptr) {
   __syncwarp();   // the previous batch has been read by every lane
-  if (lane < n_here) staged[lane].rec = __ldg(reinterpret_cast<const uint4*>(&a.cands[last_rec - lane]));
+  if (lane < n_here) staged[lane].rec = __ldg(reinterpret_cast<const uint4*>(&a.cands[last_rec - (listed ? listed[lane] : lane)]));
   __syncwarp();
   #pragma unroll 1
   for (uint32_t t = lane; t < n_here * 3u; t += 32) {
     const uint32_t r = t / 3u, j = t - r * 3u;
     if (j < (staged[r].rec.x >> 24)) {
-      const uint32_t child = __ldg(&a.cands[last_rec - r].child[j]);
+      const uint32_t child = __ldg(&a.cands[last_rec - (listed ? listed[r] : r)].child[j]);
       if (kAll && child >= lo) {
         stage_child(staged[r], j, a.sspec[child].emask, a.temp + a.temp_cap + a.sspec[child].erow, false);
       } else {
@@ -1118,7 +1127,7 @@ __device__ __noinline__ void phase_sweep(const HotArgs a, int mode, uint32_t lo,
     const uint2 cl = *reinterpret_cast<const uint2*>(&a.hdrs[i].cand_off);
     const uint32_t n_late = a.sspec[i].n_late, last = cl.x + cl.y - 1;   // the records with a same-stage child are the last ones
     const uint4 m = *reinterpret_cast<const uint4*>(&a.hdrs[i]);
-    uint32_t n_aff = 0;
+    uint32_t n_aff = 0, n_listed = 0;   // n_listed: records with a changed child, if a batch holds them
     if (!kAll && mode == SWEEP_NEW) {
       if (lane == 0) {
         const uint4 om = a.sspec[i].old_mask;
@@ -1149,9 +1158,20 @@ __device__ __noinline__ void phase_sweep(const HotArgs a, int mode, uint32_t lo,
       __syncwarp();
       // per such child and memory, the codes of this grid that read one of its changed slots
       if (n_aff <= kMaxAffected) {
+        const uint32_t r_own = lane < n_aff ? ws.who[lane] & 0xFFFFu : 0xFFFFu;
+        const uint32_t r_prev = __shfl_up_sync(0xFFFFFFFFu, r_own, 1);
+        const bool fresh = lane < n_aff && (lane == 0 || r_prev != r_own);   // a record's children follow one another
+        const uint32_t firsts = __ballot_sync(0xFFFFFFFFu, fresh), at = __popc(firsts & (0xFFFFFFFFu >> (31 - lane))) - 1;
+        if (__popc(firsts) <= kBatch) {
+          n_listed = __popc(firsts);
+          if (fresh) ws.listed[at] = r_own;
+        }
+        __syncwarp();
+        if (lane < n_aff) ws.who[lane] |= at << 20;
+        __syncwarp();
         #pragma unroll 1
         for (uint32_t t = lane; t < n_aff * 4u; t += 32) {
-          const uint32_t k = t & 3u, r = ws.who[t >> 2] & 0xFFFFu, j = ws.who[t >> 2] >> 16;
+          const uint32_t k = t & 3u, r = ws.who[t >> 2] & 0xFFFFu, j = (ws.who[t >> 2] >> 16) & 0xFu;
           const CandRec* const rec = &a.cands[last - r];
           const uint4 c = __ldg(reinterpret_cast<const uint4*>(rec));
           const uint32_t child = __ldg(&rec->child[j]), level = c.z & 0xFFu;
@@ -1197,7 +1217,7 @@ __device__ __noinline__ void phase_sweep(const HotArgs a, int mode, uint32_t lo,
     if (l_begin == l_end) continue;
     const bool single = n_late <= (uint32_t)kBatch;   // all records staged once for the whole item
     stage_slot_codes(ws.codes, m, n0, n1, n2, n3, lane);
-    const bool bounded = l_end - l_begin > kBoundCells && (kAll || single);
+    const bool bounded = l_end - l_begin > kBoundCells && (kAll || single) && !n_listed;
     const uint32_t cmax = bounded ? top_codes(codes, l_begin, l_end, n0, n1, n2, z0, z1, z2, z3) : 0u;
     uint4 ch = make_uint4(0, 0, 0, 0);   // codes of the slots of the cells that change
     if (kAll) {
@@ -1236,7 +1256,7 @@ __device__ __noinline__ void phase_sweep(const HotArgs a, int mode, uint32_t lo,
     for (;;) {
       // the next cells to solve, one per lane, collected from those that qualify
       bool live;
-      uint32_t slots;
+      uint32_t slots, reads;
       {
 #pragma unroll 1
         while (queued < 32 && c0 < l_end) {
@@ -1255,12 +1275,16 @@ __device__ __noinline__ void phase_sweep(const HotArgs a, int mode, uint32_t lo,
 #pragma unroll 1
             for (uint32_t e = 0; e < n_aff; e++) {
               const uint4 f = ws.affected[e];
-              hit |= (f.x >> k0) & (f.y >> k1) & (f.z >> k2) & (f.w >> k3);
+              hit |= ((f.x >> k0) & (f.y >> k1) & (f.z >> k2) & (f.w >> k3) & 1u) << (ws.who[e] >> 20);
             }
           }
-          const bool again = in && (hit & 1u);
+          const bool again = in && (mode == SWEEP_NEW ? hit & 1u : hit);
           const uint32_t who = __ballot_sync(0xFFFFFFFFu, again);
-          if (again) ws.queue[queued + __popc(who & ((1u << lane) - 1u))] = s0 | (s1 << 8) | (s2 << 16) | (s3 << 24);
+          if (again) {
+            const uint32_t at = queued + __popc(who & ((1u << lane) - 1u));
+            ws.queue[at] = s0 | (s1 << 8) | (s2 << 16) | (s3 << 24);
+            ws.reads[at] = (uint16_t)hit;
+          }
           queued += __popc(who);
           c0 += 32;
         }
@@ -1268,12 +1292,19 @@ __device__ __noinline__ void phase_sweep(const HotArgs a, int mode, uint32_t lo,
         __syncwarp();
         live = lane < queued;
         slots = live ? ws.queue[lane] : (z0 | (z1 << 8) | (z2 << 16) | (z3 << 24));
-        const uint32_t rest_of = ws.queue[32 + lane];
+        reads = live ? ws.reads[lane] : 0u;
+        const uint32_t rest_of = ws.queue[32 + lane], rest_reads = ws.reads[32 + lane];
         __syncwarp();
         queued = queued > 32 ? queued - 32 : 0;
-        if (lane < queued) ws.queue[lane] = rest_of;
+        if (lane < queued) {
+          ws.queue[lane] = rest_of;
+          ws.reads[lane] = (uint16_t)rest_reads;
+        }
       }
-      if (single && !staged_yet) {
+      if (n_listed) {
+        if (!staged_yet) stage_late_batch<false>(a, lo, staged, last, n_listed, lane, ws.listed);
+        staged_yet = true;
+      } else if (single && !staged_yet) {
         stage_late_batch<false>(a, lo, staged, last, n_late, lane);
         if (bounded) n_apply = stage_bounds<true>(ws, n_late, cmax, lane);
         staged_yet = true;
@@ -1285,17 +1316,41 @@ __device__ __noinline__ void phase_sweep(const HotArgs a, int mode, uint32_t lo,
       MrlRow* const at = grid + (((s3 * n2 + s2) * n1 + s1) * n0 + s0);
       Best best = {MRL_UNSAT, MRL_UNSAT, MRL_UNSAT};
       uint4 was = make_uint4(MRL_UNSAT, MRL_UNSAT, MRL_UNSAT, 0u);
-      if (live) {
-        const uint32_t i0 = __popc(em.x & bm0) - 1, i1 = __popc(em.y & bm1) - 1, i2 = __popc(em.z & bm2) - 1, i3 = __popc(em.w & bm3) - 1;
-        const uint4 f = ld_row(egrid + (((i3 * __popc(em.z) + i2) * __popc(em.y) + i1) * __popc(em.x) + i0));
-        best.main = f.x; best.peaks = f.y; best.tail = f.z;
-        was = ld_row(at);   // only this warp writes the cell in this sweep
-      }
+      if (live) was = ld_row(at);   // only this warp writes the cell in this sweep
+      bool whole = live;            // solve it from all its records
+      if (n_listed) {
+        // The other records cost what they did when the cell was last solved, so the cell's row still is
+        // the best of them, unless it came from one of these: then these alone decide as long as they
+        // reach the row again, and all records do where they fall short of it.
+        const uint32_t any = __reduce_or_sync(0xFFFFFFFFu, reads);
+        bool own = false;
 #pragma unroll 1
-      for (uint32_t b = 0; b < n_late; b += kBatch) {
-        const uint32_t n_here = min((uint32_t)kBatch, n_late - b);
-        if (!single) stage_late_batch<false>(a, lo, staged, last - b, n_here, lane);
-        eval_batch<true>(ws, single ? n_apply : n_here, bounded, live, cpack, bm0, bm1, bm2, bm3, best, tally);
+        for (uint32_t rest = any; rest; rest &= rest - 1) {
+          const uint32_t r = __ffs(rest) - 1;
+          own |= ((reads >> r) & 1u) && (staged[r].rec.x & 0xFFFFu) == (was.z & 0xFFFFu);
+        }
+        own = own && was.z != MRL_UNSAT;
+        if (!own) { best.main = was.x; best.peaks = was.y; best.tail = was.z; }
+#pragma unroll 1
+        for (uint32_t rest = any; rest; rest &= rest - 1) {
+          const uint32_t r = __ffs(rest) - 1;
+          if ((reads >> r) & 1u) eval_staged<true>(staged[r], cpack, bm0, bm1, bm2, bm3, best, tally);
+        }
+        whole = own && key_less(was.x, was.y, was.z, best);
+      }
+      if (__any_sync(0xFFFFFFFFu, whole)) {
+        if (whole) {
+          const uint32_t i0 = __popc(em.x & bm0) - 1, i1 = __popc(em.y & bm1) - 1, i2 = __popc(em.z & bm2) - 1, i3 = __popc(em.w & bm3) - 1;
+          const uint4 f = ld_row(egrid + (((i3 * __popc(em.z) + i2) * __popc(em.y) + i1) * __popc(em.x) + i0));
+          best.main = f.x; best.peaks = f.y; best.tail = f.z;
+        }
+#pragma unroll 1
+        for (uint32_t b = 0; b < n_late; b += kBatch) {
+          const uint32_t n_here = min((uint32_t)kBatch, n_late - b);
+          if (!single || n_listed) stage_late_batch<false>(a, lo, staged, last - b, n_here, lane);
+          eval_batch<true>(ws, single && !n_listed ? n_apply : n_here, bounded, whole, cpack, bm0, bm1, bm2, bm3, best, tally);
+        }
+        if (n_listed) staged_yet = false;   // the listed ones have been overwritten
       }
       if (live && (best.main != was.x || best.peaks != was.y || best.tail != was.z)) {
         st_row_shared(at, make_uint4(best.main, best.peaks, best.tail, 0u));
@@ -1519,7 +1574,6 @@ __device__ __noinline__ void phase_count(const StageArgs& a, uint32_t lo, uint32
 // owner's rows onto them). Returns the rows that this block's Specs take.
 __device__ __noinline__ unsigned long long phase_compact(const StageArgs& a, uint32_t lo, uint32_t hi, unsigned long long first_row,
                                                          unsigned long long* block_bytes) {
-  __shared__ uint32_t off[kStageBlock];
   __shared__ uint32_t warp_base[kStageBlock / 32 + 1];
   const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   WarpScratch& ws = warp_scratch();
@@ -1539,7 +1593,7 @@ __device__ __noinline__ unsigned long long phase_compact(const StageArgs& a, uin
     }
     if (!few) {
       __syncthreads();   // the run before has been read
-      off[threadIdx.x] = inc - n_own;
+      ws.who[lane] = inc - n_own;   // (the sweeps' scratch is free here)
       if (lane == 31) warp_base[warp] = inc;
       __syncthreads();
       if (warp == 0) {
@@ -1558,7 +1612,7 @@ __device__ __noinline__ unsigned long long phase_compact(const StageArgs& a, uin
 #pragma unroll 1
     for (uint32_t k = warp; k < here; k += kStageBlock / 32) {
       const uint32_t i = base + k;
-      const uint32_t place = few ? __shfl_sync(0xFFFFFFFFu, inc - n_own, k) : warp_base[k >> 5] + off[k];
+      const uint32_t place = few ? __shfl_sync(0xFFFFFFFFu, inc - n_own, k) : warp_base[k >> 5] + reinterpret_cast<const WarpScratch*>(&ws - warp)[k >> 5].who[k & 31u];
       const unsigned long long fbase = first_row + taken + place;
       const uint4 fm = a.rmask[i], tm = *reinterpret_cast<const uint4*>(&a.hdrs[i]);
       const unsigned long long tbase = a.hdrs[i].row_base;
