@@ -462,12 +462,20 @@ __device__ __forceinline__ bool is_late(const uint4 a) { return (a.z >> 24) & 1u
 // The Specs a warp of a per-Spec phase takes at a time: as many as keep all warps busy, at most one
 // per lane.
 __device__ __forceinline__ uint32_t group_size(uint32_t n, uint32_t gwarps) { return max(1u, min(32u, (n + gwarps - 1) / gwarps)); }
-// Cells per work item: a work item's records are staged once, so long items where there are enough
-// of them; one step of the warp where Specs are few. Grids have 100 to 600 cells on average.
-__device__ __forceinline__ uint32_t item_size(uint32_t n, uint32_t gwarps) {
-  if (n >= gwarps * (MRL_ITEM_CELLS / 128u)) return MRL_ITEM_CELLS;
-  return max(32u, n * 128u / gwarps & ~31u);
+// Cells per work item of a grid, as a power of two times 32 (0 to 5: 32 to MRL_ITEM_CELLS cells). An item's
+// records are staged and bounded once, so items are long while there are enough of them: some four for
+// every warp if the stage's other grids are as large as this one, and 128 cells a grid, the average, are
+// taken where it is smaller or has more same-stage records than a batch (then its cells cost several
+// times those of others, and long items leave warps idle at the barrier). 8x8x8 Matmul 65.0 ms by the
+// number of Specs alone, 60.4 with four items a warp, 64.0 with one, 68.6 with sixteen; 16x16 Move 8.4,
+// 8.8, 9.8 and 9.1, which is why such Specs keep to the number alone.
+__device__ __forceinline__ uint32_t item_log(unsigned long long cells, uint32_t n_late, uint32_t n, uint32_t gwarps) {
+  const unsigned long long share = (n_late > 16u ? 128ull : max(128ull, cells / 4)) * n / gwarps;
+  return share >= MRL_ITEM_CELLS ? 5u : (share < 32u ? 0u : 26u - __clz((uint32_t)share));
 }
+// An item's first cell, and its size; first_cell has the size's log in bits 1 to 3 (bit 0: the grid is new).
+__device__ __forceinline__ uint32_t item_first(const WorkItem& it) { return it.first_cell & ~31u; }
+__device__ __forceinline__ uint32_t item_cells(const WorkItem& it) { return 32u << ((it.first_cell >> 1) & 7u); }
 
 // One pass over the records of a Spec, a record per lane: the breakpoints of the records whose children
 // all lie in finished stages (they come first), the corner of those, and of the others with nothing
@@ -526,9 +534,10 @@ __device__ __noinline__ void phase_records(const StageArgs& a, StageCtl* sc, uin
 // the lane's first row, and items at the end of the list. What does not fit is counted and left out;
 // the totals are checked behind the next barrier.
 __device__ __forceinline__ unsigned long long place_grids(const StageArgs& a, StageCtl* sc, unsigned long long* row_cursor, uint32_t spec, unsigned long long cells,
-                                                          unsigned long long item_cells_of, uint32_t item_cells, uint32_t flag, uint32_t lane) {
+                                                          unsigned long long item_cells_of, uint32_t log, uint32_t flag, uint32_t lane) {
   unsigned long long inc = cells;
-  uint32_t items = (uint32_t)((item_cells_of + item_cells - 1) / item_cells), iinc = items;
+  uint32_t items = (uint32_t)((item_cells_of + (32u << log) - 1) >> (5u + log)), iinc = items;
+  flag |= log << 1;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
     const unsigned long long t = __shfl_up_sync(0xFFFFFFFFu, inc, o);
@@ -555,7 +564,7 @@ __device__ __forceinline__ unsigned long long place_grids(const StageArgs& a, St
       if (at + w < a.item_cap) {
         WorkItem it;
         it.spec = sp;
-        it.first_cell = (w * item_cells) | fl;
+        it.first_cell = (w * item_cells(WorkItem{0, fl})) | fl;
         a.items[at + w] = it;
       }
   }
@@ -566,7 +575,7 @@ __device__ __forceinline__ unsigned long long place_grids(const StageArgs& a, St
 // of the unordered phase, its rows and work items.
 __device__ __noinline__ void phase_place_early(const StageArgs& a, StageCtl* sc, uint32_t lo, uint32_t hi, uint32_t gwarp, uint32_t gwarps, bool any_late) {
   const uint32_t lane = threadIdx.x & 31;
-  const uint32_t G = group_size(hi - lo, gwarps), item_cells = item_size(hi - lo, gwarps);
+  const uint32_t G = group_size(hi - lo, gwarps);
   #pragma unroll 1
   for (uint32_t base = lo + gwarp * G; base < hi; base += gwarps * G) {
     const uint32_t i = base + lane;
@@ -601,7 +610,7 @@ __device__ __noinline__ void phase_place_early(const StageArgs& a, StageCtl* sc,
       m = clip_at_corner(m, corner);
       cells = cells_of(m);
     }
-    const unsigned long long row = place_grids(a, sc, &sc->rows_early, i, cells, cells, item_cells, 0, lane);
+    const unsigned long long row = place_grids(a, sc, &sc->rows_early, i, cells, cells, item_log(cells, n_late, hi - lo, gwarps), 0, lane);
     if (mine) {
       StageSpec& s = a.sspec[i - lo];
       s.emask = m;
@@ -620,7 +629,7 @@ __device__ __noinline__ void phase_place_early(const StageArgs& a, StageCtl* sc,
 // A Spec without such records is finished: its grid is that of the unordered phase.
 __device__ __noinline__ void phase_place_late(const StageArgs& a, StageCtl* sc, uint32_t lo, uint32_t hi, uint32_t gwarp, uint32_t gwarps, uint32_t pass) {
   const uint32_t lane = threadIdx.x & 31;
-  const uint32_t G = group_size(hi - lo, gwarps), item_cells = item_size(hi - lo, gwarps);
+  const uint32_t G = group_size(hi - lo, gwarps);
   #pragma unroll 1
   for (uint32_t base = lo + gwarp * G; base < hi; base += gwarps * G) {
     const uint32_t i = base + lane;
@@ -662,7 +671,7 @@ __device__ __noinline__ void phase_place_late(const StageArgs& a, StageCtl* sc, 
       fresh = !pass || nm.x != old.x || nm.y != old.y || nm.z != old.z || nm.w != old.w;
       cells = cells_of(nm);
     }
-    const unsigned long long row = place_grids(a, sc, &sc->rows_late, i, fresh ? cells : 0ull, cells, item_cells, fresh ? 1u : 0u, lane);
+    const unsigned long long row = place_grids(a, sc, &sc->rows_late, i, fresh ? cells : 0ull, cells, item_log(cells, n_late, hi - lo, gwarps), fresh ? 1u : 0u, lane);
     if (fresh) {
       StageSpec& s = a.sspec[i - lo];
       s.old_mask = old;
@@ -713,7 +722,7 @@ struct HotArgs {   // what the solve phases read, by value: registers instead of
   unsigned long long temp_cap;   // the grids of the unordered phase start here
   StageSpec* sspec;              // already offset: indexed by Spec id
   const WorkItem* items;
-  uint32_t n_items, item_cells;
+  uint32_t n_items;
   uint32_t* next_item;
 };
 
@@ -1038,8 +1047,8 @@ __device__ __noinline__ void phase_early(const HotArgs a, unsigned long long* bl
     const uint4 m = sp.emask;
     const uint2 cl = *reinterpret_cast<const uint2*>(&a.hdrs[it.spec].cand_off);
     stage_slot_codes(ws.codes, m, __popc(m.x), __popc(m.y), __popc(m.z), __popc(m.w), lane);
-    solve_early_cells(a, ws, cl.x, cl.y - sp.n_late, m, sp.corner, a.temp + a.temp_cap + sp.erow, it.first_cell,
-                      min((uint32_t)cells_of(m), it.first_cell + a.item_cells), tally, lane);
+    solve_early_cells(a, ws, cl.x, cl.y - sp.n_late, m, sp.corner, a.temp + a.temp_cap + sp.erow, item_first(it),
+                      min((uint32_t)cells_of(m), item_first(it) + item_cells(it)), tally, lane);
   } while (next_item(a, w, lane));
   add_tally(tally, &block_stats[0], &block_stats[1], lane);
 }
@@ -1122,7 +1131,7 @@ __device__ __noinline__ void phase_sweep(const HotArgs a, int mode, uint32_t lo,
 #pragma unroll 1
   do {
     const WorkItem it = a.items[w];
-    const uint32_t i = it.spec, first_cell = it.first_cell & ~31u;
+    const uint32_t i = it.spec, first_cell = item_first(it);
     if (!kAll && mode == SWEEP_NEW && !(it.first_cell & 1u)) continue;   // the grid did not grow
     const uint2 cl = *reinterpret_cast<const uint2*>(&a.hdrs[i].cand_off);
     const uint32_t n_late = a.sspec[i].n_late, last = cl.x + cl.y - 1;   // the records with a same-stage child are the last ones
@@ -1200,9 +1209,9 @@ __device__ __noinline__ void phase_sweep(const HotArgs a, int mode, uint32_t lo,
                    z3 = corner_of(corner, 3) ? 1u : 0u;
     const uint32_t v0 = n0 - z0, v1 = n1 - z1, v2 = n2 - z2, v3 = n3 - z3;
     const uint32_t live_cells = none ? 0u : v0 * v1 * v2 * v3;
-    const uint32_t c_hi = min(cells, first_cell + a.item_cells);
+    const uint32_t c_hi = min(cells, first_cell + item_cells(it));
     uint32_t l_begin = 0, l_end = live_cells;
-    if (cells > a.item_cells) {   // several items
+    if (cells > item_cells(it)) {   // several items
       l_begin = (uint32_t)((unsigned long long)live_cells * first_cell / cells);
       l_end = (uint32_t)((unsigned long long)live_cells * c_hi / cells);
     }
@@ -1378,13 +1387,13 @@ __device__ __noinline__ void phase_refine(const HotArgs a) {
   do {
     const WorkItem it = a.items[w];
     if (!(it.first_cell & 1u)) continue;
-    const uint32_t i = it.spec, first_cell = it.first_cell & ~31u;
+    const uint32_t i = it.spec, first_cell = item_first(it);
     const uint4 m = *reinterpret_cast<const uint4*>(&a.hdrs[i]);
     MrlRow* const grid = a.temp + (a.hdrs[i].row_base & ~MRL_TEMP_FLAG);
     const uint4 om = a.sspec[i].old_mask;
     const unsigned long long obase = a.sspec[i].old_row;
     const uint32_t n0 = __popc(m.x), n1 = __popc(m.y), n2 = __popc(m.z), n3 = __popc(m.w);
-    const uint32_t c_end = min(n0 * n1 * n2 * n3, first_cell + a.item_cells);
+    const uint32_t c_end = min(n0 * n1 * n2 * n3, first_cell + item_cells(it));
     #pragma unroll 1
     for (uint32_t cell = first_cell + lane; cell < c_end; cell += 32) {
       uint32_t s0, s1, s2, s3;
@@ -1442,12 +1451,12 @@ __device__ __noinline__ void phase_real_masks(const HotArgs a, uint4* rmask, boo
 #pragma unroll 1
   do {
     const WorkItem it = a.items[w];
-    const uint32_t i = it.spec, first_cell = it.first_cell & ~31u;
+    const uint32_t i = it.spec, first_cell = item_first(it);
     if (only_dirty && !a.sspec[i].dirty) continue;
     const uint4 m = kEarly ? a.sspec[i].emask : *reinterpret_cast<const uint4*>(&a.hdrs[i]);
     const MrlRow* const grid = kEarly ? a.temp + a.temp_cap + a.sspec[i].erow : a.temp + (a.hdrs[i].row_base & ~MRL_TEMP_FLAG);
     stage_slot_codes(ws.codes, m, __popc(m.x), __popc(m.y), __popc(m.z), __popc(m.w), lane);
-    const uint4 real = real_breakpoints(ws.codes, m, grid, first_cell, min((uint32_t)cells_of(m), first_cell + a.item_cells), lane);
+    const uint4 real = real_breakpoints(ws.codes, m, grid, first_cell, min((uint32_t)cells_of(m), first_cell + item_cells(it)), lane);
     if (lane == 0) {
       uint32_t* const out = reinterpret_cast<uint32_t*>(&rmask[i]);
       if (real.x & ~1u) atomicOr(out, real.x);
@@ -1487,7 +1496,8 @@ __device__ __noinline__ void phase_early_fused(const StageArgs& a, const HotArgs
     m = clip_at_corner(m, corner);
     const unsigned long long cells = cells_of(m);
     const bool here = cells <= kInlineCells;
-    const uint32_t n_items = here ? 0u : (uint32_t)((cells + h.item_cells - 1) / h.item_cells);
+    const uint32_t log = item_log(cells, n_late, hi - lo, gwarps);
+    const uint32_t n_items = here ? 0u : (uint32_t)((cells + (32u << log) - 1) >> (5u + log));
     unsigned long long row = 0;
     uint32_t item0 = 0;
     if (lane == 0) {
@@ -1502,7 +1512,7 @@ __device__ __noinline__ void phase_early_fused(const StageArgs& a, const HotArgs
       if (at < a.item_cap) {
         WorkItem it;
         it.spec = i;
-        it.first_cell = w * h.item_cells;
+        it.first_cell = (w << (5u + log)) | (log << 1);
         a.items[at] = it;
       }
     }
@@ -1761,7 +1771,7 @@ __global__ void __launch_bounds__(kStageBlock, 1) stage_kernel(const __grid_cons
       uint32_t ph = 0;   // phases that hand out items take the counters in turn; one is cleared four phases ahead
       HotArgs h;
       h.hdrs = a.hdrs; h.cands = a.cands; h.rows = a.rows; h.temp = a.temp; h.temp_cap = a.temp_cap; h.sspec = a.sspec - lo;
-      h.items = a.items; h.item_cells = item_size(hi - lo, gwarps); h.n_items = 0; h.next_item = nullptr;
+      h.items = a.items; h.n_items = 0; h.next_item = nullptr;
       auto hand_out = [&](uint32_t n_items) {
         h.n_items = n_items;
         h.next_item = &sc->next_item[ph & 7];

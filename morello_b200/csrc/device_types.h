@@ -53,8 +53,8 @@ struct CandRec {
 };
 
 // A piece of one Spec's grid for a solve phase: consecutive cells from
-// first_cell on, at most MRL_ITEM_CELLS of them (the stage kernel picks the size, a multiple of 32;
-// bit 0 of first_cell: the grid is new in this pass). Warps take items as they finish others.
+// first_cell on, at most MRL_ITEM_CELLS of them (the stage kernel picks the size, 32 << bits 1 to 3 of
+// first_cell; bit 0: the grid is new in this pass). Warps take items as they finish others.
 #define MRL_ITEM_CELLS 1024u
 struct WorkItem {
   uint32_t spec;
