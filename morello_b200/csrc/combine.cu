@@ -1,32 +1,30 @@
 // The CUDA side of the synthesis-database fill (sm_100a).
 //
-// Specs are processed stage by stage (plan.hpp). One cooperative launch solves a whole stage
-// on the device, with grid-wide barriers between its phases and nothing for the host to decide.
+// Specs are processed stage by stage (plan.hpp). A team of blocks solves a whole stage on the device,
+// with barriers between its phases and nothing for the host to decide.
 // A limits grid of a Spec = per memory the lattice codes at which its result can change; a cell
 // = one combination of slots; evaluating a candidate record at a cell = feasibility under the
 // cell's limits, gather of the child rows at the children's limits, combine into a Cost,
 // lexicographic minimum.
 //   0. corners: below its corner a Spec has no implementation at all; every grid of the stage is
-//      clipped there (phase_minsat, phase_corner);
+//      clipped there (phase_minsat, phase_records, phase_place_early);
 //   1. once per stage, the records whose children all lie in earlier stages are solved on a grid
 //      of their own - their thresholds plus the (shifted) breakpoints of those children's
 //      finished tables - in no particular order: a warp takes a piece of one Spec's grid, stages
-//      the Spec's records and the headers of their children in shared memory, and its lanes take
-//      32 cells at a time and walk the staged records together (phase_derive_early,
-//      phase_place, phase_early); the real breakpoints of the result are found at once
-//      (phase_real_masks);
+//      the Spec's records and the headers of their children in shared memory, orders the records by
+//      a lower bound on their cost there, and its lanes take 32 cells at a time and walk the staged
+//      records together as far as one can still gain (phase_early; phase_early_fused for small
+//      teams); the real breakpoints of the result are found at once (phase_real_masks);
 //   2. the rest - relayout Moves, whose body is a Spec of the same stage at strictly lower limits
 //      - is solved on working grids: the real breakpoints of step 1's result, the thresholds of
-//      those records and the shifted breakpoints of their children (phase_derive_late). Every
-//      working cell starts from step 1's result at its limits (phase_late_init) and is recomputed
-//      in place, sweep after sweep, from that and its records at the children's current values,
-//      until a sweep changes nothing (phase_late): the dependencies between cells form no cycle,
-//      so that fixpoint is the direct solve;
+//      those records and the shifted breakpoints of their children (phase_place_late), in sweeps
+//      until one changes nothing (phase_sweep): the dependencies between cells form no cycle, so
+//      that fixpoint is the direct solve;
 //   3. breakpoints at which some pair of neighbouring cells differs are real
 //      (phase_real_masks); 2-3 repeat for the Specs whose working grid still lacks a breakpoint
-//      that a same-stage child turned out to have, and for the Specs above them (phase_spread);
-//   4. the working grids are compacted to the real breakpoints and appended to the table
-//      (phase_final_count, phase_scan_sums, phase_compact).
+//      that a same-stage child turned out to have (phase_check_grids, phase_refine);
+//   4. the grids are compacted to the real breakpoints and appended to the table (phase_count,
+//      phase_compact).
 // Step 3's fixpoint is exact: when every Spec's grid contains all thresholds and all shifted
 // breakpoints of the computed tables of its children, induction over the limits lattice shows
 // every computed cell equals the direct solve at every limit inside it.
