@@ -1724,8 +1724,9 @@ __device__ __noinline__ void warm_l1(const StageArgs& a) {
 
 // A run of stages, each start to finish, by one team of blocks: the grid (cooperative launch), one
 // cluster, or one block. Every thread of the team reaches every barrier: what decides the control
-// flow (totals, the sweep that last changed a cell, the error word) is read from device memory after
-// a barrier and written again only after a later one, so all threads take the same branches.
+// flow (totals, the error word) is read from device memory after a barrier and written again only after
+// a later one, so all threads take the same branches. The one exception is the sweep that last changed a
+// cell (sweep_changed_a_cell).
 //
 // What bounds a small stage is the number of barriers: a grid-wide one takes 2 us and more, and a
 // 2x2x2 Matmul search has 86 stages of 9 Specs on average. So the team fits the stage - a cluster's
@@ -1860,7 +1861,7 @@ __global__ void __launch_bounds__(kStageBlock, 1) stage_kernel(const __grid_cons
             else phase_sweep<false>(h, first ? SWEEP_NEW : SWEEP_CHANGED, lo, before, now, sweep, &sc->any_changed, block_stats);
             team_sync();
             MARK(first ? MRL_PH_SWEEP_FIRST : MRL_PH_SWEEP_MORE);
-            if (get(&sc->any_changed) != sweep) break;   // nothing changed anywhere: the stage's cells are consistent
+            if (!sweep_changed_a_cell(get(&sc->any_changed), sweep)) break;   // nothing changed anywhere: the stage's cells are consistent
             if (sweep - sweep_before >= (uint32_t)kMaxSweeps) {   // more sweeps than the limits lattice has diagonals: give up rather than spin
               failed = true;
               if (gtid == 0) { ctl->failed_stage = st; ctl->error |= MRL_ERR_PASSES; }

@@ -104,10 +104,18 @@ struct StageCtl {                    // of one stage; zero at its start
   unsigned long long rows_late;      // working rows handed out
   uint32_t n_items;                  // work items listed
   uint32_t any_late;                 // stage + 1 when some Spec of it has a record with a same-stage child
-  uint32_t any_changed;              // last relaxation sweep that changed a cell
+  uint32_t any_changed;              // last relaxation sweep that changed a cell; only grows within a stage
   uint32_t grew;                     // pass + 1 when a grid has to grow after it
   uint32_t next_item[8];             // item hand-out of a phase; the phases take turns
 };
+// Whether a relaxation sweep changed a cell, from StageCtl::any_changed as read behind the sweep's barrier.
+// Nothing separates that read from the next sweep of the threads that have made it already, so the word may
+// hold the next sweep's number by then - which is only ever stored where this one changed something.
+#ifdef __CUDACC__
+__host__ __device__
+#endif
+inline bool sweep_changed_a_cell(uint32_t any_changed, uint32_t sweep) { return any_changed >= sweep; }
+
 struct FillCtl {
   StageCtl stage;
   // -- sticky over a fill
