@@ -531,7 +531,7 @@ __device__ __noinline__ void phase_records(const StageArgs& a, StageCtl* sc, uin
 // Rows and work items for the grids of up to 32 Specs, one per lane (`cells` 0: none), by one warp:
 // the lane's first row, and items at the end of the list. What does not fit is counted and left out;
 // the totals are checked behind the next barrier.
-__device__ __forceinline__ unsigned long long place_grids(const StageArgs& a, StageCtl* sc, unsigned long long* row_cursor, uint32_t spec, unsigned long long cells,
+__device__ __forceinline__ unsigned long long place_grids(const StageArgs& a, unsigned long long* row_cursor, uint32_t* item_cursor, uint32_t spec, unsigned long long cells,
                                                           unsigned long long item_cells_of, uint32_t log, uint32_t flag, uint32_t lane) {
   unsigned long long inc = cells;
   uint32_t items = (uint32_t)((item_cells_of + (32u << log) - 1) >> (5u + log)), iinc = items;
@@ -546,7 +546,7 @@ __device__ __forceinline__ unsigned long long place_grids(const StageArgs& a, St
   uint32_t item0 = 0;
   if (lane == 31) {
     if (inc) row0 = atomicAdd(row_cursor, inc);
-    if (iinc) item0 = atomicAdd(&sc->n_items, iinc);
+    if (iinc) item0 = atomicAdd(item_cursor, iinc);
   }
   row0 = __shfl_sync(0xFFFFFFFFu, row0, 31);
   item0 = __shfl_sync(0xFFFFFFFFu, item0, 31);
@@ -608,7 +608,7 @@ __device__ __noinline__ void phase_place_early(const StageArgs& a, StageCtl* sc,
       m = clip_at_corner(m, corner);
       cells = cells_of(m);
     }
-    const unsigned long long row = place_grids(a, sc, &sc->rows_early, i, cells, cells, item_log(cells, n_late, hi - lo, gwarps), 0, lane);
+    const unsigned long long row = place_grids(a, &sc->rows_early, &sc->n_items_early, i, cells, cells, item_log(cells, n_late, hi - lo, gwarps), 0, lane);
     if (mine) {
       StageSpec& s = a.sspec[i - lo];
       s.emask = m;
@@ -669,7 +669,7 @@ __device__ __noinline__ void phase_place_late(const StageArgs& a, StageCtl* sc, 
       fresh = !pass || nm.x != old.x || nm.y != old.y || nm.z != old.z || nm.w != old.w;
       cells = cells_of(nm);
     }
-    const unsigned long long row = place_grids(a, sc, &sc->rows_late, i, fresh ? cells : 0ull, cells, item_log(cells, n_late, hi - lo, gwarps), fresh ? 1u : 0u, lane);
+    const unsigned long long row = place_grids(a, &sc->rows_late, &sc->n_items, i, fresh ? cells : 0ull, cells, item_log(cells, n_late, hi - lo, gwarps), fresh ? 1u : 0u, lane);
     if (fresh) {
       StageSpec& s = a.sspec[i - lo];
       s.old_mask = old;
@@ -1500,7 +1500,7 @@ __device__ __noinline__ void phase_early_fused(const StageArgs& a, const HotArgs
     uint32_t item0 = 0;
     if (lane == 0) {
       row = atomicAdd(&sc->rows_early, cells);
-      if (n_items) item0 = atomicAdd(&sc->n_items, n_items);
+      if (n_items) item0 = atomicAdd(&sc->n_items_early, n_items);
     }
     row = __shfl_sync(0xFFFFFFFFu, row, 0);
     item0 = __shfl_sync(0xFFFFFFFFu, item0, 0);
@@ -1807,7 +1807,7 @@ __global__ void __launch_bounds__(kStageBlock, 1) stage_kernel(const __grid_cons
         MARK(MRL_PH_SETUP);
       }
       const unsigned long long cells = get(&sc->rows_early);
-      const uint32_t n_early_items = get(&sc->n_items);
+      const uint32_t n_early_items = get(&sc->n_items_early);
       failed = too_small(cells, 0, n_early_items);
       if (!failed && cells) {
         st_cells += cells;
@@ -1817,7 +1817,6 @@ __global__ void __launch_bounds__(kStageBlock, 1) stage_kernel(const __grid_cons
           phase_early(h, block_stats);
           team_sync();
           MARK(MRL_PH_EARLY);
-          if (gtid == 0) sc->n_items = 0;   // read above, behind a barrier; used again from phase_place_late on
           hand_out(n_early_items);
           phase_real_masks<true>(h, a.rmask, false);
           team_sync();
@@ -1931,7 +1930,7 @@ __global__ void __launch_bounds__(kStageBlock, 1) stage_kernel(const __grid_cons
           ctl->stage_first_row = final_top;
           ctl->stage_rows = total;
           sc->rows_early = sc->rows_late = 0;
-          sc->n_items = sc->any_changed = sc->grew = 0;
+          sc->n_items_early = sc->n_items = sc->any_changed = sc->grew = 0;
 #pragma unroll
           for (int k = 0; k < 8; k++) sc->next_item[k] = 0;
         }

@@ -102,7 +102,9 @@ enum {
 struct StageCtl {                    // of one stage; zero at its start
   unsigned long long rows_early;     // rows handed out to the grids of the unordered phase
   unsigned long long rows_late;      // working rows handed out
-  uint32_t n_items;                  // work items listed
+  uint32_t n_items_early;            // work items listed for the grids of the unordered phase
+  uint32_t n_items;                  // ... for the working grids. A word of its own: a stage whose unordered phase left
+                                     // no items adds to it while slower threads still read how many that phase left
   uint32_t any_late;                 // stage + 1 when some Spec of it has a record with a same-stage child
   uint32_t any_changed;              // last relaxation sweep that changed a cell; only grows within a stage
   uint32_t grew;                     // pass + 1 when a grid has to grow after it

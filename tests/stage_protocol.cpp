@@ -36,6 +36,27 @@ static bool sweeps(World& w, Thread& t, uint32_t branch) {
   }
 }
 
+// From the unordered phase to the working grids: its work items are counted, a barrier, every thread reads
+// the count and takes part in solving them (and another barrier) if there are any; then items for the
+// working grids are counted, a barrier, and that count is read. The small teams solve grids where they
+// count them, so a stage may leave no items of the first kind.
+static bool items(World& w, Thread& t, uint32_t branch) {
+  switch (t.pc) {
+    case 0:
+      w.ctl.n_items_early += branch;
+      t.pc = 1;
+      t.waiting = 1;
+      return true;
+    case 1:
+      t.seen_early = w.ctl.n_items_early;
+      t.pc = t.seen_early ? 2 : 3;
+      return false;
+    case 2: t.pc = 3; t.waiting = 1; return false;
+    case 3: w.ctl.n_items++; t.pc = 4; t.waiting = 1; return false;
+    default: t.seen_late = w.ctl.n_items; t.done = 1; return false;
+  }
+}
+
 static std::set<std::string> g_seen;
 static long g_states = 0;
 
@@ -72,6 +93,7 @@ int main(int argc, char** argv) {
   memset(&w, 0, sizeof(w));
   Step step = nullptr;
   if (argc == 2 && !strcmp(argv[1], "sweeps")) step = sweeps;
+  if (argc == 2 && !strcmp(argv[1], "items")) step = items;
   if (!step) return 2;
   const bool ok = explore(w, step);
   printf("%ld states\n", g_states);

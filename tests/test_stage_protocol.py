@@ -19,7 +19,7 @@ def explorer(tmp_path_factory):
     return exe
 
 
-@pytest.mark.parametrize("model", ["sweeps"])
+@pytest.mark.parametrize("model", ["sweeps", "items"])
 def test_threads_agree_in_every_order(explorer, model):
     res = subprocess.run([explorer, model], capture_output=True, text=True, timeout=60)
     assert res.returncode == 0, res.stdout
