@@ -122,9 +122,11 @@ long mrl_tabulate(const uint8_t* blob, size_t len, uint8_t* out, size_t cap);
 int mrl_top_down_many(mrl_ctx* ctx, const uint8_t* blobs, const uint64_t* blob_off, size_t n, const uint64_t* limits,
                       mrl_decision* out);
 
-/* Cross-check modes of the host planner (tests): same plan, built the slow way. Bit 0: tabulate
+/* Cross-check modes (tests): same plan, built the slow way, and same tables. Bit 0: tabulate
  * both dtypes of a mirrored goal set instead of deriving f32 records from u32 ones; bit 1:
- * tabulate every Spec from scratch instead of re-using per-operand results. */
+ * tabulate every Spec from scratch instead of re-using per-operand results; bit 2: plan on the host also
+ * where the device would. Bit 3: fills take the ways of large ones (candidate records planned on the host go
+ * up in the background whatever their size). */
 int mrl_set_plan_flags(mrl_ctx* ctx, uint32_t flags);
 
 /* No counterpart in the reference. Same inputs, outputs and results as mrl_top_down_many, for
@@ -152,7 +154,8 @@ int mrl_precompute(mrl_ctx* ctx, uint32_t size, int through, int dtype_mask);
  * host, copy the plan to the device, fill (may be repeated). Gigabytes of candidate records keep
  * going up in the background after mrl_upload has returned, in stage order; a fill waits stage by
  * stage for the records it needs, so its first stages overlap the copy. Calls that replace the
- * plan or read the device records (mrl_plan_*, mrl_verify, mrl_device_cands) wait for the copy. */
+ * plan or read the device records (mrl_plan_*, mrl_verify, mrl_device_cands, mrl_get_impl) wait for the
+ * copy. */
 int mrl_plan_precompute(mrl_ctx* ctx, uint32_t size, int through, int dtype_mask);
 int mrl_plan_goals(mrl_ctx* ctx, const uint8_t* blobs, const uint64_t* blob_off, size_t n);
 int mrl_upload(mrl_ctx* ctx);

@@ -35,7 +35,7 @@ struct mrl_ctx {
   mrl_stats stats;
   std::string err;
   uint32_t rank = 0, world = 1;
-  uint32_t plan_flags = 0;        // PLAN_NO_TWINS | PLAN_NO_MEMO
+  uint32_t plan_flags = 0;        // PLAN_* and FILL_SMALL_START
   bool cands_elsewhere = false;   // adopted plan whose candidate records only exist on the planning rank
   bool table_only = false;        // loaded from a file without a matching plan: lookups only
 };
@@ -146,7 +146,7 @@ int set_plan(mrl_ctx* ctx, Job&& job) {
   const double t0 = now_s();
   double goal_seconds = 0;
   OpTables tab;
-  bool factored = ctx->device >= 0 && ctx->world == 1 && ctx->plan_flags == 0;
+  bool factored = ctx->device >= 0 && ctx->world == 1 && !(ctx->plan_flags & ~(uint32_t)FILL_SMALL_START);
   if (factored) {
     try {
       if (job.precompute) tab.build_precompute(job.size, job.through, job.dtypes);
@@ -366,8 +366,9 @@ int mrl_plan_goals(mrl_ctx* ctx, const uint8_t* blobs, const uint64_t* blob_off,
 
 int mrl_set_plan_flags(mrl_ctx* ctx, uint32_t flags) {
   if (!ctx) return -1;
-  if (flags & ~(uint32_t)(PLAN_NO_TWINS | PLAN_NO_MEMO)) return fail(ctx, -1, "unknown plan flag");
+  if (flags & ~(uint32_t)(PLAN_NO_TWINS | PLAN_NO_MEMO | PLAN_ON_HOST | FILL_SMALL_START)) return fail(ctx, -1, "unknown plan flag");
   ctx->plan_flags = flags;
+  ctx->dev.small_start((flags & FILL_SMALL_START) != 0);
   return 0;
 }
 
@@ -476,7 +477,7 @@ int mrl_top_down_many_noalloc(mrl_ctx* ctx, const uint8_t* blobs, const uint64_t
     std::vector<LogicalSpec> goals;
     if (parse_goals(blobs, blob_off, n, goals) != 0) return fail(ctx, -4, "goal Spec is not canonicalizable");
     // A plan of its own: the context's tables (and their device memory) are left as they are.
-    if (ctx->plan_flags == 0) {
+    if (!(ctx->plan_flags & ~(uint32_t)FILL_SMALL_START)) {
       char err[256] = {0};
       int rc = 1;
       std::vector<uint64_t> specs;

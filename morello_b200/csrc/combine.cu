@@ -2474,10 +2474,10 @@ int DeviceFill::upload(const Plan& plan, bool skip_cands) {
       // 11 GB/s, so four threads copy them on their own streams, piece by piece in id order, and
       // go on after this call has returned (wait_cands_).
       const size_t total = n_cand_bytes_;
-      if (fixed_ || total < (size_t(1) << 30)) {
+      if (fixed_ || (total < (size_t(1) << 30) && !small_start_)) {
         CK(cudaMemcpyAsync(d_cands_, plan.cands.data(), total, cudaMemcpyHostToDevice, stream_));
       } else {
-        up_piece_bytes_ = size_t(128) << 20;
+        up_piece_bytes_ = small_start_ ? size_t(64) << 10 : size_t(128) << 20;
         up_pieces_ = (total + up_piece_bytes_ - 1) / up_piece_bytes_;
         up_done_.reset(new std::atomic<uint8_t>[up_pieces_]);
         for (size_t k = 0; k < up_pieces_; k++) up_done_[k].store(0, std::memory_order_relaxed);
@@ -3019,6 +3019,7 @@ int DeviceFill::walk(uint64_t root, bool packed, uint32_t cpack, std::vector<Wal
   std::lock_guard<std::mutex> guard(lookup_mu_);
   CK(cudaSetDevice(device_));
   if (packed && !tab_) { snprintf(err_, sizeof(err_), "no plan made on the device"); return -3; }
+  if (wait_upload()) return -1;   // a table that was loaded may be here before the records are
   const size_t head = align256(sizeof(uint32_t)), bytes = head + kWalkMost * sizeof(WalkNode), first = head + 96 * sizeof(WalkNode);
   int rc;
   if ((rc = reserve_(b_lookup_, bytes, false)) || (rc = reserve_host_(bytes))) return rc;

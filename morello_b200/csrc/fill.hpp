@@ -61,6 +61,8 @@ class DeviceFill {
   // skip_cands: the candidate records are not on this host; the caller fills device_cands()
   // itself (e.g. a broadcast from the rank that planned) and then calls cands_arrived().
   int upload(const Plan& plan, bool skip_cands = false);
+  // For tests: records go up in the background whatever their size, in pieces of 64 KB.
+  void small_start(bool on) { small_start_ = on; }
   // Plans the job on the device (devplan.cu): ids, headers and candidate records are worked out
   // there from the factored tables. On return the plan's sizes are known; prepare_fill() then does
   // for it what upload() does for a host plan. 1: not covered, or the fixed buffer is too small -
@@ -145,6 +147,7 @@ class DeviceFill {
 
   int device_ = 0;
   bool fixed_ = false;            // carved from an attached buffer: no growth
+  bool small_start_ = false;
   unsigned char* buf_ = nullptr;  // attached buffer
   size_t buf_bytes_ = 0, buf_off_ = 0;
   // buffers, and what lies in them

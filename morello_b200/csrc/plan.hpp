@@ -164,6 +164,8 @@ struct Plan {
 enum : u32 {
   PLAN_NO_TWINS = 1,   // tabulate both dtypes of a mirrored goal set instead of deriving one from the other
   PLAN_NO_MEMO = 2,    // tabulate every Spec from scratch instead of re-using per-operand results
+  PLAN_ON_HOST = 4,    // plan on the host also where the device would
+  FILL_SMALL_START = 8,   // small plans take the ways of large ones (DeviceFill::small_start)
 };
 
 // Top limits are Avx2Target::max_mem() unless overridden. mirror_dtype >= 0: the goals come in

@@ -130,9 +130,9 @@ class SynthesisDatabase:
             err.status = rc
             raise err
 
-    def set_plan_flags(self, no_twins: bool = False, no_memo: bool = False):
-        """Cross-check modes of the host planner: the same plan built the slow way."""
-        self._check(self._lib.mrl_set_plan_flags(self._ctx, int(no_twins) | (int(no_memo) << 1)))
+    def set_plan_flags(self, no_twins: bool = False, no_memo: bool = False, on_host: bool = False, small_start: bool = False):
+        """Cross-check modes: the same plan built the slow way, and small fills taking the ways of large ones."""
+        self._check(self._lib.mrl_set_plan_flags(self._ctx, int(no_twins) | (int(no_memo) << 1) | (int(on_host) << 2) | (int(small_start) << 3)))
 
     # --- search::top_down_many / top_down ---
     def top_down_many(self, goals: Sequence[bytes], limits: Optional[Sequence[Sequence[int]]] = None) -> List[Decision]:
