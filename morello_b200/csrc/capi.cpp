@@ -377,7 +377,10 @@ int mrl_upload(mrl_ctx* ctx) {
   if (ctx->device < 0) return fail(ctx, -2, "planning-only context: no device to fill on");
   if (!ctx->planned) return fail(ctx, -1, "nothing planned");
   if (ctx->table_only) return fail(ctx, -1, "the tables were loaded from a file without their plan: nothing to upload or fill");
-  return upload_plan(ctx);
+  const int rc = upload_plan(ctx);
+  if (rc) return rc;
+  if (ctx->dev.sync() != 0) return fail(ctx, -2, ctx->dev.error());   // mrl_set_stream may follow
+  return 0;
 }
 
 int mrl_fill(mrl_ctx* ctx) {

@@ -2674,6 +2674,11 @@ int DeviceFill::prepare_fill() {
   return 0;
 }
 
+int DeviceFill::sync() {
+  CK(cudaStreamSynchronize(stream_));
+  return 0;
+}
+
 int DeviceFill::cands_arrived() {
   CK(cudaSetDevice(device_));
   if (cands_present_) return 0;

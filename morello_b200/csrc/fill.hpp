@@ -68,7 +68,10 @@ class DeviceFill {
   // for it what upload() does for a host plan. 1: not covered, or the fixed buffer is too small -
   // plan on the host.
   int plan(const OpTables& tab);
+  // What it enqueues may still be under way on return: fills on the same stream follow it, and a caller
+  // that may put another stream in its place waits with sync().
   int prepare_fill();
+  int sync();
   struct StageIds { uint32_t lo, hi; uint64_t cand_end; uint32_t team; };
   const std::vector<StageIds>& stages() const { return stages_; }
   uint64_t n_goals() const { return n_goals_; }
