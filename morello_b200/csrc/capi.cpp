@@ -6,6 +6,7 @@
 #include <chrono>
 #include <cstdio>
 #include <cstdlib>
+#include <mutex>
 #include <thread>
 
 using namespace mrl;
@@ -29,7 +30,12 @@ struct mrl_ctx {
   bool host_plan = false;         // `plan` holds the current job
   Job job;
   OpTables tab;                   // of a plan made on the device
-  std::vector<uint64_t> specs;    // its Specs by id (packed), once they were asked for
+  // Worked out when they are first asked for, by whichever thread asks (lazy_mu): of a plan made on the
+  // device its Specs by id (packed), and its families with the first one of every stage.
+  std::mutex lazy_mu;
+  std::vector<uint64_t> specs;
+  std::vector<Family> families;
+  std::vector<uint32_t> family_lo;
   bool planned = false, uploaded = false, filled = false;
   DeviceFill dev;
   mrl_stats stats;
@@ -133,7 +139,7 @@ Plan plan_on_host(const mrl_ctx* ctx, const Job& job, double* goal_seconds) {
   return build_plan(goals, ctx->n_threads, nullptr, ctx->rank, ctx->world, mirror, ctx->plan_flags);
 }
 
-// The host's form of a plan that was made on the device (sharding tables, plan sharing).
+// The host's form of a plan that was made on the device (plan sharing).
 void need_host_plan(mrl_ctx* ctx) {
   if (!ctx->on_device || ctx->host_plan) return;
   double goal_seconds = 0;
@@ -163,6 +169,8 @@ int set_plan(mrl_ctx* ctx, Job&& job) {
   ctx->table_only = false;
   ctx->on_device = ctx->host_plan = false;
   ctx->specs.clear();
+  ctx->families.clear();
+  ctx->family_lo.clear();
   ctx->job = std::move(job);
   memset(&ctx->stats, 0, sizeof(ctx->stats));
   ctx->dev.wait_upload();   // a background upload may still be reading the old plan
@@ -203,13 +211,41 @@ uint64_t spec_count(const mrl_ctx* ctx) { return ctx->on_device ? ctx->dev.n_spe
 uint32_t top_code_of(const mrl_ctx* ctx, int k) { return ctx->on_device ? ctx->tab.top_code[k] : ctx->plan.top_code[k]; }
 
 // Specs by id. The packed Specs of a plan made on the device are fetched once.
+void fetch_specs(mrl_ctx* ctx) {   // lazy_mu is held
+  if (ctx->specs.size() == ctx->dev.n_specs()) return;
+  std::vector<uint64_t> specs(ctx->dev.n_specs());
+  if (ctx->dev.read_specs(specs.data()) != 0) throw ModelError(ctx->dev.error());
+  ctx->specs.swap(specs);
+}
 void need_specs(mrl_ctx* ctx) {
-  if (!ctx->on_device || ctx->specs.size() == ctx->dev.n_specs()) return;
-  ctx->specs.resize(ctx->dev.n_specs());
-  if (ctx->dev.read_specs(ctx->specs.data()) != 0) {
-    ctx->specs.clear();
-    throw ModelError(ctx->dev.error());
+  if (!ctx->on_device) return;
+  std::lock_guard<std::mutex> guard(ctx->lazy_mu);
+  fetch_specs(ctx);
+}
+// Families of a plan made on the device: the runs of a stage's Specs with one dtype and shape (plan.cpp);
+// such a plan is not sharded, so all are owned by rank 0.
+void need_families(mrl_ctx* ctx) {
+  if (!ctx->on_device) return;
+  std::lock_guard<std::mutex> guard(ctx->lazy_mu);
+  if (!ctx->family_lo.empty()) return;
+  fetch_specs(ctx);
+  std::vector<Family> fams;
+  std::vector<uint32_t> lo;
+  for (const DeviceFill::StageIds& st : ctx->dev.stages()) {
+    lo.push_back((uint32_t)fams.size());
+    for (uint32_t i = st.lo; i < st.hi; i++) {
+      if (i == st.lo || (ctx->specs[i] >> 48) != (ctx->specs[i - 1] >> 48)) {
+        Family f;
+        f.spec_lo = i;
+        f.stage = (uint32_t)lo.size() - 1;
+        fams.push_back(f);
+      }
+      fams.back().spec_hi = i + 1;
+    }
   }
+  lo.push_back((uint32_t)fams.size());
+  ctx->families.swap(fams);
+  ctx->family_lo.swap(lo);
 }
 LogicalSpec spec_at(const mrl_ctx* ctx, uint64_t id) { return ctx->on_device ? ctx->tab.spec_of(ctx->specs[id]) : ctx->plan.specs[id]; }
 uint64_t job_fingerprint(mrl_ctx* ctx) {
@@ -594,22 +630,32 @@ int mrl_plan_adopt_done(mrl_ctx* ctx, double plan_seconds) {
 
 uint64_t mrl_num_stages(const mrl_ctx* ctx) { return ctx && ctx->planned ? (ctx->on_device ? ctx->dev.stages().size() : ctx->plan.stages.size()) : 0; }
 
-// Families and owners are of the host's form of a plan.
-static bool host_plan_ready(const mrl_ctx* ctx) {
-  if (!ctx || !ctx->planned) return false;
+static const std::vector<Family>* families_of(const mrl_ctx* ctx) {
+  if (!ctx || !ctx->planned) return nullptr;
   try {
-    need_host_plan(const_cast<mrl_ctx*>(ctx));
-    return true;
+    need_families(const_cast<mrl_ctx*>(ctx));
+    return ctx->on_device ? &ctx->families : &ctx->plan.families;
   } catch (const std::exception&) {
-    return false;
+    return nullptr;
   }
 }
 
-uint64_t mrl_num_families(const mrl_ctx* ctx) { return host_plan_ready(ctx) ? ctx->plan.families.size() : 0; }
+uint64_t mrl_num_families(const mrl_ctx* ctx) {
+  const std::vector<Family>* const f = families_of(ctx);
+  return f ? f->size() : 0;
+}
 
 int mrl_stage_info(const mrl_ctx* ctx, uint64_t stage, uint32_t* spec_lo, uint32_t* spec_hi, uint32_t* family_lo,
                    uint32_t* family_hi) {
-  if (!host_plan_ready(ctx) || stage >= ctx->plan.stages.size()) return -1;
+  if (stage >= mrl_num_stages(ctx)) return -1;
+  if (ctx->on_device) {
+    if ((family_lo || family_hi) && !families_of(ctx)) return -2;
+    if (spec_lo) *spec_lo = ctx->dev.stages()[stage].lo;
+    if (spec_hi) *spec_hi = ctx->dev.stages()[stage].hi;
+    if (family_lo) *family_lo = ctx->family_lo[stage];
+    if (family_hi) *family_hi = ctx->family_lo[stage + 1];
+    return 0;
+  }
   const Stage& st = ctx->plan.stages[stage];
   if (spec_lo) *spec_lo = st.spec_lo;
   if (spec_hi) *spec_hi = st.spec_hi;
@@ -620,8 +666,9 @@ int mrl_stage_info(const mrl_ctx* ctx, uint64_t stage, uint32_t* spec_lo, uint32
 
 int mrl_family_info(const mrl_ctx* ctx, uint64_t family, uint32_t* stage, uint32_t* owner, uint32_t* spec_lo,
                     uint32_t* spec_hi) {
-  if (!host_plan_ready(ctx) || family >= ctx->plan.families.size()) return -1;
-  const Family& f = ctx->plan.families[family];
+  const std::vector<Family>* const all = families_of(ctx);
+  if (!all || family >= all->size()) return -1;
+  const Family& f = (*all)[family];
   if (stage) *stage = f.stage;
   if (owner) *owner = f.owner;
   if (spec_lo) *spec_lo = f.spec_lo;
