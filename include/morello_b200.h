@@ -88,7 +88,9 @@ enum { MRL_MEM_RF = 0, MRL_MEM_VRF = 1, MRL_MEM_L1 = 2, MRL_MEM_GL = 3 };
 enum { MRL_THROUGH_MOVE = 0, MRL_THROUGH_ZERO = 1, MRL_THROUGH_MATMUL = 2 };
 
 /* Replaces FilesDatabase::new (morello/src/db/mod.rs:350-380): one context = one in-memory
- * database on one GPU. n_threads = host threads for planning (0 = all cores). */
+ * database on one GPU. n_threads = host threads for planning (0 = all cores). A context's device buffers
+ * stay from one plan to the next: each is at most 256 MB or four times what the present plan asks for, and
+ * mrl_ctx_destroy gives them back. */
 int mrl_ctx_create(int device, int n_threads, mrl_ctx** out);
 /* Replaces Drop for FilesDatabase (morello/src/db/mod.rs:1154-1167); frees device memory. */
 void mrl_ctx_destroy(mrl_ctx* ctx);

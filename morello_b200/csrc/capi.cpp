@@ -102,7 +102,7 @@ int dev_rc(int rc) { return (rc == -5 || rc == -6 || rc == -3) ? rc : -2; }
 
 int upload_plan(mrl_ctx* ctx) {
   double t0 = now_s();
-  ctx->filled = false;
+  ctx->uploaded = ctx->filled = false;   // a failure leaves no buffers to fill with
   int rc = ctx->on_device ? ctx->dev.prepare_fill() : ctx->dev.upload(ctx->plan, ctx->cands_elsewhere);
   if (rc != 0) return fail(ctx, dev_rc(rc), ctx->dev.error());
   ctx->uploaded = true;

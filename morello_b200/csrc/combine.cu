@@ -2233,10 +2233,12 @@ void DeviceFill::drop_(DevBuf& b) {
 
 // A cudaMalloc or cudaFree costs 50 us to milliseconds (seconds, in the tail) against the 1 to 60
 // ms of a small fill, and a plan has some twenty buffers, so buffers stay from plan to plan. What
-// a large plan leaves behind is given back when the next plan needs less than 1/16 of it.
+// a large plan leaves behind is given back when the next plan needs less than a quarter of it (a fill that
+// had to enlarge a buffer keeps it for the next one of its size, which asks for the first size again).
+bool DeviceFill::oversized_(const DevBuf& b, size_t bytes) { return b.cap > (size_t(256) << 20) && b.cap / 4 > bytes; }
 int DeviceFill::reserve_(DevBuf& b, size_t bytes, bool give_back) {
   bytes = std::max<size_t>(bytes, 256);
-  if (!fixed_ && b.cap >= bytes && !(give_back && b.cap > (size_t(256) << 20) && b.cap / 16 > bytes)) return 0;
+  if (!fixed_ && b.cap >= bytes && !(give_back && oversized_(b, bytes))) return 0;
   if (!fixed_ && b.p) {
     CK(cudaStreamSynchronize(stream_));
     drop_(b);
@@ -2262,6 +2264,15 @@ int DeviceFill::reserve_host_(size_t bytes) {
   const size_t want = std::max<size_t>(bytes + bytes / 2, size_t(64) << 10);
   CK(cudaHostAlloc(&h_stage_, want, cudaHostAllocDefault));
   h_stage_bytes_ = want;
+  return 0;
+}
+
+int DeviceFill::drop_all_() {
+  begin_plan_();
+  CK(cudaStreamSynchronize(stream_));
+  for (DevBuf* b : {&b_ctl_, &b_hdrs_, &b_cands_, &b_spec_, &b_stage_specs_, &b_mine_, &b_stages_, &b_items_, &b_temp_, &b_rows_,
+                    &b_lookup_, &b_tables_, &b_bits_, &b_rank_, &b_desc_, &b_stage_lo_})
+    drop_(*b);
   return 0;
 }
 
@@ -2395,6 +2406,8 @@ int DeviceFill::working_buffers_(bool with_mine, uint32_t world) {
   if (with_mine) {
     if ((rc = reserve_(b_mine_, n))) return rc;
     d_mine_ = static_cast<uint8_t*>(b_mine_.p);
+  } else {
+    drop_(b_mine_);
   }
   if (fixed_) {
     // Everything left is split once: lookup staging, work items, working rows and final rows.
@@ -2443,7 +2456,17 @@ int DeviceFill::working_buffers_(bool with_mine, uint32_t world) {
 
 int DeviceFill::upload(const Plan& plan, bool skip_cands) {
   CK(cudaSetDevice(device_));
+  int rc = upload_(plan, skip_cands);
+  if (rc == -6) {   // what earlier plans left may be in the way
+    if (drop_all_() != 0) return -1;
+    rc = upload_(plan, skip_cands);
+  }
+  return rc;
+}
+
+int DeviceFill::upload_(const Plan& plan, bool skip_cands) {
   begin_plan_();
+  if (!fixed_) for (DevBuf* b : {&b_tables_, &b_bits_, &b_rank_, &b_desc_, &b_stage_lo_}) drop_(*b);   // of plans made on the device
   n_specs_ = (uint32_t)plan.hdrs.size();
   top_pack_ = plan.top_pack();
   n_goals_ = plan.stats.n_goal_specs;
@@ -2543,10 +2566,13 @@ int DeviceFill::upload(const Plan& plan, bool skip_cands) {
 int DeviceFill::plan(const OpTables& tab) {
   CK(cudaSetDevice(device_));
   int rc = plan_(tab);
-  if (rc == -6) rc = 1;   // no room for the planning buffers: the host planner needs none of them
-  if (rc == 1 && !fixed_) {
-    CK(cudaStreamSynchronize(stream_));
-    for (DevBuf* b : {&b_tables_, &b_bits_, &b_rank_, &b_desc_, &b_stage_lo_}) drop_(*b);
+  if (rc == -6) {   // what earlier plans left may be in the way
+    if (drop_all_() != 0) return -1;
+    rc = plan_(tab);
+  }
+  if (rc == -6) {   // no room for the planning buffers: the host planner needs none of them
+    if (drop_all_() != 0) return -1;
+    rc = 1;
   }
   return rc;
 }
@@ -2619,7 +2645,6 @@ int DeviceFill::plan_(const OpTables& tab) {
     const uint64_t most = (uint64_t)tab.n_positions * tab.max_records;
     want_specs = std::min<uint64_t>(tab.n_positions, 1u << 16);
     want_cands = std::min<uint64_t>(most, 1u << 17);
-    if (b_cands_.cap > (size_t(256) << 20) && b_cands_.cap / sizeof(CandRec) / 16 > most) drop_(b_cands_);   // of a far larger plan
   }
   int phases = fixed_ ? DPP_CLOSURE : DPP_CLOSURE | DPP_SPECS | DPP_RECORDS;
   for (int attempt = 0;; attempt++) {
@@ -2637,12 +2662,16 @@ int DeviceFill::plan_(const OpTables& tab) {
     CK(launch_plan_kernel(a, blocks(attempt == 0 ? tab.n_positions / 2 : want_specs), stream_));
     CK(cudaMemcpyAsync(h_stage_, res, back, cudaMemcpyDeviceToHost, stream_));
     CK(cudaStreamSynchronize(stream_));
-    if (ctl->n_specs > 0xFFFFFFF0u || ctl->n_cands > 0xFFFFFFFFull || attempt > 3) return 1;
+    if (ctl->n_specs > 0xFFFFFFF0u || ctl->n_cands > 0xFFFFFFFFull || attempt > 4) return 1;
     want_specs = ctl->n_specs;
     want_cands = ctl->n_cands;
     if (ctl->n_specs > a.cap_specs || !b_hdrs_.p) phases = fixed_ ? DPP_SPECS : DPP_SPECS | DPP_RECORDS;
     else if (ctl->n_cands > a.cap_cands || !b_cands_.p || !(phases & DPP_RECORDS)) phases = DPP_RECORDS;
-    else break;
+    else if (!fixed_ && (oversized_(b_hdrs_, want_specs * sizeof(SpecHdr)) || oversized_(b_desc_, want_specs * sizeof(u64)) ||
+                         oversized_(b_cands_, want_cands * sizeof(CandRec)))) {   // of a far larger plan; the closure stays
+      for (DevBuf* b : {&b_hdrs_, &b_desc_, &b_cands_}) drop_(*b);
+      phases = DPP_SPECS | DPP_RECORDS;
+    } else break;
     if (phases == DPP_RECORDS && (rc = reserve_(b_cands_, std::max<uint64_t>(want_cands, 1) * sizeof(CandRec), false))) return rc == -5 ? 1 : rc;
   }
   d_hdrs_ = a.hdrs;
@@ -2667,6 +2696,11 @@ int DeviceFill::plan_(const OpTables& tab) {
 int DeviceFill::prepare_fill() {
   CK(cudaSetDevice(device_));
   int rc = working_buffers_(false, 1);
+  if (rc == -6) {   // the ones of earlier plans may be in the way
+    CK(cudaStreamSynchronize(stream_));
+    for (DevBuf* b : {&b_items_, &b_temp_, &b_rows_, &b_lookup_, &b_bits_}) drop_(*b);
+    rc = working_buffers_(false, 1);
+  }
   if (rc) return rc;
   CK(cudaMemsetAsync(d_ctl_, 0, 512, stream_));
   cands_present_ = true;

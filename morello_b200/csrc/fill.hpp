@@ -130,13 +130,18 @@ class DeviceFill {
   uint32_t n_specs() const { return n_specs_; }
 
  private:
-  // A device buffer that stays from one plan to the next while its size is of the right order.
+  // A device buffer that stays from one plan to the next. A context keeps no buffer of more than 256 MB
+  // and four times what its present plan asks for, and what it does keep is given back before it reports
+  // that the device is out of memory.
   struct DevBuf { void* p = nullptr; size_t cap = 0; };
   int reserve_(DevBuf& b, size_t bytes, bool give_back = true);
+  static bool oversized_(const DevBuf& b, size_t bytes);
   void drop_(DevBuf& b);
+  int drop_all_();   // buffers and the plan in them
   int alloc_(void** p, size_t bytes);
   void begin_plan_();
   int plan_(const OpTables& tab);
+  int upload_(const Plan& plan, bool skip_cands);
   int working_buffers_(bool sharded_mine, uint32_t world);
   int launch_stages_(uint32_t from, uint32_t to, int team, int blocks, bool solve, bool place);
   int blocks_of_(int team) const;
