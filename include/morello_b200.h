@@ -128,7 +128,7 @@ int mrl_top_down_many(mrl_ctx* ctx, const uint8_t* blobs, const uint64_t* blob_o
  * both dtypes of a mirrored goal set instead of deriving f32 records from u32 ones; bit 1:
  * tabulate every Spec from scratch instead of re-using per-operand results; bit 2: plan on the host also
  * where the device would. Bit 3: fills take the ways of large ones (candidate records planned on the host go
- * up in the background whatever their size). */
+ * up in the background whatever their size; buffers start small and are enlarged during the fill). */
 int mrl_set_plan_flags(mrl_ctx* ctx, uint32_t flags);
 
 /* No counterpart in the reference. Same inputs, outputs and results as mrl_top_down_many, for

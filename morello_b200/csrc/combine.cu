@@ -2430,7 +2430,8 @@ int DeviceFill::working_buffers_(bool with_mine, uint32_t world) {
     const uint64_t shard = std::max<uint32_t>(1, world);
     const uint64_t stage_part = ((uint64_t)max_stage_ * 3 / 2 + shard - 1) / shard;   // Specs of the largest stage a rank solves, with slack
     uint64_t temp = std::max<uint64_t>(1u << 20, stage_part * 1000), rows = std::max<uint64_t>(1u << 20, (uint64_t)n_specs_ * 48);
-    if (temp * 2 * sizeof(MrlRow) > b_temp_.cap || rows * sizeof(MrlRow) > b_rows_.cap) {
+    if (small_start_) temp = rows = 512;
+    else if (temp * 2 * sizeof(MrlRow) > b_temp_.cap || rows * sizeof(MrlRow) > b_rows_.cap) {
       size_t free_b = 0, total_b = 0;
       CK(cudaMemGetInfo(&free_b, &total_b));
       free_b += b_temp_.cap + b_rows_.cap;

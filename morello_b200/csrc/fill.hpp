@@ -61,7 +61,8 @@ class DeviceFill {
   // skip_cands: the candidate records are not on this host; the caller fills device_cands()
   // itself (e.g. a broadcast from the rank that planned) and then calls cands_arrived().
   int upload(const Plan& plan, bool skip_cands = false);
-  // For tests: records go up in the background whatever their size, in pieces of 64 KB.
+  // For tests: records go up in the background whatever their size, in pieces of 64 KB, and fills start with
+  // room for a few hundred rows.
   void small_start(bool on) { small_start_ = on; }
   // Plans the job on the device (devplan.cu): ids, headers and candidate records are worked out
   // there from the factored tables. On return the plan's sizes are known; prepare_fill() then does

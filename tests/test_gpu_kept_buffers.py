@@ -77,3 +77,26 @@ def test_what_a_context_keeps_is_not_in_its_own_way(built_extension):
         del rest
         torch.cuda.empty_cache()
         db.close()
+
+
+@pytest.mark.parametrize("kind,dtypes,shape", [
+    ("MATMUL", ("U32",), [1, 2, 2, 2]),           # one launch of all stages, by a block
+    ("MATMUL", ("U32", "F32"), [1, 2, 8, 4]),     # launches of several stages, by teams of all sizes
+    ("MOVE", ("F32",), [16, 16]),
+])
+def test_fills_that_enlarge_their_buffers(built_extension, kind, dtypes, shape):
+    import morello_b200 as m
+    goals = [m.simple_spec(getattr(m, "KIND_" + kind), getattr(m, "DTYPE_" + d), shape, m.GL) for d in dtypes]
+    solo = m.SynthesisDatabase(device=0)
+    want = solo.top_down_many(goals)
+    assert solo.stats()["n_buffer_growths"] == 0
+    for on_host in (False, True):
+        db = m.SynthesisDatabase(device=0)
+        db.set_plan_flags(on_host=on_host, small_start=True)
+        assert db.top_down_many(goals) == want
+        assert db.stats()["n_buffer_growths"] > 0
+        assert db.checksum() == solo.checksum()
+        db.fill()                                  # the enlarged buffers stay
+        assert db.stats()["n_buffer_growths"] == 0 and db.checksum() == solo.checksum()
+        db.close()
+    solo.close()
