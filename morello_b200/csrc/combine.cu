@@ -2261,7 +2261,7 @@ int DeviceFill::reserve_host_(size_t bytes) {
   if (h_stage_) cudaFreeHost(h_stage_);
   h_stage_ = nullptr;
   h_stage_bytes_ = 0;
-  const size_t want = std::max<size_t>(bytes + bytes / 2, size_t(64) << 10);
+  const size_t want = std::max<size_t>(bytes + std::min<size_t>(bytes / 2, size_t(1) << 20), size_t(64) << 10);
   CK(cudaHostAlloc(&h_stage_, want, cudaHostAllocDefault));
   h_stage_bytes_ = want;
   return 0;
@@ -3086,10 +3086,12 @@ int DeviceFill::walk(uint64_t root, bool packed, uint32_t cpack, std::vector<Wal
 
 // Device memory into pageable memory of the caller's, which is often fresh: the driver's own staging
 // runs on one thread, and half of its time goes into page faults. Large parts are brought over in
-// pieces by a few threads, each through two pinned buffers of its own.
+// pieces by a few threads, each through two pinned buffers of its own. Pinning them is most of a database's
+// first export: 57 MB of rows take 14 ms the first time and 5.8 then with pieces of 1 MB, 20 and 5.7 with 2 MB,
+// 13 and 6.7 with 512 KB.
 int DeviceFill::read_bulk_(void* out, const void* src, size_t bytes) {
-  const size_t piece = size_t(2) << 20;
-  if (bytes < 4 * piece || fixed_) {
+  const size_t piece = size_t(1) << 20;
+  if (bytes < 8 * piece || fixed_) {
     if (bytes) CK(cudaMemcpyAsync(out, src, bytes, cudaMemcpyDeviceToHost, stream_));
     CK(cudaStreamSynchronize(stream_));
     return 0;
