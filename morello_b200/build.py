@@ -9,8 +9,9 @@ CSRC = os.path.join(HERE, "csrc")
 LIB_DIR = os.path.join(HERE, "_lib")
 LIB_PATH = os.path.join(LIB_DIR, "libmorello_b200.so")
 SOURCES = ["combine.cu", "devplan.cu", "plan.cpp", "optable.cpp", "capi.cpp"]
-# the Python mirror's query calls (CPython C API); loaded as morello_b200._lib's helper, not as a package
-PYHOST_PATH = os.path.join(LIB_DIR, "_pyhost.so")
+# The Python mirror's query calls (CPython C API); loaded as morello_b200._lib's helper, not as a package. The
+# name carries the interpreter's ABI, so that one built for another interpreter is not taken.
+PYHOST_PATH = os.path.join(LIB_DIR, "_pyhost" + sysconfig.get_config_var("EXT_SUFFIX"))
 
 
 def _nvcc():
@@ -20,10 +21,15 @@ def _nvcc():
     return nvcc
 
 
+def _has_python_headers():
+    return os.path.exists(os.path.join(sysconfig.get_paths()["include"], "Python.h"))
+
+
 def needs_build():
-    if not os.path.exists(LIB_PATH) or not os.path.exists(PYHOST_PATH):
+    targets = [LIB_PATH] + ([PYHOST_PATH] if _has_python_headers() else [])
+    if not all(os.path.exists(t) for t in targets):
         return True
-    built = min(os.path.getmtime(LIB_PATH), os.path.getmtime(PYHOST_PATH))
+    built = min(os.path.getmtime(t) for t in targets)
     deps = []
     for root, _dirs, files in os.walk(CSRC):
         deps += [os.path.join(root, f) for f in files]
@@ -32,7 +38,9 @@ def needs_build():
 
 
 def build(force=False, verbose=False):
-    """nvcc -gencode arch=compute_100a,code=sm_100a ... -shared -> morello_b200/_lib/."""
+    """nvcc -gencode arch=compute_100a,code=sm_100a ... -shared -> morello_b200/_lib/. The helper of the
+    Python mirror's query calls needs the interpreter's headers; without them it is left out, and the mirror
+    packs its queries in Python."""
     if not force and not needs_build():
         return LIB_PATH
     os.makedirs(LIB_DIR, exist_ok=True)
@@ -46,8 +54,9 @@ def build(force=False, verbose=False):
     res = subprocess.run(cmd, capture_output=True, text=True)
     if res.returncode != 0:
         raise RuntimeError("nvcc failed:\n" + res.stdout + res.stderr)
-    res = subprocess.run(["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-I" + sysconfig.get_paths()["include"],
-                          os.path.join(CSRC, "pyhost.cpp"), "-o", PYHOST_PATH], capture_output=True, text=True)
-    if res.returncode != 0:
-        raise RuntimeError("g++ failed:\n" + res.stdout + res.stderr)
+    if _has_python_headers():
+        res = subprocess.run([_nvcc(), "-O2", "-std=c++17", "-Xcompiler", "-fPIC", "-shared", "-I" + sysconfig.get_paths()["include"],
+                              os.path.join(CSRC, "pyhost.cpp"), "-o", PYHOST_PATH], capture_output=True, text=True)
+        if res.returncode != 0:
+            raise RuntimeError("nvcc failed:\n" + res.stdout + res.stderr)
     return LIB_PATH

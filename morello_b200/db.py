@@ -75,16 +75,6 @@ def tabulate(blob: bytes):
     return out
 
 
-def _pack(blobs: Sequence[bytes]):
-    off = (C.c_uint64 * (len(blobs) + 1))()
-    pos = 0
-    for i, b in enumerate(blobs):
-        off[i] = pos
-        pos += len(b)
-    off[len(blobs)] = pos
-    return b"".join(blobs), off
-
-
 class SynthesisDatabase:
     """An in-memory synthesis database living on one GPU.
 
@@ -96,7 +86,7 @@ class SynthesisDatabase:
 
     def __init__(self, device: int = 0, threads: int = 0):
         self._lib = L.load()
-        self._call_many = L.pyhost().call_many
+        self._call_many = L.call_many()
         self._fn = {name: C.cast(getattr(self._lib, name), C.c_void_p).value
                     for name in ("mrl_top_down_many", "mrl_top_down_many_noalloc", "mrl_get_many")}
         self._ctx = C.c_void_p()
@@ -162,7 +152,7 @@ class SynthesisDatabase:
         self._check(self._lib.mrl_plan_precompute(self._ctx, size, through, self._dtype_mask(dtypes)))
 
     def plan_goals(self, goals: Sequence[bytes]):
-        data, off = _pack(goals)
+        data, off = L.pack(goals)
         self._check(self._lib.mrl_plan_goals(self._ctx, data, off, len(goals)))
 
     def upload(self):
