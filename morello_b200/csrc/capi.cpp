@@ -1130,10 +1130,12 @@ int mrl_load(mrl_ctx* ctx, const char* path) {
         new (&specs[i]) LogicalSpec(LogicalSpec::from_key(blobs.substr(lo, blob_end[i] - lo)));
       }
       for (uint64_t i = 0; i < n; i++) { hdrs[i].cand_off = 0; hdrs[i].ncand = 0; }
-      ctx->dev.wait_upload();
-      ctx->plan = table_only_plan(std::move(specs), std::move(hdrs), fh.top_code, ctx->n_threads);
-      if (ctx->plan.fingerprint(ctx->n_threads) != fh.fingerprint) return fail(ctx, -8, "the database file is corrupt (Spec fingerprint)");
+      Plan loaded = table_only_plan(std::move(specs), std::move(hdrs), fh.top_code, ctx->n_threads);
+      if (loaded.fingerprint(ctx->n_threads) != fh.fingerprint) return fail(ctx, -8, "the database file is corrupt (Spec fingerprint)");
+      ctx->dev.wait_upload();   // of the plan that is replaced
+      ctx->plan = std::move(loaded);
       ctx->planned = ctx->host_plan = true;
+      ctx->uploaded = ctx->filled = false;
       ctx->on_device = false;
       ctx->table_only = true;
       ctx->cands_elsewhere = false;
@@ -1151,6 +1153,7 @@ int mrl_load(mrl_ctx* ctx, const char* path) {
       // the plan's own candidate ranges stay; masks and first rows come from the file
       std::vector<SpecHdr> own(n);
       if (ctx->dev.read_hdrs(own.data()) != 0) return fail(ctx, -2, ctx->dev.error());
+      ctx->filled = false;
       for (uint64_t i = 0; i < n; i++) { hdrs[i].cand_off = own[i].cand_off; hdrs[i].ncand = own[i].ncand; }
       if (ctx->dev.load_table(hdrs.data(), rows.data(), fh.n_rows) != 0) return fail(ctx, -2, ctx->dev.error());
     }
@@ -1164,8 +1167,7 @@ int mrl_load(mrl_ctx* ctx, const char* path) {
       return fail(ctx, -8, "the database file is corrupt (contents do not match their checksum)");
     }
     return 0;
-  } catch (const std::exception& e) {
-    ctx->filled = false;
+  } catch (const std::exception& e) {   // by the Specs of the file: nothing is replaced yet
     return fail(ctx, -8, std::string("the database file is corrupt: ") + e.what());
   }
 }
