@@ -46,13 +46,14 @@ typedef struct mrl_stats {
   uint64_t n_candidates_evaluated; /* candidate records evaluated by those solves */
   uint64_t n_rows_gathered;    /* child rows they read */
   uint64_t n_passes;           /* solve passes of the last fill, summed over stages */
-  uint64_t n_launches;         /* kernel launches of the last fill (one per stage; in small plans one per run of stages) */
-  uint64_t n_grid_syncs;       /* grid-wide barriers inside those launches */
+  uint64_t n_launches;         /* kernel launches of the last fill (one per stage; up to 262 144 Specs one per run of stages) */
+  uint64_t n_grid_syncs;       /* barriers inside those launches that span a stage's team of blocks: one, a cluster of
+                                * eight, or the whole grid */
   uint64_t algorithmic_bytes;  /* of the finished table: per final row 12 bytes out, 16 per candidate record of
                                 * its Spec, 16 per child of each candidate that fits the row's limits */
   uint64_t h2d_bytes;          /* bytes copied host->device by the last upload */
   uint64_t d2h_bytes;          /* bytes copied device->host by the last query */
-  double plan_seconds;         /* host: closure, candidate tabulation, stage order */
+  double plan_seconds;         /* closure, candidate records, stage order (on the device or the host) */
   double upload_seconds;
   double fill_ms;              /* device time of the last fill (CUDA events on the launch stream) */
   double combine_ms;           /* of which inside the solve phases (device timer) */
@@ -152,9 +153,11 @@ int mrl_top_down_many_noalloc(mrl_ctx* ctx, const uint8_t* blobs, const uint64_t
  * dtype_mask: bit 0 = u32, bit 1 = f32 (DTYPES, precompute/src/main.rs:55). */
 int mrl_precompute(mrl_ctx* ctx, uint32_t size, int through, int dtype_mask);
 
-/* The three steps of the two calls above, exposed separately for measurement: plan on the
- * host, copy the plan to the device, fill (may be repeated). Gigabytes of candidate records keep
- * going up in the background after mrl_upload has returned, in stage order; a fill waits stage by
+/* The three steps of the two calls above, exposed separately for measurement: plan, make the plan ready
+ * on the device, fill (may be repeated). Plans for one GPU are made on the device. Those of sharded fills, of
+ * planning-only contexts, of the cross-check modes and of jobs that the device cannot plan are made on the
+ * host and copied by mrl_upload; gigabytes of their candidate records keep
+ * going up in the background after it has returned, in stage order; a fill waits stage by
  * stage for the records it needs, so its first stages overlap the copy. Calls that replace the
  * plan or read the device records (mrl_plan_*, mrl_verify, mrl_device_cands, mrl_get_impl) wait for the
  * copy. */

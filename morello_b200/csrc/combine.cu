@@ -177,14 +177,10 @@ __device__ __forceinline__ uint4 lookup(const SpecHdr* hdrs, const MrlRow* rows,
   return *reinterpret_cast<const uint4*>(row_of(rows, temp, m, base, b0, b1, b2, b3));
 }
 
-// One candidate record of a Spec at one limits point: feasibility under the limits, the child
-// rows at the children's limits, the combined Cost, and the running minimum. The fill is bound by
-// the latency of dependent loads (record -> child header -> child row), so the headers of all
-// children are requested together, then all rows: two round trips per candidate whatever the
-// number of children.
-// kFinished: every child lies in a finished stage, so headers and rows are read-only for the whole
-// launch and may take the non-coherent load path.
-template <bool kFinished>
+// One candidate record of a Spec at one limits point, for the verifier (the fill's is eval_staged):
+// feasibility under the limits, the child rows at the children's limits, the combined Cost, and the
+// running minimum. The headers of all children are requested together, then all rows: two round trips
+// per candidate whatever the number of children.
 __device__ __forceinline__ void eval_candidate(const SpecHdr* hdrs, const CandRec* __restrict__ cands, const MrlRow* rows,
                                                const MrlRow* temp, uint32_t rec, const uint4 a, uint32_t cpack,
                                                uint32_t bm0, uint32_t bm1, uint32_t bm2, uint32_t bm3, Best& best,
@@ -216,25 +212,13 @@ __device__ __forceinline__ void eval_candidate(const SpecHdr* hdrs, const CandRe
     }
     const uint4 b = __ldg(reinterpret_cast<const uint4*>(&cands[rec]) + 1);
     const uint32_t ch1 = nchild > 1 ? b.y : b.x, ch2 = nchild > 2 ? b.z : b.x;   // absent children repeat the first
-    uint4 m0, m1, m2, r0, r1, r2;
-    unsigned long long base0, base1, base2;
-    if (kFinished) {
-      m0 = __ldg(reinterpret_cast<const uint4*>(&hdrs[b.x]));
-      m1 = __ldg(reinterpret_cast<const uint4*>(&hdrs[ch1]));
-      m2 = __ldg(reinterpret_cast<const uint4*>(&hdrs[ch2]));
-      base0 = __ldg(&hdrs[b.x].row_base); base1 = __ldg(&hdrs[ch1].row_base); base2 = __ldg(&hdrs[ch2].row_base);
-      r0 = __ldg(reinterpret_cast<const uint4*>(row_of(rows, temp, m0, base0, c0, c1, c2, c3)));
-      r1 = __ldg(reinterpret_cast<const uint4*>(row_of(rows, temp, m1, base1, c0, c1, c2, c3)));
-      r2 = __ldg(reinterpret_cast<const uint4*>(row_of(rows, temp, m2, base2, c0, c1, c2, c3)));
-    } else {
-      m0 = *reinterpret_cast<const uint4*>(&hdrs[b.x]);
-      m1 = *reinterpret_cast<const uint4*>(&hdrs[ch1]);
-      m2 = *reinterpret_cast<const uint4*>(&hdrs[ch2]);
-      base0 = hdrs[b.x].row_base; base1 = hdrs[ch1].row_base; base2 = hdrs[ch2].row_base;
-      r0 = *reinterpret_cast<const uint4*>(row_of(rows, temp, m0, base0, c0, c1, c2, c3));
-      r1 = *reinterpret_cast<const uint4*>(row_of(rows, temp, m1, base1, c0, c1, c2, c3));
-      r2 = *reinterpret_cast<const uint4*>(row_of(rows, temp, m2, base2, c0, c1, c2, c3));
-    }
+    const uint4 m0 = *reinterpret_cast<const uint4*>(&hdrs[b.x]);
+    const uint4 m1 = *reinterpret_cast<const uint4*>(&hdrs[ch1]);
+    const uint4 m2 = *reinterpret_cast<const uint4*>(&hdrs[ch2]);
+    const unsigned long long base0 = hdrs[b.x].row_base, base1 = hdrs[ch1].row_base, base2 = hdrs[ch2].row_base;
+    const uint4 r0 = *reinterpret_cast<const uint4*>(row_of(rows, temp, m0, base0, c0, c1, c2, c3));
+    const uint4 r1 = *reinterpret_cast<const uint4*>(row_of(rows, temp, m1, base1, c0, c1, c2, c3));
+    const uint4 r2 = *reinterpret_cast<const uint4*>(row_of(rows, temp, m2, base2, c0, c1, c2, c3));
     tally.lookups += nchild;
     if (r0.z == MRL_UNSAT || r1.z == MRL_UNSAT || r2.z == MRL_UNSAT) return;
     uint32_t depth;
@@ -276,7 +260,7 @@ __device__ __forceinline__ Best solve_point(const SpecHdr* hdrs, const CandRec* 
   Best best = {MRL_UNSAT, MRL_UNSAT, MRL_UNSAT};
   for (uint32_t ci = 0; ci < cl.y; ci++) {
     const uint4 a = __ldg(reinterpret_cast<const uint4*>(&cands[cl.x + ci]));
-    eval_candidate<false>(hdrs, cands, rows, temp, cl.x + ci, a, cpack, bm0, bm1, bm2, bm3, best, tally);
+    eval_candidate(hdrs, cands, rows, temp, cl.x + ci, a, cpack, bm0, bm1, bm2, bm3, best, tally);
   }
   return best;
 }
@@ -2597,8 +2581,8 @@ int DeviceFill::plan_(const OpTables& tab) {
   if ((rc = reserve_host_(std::max(bytes, back)))) return rc;
   for (const Part& q : parts) if (q.bytes) memcpy(static_cast<unsigned char*>(h_stage_) + q.off, q.src, q.bytes);
   const size_t word_bytes = align256((size_t)n_words * sizeof(u32));
-  // The closure's queue has room for every position (size 8 in one dtype: 1.9 GB), so it lies in the
-  // working rows, which are idle until the fill; a fixed buffer carves those last.
+  // The closure's queue has room for every position (8 bytes each: 63 MB at size 8 in one dtype), and lies in
+  // the working rows, which are far larger and idle until the fill; a fixed buffer carves those last.
   const size_t queue_bytes = (size_t)tab.n_positions * sizeof(u64);
   if (!fixed_ && (rc = reserve_(b_temp_, queue_bytes, false))) return rc;
   if ((rc = reserve_(b_ctl_, 512)) || (rc = reserve_(b_tables_, bytes)) || (rc = reserve_(b_bits_, word_bytes + (fixed_ ? queue_bytes : 0))) ||
@@ -2621,7 +2605,6 @@ int DeviceFill::plan_(const OpTables& tab) {
   a.products = reinterpret_cast<const DpProduct*>(base + parts[7].off);
   a.lists = reinterpret_cast<const u16*>(base + parts[8].off);
   a.seeds = reinterpret_cast<const u64*>(base + parts[9].off);
-  a.t.n_positions = tab.n_positions;
   a.n_stages = n_stages;
   a.n_products = (u32)tab.products.size();
   a.n_seeds = (u32)tab.seeds.size();
@@ -2792,8 +2775,7 @@ int DeviceFill::begin_fill() {
   return 0;
 }
 
-// One launch of the stage kernel for the stages [from, to), by a team that fits them (see the
-// thresholds in run).
+// One launch of the stage kernel for the stages [from, to), by a team that fits them (team_of_stage).
 int DeviceFill::launch_stages_(uint32_t from, uint32_t to, int team, int blocks, bool solve, bool place) {
   StageArgs a;
   a.hdrs = d_hdrs_; a.cands = d_cands_; a.rmask = d_rmask_; a.mine = d_mine_; a.items = d_items_; a.rows = d_rows_; a.temp = d_temp_;

@@ -16,8 +16,7 @@ struct MrlRow {
   uint32_t main;   // saturating u32 main cost
   uint32_t peaks;  // RF<<24 | VRF<<16 | L1 code<<8 | GL code   (peak memory, as lattice codes)
   uint32_t tail;   // depth<<16 | action number; 0xFFFFFFFF = no implementation
-  uint32_t aux;    // finished table: 0. Working rows of the stage being solved: index of the winning
-                   // candidate record within its Spec (0xFFFFFFFF when there is none).
+  uint32_t aux;    // 0 (1 in a lookup's answer for a Spec that does not exist).
                    // 12 bytes of payload in a 16-byte slot: one aligned vector load per gather.
 };
 #define MRL_UNSAT 0xFFFFFFFFu
@@ -132,7 +131,7 @@ struct FillCtl {
   unsigned long long st_lookups;     // child rows gathered
   unsigned long long st_passes;
   unsigned long long st_final_bytes; // algorithmic bytes of the finished rows (see fill.hpp)
-  unsigned long long st_syncs;       // grid-wide barriers executed
+  unsigned long long st_syncs;       // barriers of a stage's team executed (a grid, a cluster or a block)
   unsigned long long st_sweeps;      // relaxation sweeps, all passes
   unsigned long long st_early_cells; // of st_cells: cells of the grids of the unordered phase
   unsigned long long st_late_cands;  // of st_cands: evaluated by the sweeps

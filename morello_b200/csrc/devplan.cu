@@ -11,8 +11,8 @@
 // The host planner (plan.cpp) builds the same arrays from tabulated Specs; the two agree byte for
 // byte.
 //
-// What bounds it: latency of dependent table and bitmap reads that hit L1 and L2 (the tables of a
-// size-8 precompute are 5 MB, its bitmap 58 MB); the records, 32 bytes each, are the only large
+// What bounds it: latency of dependent table and bitmap reads that hit L1 and L2 (at size 8 in one dtype
+// the tables are 1.0 MB and the bitmap another); the records, 32 bytes each, are the only large
 // stream and are written once.
 //
 // Restates for the device: morello/src/target/cpu.rs:455-823 (action order),

@@ -14,7 +14,6 @@ struct DpTables {   // device copies
   const DpFam* fams;
   const u16* fam_child;
   const uint2* rank;   // per 32 positions: which exist, and how many exist before them
-  u32 n_positions;
 };
 
 // Position of a Spec given by family and local operand indices (optable.hpp: level rank, then

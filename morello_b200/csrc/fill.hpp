@@ -38,7 +38,7 @@ struct FillStats {
   uint64_t late_items = 0;      // work items the sweeps evaluated
   uint64_t growths = 0;         // times a buffer had to be enlarged (the stage that asked is solved again)
   uint64_t sweeps = 0;          // relaxation sweeps of the candidates with a same-stage child
-  uint64_t grid_syncs = 0;      // grid-wide barriers inside the stage kernels
+  uint64_t grid_syncs = 0;      // team-wide barriers inside the stage kernels
   float fill_ms = 0;            // device time of the whole fill (CUDA events on the launch stream)
   float combine_ms = 0;         // device time inside the solve phases (device timer)
   float early_ms = 0;           // of which the unordered phase

@@ -19,7 +19,7 @@ def _goals(m):
     }
 
 
-@pytest.mark.parametrize("job", ["mixed", "one", "relayouts", "long", (1, 0), (2, 2), (4, 1), (4, 2)])
+@pytest.mark.parametrize("job", ["mixed", "one", "relayouts", "long", (1, 0), (2, 2), (4, 1), (4, 2), (8, 1)])
 def test_device_plan_equals_host_plan(job):
     import torch
     import morello_b200 as m
