@@ -369,8 +369,9 @@ def cuda_arm(args):
                      "algorithmic_bytes_how": ("final table rows only: per row 12 B out, 16 B per candidate record of its "
                                                "Spec, 16 B per child of each candidate that fits the row's limits"),
                      "kernel_ms_per_step": kernel_ms, "kernel_launches_per_step": launches // args.steps,
-                     "limiter": ("instruction issue (55-60 % of cycles in the stages that carry the time) and the latency of "
-                                 "dependent loads at 32 resident warps per SM; DRAM at 0.13 of peak (profiles/)")},
+                     "limiter": ("instruction issue (42 % of cycles in the longest launch of an 8x8x8 Matmul search), the latency "
+                                 "of dependent loads at 32 resident warps per SM (38 % of a warp's time) and barriers (23 %): "
+                                 "profiles/stage_kernel_matmul_8x8x8_sections.md")},
         "parity": parity,
         "clocks": clocks,
     }
@@ -382,17 +383,6 @@ def cuda_arm(args):
             n_lookups, n_bad = compare_with_oracle_puts(db, o)
             o.close()
             parity["oracle_put_corners_checked"], parity["oracle_mismatches"] = n_lookups, n_bad
-        traffic_path = os.path.join(ROOT, "profiles", "traffic.json")
-        if os.path.exists(traffic_path):
-            with open(traffic_path) as f:
-                t = json.load(f).get(str(SIZE) if THROUGH == 2 else "")
-            if t and "dram_bytes_per_cell" in t:  # measured DRAM bytes per solved working cell on a small case, scaled to this step (see the file's "how")
-                traffic = t["dram_bytes_per_cell"] * sum(cells_by_rank)
-                line["roofline"]["traffic"] = traffic
-                line["roofline"]["traffic_how"] = ("DRAM bytes of one single-GPU fill of this workload (one ncu pass per launch), "
-                                                   "scaled by the working cells solved: profiles/traffic.json")
-                line["roofline"]["dram_GBps"] = traffic / world / (kernel_ms * 1e-3) / 1e9   # per GPU
-                line["roofline"]["dram_frac_of_peak"] = traffic / world / (kernel_ms * 1e-3) / 1e9 / hbm_gbs
         sys.stdout.flush()
         os.dup2(real_stdout, 1)
         print(json.dumps(line), flush=True)

@@ -2,8 +2,8 @@
 // and limits are packed into the C ABI's arrays, the library's entry point is called without the
 // interpreter lock, and its decisions come back as instances of the caller's class.
 //
-// In Python this took 1.8 us per query (0.35 packing, 1.45 making the dataclass instances) against 0.09 us
-// for the lookup itself; here it takes 0.3.
+// In Python this took 1.8 us per query (0.35 packing, 1.45 making the dataclass instances); 16 384 queries
+// took 29.6 ms with the lookups, and take 5.9 here (0.36 us each, of which the library's lookup is 0.09).
 #define PY_SSIZE_T_CLEAN
 #include <Python.h>
 #include <stdint.h>
