@@ -41,6 +41,7 @@
 #include "device_types.h"
 #include "fill.hpp"
 #include "devplan.hpp"
+#include "host_threads.hpp"
 #include "../../include/morello_b200.h"
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
@@ -3073,15 +3074,14 @@ int DeviceFill::walk(uint64_t root, bool packed, uint32_t cpack, std::vector<Wal
 // 13 and 6.7 with 512 KB.
 int DeviceFill::read_bulk_(void* out, const void* src, size_t bytes) {
   const size_t piece = size_t(1) << 20;
-  if (bytes < 8 * piece || fixed_) {
+  const int n_threads = 4;
+  if (bytes < 8 * piece || fixed_ || reserve_host_(n_threads * 2 * piece) != 0) {
+    cudaGetLastError();   // no pinned memory to be had is no reason to refuse
     if (bytes) CK(cudaMemcpyAsync(out, src, bytes, cudaMemcpyDeviceToHost, stream_));
     CK(cudaStreamSynchronize(stream_));
     return 0;
   }
   CK(cudaStreamSynchronize(stream_));
-  const int n_threads = 4;
-  int rc = reserve_host_(n_threads * 2 * piece);
-  if (rc) return rc;
   std::atomic<size_t> next{0};
   std::atomic<int> error{0};
   const size_t pieces = (bytes + piece - 1) / piece;
@@ -3114,10 +3114,7 @@ int DeviceFill::read_bulk_(void* out, const void* src, size_t bytes) {
     for (cudaEvent_t v : ev) if (v) cudaEventDestroy(v);
     if (e != cudaSuccess) error.store((int)e);
   };
-  std::vector<std::thread> pool;
-  for (int t = 1; t < n_threads; t++) pool.emplace_back(work, t);
-  work(0);
-  for (auto& th : pool) th.join();
+  on_threads(n_threads, work);
   CK((cudaError_t)error.load());
   return 0;
 }
